@@ -1,0 +1,50 @@
+"""Kernels at the edges of their tiles and dispatch rules, against the oracle.
+
+Where the inputs are small integers the sums are exact in FP32 below 2^24, so
+the outputs must equal the oracle's bit for bit: one decision taken
+differently changes an output by at least 1.
+"""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from totri_gb300.totri_cpp import reconstruct as K
+
+pytestmark = pytest.mark.gpu
+
+
+def cu(a):
+    return torch.as_tensor(np.ascontiguousarray(a)).cuda()
+
+
+def points(g, n, z=0.0):
+    return np.stack([g.uniform(-1, 1, n), g.uniform(-1, 1, n), np.full(n, z)], 1).astype(np.float32)
+
+
+# (D, H, W), S, T, bin width: depths around the column of 4 voxels, one scan
+# point to just past a tile of 8, one voxel row to several slices of the voxels,
+# 512 and 1,024 threads per CTA (histograms below and above 100 KB)
+ADJOINT = [((1, 1, 1), 1, 1, 0.02), ((3, 2, 5), 7, 40, 0.05), ((4, 1, 33), 8, 300, 0.01),
+           ((5, 17, 3), 9, 300, 0.01), ((37, 40, 44), 17, 500, 0.008),
+           ((9, 8, 70), 12, 3300, 0.0012), ((64, 48, 40), 3, 6400, 0.0006)]
+
+
+@pytest.mark.parametrize("shape,S,T,bw", ADJOINT)
+@pytest.mark.parametrize("origin", [False, True])
+def test_velten_adjoint_edges(cuda_lib, shape, S, T, bw, origin):
+    g = np.random.default_rng(S * 1000 + T)
+    sp = points(g, S)
+    so = points(g, S, -0.3) if origin else None
+    st, en, bo = (-0.5, -0.4, 0.5), (0.45, 0.5, 1.4), 0.013
+    # a single-voxel axis has no spacing (0 / 0): its voxels fall in no bin
+    vol = g.integers(-3, 4, shape).astype(np.float64)
+    ref = oracle.bp_confocal_velten_adjoint(vol, sp, so, T, st, en, bw, bo)
+    out = torch.full((2, T, S), 7.0, device="cuda")
+    both = np.stack([vol, 2 * vol]).astype(np.float32)
+    so_t = cu(np.stack([so, so])) if origin else torch.empty((2, 0, 3), device="cuda")
+    K.backprojection_confocal_velten_adjoint(cu(both), cu(np.stack([sp, sp])), so_t, out, st, en,
+                                             bw, bo)
+    got = out.double().cpu().numpy()
+    assert np.array_equal(got[0], ref)
+    assert np.array_equal(got[1], 2 * ref)
