@@ -48,3 +48,39 @@ def test_velten_adjoint_edges(cuda_lib, shape, S, T, bw, origin):
     got = out.double().cpu().numpy()
     assert np.array_equal(got[0], ref)
     assert np.array_equal(got[1], 2 * ref)
+
+
+# (D, H, W), S, T, bin width, offset, z of the scan points: partial voxel
+# blocks; one point, an odd count and counts around the tiles of 8, 16 and 32 and
+# the batch of 256; bins of the whole volume before or past [0, T) and across its
+# ends (rows staged as zeros); windows too small for a block (exact chain in
+# place); scan points inside the volume (no window)
+FORWARD = [((5, 3, 2), 1, 50, 0.05, 0.0, 0.0), ((16, 8, 8), 33, 300, 0.01, 0.0, 0.0),
+           ((17, 9, 10), 255, 300, 0.01, 0.5, 0.0), ((30, 20, 12), 257, 200, 0.004, 1.2, 0.0),
+           ((24, 24, 24), 47, 64, 0.02, 3.9, 0.0), ((24, 24, 24), 47, 64, 0.02, -1.5, 0.0),
+           ((20, 20, 20), 31, 4000, 0.0008, 0.0, 0.0), ((9, 9, 9), 19, 4096, 0.0002, 1.0, 0.0),
+           ((12, 11, 10), 21, 100, 0.02, 0.0, 0.9), ((1, 9, 9), 9, 100, 0.02, 0.0, 0.0)]
+
+
+@pytest.mark.parametrize("shape,S,T,bw,bo,z", FORWARD)
+@pytest.mark.parametrize("origin", [False, True])
+def test_velten_forward_edges(cuda_lib, shape, S, T, bw, bo, z, origin):
+    from totri_gb300 import autotune
+    g = np.random.default_rng(S * 1000 + T)
+    sp = points(g, S, z)
+    so = points(g, S, -0.3) if origin else None
+    st, en = (-0.5, -0.4, 0.5), (0.45, 0.5, 1.4)
+    tr = g.integers(0, 16, (T, S)).astype(np.float32)
+    ref = oracle.bp_confocal_velten(tr, sp, so, shape, st, en, bw, bo)
+    so_t = cu(so[None]) if origin else torch.empty((1, 0, 3), device="cuda")
+    try:
+        for vz, n in ((0, 0), (2, 8), (4, 8), (4, 16), (4, 32)):
+            autotune.set_tile("backprojection.velten.vz", vz)
+            autotune.set_tile("backprojection.velten.points", n)
+            out = torch.full((1,) + shape, 7.0, device="cuda")
+            K.backprojection_confocal_velten_forward(cu(tr[None]), cu(sp[None]), so_t, out, st, en,
+                                                     bw, bo)
+            assert np.array_equal(out[0].double().cpu().numpy(), ref)
+    finally:
+        autotune.set_tile("backprojection.velten.vz", 0)
+        autotune.set_tile("backprojection.velten.points", 0)

@@ -54,6 +54,7 @@ __device__ __forceinline__ int nearest_bin(float dist, float bw, float bo) {
 // so the bins are those of the exact chain everywhere.
 struct FastBin {
   float inv_bw, nbo, k1, k2;
+  float kc, kb;  // box_bins' margin: kc dist + kb
 };
 
 inline FastBin make_fast_bin(float bw, float bo) {
@@ -64,6 +65,8 @@ inline FastBin make_fast_bin(float bw, float bo) {
   const bool ok = bw > 0.f && std::isfinite(f.inv_bw) && std::isfinite(f.nbo);
   f.k1 = ok ? 32.f * u * f.inv_bw : INFINITY;
   f.k2 = ok ? 32.f * u * std::fabs(bo) * f.inv_bw + 1e-6f : INFINITY;
+  f.kc = ok ? 16.f * u * f.inv_bw : INFINITY;
+  f.kb = ok ? 16.f * u * std::fabs(bo) * f.inv_bw + 1e-6f : INFINITY;
   return f;
 }
 
@@ -86,32 +89,44 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
   return r;
 }
 
-// velten_bin for the voxels of a column, with the margin m bounded once per
-// tile (the tiled kernel derives it from the distance and bin bounds of its
-// voxel block, 2% above velten_bin's per-pair margin there) and the +1/2 of
-// the bin coordinate folded away. r2, the squared distance in x and y, is
-// shared by the column's voxels (one fused multiply-add per voxel adds dz^2;
-// the sum of squares keeps three roundings). The bin is rounded without the
-// conversion units: v = dist / bw - bo / bw plus 1.5 2^23 holds rint(v) in
-// its low mantissa bits for |v| < 2^22, and floor(v + 1/2) = rint(v) wherever
-// v + 1/2 is farther than the margin from an integer, which is the test
-// |v - rint(v)| < 1/2 - m (`half_m`; <= 0 sends every pair of a tile to the
-// exact chain). The bins are those of the exact chain everywhere.
-__device__ __forceinline__ int velten_bin_col(fv3 q, float od2, fv3 p, float r2, float bw,
-                                              float bo, float inv_bw, float nbo, float half_m) {
-  const float dz = q.z - p.z;
-  const float d2 = fmaf(dz, dz, r2);
-  const float dist = fmaf(2.f, d2 * rsqrt_approx(d2), od2);
-  const float v = fmaf(dist, inv_bw, nbo);
-  const float x = v + 12582912.f;  // 1.5 2^23
-  const float rr = v - (x - 12582912.f);
-  if (fabsf(rr) < half_m) return __float_as_int(x) - 0x4B400000;
-  return nearest_bin(xadd(od2, xmul(2.f, xlen(xsub3(q, p)))), bw, bo);
+// max(m, |a|, |b|) in one instruction.
+__device__ __forceinline__ float absmax3(float m, float a, float b) {
+  float r;
+  asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(m), "f"(a), "f"(b));
+  return r;
 }
 
-// velten_bin_col for two voxels of the column at once: the same operations
-// on (voxel a, voxel b) pairs with paired FP32 instructions (each rounds as
-// its scalar form), the reciprocal square roots and the decisions per voxel.
+// The float at shared-memory address `at` (the caller orders it after the
+// barrier that follows the writes).
+__device__ __forceinline__ float lds(uint32_t at) {
+  float r;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(r) : "r"(at));
+  return r;
+}
+
+// Copies 4 bytes (or, with bytes = 0, writes 4 zero bytes) to shared memory
+// without passing through a register.
+__device__ __forceinline__ void cp_async4(uint32_t dst, const float* src, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes)
+               : "memory");
+}
+
+// Square root within 2^-23 (the caller keeps x in the normal range).
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// velten_bin for two voxels of a column at once with paired FP32 instructions,
+// the margin bounded once per box of voxels (box_bins) and the +1/2 of the bin
+// coordinate folded away. r2, the squared distance in x and y, is shared by
+// the column's voxels. The bin is rounded without the conversion units: v =
+// dist / bw - bo / bw plus 1.5 2^23 holds rint(v) in its low mantissa bits for
+// |v| < 2^22, and floor(v + 1/2) = rint(v) wherever v + 1/2 is farther than
+// the margin from an integer, which is the test |v - rint(v)| < 1/2 - m
+// (`half_m`; <= 0 sends every pair to the exact chain). The bins are those of
+// the exact chain everywhere.
 __device__ __forceinline__ void velten_bin_col2(fv3 q, float od2, fv3 pa, fv3 pb, float r2,
                                                 float bw, float bo, float inv_bw, float nbo,
                                                 float half_m, int& ta, int& tb) {
@@ -143,14 +158,21 @@ struct Pts3 {  // [B, n, 3] with strides
   }
 };
 
-// Bin coordinates that a scan point q with origin term od2 can reach in a box
-// of voxels, [cmin, cmax] (NaN where they are not defined), and the margin
-// that velten_bin_col needs there: velten_bin's k1 dist + k2 + 1e-6 |c| at the
-// largest distance and |c| of the box, with 2% slack for the rounding of these
-// bounds; infinite (every pair takes the exact chain) where the bounds are not
-// finite or the bins reach 2^21, the range of the rounding by addition.
+// Bin coordinates (+1/2) that a scan point q with origin term od2 can reach in
+// a box of voxels, [cmin, cmax] (NaN where they are not defined), and the
+// margin of the fast bins there. With u = 2^-24 and dist = 2 s + od2, the exact
+// chain's own roundings move the coordinate by at most 5 u 2s + 4 u od2 + 3 u
+// |bo| (over bw; plus u/2), the fast paths' by 6.2 u 2s + 3 u od2 + 4 u |bo|
+// (root: 2^-22.9 from rsqrt and one product), and the two sums of squares
+// differ by at most 6 u, 3 u in the root: 14.2 u (dist + |bo|) / bw in all. The
+// margin is 16 u of the largest distance of the box, 2% wider still for the
+// rounding of these bounds, plus 1e-6; infinite (every pair takes the exact
+// chain) where the bounds are not finite or the bins reach 2^21, the range of
+// the rounding by addition. With the previous 32 u dist / bw + 1e-6 |c|, three
+// times as wide, a warp left the fast path three times as often.
 struct BoxBins {
   float cmin, cmax, margin;
+  bool away;  // the box keeps a normal distance from the point
 };
 __device__ __forceinline__ BoxBins box_bins(fv3 q, float od2, fv3 lo, fv3 hi, float bw, float bo,
                                             const FastBin& fb) {
@@ -160,13 +182,16 @@ __device__ __forceinline__ BoxBins box_bins(fv3 q, float od2, fv3 lo, fv3 hi, fl
   const float fx = fmaxf(fabsf(lo.x - q.x), fabsf(hi.x - q.x));
   const float fy = fmaxf(fabsf(lo.y - q.y), fabsf(hi.y - q.y));
   const float fz = fmaxf(fabsf(lo.z - q.z), fabsf(hi.z - q.z));
+  const float e2 = ex * ex + ey * ey + ez * ez, f2 = fx * fx + fy * fy + fz * fz;
   BoxBins r;
-  r.cmin = (od2 + 2.f * sqrtf(ex * ex + ey * ey + ez * ez) - bo) / bw + 0.5f;
-  r.cmax = (od2 + 2.f * sqrtf(fx * fx + fy * fy + fz * fz) - bo) / bw + 0.5f;
-  const float dmax = fmaf(r.cmax - 0.5f, bw, bo);
+  r.cmin = (od2 + 2.f * sqrtf(e2) - bo) / bw + 0.5f;
+  r.cmax = (od2 + 2.f * sqrtf(f2) - bo) / bw + 0.5f;
+  const float dmax = fmaf(2.f, sqrtf(f2), od2);
   const float cabs = fmaxf(fabsf(r.cmin), fabsf(r.cmax));
-  r.margin = 1.02f * (fmaf(fb.k1, fabsf(dmax), fb.k2) + 1e-6f * cabs);
-  if (!(r.margin == r.margin) || !(cabs < 2097152.f)) r.margin = INFINITY;
+  r.margin = 1.02f * fmaf(fb.kc, dmax, fb.kb);
+  if (!(r.margin == r.margin) || !(cabs < 2097152.f) || !(r.cmin == r.cmin))
+    r.margin = INFINITY;
+  r.away = e2 > 1e-30f;
   return r;
 }
 
@@ -204,260 +229,252 @@ __global__ void __launch_bounds__(256) velten_confocal_kernel(Grid g, int b, int
   if (v < nv) vol[(size_t)b * nv + v] = value;
 }
 
-// Tiled Velten confocal: one CTA of 256 threads per 8x8x(4 VZ) block of
-// voxels, each thread VZ voxels 4 apart in z (default VZ = 4: 42.7 ms against
-// 51.1 ms for one voxel per thread and 46.3 ms for 8 on 128^3 voxels x 16,384
-// points, as the staged window and each scan point's shared-memory load serve
-// more voxels), scan points in tiles of 32. Per tile, warp 0 bounds the bins
-// the block can reach from each point (distance from the point to the block's
-// box, one bin of margin each side) and the CTA stages the union of those
-// rows of the tile's 32 transient columns in shared memory with coalesced
-// 128-byte row reads (row stride 33, so lanes reading different bins of one
-// column hit different banks). Voxels then read their bin from shared memory;
-// a bin outside the staged rows is read from global memory, so the window
-// only affects speed. The sum runs over the scan points in the same order as
-// velten_confocal_kernel, so the two give identical volumes.
+// Tiled Velten confocal: one CTA of 256 threads per 8 x 8 x (4 VZ) block of
+// voxels, each thread VZ voxels of a column, 4 apart in z, and the scan points
+// in tiles of ST. Every point of a tile has a window of kWinFloats / ST rows of
+// its transient column in shared memory, which holds every bin that the block
+// can reach from it (box_bins, one bin more each side); bins outside [0, T) are
+// staged as zeros. So a fast bin needs no range test: its shared-memory address
+// is one shift and add away from the rounded coordinate. A window starts at
+// the first bin of its group of 8 neighbouring points (whose 8 columns of a row
+// are one 32-byte sector) or, when a group's bins overflow it, of its own point.
+// Tiles whose windows cannot hold their bins, or with bins that need the exact
+// chain throughout, read the transient in place (velten_tile_direct).
+// Descriptors of 256 points are prepared at a time, one per thread.
 //
-// A tile whose union exceeds kWinRows (fine bins: the union of 32 points
-// spans 2-4x the rows of 8 consecutive points) stages per group of
-// consecutive points instead: 4 groups of 8, whose 8 columns of a row are one
-// full 32-byte sector, when every group's union fits its part of the window;
-// else 8 groups of 4; else one window per point, cut to its first rows. With
-// one union per tile, 4,096 bins of 1.25 mm over 128^3 voxels from 128x128
-// points took 4.6x the time of 1,024 bins. The group windows are compiled
-// in only with kGrouped: their code alone, never taken, made the kernel 10%
-// slower at 1,024 bins (38.3 -> 42.8 ms), so the host launches them when a
-// point's bins over the voxel block alone span more than about 100 rows.
-constexpr int kBX = 8, kBY = 8, kBZ = 4, kST = 32, kWinRows = 256;
-constexpr int kWinFloats = kWinRows * (kST + 1);
+// What bounds it: instruction issue (73% of slots with 40 warps per SM). Pairs
+// within the margin of a bin boundary (about 1e-3 of them at 5 mm bins) take the
+// exact chain, one lane at a time, about a tenth of the instructions. 128^3
+// voxels x 16,384 points: 33.4 -> 17.2 ms at 1,024 bins and 61.1 -> 26.3 ms at
+// 4,096, against a kernel that tested every pair's margin and window row with
+// branches. On the way: registers for 5 CTAs per SM (48), 18.1 ms, for 4, 19.4,
+// for 6, 20.5; 8 voxels per thread 18.4 ms; the boundary test per point instead
+// of per two points 19.8 ms; staging through registers instead of cp.async
+// 18.1 ms. The sum runs over the scan points in the order of
+// velten_confocal_kernel, so the two give identical volumes.
+constexpr int kBX = 8, kBY = 8, kBZ = 4, kWinFloats = 6176, kBatch = 256;
+// rows of a window: an odd count, so neighbouring points' windows start on
+// different banks (staging writes one row of 32 points)
+__host__ __device__ constexpr int win_rows(int ST) { return (kWinFloats / ST - 1) | 1; }
 
-// rows of a bin span [lo, hi]; an empty span (lo = INT_MAX, hi = INT_MIN)
-// has none, and its difference is never formed (it overflows)
-__device__ __forceinline__ int span_rows(int lo, int hi) { return hi >= lo ? hi - lo + 1 : 0; }
-
-// Group windows: group g of COLS points holds rows [grp[g].x, grp[g].x +
-// grp[g].y) of its columns at win + g REGION, row stride STRIDE (COLS + 1,
-// odd, for COLS > 1). REGION = COLS mod 32, so one row of all groups, as
-// staged, lands on 32 distinct banks; 4 x 2088, 8 x 1028 and 32 x 257 floats
-// fit kWinFloats.
-template <int COLS, int STRIDE, int REGION>
-__device__ __forceinline__ void velten_group_stage(float* win, const int2* grp, int cnt, int rows_max,
-                                                   const float* __restrict__ trb, int S, int s0) {
-  const int k = threadIdx.x & 31;  // a warp stages one row of every group
-  const int2 d = grp[k / COLS];
-  const int rows = k < cnt ? d.y : 0;
-  float* dst = win + (k / COLS) * REGION + k % COLS;
-  for (int r = threadIdx.x >> 5; r < rows_max; r += blockDim.x >> 5)
-    if (r < rows) dst[r * STRIDE] = __ldg(trb + (size_t)(d.x + r) * S + s0 + k);
-}
-
-// The samples of a tile with group windows. Points j >= cnt of a partial
-// tile carry a NaN distance, whose bin (-1) is neither staged nor in [0, T):
-// they add nothing.
-template <int COLS, int STRIDE, int REGION, int VZ, bool kPair>
-__device__ __forceinline__ void velten_group_samples(const float* win, const float4* pts,
-                                                     const int2* grp, const fv3 (&p)[VZ],
-                                                     float (&value)[VZ], int cnt, int T, int S,
-                                                     int s0, float bw, float bo, float inv_bw,
-                                                     float nbo, float half_m,
-                                                     const float* __restrict__ trb) {
-  for (int j0 = 0; j0 < cnt; j0 += COLS) {
-    const int2 d = grp[j0 / COLS];
-    const float* wg = win + (j0 / COLS) * REGION;
-#pragma unroll 1
-    for (int c = 0; c < COLS; ++c) {
-      const float4 q = pts[j0 + c];
-      const float dx = q.x - p[0].x, dy = q.y - p[0].y;
-      const float r2 = fmaf(dx, dx, dy * dy);
-      auto add = [&](int v, int t) {
-        const unsigned r = (unsigned)t - (unsigned)d.x;
-        if (r < (unsigned)d.y) value[v] += wg[r * STRIDE + c];
-        else if ((unsigned)t < (unsigned)T)
-          value[v] += __ldg(trb + (size_t)t * S + s0 + j0 + c);
-      };
-      if constexpr (kPair) {
-#pragma unroll
-        for (int v = 0; v < VZ; v += 2) {
-          int ta, tb;
-          velten_bin_col2(mkv(q.x, q.y, q.z), q.w, p[v], p[v + 1], r2, bw, bo, inv_bw, nbo,
-                          half_m, ta, tb);
-          add(v, ta);
-          add(v + 1, tb);
-        }
-      } else {
-#pragma unroll
-        for (int v = 0; v < VZ; ++v)
-          add(v, velten_bin_col(mkv(q.x, q.y, q.z), q.w, p[v], r2, bw, bo, inv_bw, nbo, half_m));
-      }
+// One tile of scan points [s0, s0 + cnt) against the thread's voxels, bins by
+// velten_bin and read in place.
+template <int VZ>
+__device__ __noinline__ void velten_tile_direct(int b, int T, int S, Pts3 sp, Pts3 so,
+                                                int has_origin, float bw, float bo,
+                                                const FastBin& fb, const float* __restrict__ trb,
+                                                int s0, int cnt, const fv3* p, float* value) {
+  for (int j = 0; j < cnt; ++j) {
+    const fv3 q = sp.at(b, s0 + j);
+    const float od2 = xmul(2.f, has_origin ? xlen(xsub3(q, so.at(b, s0 + j))) : 0.f);
+    for (int v = 0; v < VZ; ++v) {
+      const int t = velten_bin(q, od2, p[v], bw, bo, fb);
+      if ((unsigned)t < (unsigned)T) value[v] += __ldg(trb + (size_t)t * S + s0 + j);
     }
   }
 }
 
-template <int VZ, int kOcc = 1, bool kGrouped = false, bool kPair = false>
-__global__ void __launch_bounds__(256, kOcc) velten_confocal_tiled_kernel(
+enum : int { kTileSkip = 0, kTileFast = 1, kTileDirect = 2 };
+
+template <int VZ, int ST>
+__global__ void __launch_bounds__(256, 5) velten_confocal_tiled_kernel(
     Grid g, int b, int T, int S, Pts3 sp, Pts3 so, int has_origin, float bw, float bo,
     FastBin fb, const float* __restrict__ tr, float* __restrict__ vol) {
+  using u64 = unsigned long long;
+  constexpr int kRows = win_rows(ST), kTiles = kBatch / ST;
   __shared__ float win[kWinFloats];
-  __shared__ float4 pts[kST];
-  __shared__ int2 grp[kST];  // group windows: first staged bin, staged rows
-  __shared__ int span[2];
-  __shared__ int tile_cols;  // 32: one window; 8, 4, 1: points per group window
-  __shared__ int tile_rows;  // group windows: the most rows any group stages
-  __shared__ float tile_margin;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ float4 pa[kBatch];  // x, y, window address less the bin bias, 1/2 - margin
+  __shared__ float4 pb[kBatch];  // z, z, od2 / bw - bo / bw twice
+  __shared__ int2 prow[kBatch];  // first staged bin, staged rows
+  __shared__ int tile_mode[kTiles], tile_inner[kTiles];
+  const int lane = threadIdx.x & 31;
   const int x0 = blockIdx.x * kBX, y0 = blockIdx.y * kBY, z0 = blockIdx.z * kBZ * VZ;
   const int x = x0 + (threadIdx.x & 7), y = y0 + ((threadIdx.x >> 3) & 7);
-  // voxels z0 + (threadIdx.x >> 6) + kBZ v, v < VZ: one bin window and one
-  // scan-point load serve VZ voxels
-  bool inside[VZ];
-  fv3 p[VZ];
+  const int zt = z0 + (threadIdx.x >> 6);  // voxels zt + kBZ v
+  // Voxels past the volume's edge compute on a clamped position (inside the
+  // block's box) and are never written.
+  const fv3 p0 = voxel_point(g, min(x, g.W - 1), min(y, g.H - 1), 0);
+  float npz[VZ];  // negated
 #pragma unroll
-  for (int v = 0; v < VZ; ++v) {
-    const int z = z0 + (threadIdx.x >> 6) + kBZ * v;
-    inside[v] = x < g.W && y < g.H && z < g.D;
-    p[v] = voxel_point(g, min(x, g.W - 1), min(y, g.H - 1), min(z, g.D - 1));
-  }
-  // the block's box: voxel coordinates are monotone in the index
-  const fv3 ca = voxel_point(g, x0, y0, z0);
-  const fv3 cb = voxel_point(g, min(x0 + kBX, g.W) - 1, min(y0 + kBY, g.H) - 1,
-                             min(z0 + kBZ * VZ, g.D) - 1);
-  const fv3 lo = mkv(fminf(ca.x, cb.x), fminf(ca.y, cb.y), fminf(ca.z, cb.z));
-  const fv3 hi = mkv(fmaxf(ca.x, cb.x), fmaxf(ca.y, cb.y), fmaxf(ca.z, cb.z));
+  for (int v = 0; v < VZ; ++v) npz[v] = -grid_coord(g.sz, g.ez, g.D, min(zt + kBZ * v, g.D - 1));
   const float* trb = tr + (size_t)b * T * S;
-  float value[VZ];
+  const u64 slope = f2pack(2.f * fb.inv_bw, 2.f * fb.inv_bw);
+  const u64 big = f2pack(12582912.f, 12582912.f);  // 1.5 2^23
+  u64 value[VZ / 2];
 #pragma unroll
-  for (int v = 0; v < VZ; ++v) value[v] = 0.f;
-  for (int s0 = 0; s0 < S; s0 += kST) {
-    const int cnt = min(kST, S - s0);
-    __syncthreads();  // the previous tile is consumed
-    if (warp == 0) {
-      int tlo = INT_MAX, thi = INT_MIN;
-      float mrg = 0.f;  // margin bound of this lane's pairs (infinite: exact chain)
-      float4 pt = make_float4(0.f, 0.f, 0.f, __int_as_float(0x7fc00000));  // NaN distance
-      if (lane < cnt) {
-        const fv3 q = sp.at(b, s0 + lane);
-        const float od2 = xmul(2.f, has_origin ? xlen(xsub3(q, so.at(b, s0 + lane))) : 0.f);
-        pt = make_float4(q.x, q.y, q.z, od2);
+  for (int v = 0; v < VZ / 2; ++v) value[v] = 0ull;
+  for (int i0 = 0; i0 < S; i0 += kBatch) {
+    __syncthreads();  // the previous descriptors are consumed
+    {
+      const int i = i0 + threadIdx.x;
+      const bool live = i < S;
+      int lo1 = INT_MAX, hi1 = INT_MIN;
+      bool fast = true;
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f), c = a;
+      if (live) {
+        const fv3 q = sp.at(b, i);
+        const float od2 = has_origin ? xmul(2.f, xlen(xsub3(q, so.at(b, i)))) : 0.f;
+        // the block's box: voxel coordinates are monotone in the index
+        const fv3 ca = voxel_point(g, x0, y0, z0);
+        const fv3 cb = voxel_point(g, min(x0 + kBX, g.W) - 1, min(y0 + kBY, g.H) - 1,
+                                   min(z0 + kBZ * VZ, g.D) - 1);
+        const fv3 lo = mkv(fminf(ca.x, cb.x), fminf(ca.y, cb.y), fminf(ca.z, cb.z));
+        const fv3 hi = mkv(fmaxf(ca.x, cb.x), fmaxf(ca.y, cb.y), fmaxf(ca.z, cb.z));
         const BoxBins bb = box_bins(q, od2, lo, hi, bw, bo, fb);
-        if (bb.cmin == bb.cmin && bb.cmax == bb.cmax && bb.cmax >= -1.f &&
-            bb.cmin <= (float)T + 1.f) {
-          tlo = max((int)floorf(fmaxf(bb.cmin, -2.f)) - 1, 0);
-          thi = min((int)floorf(fminf(bb.cmax, (float)T + 2.f)) + 1, T - 1);
+        fast = bb.margin < 0.25f && bb.away;  // so |cmin|, |cmax| < 2^21
+        lo1 = hi1 = 0;
+        if (fast) {
+          lo1 = (int)floorf(bb.cmin) - 1;
+          hi1 = (int)floorf(bb.cmax) + 1;
         }
-        mrg = bb.margin;
+        a = make_float4(q.x, q.y, 0.f, 0.5f - bb.margin);
+        const float c0 = fmaf(od2, fb.inv_bw, fb.nbo);
+        c = make_float4(q.z, q.z, c0, c0);
       }
-      if (kGrouped || lane < cnt) pts[lane] = pt;
-      const int lo1 = tlo, hi1 = thi;
-      int lo4 = 0, hi4 = 0, lo8 = 0, hi8 = 0;
-      if constexpr (kGrouped) {
-        // unions of aligned groups of 4, 8 and 32 lanes (each within [0, T) or empty)
-        for (int o = 1; o < 32; o <<= 1) {
-          tlo = min(tlo, __shfl_xor_sync(0xffffffffu, tlo, o));
-          thi = max(thi, __shfl_xor_sync(0xffffffffu, thi, o));
-          mrg = fmaxf(mrg, __shfl_xor_sync(0xffffffffu, mrg, o));
-          if (o == 2) lo4 = tlo, hi4 = thi;
-          if (o == 4) lo8 = tlo, hi8 = thi;
+      int lo8 = lo1, hi8 = hi1;
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) {
+        lo8 = min(lo8, __shfl_xor_sync(0xffffffffu, lo8, o));
+        hi8 = max(hi8, __shfl_xor_sync(0xffffffffu, hi8, o));
+      }
+      // (a dead point's span is empty, and its difference never formed)
+      const int rows1 = hi1 >= lo1 ? hi1 - lo1 + 1 : 0, rows8 = hi8 >= lo8 ? hi8 - lo8 + 1 : 0;
+      const unsigned mine = ST == 32 ? 0xffffffffu : ((1u << (ST & 31)) - 1u) << (lane & ~(ST - 1));
+      const bool in8 = !(__ballot_sync(0xffffffffu, rows8 > kRows) & mine);
+      const bool in1 = !(__ballot_sync(0xffffffffu, rows1 > kRows) & mine);
+      const bool all_fast = !(__ballot_sync(0xffffffffu, !fast) & mine);
+      const bool some = (__ballot_sync(0xffffffffu, hi1 >= 0 && lo1 < T && live) & mine) != 0;
+      const int first = in8 ? lo8 : lo1;
+      const int rows = in8 ? rows8 : rows1;
+      const bool inner =
+          (__ballot_sync(0xffffffffu, !live || first < 0 || first + rows > T) & mine) == 0;
+      const uint32_t base = (uint32_t)__cvta_generic_to_shared(win) +
+                            4u * (uint32_t)((threadIdx.x & (ST - 1)) * kRows);
+      const uint32_t bias = 4u * (0x4B400000u + (uint32_t)first);
+      if (live) {
+        a.z = __uint_as_float(base - bias);
+        pa[threadIdx.x] = a;
+        pb[threadIdx.x] = c;
+        prow[threadIdx.x] = make_int2(first, rows);
+        if (i == S - 1 && !(threadIdx.x & 1)) {
+          // the odd last point's companion: the same point and rows in the
+          // next window, which is staged as zeros
+          a.z = __uint_as_float(base + 4u * kRows - bias);
+          pa[threadIdx.x + 1] = a;
+          pb[threadIdx.x + 1] = c;
+          prow[threadIdx.x + 1] = make_int2(-(1 << 30), rows);
         }
-      } else {
-        for (int o = 16; o > 0; o >>= 1) {
-          tlo = min(tlo, __shfl_xor_sync(0xffffffffu, tlo, o));
-          thi = max(thi, __shfl_xor_sync(0xffffffffu, thi, o));
-          mrg = fmaxf(mrg, __shfl_xor_sync(0xffffffffu, mrg, o));
-        }
+      } else if (i > S || !(threadIdx.x & 1)) {
+        prow[threadIdx.x] = make_int2(0, 0);
       }
-      constexpr int kR8 = 232, kR4 = 205, kR1 = 257;  // rows of 2088 / 9, 1028 / 5, 257
-      int cols = 32, grows = 0;
-      if (kGrouped && span_rows(tlo, thi) > kWinRows) {
-        int glo;
-        if (__all_sync(0xffffffffu, span_rows(lo8, hi8) <= kR8))
-          cols = 8, glo = lo8, grows = span_rows(lo8, hi8);
-        else if (__all_sync(0xffffffffu, span_rows(lo4, hi4) <= kR4))
-          cols = 4, glo = lo4, grows = span_rows(lo4, hi4);
-        else
-          cols = 1, glo = lo1, grows = min(span_rows(lo1, hi1), kR1);
-        if ((lane & (cols - 1)) == 0) grp[lane / cols] = make_int2(glo, grows);
-        for (int o = 16; o > 0; o >>= 1) grows = max(grows, __shfl_xor_sync(0xffffffffu, grows, o));
-      }
-      if (lane == 0) {
-        span[0] = tlo;
-        span[1] = thi;
-        tile_cols = cols;
-        tile_rows = grows;
-        tile_margin = mrg;
+      if ((threadIdx.x & (ST - 1)) == 0) {
+        const int tile = threadIdx.x / ST;
+        tile_mode[tile] = !(all_fast && in1) ? kTileDirect : (some ? kTileFast : kTileSkip);
+        tile_inner[tile] = inner;
       }
     }
     __syncthreads();
-    // one unsigned compare accepts a staged row (the windows lie in [0, T));
-    // anything else is read from global memory if it is a bin at all. Voxels
-    // past the volume's edge compute on a clamped position and are never
-    // written.
-    const int cols = tile_cols;
-    if (!kGrouped || cols == 32) {
-      // (with kGrouped a tile takes this path only when its union fits)
-      const int tlo = span[0], thi = span[1];
-      const int rows = (tlo >= 0 && thi < T && thi >= tlo) ? thi - tlo + 1 : 0;
-      const bool staged = rows > 0 && rows <= kWinRows;
-      if (staged)
-        for (int i = threadIdx.x; i < rows * kST; i += blockDim.x) {
-          const int r = i >> 5, c = i & 31;
-          win[r * (kST + 1) + c] = c < cnt ? __ldg(trb + (size_t)(tlo + r) * S + s0 + c) : 0.f;
+    for (int t0 = 0; t0 < kBatch && i0 + t0 < S; t0 += ST) {
+      const int cnt = min(ST, S - i0 - t0);
+      const int mode = tile_mode[t0 / ST];
+      if (mode == kTileSkip) continue;  // every bin is outside [0, T)
+      if (mode == kTileDirect) {
+        fv3 p[VZ];
+        float val[VZ];
+#pragma unroll
+        for (int v = 0; v < VZ; v += 2) f2unpack(value[v / 2], val[v], val[v + 1]);
+#pragma unroll
+        for (int v = 0; v < VZ; ++v) p[v] = mkv(p0.x, p0.y, -npz[v]);
+        velten_tile_direct<VZ>(b, T, S, sp, so, has_origin, bw, bo, fb, trb, i0 + t0, cnt, p, val);
+#pragma unroll
+        for (int v = 0; v < VZ; v += 2) value[v / 2] = f2pack(val[v], val[v + 1]);
+        continue;
+      }
+      __syncthreads();  // the previous tile's windows are consumed
+      {
+        constexpr int kSub = 32 / ST, kStep = 8 * kSub;  // rows a warp, the CTA takes at once
+        const int k = lane & (ST - 1);
+        const int2 d = prow[t0 + k];
+        const int r0 = (threadIdx.x >> 5) * kSub + lane / ST;
+        uint32_t dst = (uint32_t)__cvta_generic_to_shared(win) + 4u * (uint32_t)(k * kRows + r0);
+        const float* src = trb + i0 + t0 + k + ((int64_t)d.x + r0) * S;
+        const int64_t step = (int64_t)kStep * S;
+        if (tile_inner[t0 / ST]) {  // every row is a bin
+#pragma unroll 4
+          for (int r = r0; r < d.y; r += kStep, dst += 4u * kStep, src += step)
+            cp_async4(dst, src, 4);
+        } else {
+          for (int r = r0; r < d.y; r += kStep, dst += 4u * kStep, src += step) {
+            const bool bin = (unsigned)(d.x + r) < (unsigned)T;
+            cp_async4(dst, bin ? src : trb, bin ? 4 : 0);
+          }
         }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+      }
       __syncthreads();
-      const unsigned srows = staged ? (unsigned)rows : 0u;
-      const float half_m = 0.5f - tile_margin;
-      for (int j = 0; j < cnt; ++j) {
-        const float4 q = pts[j];
-        const float dx = q.x - p[0].x, dy = q.y - p[0].y;
-        const float r2 = fmaf(dx, dx, dy * dy);
-        if constexpr (kPair) {
+      // two points at a time: one test sends the lanes with a bin near a
+      // boundary (in either point) to the exact chain. An odd last point is
+      // joined by the dead one after it, whose window holds zeros.
+#pragma unroll 1
+      for (int j = 0; j < cnt; j += 2) {
+        float w[2][VZ], off[2][VZ];
+        float far = 0.f, near = 1.f;
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          const float4 a = pa[t0 + j + m], c = pb[t0 + j + m];
+          const float dx = a.x - p0.x, dy = a.y - p0.y;
+          const float r2 = fmaf(dx, dx, dy * dy);
+          const uint32_t base = __float_as_uint(a.z);
+          near = fminf(near, a.w);
 #pragma unroll
           for (int v = 0; v < VZ; v += 2) {
-            int t[2];
-            velten_bin_col2(mkv(q.x, q.y, q.z), q.w, p[v], p[v + 1], r2, bw, bo, fb.inv_bw,
-                            fb.nbo, half_m, t[0], t[1]);
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const unsigned r = (unsigned)t[h] - (unsigned)tlo;
-              if (r < srows) value[v + h] += win[r * (kST + 1) + j];
-              else if ((unsigned)t[h] < (unsigned)T)
-                value[v + h] += __ldg(trb + (size_t)t[h] * S + s0 + j);
-            }
-          }
-        } else {
-#pragma unroll
-          for (int v = 0; v < VZ; ++v) {
-            const int t = velten_bin_col(mkv(q.x, q.y, q.z), q.w, p[v], r2, bw, bo, fb.inv_bw,
-                                         fb.nbo, half_m);
-            const unsigned r = (unsigned)t - (unsigned)tlo;
-            if (r < srows) value[v] += win[r * (kST + 1) + j];
-            else if ((unsigned)t < (unsigned)T) value[v] += __ldg(trb + (size_t)t * S + s0 + j);
+            const u64 dz = f2add(f2pack(c.x, c.y), f2pack(npz[v], npz[v + 1]));
+            float da, db, xa, xb;
+            f2unpack(f2fma(dz, dz, f2pack(r2, r2)), da, db);
+            const u64 q =
+                f2fma(f2pack(sqrt_approx(da), sqrt_approx(db)), slope, f2pack(c.z, c.w));
+            const u64 x = f2add(q, big);
+            f2unpack(f2sub(q, f2sub(x, big)), off[m][v], off[m][v + 1]);
+            f2unpack(x, xa, xb);
+            far = absmax3(far, off[m][v], off[m][v + 1]);
+            w[m][v] = lds(base + 4u * __float_as_uint(xa));
+            w[m][v + 1] = lds(base + 4u * __float_as_uint(xb));
           }
         }
+        if (!(far < near)) {
+#pragma unroll
+          for (int m = 0; m < 2; ++m) {
+            const float4 a = pa[t0 + j + m];
+            const fv3 q = mkv(a.x, a.y, pb[t0 + j + m].x);
+            const int i = min(i0 + t0 + j + m, S - 1);
+            const float od2 = has_origin ? xmul(2.f, xlen(xsub3(q, so.at(b, i)))) : 0.f;
+#pragma unroll
+            for (int v = 0; v < VZ; ++v) {
+              if (fabsf(off[m][v]) < a.w) continue;
+              // the exact chain's bin is in the window like every other
+              const fv3 e = xsub3(q, mkv(p0.x, p0.y, -npz[v]));
+              const float t =
+                  floorf(xadd(xdiv(xsub(xadd(od2, xmul(2.f, xlen(e))), bo), bw), 0.5f));
+              w[m][v] = lds(__float_as_uint(a.z) + 4u * __float_as_uint(t + 12582912.f));
+            }
+          }
+        }
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+          for (int v = 0; v < VZ; v += 2)
+            value[v / 2] = f2add(value[v / 2], f2pack(w[m][v], w[m][v + 1]));
       }
-    } else if (cols == 8) {
-      velten_group_stage<8, 9, 2088>(win, grp, cnt, tile_rows, trb, S, s0);
-      __syncthreads();
-      const float half_m = 0.5f - tile_margin;
-      velten_group_samples<8, 9, 2088, VZ, kPair>(win, pts, grp, p, value, cnt, T, S, s0, bw, bo, fb.inv_bw,
-                                       fb.nbo, half_m, trb);
-    } else if (cols == 4) {
-      velten_group_stage<4, 5, 1028>(win, grp, cnt, tile_rows, trb, S, s0);
-      __syncthreads();
-      const float half_m = 0.5f - tile_margin;
-      velten_group_samples<4, 5, 1028, VZ, kPair>(win, pts, grp, p, value, cnt, T, S, s0, bw, bo, fb.inv_bw,
-                                       fb.nbo, half_m, trb);
-    } else {
-      velten_group_stage<1, 1, 257>(win, grp, cnt, tile_rows, trb, S, s0);
-      __syncthreads();
-      const float half_m = 0.5f - tile_margin;
-      velten_group_samples<1, 1, 257, VZ, kPair>(win, pts, grp, p, value, cnt, T, S, s0, bw, bo, fb.inv_bw,
-                                      fb.nbo, half_m, trb);
     }
   }
+  float val[VZ];
+#pragma unroll
+  for (int v = 0; v < VZ; v += 2) f2unpack(value[v / 2], val[v], val[v + 1]);
 #pragma unroll
   for (int v = 0; v < VZ; ++v) {
-    const int z = z0 + (threadIdx.x >> 6) + kBZ * v;
-    if (inside[v]) vol[(size_t)b * g.D * g.H * g.W + ((size_t)z * g.H + y) * g.W + x] = value[v];
+    const int z = zt + kBZ * v;
+    if (x < g.W && y < g.H && z < g.D)
+      vol[(size_t)b * g.D * g.H * g.W + ((size_t)z * g.H + y) * g.W + x] = val[v];
   }
 }
 
@@ -476,7 +493,7 @@ __global__ void __launch_bounds__(256, kOcc) velten_confocal_tiled_kernel(
 // one voxel at a time, with two 64-bit divisions for the voxel's index and three
 // correctly rounded ones for its position per pair, in 8 warps per SM at 4,096
 // bins: 96 x 88 x 72 voxels x 4,320 points x 4,096 bins took 60.4 ms
-// (now 5.7 ms).
+// (now 4.5 ms; 5.7 ms with the margin of the wider bound).
 constexpr int kTS = 8, kAZ = 4;
 __global__ void __launch_bounds__(1024) velten_adjoint_kernel(Grid g, int b, int T, int S, Pts3 sp,
                                                               Pts3 so, int has_origin, float bw,
@@ -740,66 +757,52 @@ int totri_backprojection_confocal_velten_forward(const totri_array_t* transient,
   if (vz <= 0) vz = 4;
   if (vz != 1 && vz != 2 && vz != 4)
     return fail(TOTRI_ERR_INVALID_ARGUMENT, "backprojection.velten.vz must be 1, 2 or 4");
+  if (vz == 1) vz = 2;  // voxels go in pairs
   const dim3 grid((unsigned)ceil_div(g.W, bp::kBX), (unsigned)ceil_div(g.H, bp::kBY),
                   (unsigned)ceil_div(g.D, bp::kBZ * vz));
-  // Group windows when one point's bins over a voxel block alone, 2 |block
-  // diagonal| / bw, span more than 100 rows (measured on 128^3 and 192^3
-  // voxels from 128^2 and 256^2 points: whole-tile windows were faster up to
-  // 82 rows, group windows from 122); "backprojection.velten.groups" = 1
-  // forces whole-tile windows, 2 group windows.
-  int groups = tune::get("backprojection.velten.groups");
-  if (groups != 1 && groups != 2) {
-    const auto pitch = [](float a, float e, int n) {
-      return n > 1 ? std::fabs((double)e - (double)a) / (n - 1) : 0.0;
-    };
-    const double ex = bp::kBX * pitch(g.sx, g.ex, g.W), ey = bp::kBY * pitch(g.sy, g.ey, g.H);
-    const double ez = bp::kBZ * vz * pitch(g.sz, g.ez, g.D);
-    const double rows = 2.0 * std::sqrt(ex * ex + ey * ey + ez * ez) / std::fabs((double)bw);
-    groups = rows > 100.0 ? 2 : 1;
-  }
-  const bool grouped = groups == 2;
+  // Points per tile (32, 16 or 8; "backprojection.velten.points" sets it): the
+  // most whose windows are a third larger than a block's bins from one point, at
+  // most 2 |block diagonal| / bw + 4 rows, so that the bins of 8 neighbouring
+  // points mostly fit too (windows per point read the transient 4 bytes at a
+  // time). 230 rows of 385 at 16 points: 26.3 ms against 30.0 ms with 8
+  // (128^3 x 16,384 points, 4,096 bins); 385 rows of 385: 4.46 ms against 3.73 ms
+  // with 8 (96 x 88 x 72 x 4,320, 4,096 bins); 60 rows of 193 at 32 points:
+  // 17.2 ms against 18.2 ms with 16 (128^3 x 16,384, 1,024 bins).
+  const auto pitch = [](float a, float e, int n) {
+    return n > 1 ? std::fabs((double)e - (double)a) / (n - 1) : 0.0;
+  };
+  const double ex = (bp::kBX - 1) * pitch(g.sx, g.ex, g.W);
+  const double ey = (bp::kBY - 1) * pitch(g.sy, g.ey, g.H);
+  const double ez = (bp::kBZ * vz - 1) * pitch(g.sz, g.ez, g.D);
+  const double rows = 2.0 * std::sqrt(ex * ex + ey * ey + ez * ez) / std::fabs((double)bw) + 4.0;
+  int st = tune::get("backprojection.velten.points");
+  if (st != 8 && st != 16 && st != 32)
+    st = rows <= 0.75 * bp::win_rows(32) ? 32 : (rows <= 0.75 * bp::win_rows(16) ? 16 : 8);
+  const bp::FastBin fb = bp::make_fast_bin(bw, bo);
+  const float* trp = static_cast<const float*>(transient->data);
+  float* volp = static_cast<float*>(volume->data);
   for (int b = 0; b < (int)B; ++b) {
-    const bp::FastBin fb = bp::make_fast_bin(bw, bo);
-    const float* trp = static_cast<const float*>(transient->data);
-    float* volp = static_cast<float*>(volume->data);
-    // 4 voxels per thread with registers capped for 6 CTAs per SM (38, no
-    // spills; 34 KB of shared memory each): 38.2 ms against 40.4 ms uncapped
-    // (47 registers, 5 CTAs; "backprojection.velten.occupancy" = 1), the same
-    // volume bit for bit.
-#define TOTRI_VELTEN_TILED(VZ, OCC, PAIR)                                                  \
-  TOTRI_KERNEL("backprojection velten confocal", stream,                                  \
-               grouped ? (bp::velten_confocal_tiled_kernel<VZ, OCC, true, PAIR>           \
-                          <<<grid, 256, 0, stream>>>(g, b, T, (int)S, sp, so, So > 0, bw, \
-                                                     bo, fb, trp, volp))                  \
-                       : (bp::velten_confocal_tiled_kernel<VZ, OCC, false, PAIR>          \
-                          <<<grid, 256, 0, stream>>>(g, b, T, (int)S, sp, so, So > 0, bw, \
-                                                     bo, fb, trp, volp)))
-    // Bins of two voxels at a time with paired FP32 instructions
-    // (velten_bin_col2; "backprojection.velten.pair" = 2 takes them one at a
-    // time): 33.3 ms against 39.0 ms, the same volume bit for bit.
-    const bool pair = tune::get("backprojection.velten.pair") != 2;
-    const int occ = (int)tune::get("backprojection.velten.occupancy");
-    if (tiled && vz == 4 && pair && occ == 5)
-      TOTRI_VELTEN_TILED(4, 5, true);
-    else if (tiled && vz == 4 && pair && occ != 1)
-      TOTRI_VELTEN_TILED(4, 6, true);
-    else if (tiled && vz == 4 && occ != 1)
-      TOTRI_VELTEN_TILED(4, 6, false);
-    else if (tiled && vz == 4)
-      TOTRI_VELTEN_TILED(4, 1, false);
-    else if (tiled && vz == 2 && pair)
-      TOTRI_VELTEN_TILED(2, 1, true);
-    else if (tiled && vz == 2)
-      TOTRI_VELTEN_TILED(2, 1, false);
-    else if (tiled)
-      TOTRI_VELTEN_TILED(1, 1, false);
-#undef TOTRI_VELTEN_TILED
-    else
+#define TOTRI_VELTEN_TILED(VZ, ST)                                                 \
+  TOTRI_KERNEL("backprojection velten confocal", stream,                          \
+               bp::velten_confocal_tiled_kernel<VZ, ST><<<grid, 256, 0, stream>>>( \
+                   g, b, T, (int)S, sp, so, So > 0, bw, bo, fb, trp, volp))
+    if (!tiled)
       TOTRI_KERNEL("backprojection velten confocal", stream,
                    bp::velten_confocal_kernel<<<(unsigned)ceil_div(nv, 256), 256, 0, stream>>>(
-                       g, b, T, (int)S, sp, so, So > 0, bw, bo, bp::make_fast_bin(bw, bo),
-                       static_cast<const float*>(transient->data),
-                       static_cast<float*>(volume->data)));
+                       g, b, T, (int)S, sp, so, So > 0, bw, bo, fb, trp, volp));
+    else if (vz == 4 && st == 32)
+      TOTRI_VELTEN_TILED(4, 32);
+    else if (vz == 4 && st == 16)
+      TOTRI_VELTEN_TILED(4, 16);
+    else if (vz == 4)
+      TOTRI_VELTEN_TILED(4, 8);
+    else if (st == 32)
+      TOTRI_VELTEN_TILED(2, 32);
+    else if (st == 16)
+      TOTRI_VELTEN_TILED(2, 16);
+    else
+      TOTRI_VELTEN_TILED(2, 8);
+#undef TOTRI_VELTEN_TILED
   }
   return TOTRI_OK;
 }

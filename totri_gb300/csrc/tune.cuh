@@ -34,11 +34,9 @@
 //   "volume.adjoint.warps"      warps per CTA of the lanes-over-columns adjoint
 //   "volume.adjoint.slabs"      z slabs of its columns (default: slabs of <= 64 cells)
 //   "volume.exhaustive.lt"      laser points per exhaustive volume CTA (1,8,32)
-//   "backprojection.velten.mode", ".occupancy", ".vz", ".groups", ".pair"
-//                               Velten kernel variant, 1: uncapped registers (5: capped for
-//                               5 CTAs per SM), slab depth, bin windows (1 one per tile, 2 per
-//                               point group; 0: by the voxel block's span in bins), 2: bins
-//                               one voxel at a time instead of paired
+//   "backprojection.velten.mode", ".vz", ".points"
+//                               1: one voxel per thread without windows / voxels per
+//                               thread (2, 4) / scan points per tile (8, 16, 32)
 //   "rbf.cull"                  1: RBF kernels without the underflow cull
 //   "rbf.forward.vz"            1: one voxel per thread in the RBF forward (default two)
 //   "rbf.grad.pair"             2: one Gaussian per warp iteration in the RBF gradient
