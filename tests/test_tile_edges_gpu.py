@@ -10,6 +10,7 @@ import torch
 
 import oracle
 from totri_gb300.totri_cpp import reconstruct as K
+from totri_gb300.totri_cpp import render as R
 
 pytestmark = pytest.mark.gpu
 
@@ -20,6 +21,11 @@ def cu(a):
 
 def points(g, n, z=0.0):
     return np.stack([g.uniform(-1, 1, n), g.uniform(-1, 1, n), np.full(n, z)], 1).astype(np.float32)
+
+
+def rel(a, b):
+    a = np.asarray(a, np.float64)
+    return float(np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-300))
 
 
 # (D, H, W), S, T, bin width: depths around the column of 4 voxels, one scan
@@ -84,3 +90,25 @@ def test_velten_forward_edges(cuda_lib, shape, S, T, bw, bo, z, origin):
     finally:
         autotune.set_tile("backprojection.velten.vz", 0)
         autotune.set_tile("backprojection.velten.points", 0)
+
+
+# (X, Y, Z), N, T, bin width, offset: one cell pair, columns around a slab of 64
+# cells and past it, column tiles of 4 x 8 with remainders; runs of 8, 16 and 32
+# points with a remainder; bin counts around the steps of 4 and chunks of 32
+COLUMNS = [((1, 1, 2), 1, 700, 0.004, 0.0), ((4, 8, 64), 7, 161, 0.013, 0.0),
+           ((5, 9, 65), 9, 162, 0.013, -0.4), ((3, 17, 20), 300, 131, 0.017, 0.0),
+           ((13, 30, 130), 1100, 99, 0.02, 0.1), ((40, 41, 33), 2500, 64, 0.03, 0.3)]
+
+
+@pytest.mark.parametrize("shape,N,T,bw,bo", COLUMNS)
+def test_volume_adjoint_edges(cuda_lib, shape, N, T, bw, bo):
+    """Against the exact FP64 adjoint, 1e-5 (columns of up to 200 cells)."""
+    g = np.random.default_rng(N + T)
+    mp = np.stack([g.uniform(-1, 1, N), g.uniform(-1, 1, N), g.uniform(0, 0.8, N)])
+    mp = mp.astype(np.float32)
+    org, size = (-0.5, -0.5, 0.5), (1.0, 1.0, 1.0)
+    y = g.uniform(0.5, 1.5, (N, T)).astype(np.float32)
+    ref = oracle.volume_confocal_adjoint(y, shape, mp, org, size, bw, bo)
+    adj = torch.full(shape, 7.0, device="cuda")
+    R.volume_confocal_adjoint(adj, cu(mp), cu(y), org, size, bw, bo)
+    assert rel(adj.cpu().numpy(), ref) < 1e-5

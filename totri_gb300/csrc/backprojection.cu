@@ -83,19 +83,6 @@ __device__ __forceinline__ int velten_bin(fv3 q, float od2, fv3 p, float bw, flo
   return nearest_bin(xadd(od2, xmul(2.f, xlen(xsub3(q, p)))), bw, bo);
 }
 
-__device__ __forceinline__ float rsqrt_approx(float x) {
-  float r;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-
-// max(m, |a|, |b|) in one instruction.
-__device__ __forceinline__ float absmax3(float m, float a, float b) {
-  float r;
-  asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(m), "f"(a), "f"(b));
-  return r;
-}
-
 // The float at shared-memory address `at` (the caller orders it after the
 // barrier that follows the writes).
 __device__ __forceinline__ float lds(uint32_t at) {

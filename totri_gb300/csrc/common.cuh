@@ -184,6 +184,13 @@ __device__ __forceinline__ unsigned long long f2add(unsigned long long a, unsign
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
+// a + b rounded down (towards minus infinity) in each half.
+__device__ __forceinline__ unsigned long long f2add_rm(unsigned long long a,
+                                                       unsigned long long b) {
+  unsigned long long d;
+  asm("add.rm.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
 __device__ __forceinline__ unsigned long long f2sub(unsigned long long a, unsigned long long b) {
   unsigned long long d;
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
@@ -194,6 +201,20 @@ __device__ __forceinline__ unsigned long long f2mul(unsigned long long a, unsign
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
+
+// max(m, |a|, |b|) in one instruction (a NaN operand is passed over).
+__device__ __forceinline__ float absmax3(float m, float a, float b) {
+  float r;
+  asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(m), "f"(a), "f"(b));
+  return r;
+}
+// 1 / sqrt(x) within 2^-22.9 for normal x (denormals count as zero).
+__device__ __forceinline__ float rsqrt_approx(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 // Monotone float <-> int mapping for atomicMin/atomicMax on floats.
 __device__ __forceinline__ int ford(float f) {
   const int i = __float_as_int(f);

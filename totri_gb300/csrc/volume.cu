@@ -548,73 +548,117 @@ __global__ void __launch_bounds__(256) confocal_adjoint_cells_kernel(Geo g, Poin
   }
 }
 
-constexpr int kAdjUnroll = 4;  // bins per step of the lanes-over-columns adjoint
-// (8 bins per step, at 80 registers, measured the same: 65.6 against 65.8 ms)
-constexpr int kAdjTablePad = kAdjUnroll;  // table entries past the last bin
+// Table entries of two bins each: (tc^2, tc^2, 1 / tc^8, 1 / tc^8) of bins 2 i
+// and 2 i + 1, padded to a multiple of four bins.
+__host__ __device__ constexpr int adj_table(int T) { return 2 * ((T + 3) / 4); }
 
-// The bins [t0, t1] of one point for the lanes' columns, kAdjUnroll at a time:
-// the fast path without branches (a sample that is not taken adds zero to
-// cell 0), then the few samples that sit within the rounding margin of a cell
-// boundary through the exact chain. Without kCheck (the bins with
-// non-negative centres, walked last) the step may run up to kAdjUnroll - 1
-// bins past t1: those are real bins (walked with their values, and rejected
-// unless they hold a sample) up to T - 1, and table padding (tc^2 = -inf)
-// beyond it; with kCheck (the negative centres, whose later bins belong to
-// the other walk) bins past t1 are skipped. z_hat = (depth + (wz - oz)) scale
-// - 0.5: the rounding of either association is inside sample_filtered's
-// margin.
-template <bool kCheck, int U>
-__device__ __forceinline__ void adj_walk(const Geo& g, const float2* __restrict__ tab,
-                                         const float* __restrict__ row, float* col, int t0,
-                                         int t1, int lane, float ddx, float ddy, float wz,
-                                         float wzo, float pm, float wx, float wy, float x,
-                                         float y, int za, int zn) {
-  const int tend = kCheck ? t1 : g.T - 1;  // last bin whose value is read
-  float wval = 0.f;                        // bin t0 + 32 k + lane
-  for (int t = t0; t <= t1; t += U) {
-    const int wo = (t - t0) & 31;
-    if (wo == 0) wval = t + lane <= tend ? __ldg(row + t + lane) : 0.f;
-    int zi[U];
-    float w0[U], w1[U];
-    bool slow[U];
-    bool any_slow = false;
+// Adds w0 to cell row `u` and w1 to the next one of the lane's column (at
+// shared-memory address `col`, rows 128 bytes apart) when u < zn. Predicated
+// loads and stores: a select of the row or of zero weights took three more
+// instructions.
+__device__ __forceinline__ void adj_add(uint32_t col, unsigned u, unsigned zn, float w0,
+                                        float w1) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      ".reg .f32 a, b;\n\t"
+      "setp.lt.u32 p, %1, %2;\n\t"
+      "@p ld.shared.f32 a, [%0];\n\t"
+      "@p ld.shared.f32 b, [%0 + 128];\n\t"
+      "add.f32 a, a, %3;\n\t"
+      "add.f32 b, b, %4;\n\t"
+      "@p st.shared.f32 [%0], a;\n\t"
+      "@p st.shared.f32 [%0 + 128], b;\n\t"
+      "}"
+      :: "r"(col + 128u * u), "r"(u), "r"(zn), "f"(w0), "f"(w1)
+      : "memory");
+}
+
+// A point as the lane's column sees it.
+struct AdjPoint {
+  float ndx, ndy;  // minus the squared horizontal offsets (the sample chain's)
+  float wx, wy, wz;
+  float lim;       // 1/2 - margin of a cell fraction
+};
+
+// The bins [t0, t1] of one point for the lanes' columns, four at a time from
+// the multiple of four at or below t0, in pairs with paired FP32
+// instructions. `val` holds the values of the first 32 bins, one per lane;
+// each chunk of 32 passes through the warp's buffer, from where four come by
+// one broadcast read (as the table entries of two bins do), and the next chunk
+// is read ahead. floor(z_hat) is the addition of 1.5 2^23 rounded down, whose
+// low mantissa bits are the cell. A sample with d2 <= 0 has a NaN z_hat, whose
+// bits are past every cell. Samples within the rounding margin of a cell
+// boundary go through the exact chain. The step may touch up to three bins on
+// each side of [t0, t1]: without kCheck (no negative bin centres) those are real
+// bins, rejected unless they hold a sample, or table padding (tc^2 = -inf); with
+// kCheck they belong to the other walk and are skipped. Each sample's values
+// are those of sample_filtered or, near a boundary, of the exact chain, bit
+// for bit.
+template <bool kCheck>
+__device__ __forceinline__ void adj_walk(const Geo& g, const float4* __restrict__ tab,
+                                         float4* vbuf, const float* __restrict__ row,
+                                         const AdjPoint& p, int t0, int t1, float val, int lane,
+                                         uint32_t col, float x, float y, int za, int zn) {
+  using u64 = unsigned long long;
+  const u64 ndx = f2pack(p.ndx, p.ndx), ndy = f2pack(p.ndy, p.ndy);
+  const u64 wzo = f2pack(p.wz - g.oz, p.wz - g.oz), scale = f2pack(g.scale, g.scale);
+  const u64 half = f2pack(-0.5f, -0.5f);
+  const u64 big = f2pack(12582912.f, 12582912.f);  // 1.5 2^23
+  const unsigned bias = 0x4B400000u + (unsigned)za;
+  for (int c = t0 & ~3; c <= t1; c += 32) {
+    __syncwarp();
+    reinterpret_cast<float*>(vbuf)[lane] = val;
+    __syncwarp();
+    if (c + 32 <= t1) val = c + 32 + lane < g.T ? __ldg(row + c + 32 + lane) : 0.f;
+    const int n = min(32, t1 - c + 1);
+#pragma unroll 1
+    for (int s = 0; s < n; s += 4) {
+      const float4 v4 = vbuf[s >> 2];
+      unsigned u[4];
+      float w0[4], w1[4], off[4];
 #pragma unroll
-    for (int q = 0; q < U; ++q) {
-      const float val = __shfl_sync(0xffffffffu, wval, wo + q);
-      const float2 tb = (!kCheck || t + q <= t1) ? tab[t + q] : make_float2(-INFINITY, 0.f);
-      const float d2 = xsub(xsub(tb.x, ddx), ddy);
-      const bool valid = d2 > 0.f;
-      const float depth = d2 * rsqrtf(d2);  // NaN when d2 <= 0: never taken
-      const float zh = fmaf(depth + wzo, g.scale, -0.5f);
-      const float fl = floorf(zh);
-      const float fr = zh - fl;
-      const bool fast = !g.exact && fabsf(fr - 0.5f) < 0.5f - pm;
-      const int z = __float2int_rz(fl);
-      const bool ok = valid && fast && (unsigned)(z - za) < (unsigned)zn;
-      const float v = val * ((d2 * d2) * tb.y);
-      zi[q] = ok ? z - za : 0;
-      w0[q] = ok ? (1.f - fr) * v : 0.f;
-      w1[q] = ok ? fr * v : 0.f;
-      slow[q] = valid && !fast;
-      any_slow |= slow[q];
-    }
-    if (__any_sync(0xffffffffu, any_slow)) {
-#pragma unroll
-      for (int q = 0; q < U; ++q) {
-        if (!slow[q]) continue;
-        const Sample sm = sample(g, wx, wy, wz, t + q, x, y);
-        if (sm.ok && (unsigned)(sm.zi - za) < (unsigned)zn) {
-          const float vv = __ldg(row + t + q) * sm.f2;
-          zi[q] = sm.zi - za;
-          w0[q] = (1.f - sm.alpha) * vv;
-          w1[q] = sm.alpha * vv;
+      for (int h = 0; h < 2; ++h) {
+        float4 tb = tab[((c + s) >> 1) + h];
+        if (kCheck) {
+          const int t = c + s + 2 * h;
+          if (t < t0 || t > t1) tb.x = -INFINITY;
+          if (t + 1 < t0 || t + 1 > t1) tb.y = -INFINITY;
         }
+        const u64 d2 = f2add(f2add(f2pack(tb.x, tb.y), ndx), ndy);
+        float da, db, xa, xb;
+        f2unpack(d2, da, db);
+        const u64 zh = f2fma(f2fma(d2, f2pack(rsqrt_approx(da), rsqrt_approx(db)), wzo), scale,
+                             half);
+        const u64 fx = f2add_rm(zh, big);
+        const u64 fr = f2sub(zh, f2sub(fx, big));
+        f2unpack(fx, xa, xb);
+        f2unpack(f2add(fr, half), off[2 * h], off[2 * h + 1]);
+        const u64 v = f2mul(f2mul(f2mul(d2, d2), f2pack(tb.z, tb.w)),
+                            h ? f2pack(v4.z, v4.w) : f2pack(v4.x, v4.y));
+        const u64 upper = f2mul(fr, v);
+        f2unpack(upper, w1[2 * h], w1[2 * h + 1]);
+        f2unpack(f2sub(v, upper), w0[2 * h], w0[2 * h + 1]);
+        u[2 * h] = __float_as_uint(xa) - bias;
+        u[2 * h + 1] = __float_as_uint(xb) - bias;
       }
-    }
+      // (NaN fractions are passed over)
+      if (absmax3(absmax3(0.f, off[0], off[1]), off[2], off[3]) >= p.lim) {
+        unsigned slow = 0;
 #pragma unroll
-    for (int q = 0; q < U; ++q) {
-      col[zi[q] * 32] += w0[q];
-      col[zi[q] * 32 + 32] += w1[q];
+        for (int q = 0; q < 4; ++q)
+          if (fabsf(off[q]) >= p.lim) slow |= 1u << q, u[q] = 0xffffffffu;
+        do {
+          const int q = __ffs(slow) - 1;
+          slow &= slow - 1;
+          const Sample sm = sample(g, p.wx, p.wy, p.wz, c + s + q, x, y);
+          const float v = reinterpret_cast<const float*>(vbuf)[s + q] * sm.f2;
+          if (sm.ok)
+            adj_add(col, (unsigned)(sm.zi - za), (unsigned)zn, (1.f - sm.alpha) * v, sm.alpha * v);
+        } while (slow);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) adj_add(col, u[q], (unsigned)zn, w0[q], w1[q]);
     }
   }
 }
@@ -622,104 +666,134 @@ __device__ __forceinline__ void adj_walk(const Geo& g, const float2* __restrict_
 // Exact adjoint of the forward with the lanes of a warp over 32 neighbouring
 // voxel columns (an 8 x 4 tile: y fastest) and all lanes on one point and one
 // bin at a time. The point's transient row is then read once per warp (32 bins
-// per coalesced load, handed out by shuffles), and the bin's tc^2 (the sample
-// chain's FP32 value) and 1 / tc^8 come from a per-CTA table in shared memory
-// (broadcast reads), so f2 = (depth / tc^2)^4 = d2^2 / tc^8 needs no second
-// special-function op. A CTA takes one slab of the columns' cells (the
-// samples whose cell pair starts there; the pair's second cell may be the next
-// slab's first, one extra row), and each lane owns its column's cells of the
-// slab in shared memory ([cell][lane]: no bank conflicts, no atomics), one
-// copy per warp; the warps of a CTA take interleaved runs of 32 points of one
-// point group, and the CTA adds its summed columns into the volume (which the
-// launcher zeroes) with one atomic per cell when there is more than one group
-// or slab. A point's bins are those whose samples can land in the slab. Four bins per step,
-// evaluated without branches, give each lane four independent sample chains
-// (a branchy two-bin version issued 52 warp instructions per sample at 46% of
-// issue slots, latency-bound with 12 warps per SM). The bins walked for a point
-// are the union of the lanes' column spans: every valid sample of a lane lies
-// in its own span, and a sample outside it is decided (and rejected) like any
-// other, so each (column, point, bin) is counted once. Decisions are the exact
-// chain's (sample_filtered's margin, taken over the largest |tc| of the union).
-template <int U>
-__global__ void __launch_bounds__(256) confocal_adjoint_columns_kernel(
-    Geo g, Points mp, int N, int points_per_group, const float* __restrict__ tr,
+// per coalesced load), and the bin's tc^2 (the sample chain's FP32 value) and
+// 1 / tc^8 come from a per-CTA table in shared memory (broadcast reads), so f2 =
+// (depth / tc^2)^4 = d2^2 / tc^8 needs no second special-function op. A CTA
+// takes one slab of the columns' cells (the samples whose cell pair starts
+// there; the pair's second cell may be the next slab's first, one extra row),
+// and each lane owns its column's cells of the slab in shared memory
+// ([cell][lane]: no bank conflicts, no atomics), one copy per warp; the warps
+// of a CTA take interleaved runs of 32 points of one point group, and the CTA
+// adds its summed columns into the volume (which the launcher zeroes) with one
+// atomic per cell when there is more than one group or slab. A point's bins
+// are those whose samples can land in the slab: the bins walked are the union
+// of the lanes' column spans: every valid sample of a lane lies in its own
+// span, and a sample outside it is decided (and rejected) like any other, so
+// each (column, point, bin) is counted once. Decisions are the exact chain's
+// (sample_filtered's margin, taken over the largest |tc| of the union).
+// What bounds it: instruction issue and the four shared-memory accesses of a
+// sample's cell pair, about 25 warp instructions per warp-sample (55 with one
+// bin at a time in scalar instructions, the values handed out by shuffles and
+// floor and conversion on the special-function units). 128^3 voxels x 16,384
+// points x 1,024 bins: 62.8 -> 39.5 ms, at
+// 73% of the shared-memory pipe's wavefronts.
+// kSigned: there may be negative bin centres (a negative bin offset), whose bins
+// are a second walk of a point.
+template <bool kSigned>
+__global__ void __launch_bounds__(256, 3) confocal_adjoint_columns_kernel(
+    Geo g, Points mp, int N, int points_per_group, int run, const float* __restrict__ tr,
     float* __restrict__ vol, int accumulate, int slab) {
   // slab blockIdx.z: the samples in cells [za, za + zn) (cell pairs (z, z + 1)
   // with z < Z - 1), held in rows 0 .. slab of the column copies (row slab is
   // cell za + slab, the next slab's first)
   const int za = blockIdx.z * slab, zb = min(g.Z, za + slab), zn = min(zb, g.Z - 1) - za;
   const int rows = slab + 1;
-  extern __shared__ float acc[];  // [warp][rows][32], then the bin table
+  extern __shared__ float acc[];  // [warp][rows][32], [warp][32] bin values, the bin table
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  float2* tab = reinterpret_cast<float2*>(acc + (size_t)nw * rows * 32);  // [T]: tc^2, 1/tc^8
+  float4* vbuf = reinterpret_cast<float4*>(acc + (size_t)nw * rows * 32 + warp * 32);
+  float4* tab = reinterpret_cast<float4*>(acc + (size_t)nw * (rows + 1) * 32);
   const int tiles_y = (g.Y + 7) >> 3;
   const int ty = (blockIdx.x % tiles_y) * 8, tx = (blockIdx.x / tiles_y) * 4;
   const int yi = ty + (lane & 7), xi = tx + (lane >> 3);
   const bool live = xi < g.X && yi < g.Y;
   for (int j = threadIdx.x; j < nw * rows * 32; j += blockDim.x) acc[j] = 0.f;
-  for (int t = threadIdx.x; t < g.T + kAdjTablePad; t += blockDim.x) {
-    if (t >= g.T) {  // padding: no sample
-      tab[t] = make_float2(-INFINITY, 0.f);
-      continue;
+  for (int i = threadIdx.x; i < adj_table(g.T); i += blockDim.x) {
+    float tc2[2], i8[2];
+    for (int h = 0; h < 2; ++h) {
+      const int t = 2 * i + h;
+      const float tc = xadd(xmul((float)t, g.bw), g.bo);
+      tc2[h] = xmul(tc, tc);
+      const float i2 = __fdividef(1.f, tc2[h]);
+      i8[h] = (i2 * i2) * (i2 * i2);
+      if (t >= g.T) tc2[h] = -INFINITY, i8[h] = 0.f;  // padding: no sample
     }
-    const float tc = xadd(xmul((float)t, g.bw), g.bo);
-    const float tc2 = xmul(tc, tc);
-    const float i2 = __fdividef(1.f, tc2);
-    tab[t] = make_float2(tc2, (i2 * i2) * (i2 * i2));
+    tab[i] = make_float4(tc2[0], tc2[1], i8[0], i8[1]);
   }
   __syncthreads();
-  float* col = acc + (size_t)warp * rows * 32 + lane;
+  const uint32_t col = (uint32_t)__cvta_generic_to_shared(acc + (size_t)warp * rows * 32 + lane);
   const float x = centre(g.ox, g.sx, g.X, live ? xi : 0);
   const float y = centre(g.oy, g.sy, g.Y, live ? yi : 0);
+  // the columns' rectangle (centres are monotone in the index) and the slab's z
+  const float xa = centre(g.ox, g.sx, g.X, tx), xb = centre(g.ox, g.sx, g.X, min(tx + 3, g.X - 1));
+  const float ya = centre(g.oy, g.sy, g.Y, ty), yb = centre(g.oy, g.sy, g.Y, min(ty + 7, g.Y - 1));
+  const float bx0 = fminf(xa, xb), bx1 = fmaxf(xa, xb), by0 = fminf(ya, yb), by1 = fmaxf(ya, yb);
+  const float zlo = g.oz + ((float)za + 0.5f) / g.scale;
+  const float zhi = g.oz + ((float)zb + 0.5f) / g.scale;
   const float u = 5.9604645e-8f;
-  const int tz = first_nonneg_bin(g);
+  const int tz = kSigned ? first_nonneg_bin(g) : 0;
   const int i0 = blockIdx.y * points_per_group;
   const int i1 = min(N, i0 + points_per_group);
-  for (int base = i0 + warp * 32; base < i1; base += nw * 32) {
+  for (int base = i0 + warp * run; base < i1; base += nw * run) {
     // lane j loads point base + j
     const int ip = base + lane;
+    const int np = min(run, i1 - base);
     float lwx = 0.f, lwy = 0.f, lwz = 0.f;
-    if (ip < i1) {
+    if (lane < np) {
       lwx = mp.at(0, ip);
       lwy = mp.at(1, ip);
       lwz = mp.at(2, ip);
     }
-    const int np = min(32, i1 - base);
-    for (int j = 0; j < np; ++j) {
-      const float wx = __shfl_sync(0xffffffffu, lwx, j);
-      const float wy = __shfl_sync(0xffffffffu, lwy, j);
-      const float wz = __shfl_sync(0xffffffffu, lwz, j);
-      const float dx = xsub(wx, x), dy = xsub(wy, y);
-      const float ddx = live ? xmul(dx, dx) : INFINITY, ddy = live ? xmul(dy, dy) : 0.f;
-      Spans sp{1, 0, 1, 0};
-      float cl, ch;
-      if (live && zn > 0 &&
-          tc_bounds(dx * dx + dy * dy, wz, g.oz + ((float)za + 0.5f) / g.scale,
-                    g.oz + ((float)zb + 0.5f) / g.scale, cl, ch))
-        sp = tc_spans(g, tz, cl, ch, span_eps(g, ch, wz));
-      // warp union of the lanes' spans
-      const int p0 = __reduce_min_sync(0xffffffffu, sp.p0 <= sp.p1 ? sp.p0 : INT_MAX);
-      const int p1 = __reduce_max_sync(0xffffffffu, sp.p0 <= sp.p1 ? sp.p1 : -1);
-      int n0 = INT_MAX, n1 = -1;
-      if (tz > 0) {  // warp-uniform
-        n0 = __reduce_min_sync(0xffffffffu, sp.n0 <= sp.n1 ? sp.n0 : INT_MAX);
-        n1 = __reduce_max_sync(0xffffffffu, sp.n0 <= sp.n1 ? sp.n1 : -1);
-      }
-      if (p0 > p1 && n0 > n1) continue;  // warp-uniform
-      const Spans un{p0, p1, n0, n1};
-      // sample_filtered's margin over the union's largest |tc| (warp-uniform)
-      const float dmax = 1.001f * span_tc_max(g, un);
-      const float zmax = fabsf(wz) + dmax;
+    // and bounds its bins over the rectangle of the tile's columns: the nearest
+    // and the farthest horizontal distance give the union of the columns' spans
+    Spans sp{1, 0, 1, 0};
+    float lim = 0.f;
+    if (lane < np) {
+      const float ex = fmaxf(fmaxf(bx0 - lwx, lwx - bx1), 0.f);
+      const float ey = fmaxf(fmaxf(by0 - lwy, lwy - by1), 0.f);
+      const float fx = fmaxf(fabsf(lwx - bx0), fabsf(lwx - bx1));
+      const float fy = fmaxf(fabsf(lwy - by0), fabsf(lwy - by1));
+      float cl, ch, unused;
+      if (zn > 0 && zlo <= zhi && tc_bounds(ex * ex + ey * ey, lwz, zlo, zhi, cl, unused) &&
+          tc_bounds(fx * fx + fy * fy, lwz, zlo, zhi, unused, ch))
+        sp = tc_spans(g, tz, cl, ch, span_eps(g, ch, lwz));
+      // sample_filtered's margin over the spans' largest |tc|
+      const float dmax = 1.001f * span_tc_max(g, sp);
+      const float zmax = fabsf(lwz) + dmax;
       const float zhmax = (zmax + fabsf(g.oz)) * g.scale + 0.5f;
-      const float pm = 8.f * u * g.scale * (dmax + fabsf(wz) + zmax + fabsf(g.oz)) +
+      const float pm = 8.f * u * g.scale * (dmax + fabsf(lwz) + zmax + fabsf(g.oz)) +
                        4.f * u * zhmax + 1e-7f;
+      lim = g.exact || !(pm < 0.5f) ? 0.f : 0.5f - pm;
+    }
+    // a point's first 32 values are read while the point before it is walked
+    auto first = [&](int j) {
+      const int t = (__shfl_sync(0xffffffffu, sp.p0, j) & ~3) + lane;
+      return t < g.T ? __ldg(tr + (size_t)(base + j) * g.T + t) : 0.f;
+    };
+    float next = first(0);
+    for (int j = 0; j < np; ++j) {
+      const float val = next;
+      if (j + 1 < np) next = first(j + 1);
+      AdjPoint p;
+      p.wx = __shfl_sync(0xffffffffu, lwx, j);
+      p.wy = __shfl_sync(0xffffffffu, lwy, j);
+      p.wz = __shfl_sync(0xffffffffu, lwz, j);
+      p.lim = __shfl_sync(0xffffffffu, lim, j);
+      const int p0 = __shfl_sync(0xffffffffu, sp.p0, j);
+      const int p1 = __shfl_sync(0xffffffffu, sp.p1, j);
+      const float dx = xsub(p.wx, x), dy = xsub(p.wy, y);
+      p.ndx = live ? -xmul(dx, dx) : -INFINITY;
+      p.ndy = live ? -xmul(dy, dy) : 0.f;
       const float* row = tr + (size_t)(base + j) * g.T;
-      const float wzo = wz - g.oz;
-      adj_walk<false, U>(g, tab, row, col, p0, p1, lane, ddx, ddy, wz, wzo, pm, wx, wy, x, y,
-                         za, zn);
-      if (n0 <= n1)  // warp-uniform: negative bin centres (a negative bin offset)
-        adj_walk<true, U>(g, tab, row, col, n0, n1, lane, ddx, ddy, wz, wzo, pm, wx, wy, x, y,
-                          za, zn);
+      if (p0 <= p1)
+        adj_walk<kSigned>(g, tab, vbuf, row, p, p0, p1, val, lane, col, x, y, za, zn);
+      if (kSigned) {
+        const int n0 = __shfl_sync(0xffffffffu, sp.n0, j);
+        const int n1 = __shfl_sync(0xffffffffu, sp.n1, j);
+        const int t = (n0 & ~3) + lane;
+        if (n0 <= n1)
+          adj_walk<true>(g, tab, vbuf, row, p, n0, n1, t < g.T ? __ldg(row + t) : 0.f, lane, col,
+                         x, y, za, zn);
+      }
     }
   }
   __syncthreads();
@@ -904,7 +978,7 @@ int totri_volume_confocal_adjoint(const totri_array_t* vol, const totri_array_t*
   // lanes over columns: warps per CTA such that two CTAs' copies of 32
   // columns and the bin table fit an SM's shared memory
   // ("volume.adjoint.warps" overrides); bins beyond 4,096 take the atomic kernel
-  const size_t table = sizeof(float2) * ((size_t)T + volume::kAdjTablePad);
+  const size_t table = sizeof(float4) * volume::adj_table(T);
   // The columns split into slabs of at most 64 cells, a CTA per slab: each
   // warp's column copy is then 65 rows (8.3 KB), and 3 CTAs of 8 warps share
   // an SM (24 warps) instead of 2 of 6 with whole 128-cell columns. 128^3
@@ -915,7 +989,7 @@ int totri_volume_confocal_adjoint(const totri_array_t* vol, const totri_array_t*
   if (slabs <= 0) slabs = (int)ceil_div(Z, 64);
   slabs = std::min(slabs, Z);
   const int slab = (int)ceil_div(Z, slabs);
-  const size_t per_warp = (size_t)(slab + 1) * 32 * sizeof(float);
+  const size_t per_warp = (size_t)(slab + 2) * 32 * sizeof(float);  // cells and bin values
   int warps = T <= 4096 && table < 113 * 1024 ? (int)((113 * 1024 - table) / per_warp) : 0;
   if (tune::get("volume.adjoint.warps") > 0) warps = tune::get("volume.adjoint.warps");
   warps = std::min(warps, 8);
@@ -926,23 +1000,27 @@ int totri_volume_confocal_adjoint(const totri_array_t* vol, const totri_array_t*
   if (mode == 0 && warps >= 1 && T <= 4096) {
     const size_t smem = (size_t)warps * per_warp + table;
     const int64_t tiles = ceil_div(Y, 8) * ceil_div(X, 4);
-    // point groups: about 16 CTAs per SM in all, each group at least four
-    // runs of 32 points per warp
+    // point groups: about 16 CTAs per SM in all, each with at least a run of
+    // points per warp; runs of 32 points, or down to 8 while the CTAs would not
+    // fill the SMs' three places twice (41 x 37 x 53 voxels x 899 points: 0.60 -> 0.15 ms)
     const int nslab = (int)ceil_div(Z, slab);
     const int64_t want = std::max<int64_t>(1, (16 * tune::sm_count()) / (tiles * nslab));
+    int run = 32;
+    while (run > 8 && tiles * nslab * ceil_div(N, (int64_t)run * warps) < 6 * tune::sm_count())
+      run /= 2;
     const int groups =
-        (int)std::max<int64_t>(1, std::min<int64_t>(want, N / (128 * warps)));
-    const int per = (int)(ceil_div(ceil_div(N, groups), 32) * 32);
+        (int)std::max<int64_t>(1, std::min<int64_t>(want, ceil_div(N, (int64_t)run * warps)));
+    const int per = (int)(ceil_div(ceil_div(N, groups), run) * run);
     const int used = (int)ceil_div(N, per);
     const int accumulate = used > 1 || nslab > 1;
     if (accumulate) TOTRI_CUDA(cudaMemsetAsync(vd, 0, sizeof(float) * numel(vol), stream));
     const dim3 grid3((unsigned)tiles, (unsigned)used, (unsigned)nslab);
-    TOTRI_CUDA(tune::ensure_dynamic_smem(
-        reinterpret_cast<const void*>(volume::confocal_adjoint_columns_kernel<volume::kAdjUnroll>),
-        smem));
+    const auto kernel = g.bo < 0.f && !g.all_bins ? volume::confocal_adjoint_columns_kernel<true>
+                                                  : volume::confocal_adjoint_columns_kernel<false>;
+    TOTRI_CUDA(tune::ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem));
     TOTRI_KERNEL("volume confocal adjoint", stream,
-                 volume::confocal_adjoint_columns_kernel<volume::kAdjUnroll>
-                 <<<grid3, warps * 32, smem, stream>>>(g, pts, N, per, trd, vd, accumulate, slab));
+                 kernel<<<grid3, warps * 32, smem, stream>>>(g, pts, N, per, run, trd, vd,
+                                                             accumulate, slab));
     return TOTRI_OK;
   }
   if (Z <= 256 && mode == 2) {
