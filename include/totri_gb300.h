@@ -363,6 +363,24 @@ int totri_volume_exhaustive_grad_volume(const totri_array_t* transient_grad,
                                         const float volume_end[3], float bin_width,
                                         float bin_offset, void* stream);
 
+/* The same with an optional workspace of
+ * totri_volume_exhaustive_grad_scratch(S, L, T) bytes (at most 2 GiB; smaller
+ * or null: transient_grad is read in place, more slowly), which holds bins-last
+ * copies of transient_grad, one batch item and range of scan points at a time.
+ * The results are the same up to FP32 summation order. */
+size_t totri_volume_exhaustive_grad_scratch(int64_t num_scan_points, int64_t num_laser_points,
+                                            int64_t num_bins);
+int totri_volume_exhaustive_grad_volume_ws(const totri_array_t* transient_grad,
+                                           const totri_array_t* scan_points,
+                                           const totri_array_t* laser_points,
+                                           const totri_array_t* scan_origin,
+                                           const totri_array_t* laser_origin,
+                                           const totri_array_t* volume_grad,
+                                           const float volume_start[3],
+                                           const float volume_end[3], float bin_width,
+                                           float bin_offset, void* workspace,
+                                           size_t workspace_bytes, void* stream);
+
 /* ----------------------------------------------------------------------- */
 /* reconstruct: backprojection                                              */
 

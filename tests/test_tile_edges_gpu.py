@@ -112,3 +112,40 @@ def test_volume_adjoint_edges(cuda_lib, shape, N, T, bw, bo):
     adj = torch.full(shape, 7.0, device="cuda")
     R.volume_confocal_adjoint(adj, cu(mp), cu(y), org, size, bw, bo)
     assert rel(adj.cpu().numpy(), ref) < 1e-5
+
+
+# (D, H, W), S, L, T, bin width, offset: voxel blocks of 8 x 8 x 4 and laser groups
+# of 8 with remainders; one scan point to several slices; bins that start before
+# and end past [0, T); bins of one voxel in one bin, and past the staged 256
+PAIRS = [((1, 1, 1), 1, 1, 300, 0.02, 0.0), ((5, 9, 3), 9, 7, 500, 0.01, 0.0),
+         ((4, 8, 8), 33, 8, 120, 0.02, 1.3), ((9, 11, 17), 70, 9, 60, 0.05, 0.9),
+         ((6, 7, 9), 5, 17, 3000, 0.0011, 0.5), ((6, 7, 9), 6, 3, 1500, 0.002, 1.0),
+         ((7, 6, 5), 4, 2, 40, 0.4, -0.3)]
+
+
+@pytest.mark.parametrize("shape,S,L,T,bw,bo", PAIRS)
+def test_volume_pairs_edges(cuda_lib, shape, S, L, T, bw, bo):
+    """Forward and gradient of the exhaustive volume render against the FP64
+    oracle, 1e-5; the gradient with and without its workspace."""
+    from totri_gb300 import _lib
+    g = np.random.default_rng(S + T)
+    sp, lp = points(g, S), points(g, L)
+    vol = g.uniform(0.5, 1.5, (2,) + shape).astype(np.float32)
+    st, en = (-0.5, -0.4, 0.5), (0.45, 0.5, 1.4)
+    spt, lpt = (cu(np.stack([p.T, p.T])) for p in (sp, lp))
+    none = torch.empty((2, 3, 0), device="cuda")
+    out = torch.full((2, T, S, L), 7.0, device="cuda")
+    R.volume_render_exhaustive_forward(cu(vol), spt, lpt, none, none, out, st, en, bw, bo)
+    tg = g.uniform(0.5, 1.5, (2, T, S, L)).astype(np.float32)
+    grad = torch.full((2,) + shape, 7.0, device="cuda")
+    R.volume_render_exhaustive_grad_volume(cu(tg), spt, lpt, none, none, grad, st, en, bw, bo)
+    inplace = torch.full((2,) + shape, 7.0, device="cuda")
+    _lib.check(cuda_lib.totri_volume_exhaustive_grad_volume(
+        *[_lib.array(t) for t in (cu(tg), spt, lpt, none, none, inplace)], _lib.vec3(st),
+        _lib.vec3(en), bw, bo, _lib.stream_of(inplace.device)))
+    for b in range(2):
+        ref = oracle.volume_exhaustive_forward(vol[b], sp.T, lp.T, T, st, en, bw, bo)
+        assert rel(out[b].cpu().numpy(), ref) < 1e-5
+        ref = oracle.volume_exhaustive_adjoint(tg[b], shape, sp.T, lp.T, st, en, bw, bo)
+        assert rel(grad[b].cpu().numpy(), ref) < 1e-5
+        assert rel(inplace[b].cpu().numpy(), ref) < 1e-5

@@ -83,21 +83,6 @@ __device__ __forceinline__ int velten_bin(fv3 q, float od2, fv3 p, float bw, flo
   return nearest_bin(xadd(od2, xmul(2.f, xlen(xsub3(q, p)))), bw, bo);
 }
 
-// The float at shared-memory address `at` (the caller orders it after the
-// barrier that follows the writes).
-__device__ __forceinline__ float lds(uint32_t at) {
-  float r;
-  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(r) : "r"(at));
-  return r;
-}
-
-// Copies 4 bytes (or, with bytes = 0, writes 4 zero bytes) to shared memory
-// without passing through a register.
-__device__ __forceinline__ void cp_async4(uint32_t dst, const float* src, int bytes) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes)
-               : "memory");
-}
-
 // Square root within 2^-23 (the caller keeps x in the normal range).
 __device__ __forceinline__ float sqrt_approx(float x) {
   float r;
@@ -396,7 +381,7 @@ __global__ void __launch_bounds__(256, 5) velten_confocal_tiled_kernel(
             cp_async4(dst, bin ? src : trb, bin ? 4 : 0);
           }
         }
-        asm volatile("cp.async.wait_all;" ::: "memory");
+        cp_async_wait_all();
       }
       __syncthreads();
       // two points at a time: one test sends the lanes with a bin near a

@@ -115,6 +115,19 @@ __device__ __forceinline__ float xfma(float a, float b, float c) { return __fmaf
 __device__ __forceinline__ float xsqrt(float a) { return __fsqrt_rn(a); }
 __device__ __forceinline__ float xrcp(float a) { return __frcp_rn(a); }
 
+// a / b for a fixed divisor b with y = 1 / b correctly rounded: two steps of
+// the remainder correction q + (a - b q) y, the remainder exact in a fused
+// multiply-add. The first brings q within one ulp of a / b, from where the
+// second gives the correctly rounded quotient (Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990, theorem
+// on division with a correctly rounded reciprocal). For b, a and the quotient
+// within 2^-60 .. 2^60 or a = 0; a NaN or infinite a gives NaN.
+__device__ __forceinline__ float div_fixed(float a, float b, float y) {
+  float q = __fmul_rn(a, y);
+  q = __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
+  return __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
+}
+
 struct fv3 {
   float x, y, z;
 };
@@ -213,6 +226,36 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
+}
+
+// The float at shared-memory address `at` (the caller orders it after the
+// barrier that follows the writes).
+__device__ __forceinline__ float lds(uint32_t at) {
+  float r;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(r) : "r"(at));
+  return r;
+}
+
+// Minimum and maximum that give NaN when an operand is NaN.
+__device__ __forceinline__ float min_nan(float a, float b) {
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
+// Copies 4 bytes (or, with bytes = 0, writes 4 zero bytes) to shared memory
+// without passing through a register.
+__device__ __forceinline__ void cp_async4(uint32_t dst, const float* src, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 // Monotone float <-> int mapping for atomicMin/atomicMax on floats.

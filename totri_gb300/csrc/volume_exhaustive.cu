@@ -7,10 +7,14 @@
 // and a tile of laser points, walks the occupied voxels and splats each
 // voxel's path-length interval into a shared [T][tile] histogram that is
 // flushed with row stores; the adjoint (the forward is linear in the volume)
-// gathers per voxel.
+// gathers per voxel. A voxel's path length is the sum of a scan and a laser
+// distance, so each distance is taken once and serves a whole tile of pairs.
+#include <algorithm>
+#include <cmath>
 #include <string>
 
 #include "capi_common.cuh"
+#include "mesh_kernels.cuh"
 #include "tune.cuh"
 
 namespace totri {
@@ -19,6 +23,7 @@ namespace vexh {
 struct Geo {
   int D, H, W, S, L, T;
   float sx, sy, sz, ex, ey, ez, bw, bo;
+  float inv_bw;  // 1 / bw for div_fixed; NaN where it does not apply (every pair is exact)
 };
 
 struct Pts {  // [B, 3, n] with strides
@@ -36,27 +41,45 @@ struct Interval {
   float bf0, bf1, range;
 };
 
-// Path-length interval of voxel (xi, yi, zi) for the pair (s, l), binned
-// (volume_cuda.cu:314-364); FP32 decisions as in the oracle.
-__device__ __forceinline__ Interval interval(const Geo& g, fv3 sc, fv3 lc, int xi, int yi,
-                                             int zi) {
-  Interval r{false, 0, 0, 0.f, 0.f, 0.f};
+// The two ends of a voxel's z extent (volume_cuda.cu:314-330), each value with
+// one rounding per operation.
+struct Ends {
+  fv3 p0, p1;
+};
+__device__ __forceinline__ Ends voxel_ends(const Geo& g, int xi, int yi, int zi) {
   const float xf = xadd(g.sx, xmul(xdiv(xadd((float)xi, 0.5f), (float)g.W), xsub(g.ex, g.sx)));
   const float yf = xadd(g.sy, xmul(xdiv(xadd((float)yi, 0.5f), (float)g.H), xsub(g.ey, g.sy)));
   const float zf = xadd(g.sz, xmul(xdiv(xadd((float)zi, 0.5f), (float)g.D), xsub(g.ez, g.sz)));
   const float half = xmul(xdiv(0.5f, (float)g.D), xsub(g.ez, g.sz));
-  const float zf0 = xsub(zf, half), zf1 = xadd(zf, half);
-  const fv3 p0 = mkv(xf, yf, zf0), p1 = mkv(xf, yf, zf1);
-  float d0 = xadd(xlen(xsub3(sc, p0)), xlen(xsub3(lc, p0)));
-  float d1 = xadd(xlen(xsub3(sc, p1)), xlen(xsub3(lc, p1)));
+  return Ends{mkv(xf, yf, xsub(zf, half)), mkv(xf, yf, xadd(zf, half))};
+}
+
+// Path-length interval of a voxel for a pair whose path lengths to its two
+// ends are d0 and d1, binned (volume_cuda.cu:331-364); FP32 decisions as in the
+// oracle. The quotients come from div_fixed and the floors from an addition
+// of 1.5 2^23 rounded down while both bin coordinates lie within 2^21, from
+// the correctly rounded division and floorf otherwise (NaN and infinities too):
+// the same values either way.
+__device__ __forceinline__ Interval interval(const Geo& g, float d0, float d1) {
+  Interval r{false, 0, 0, 0.f, 0.f, 0.f};
   if (d1 < d0) {
     const float t = d0;
     d0 = d1;
     d1 = t;
   }
-  float bf0 = xdiv(xsub(d0, g.bo), g.bw), bf1 = xdiv(xsub(d1, g.bo), g.bw);
+  float bf0 = div_fixed(xsub(d0, g.bo), g.bw, g.inv_bw);
+  float bf1 = div_fixed(xsub(d1, g.bo), g.bw, g.inv_bw);
+  int first, last;
+  if (bf0 > -2097152.f && bf1 < 2097152.f) {
+    first = __float_as_int(__fadd_rd(bf0, 12582912.f)) - 0x4B400000;
+    last = __float_as_int(__fadd_rd(bf1, 12582912.f)) - 0x4B400000;
+  } else {
+    bf0 = xdiv(xsub(d0, g.bo), g.bw);
+    bf1 = xdiv(xsub(d1, g.bo), g.bw);
+    first = (int)floorf(bf0);
+    last = (int)floorf(bf1);
+  }
   const float range = xsub(bf1, bf0);
-  int first = (int)floorf(bf0), last = (int)floorf(bf1);
   if (first < 0) {
     if (last < 0) return r;
     bf0 = 0.f;
@@ -100,17 +123,33 @@ __global__ void __launch_bounds__(256) forward_kernel(Geo g, int b, const float*
   for (int j = threadIdx.x; j < g.T * LT; j += blockDim.x) hist[j] = 0.f;
   __syncthreads();
   const uint32_t nnz = *count;
-  const int ll = threadIdx.x % LT;
-  const int l = l0 + ll;
-  if (l < g.L) {
-    const fv3 sc = sp.at(b, s), lc = lp.at(b, l);
-    for (uint32_t v = threadIdx.x / LT; v < nnz; v += blockDim.x / LT) {
-      const uint32_t lin = __ldg(list + v);
-      const int xi = (int)(lin % g.W), yi = (int)((lin / g.W) % g.H);
-      const int zi = (int)(lin / ((uint32_t)g.W * g.H));
-      const Interval iv = interval(g, sc, lc, xi, yi, zi);
+  // a thread takes one occupied voxel at a time to every laser of the tile, in
+  // an order that starts at its lane: the lanes of a warp add to different
+  // histogram columns
+  __shared__ float laser[LT][3];
+  if (threadIdx.x < LT && l0 + (int)threadIdx.x < g.L) {
+    const fv3 q = lp.at(b, l0 + threadIdx.x);
+    laser[threadIdx.x][0] = q.x;
+    laser[threadIdx.x][1] = q.y;
+    laser[threadIdx.x][2] = q.z;
+  }
+  __syncthreads();
+  const fv3 sc = sp.at(b, s);
+  for (uint32_t v = threadIdx.x; v < nnz; v += blockDim.x) {
+    const uint32_t lin = __ldg(list + v);
+    const int xi = (int)(lin % g.W), yi = (int)((lin / g.W) % g.H);
+    const int zi = (int)(lin / ((uint32_t)g.W * g.H));
+    const Ends e = voxel_ends(g, xi, yi, zi);
+    const float occ = __ldg(vol + lin);
+    const float s0 = xlen(xsub3(sc, e.p0)), s1 = xlen(xsub3(sc, e.p1));
+#pragma unroll 1
+    for (int i = 0; i < LT; ++i) {
+      const int ll = (threadIdx.x + i) & (LT - 1);
+      if (l0 + ll >= g.L) continue;
+      const fv3 lc = mkv(laser[ll][0], laser[ll][1], laser[ll][2]);
+      const Interval iv = interval(g, xadd(s0, xlen(xsub3(lc, e.p0))),
+                                   xadd(s1, xlen(xsub3(lc, e.p1))));
       if (!iv.ok) continue;
-      const float occ = __ldg(vol + lin);
       float* col = hist + ll;
       if (iv.first == iv.last) {
         atomicAdd(col + iv.first * LT, occ);
@@ -131,34 +170,164 @@ __global__ void __launch_bounds__(256) forward_kernel(Geo g, int b, const float*
   }
 }
 
-// d loss / d volume: per voxel, the forward weights against transient_grad.
-__global__ void adjoint_kernel(Geo g, int B, Pts sp, Pts lp, const float* __restrict__ tg,
-                               float* __restrict__ vg) {
-  const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t nv = (int64_t)g.D * g.H * g.W;
-  if (v >= nv * B) return;
-  const int b = (int)(v / nv);
-  const int64_t lin = v - (int64_t)b * nv;
-  const int xi = (int)(lin % g.W), yi = (int)((lin / g.W) % g.H), zi = (int)(lin / ((int64_t)g.W * g.H));
+// d loss / d volume: per voxel, the forward weights against transient_grad. A
+// CTA takes a block of 8 x 8 x 4 voxels, one per thread, and the scan points of
+// its slice; a thread holds the distances of its voxel's ends to kLC lasers in
+// registers and walks the scan points, so a pair costs two additions, the
+// division by the bin width and its bins. transient_grad element (t, s, l) is
+// tg[((s - s_base) L + l) cstep + t bstep]: in bins-last order (bstep 1) the bins that
+// the block can reach in a pair are one run of memory, which a warp copies to
+// shared memory (cp.async, the next scan point's while this one's are used). A window past kRows bins, or without
+// sound bounds, is read in place. 56 x 40 x 48 voxels x 256 scan points x 36
+// lasers, 1,024 bins: 21.8 ms (four square roots and eight divisions per pair,
+// every bin another sector of the in-place order) -> 3.65 ms,
+// at 91% of issue slots: about 50 instructions per pair and 5 per bin.
+constexpr int kLC = 8, kRows = 256;
+
+// A pair's weighted bins, read in place.
+__device__ __noinline__ float pair_direct(Geo g, float d0, float d1, const float* __restrict__ col,
+                                          int64_t bstep) {
+  const Interval iv = interval(g, d0, d1);
+  if (!iv.ok) return 0.f;
+  if (iv.first == iv.last) return __ldg(col + iv.first * bstep);
+  float sum = (1.f - (iv.bf0 - (float)iv.first)) * __ldg(col + iv.first * bstep);
+  for (int t = iv.first + 1; t < iv.last; ++t) sum += __ldg(col + t * bstep);
+  sum += (iv.bf1 - (float)iv.last) * __ldg(col + iv.last * bstep);
+  return sum / iv.range;
+}
+
+__global__ void __launch_bounds__(256, 4) adjoint_kernel(Geo g, int b, Pts sp, Pts lp, int s_base,
+                                                         int s_end, int per_slice,
+                                                         const float* __restrict__ tg,
+                                                         int64_t cstep, int64_t bstep,
+                                                         float* __restrict__ vg, int accumulate) {
+  using u64 = unsigned long long;
+  __shared__ float win[2][kLC][kRows];
+  __shared__ float2 laser[kLC][256];  // distances of the thread's voxel ends to the lasers
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;  // warp w stages laser l0 + w
+  const int nbx = (g.W + 7) >> 3, nby = (g.H + 7) >> 3;
+  const int x0 = (blockIdx.x % nbx) * 8, y0 = (blockIdx.x / nbx) % nby * 8;
+  const int z0 = blockIdx.x / (nbx * nby) * 4;
+  const int xi = x0 + (threadIdx.x & 7), yi = y0 + ((threadIdx.x >> 3) & 7);
+  const int zi = z0 + (threadIdx.x >> 6);
+  // threads past the volume's edge work on a clamped voxel and write nothing
+  const Ends e = voxel_ends(g, min(xi, g.W - 1), min(yi, g.H - 1), min(zi, g.D - 1));
+  float box[6];  // of the block: voxel positions are monotone in the index
+  {
+    const Ends a = voxel_ends(g, x0, y0, z0);
+    const Ends c = voxel_ends(g, min(x0 + 8, g.W) - 1, min(y0 + 8, g.H) - 1,
+                              min(z0 + 4, g.D) - 1);
+    box[0] = fminf(a.p0.x, c.p0.x), box[3] = fmaxf(a.p0.x, c.p0.x);
+    box[1] = fminf(a.p0.y, c.p0.y), box[4] = fmaxf(a.p0.y, c.p0.y);
+    box[2] = fminf(fminf(a.p0.z, a.p1.z), fminf(c.p0.z, c.p1.z));
+    box[5] = fmaxf(fmaxf(a.p0.z, a.p1.z), fmaxf(c.p0.z, c.p1.z));
+  }
+  // nearest and farthest distance from q to the box (NaN for a NaN point)
+  auto reach = [&](fv3 q, float& near, float& far) {
+    const float ex = fmaxf(fmaxf(box[0] - q.x, q.x - box[3]), 0.f);
+    const float ey = fmaxf(fmaxf(box[1] - q.y, q.y - box[4]), 0.f);
+    const float ez = fmaxf(fmaxf(box[2] - q.z, q.z - box[5]), 0.f);
+    const float fx = fmaxf(fabsf(q.x - box[0]), fabsf(q.x - box[3]));
+    const float fy = fmaxf(fabsf(q.y - box[1]), fabsf(q.y - box[4]));
+    const float fz = fmaxf(fabsf(q.z - box[2]), fabsf(q.z - box[5]));
+    near = sqrtf(ex * ex + ey * ey + ez * ez);
+    far = sqrtf(fx * fx + fy * fy + fz * fz);
+  };
+  const int s0 = s_base + blockIdx.y * per_slice, s1 = min(s_end, s0 + per_slice);
+  const u64 nbo = f2pack(-g.bo, -g.bo), nbw = f2pack(-g.bw, -g.bw);
+  const u64 inv = f2pack(g.inv_bw, g.inv_bw), big = f2pack(12582912.f, 12582912.f);
+  const float bins = (float)min(g.T, 2097152);
   float acc = 0.f;
-  const size_t st = (size_t)g.S * g.L;
-  for (int s = 0; s < g.S; ++s) {
-    const fv3 sc = sp.at(b, s);
-    for (int l = 0; l < g.L; ++l) {
-      const Interval iv = interval(g, sc, lp.at(b, l), xi, yi, zi);
-      if (!iv.ok) continue;
-      const float* col = tg + (size_t)b * g.T * st + (size_t)s * g.L + l;
-      if (iv.first == iv.last) {
-        acc += __ldg(col + iv.first * st);
-        continue;
+  for (int l0 = 0; l0 < g.L; l0 += kLC) {
+    const int nl = min(kLC, g.L - l0);
+#pragma unroll 1
+    for (int k = 0; k < nl; ++k) {
+      const fv3 lc = lp.at(b, l0 + k);
+      laser[k][threadIdx.x] = make_float2(xlen(xsub3(lc, e.p0)), xlen(xsub3(lc, e.p1)));
+    }
+    float lnear, lfar;  // lane k: laser l0 + k
+    reach(lp.at(b, min(l0 + (lane & (kLC - 1)), g.L - 1)), lnear, lfar);
+    float snear = 0.f, sfar = 0.f;  // lane j: scan point s0 + 32 i + j
+    // Stages the windows of scan point s; lane k receives laser l0 + k's first
+    // bin and bins (none: read in place).
+    auto stage = [&](int s, int buf) {
+      if (((s - s0) & 31) == 0) reach(sp.at(b, min(s + lane, s_end - 1)), snear, sfar);
+      const float near = __shfl_sync(0xffffffffu, snear, (s - s0) & 31) + lnear;
+      const float far = __shfl_sync(0xffffffffu, sfar, (s - s0) & 31) + lfar;
+      const float c0 = (near - g.bo) / g.bw, c1 = (far - g.bo) / g.bw;
+      int2 w = make_int2(0, 0);
+      if (g.bw > 0.f && c0 > -262144.f && c1 < 262144.f) {  // (NaN: no window)
+        w.x = max((int)floorf(c0) - 1, 0);
+        w.y = min((int)floorf(c1) + 1, g.T - 1) - w.x + 1;
+        if (w.y > kRows || w.y < 0) w.y = 0;
       }
-      float sum = (1.f - (iv.bf0 - (float)iv.first)) * __ldg(col + iv.first * st);
-      for (int t = iv.first + 1; t < iv.last; ++t) sum += __ldg(col + t * st);
-      sum += (iv.bf1 - (float)iv.last) * __ldg(col + iv.last * st);
-      acc += sum / iv.range;
+      const int first = __shfl_sync(0xffffffffu, w.x, warp);
+      const int rows = __shfl_sync(0xffffffffu, w.y, warp);
+      if (l0 + warp < g.L) {
+        const float* src =
+            tg + ((int64_t)(s - s_base) * g.L + l0 + warp) * cstep + (first + lane) * bstep;
+        uint32_t dst = (uint32_t)__cvta_generic_to_shared(&win[buf][warp][lane]);
+        for (int r = lane; r < rows; r += 32, dst += 128, src += 32 * bstep)
+          cp_async4(dst, src, 4);
+      }
+      return w;
+    };
+    __syncthreads();  // the previous lasers' windows are consumed
+    int2 next = stage(s0, 0);
+    for (int s = s0; s < s1; ++s) {
+      const int2 w = next;
+      const int buf = (s - s0) & 1;
+      cp_async_wait_all();
+      __syncthreads();  // this point's windows are there, the other buffer's are consumed
+      if (s + 1 < s1) next = stage(s + 1, buf ^ 1);
+      const fv3 sc = sp.at(b, s);
+      const u64 d = f2pack(xlen(xsub3(sc, e.p0)), xlen(xsub3(sc, e.p1)));
+      float part = 0.f;
+#pragma unroll 1
+      for (int k = 0; k < nl; ++k) {
+        // interval() for bins inside [0, T): the ends' quotients in pairs
+        const float2 e2 = laser[k][threadIdx.x];
+        float da, db;
+        f2unpack(f2add(d, f2pack(e2.x, e2.y)), da, db);
+        const u64 a = f2add(f2pack(min_nan(da, db), max_nan(da, db)), nbo);
+        u64 q = f2mul(a, inv);
+        q = f2fma(f2fma(q, nbw, a), inv, q);
+        q = f2fma(f2fma(q, nbw, a), inv, q);
+        const u64 x = f2add_rm(q, big);
+        float q0, q1, x0, x1, f0, f1;
+        f2unpack(q, q0, q1);
+        f2unpack(x, x0, x1);
+        f2unpack(f2sub(q, f2sub(x, big)), f0, f1);  // the ends' bin fractions
+        const int lo = __shfl_sync(0xffffffffu, w.x, k);
+        const int rows = __shfl_sync(0xffffffffu, w.y, k);
+        if (rows > 0 && q0 >= 0.f && q1 < bins) {  // (NaN: no)
+          const int n = __float_as_int(x1) - __float_as_int(x0);
+          const uint32_t c = (uint32_t)__cvta_generic_to_shared(&win[buf][k][0]) +
+                             4u * (__float_as_uint(x0) - 0x4B400000u - (uint32_t)lo);
+          const float c0 = lds(c);
+          float sum = (1.f - f0) * c0 + f1 * lds(c + 4u * n);
+#pragma unroll 1
+          for (int i = 1; i < n; i += 4) {
+            const uint32_t ci = c + 4u * i;
+            const float v0 = lds(ci), v1 = i + 1 < n ? lds(ci + 4u) : 0.f;
+            const float v2 = i + 2 < n ? lds(ci + 8u) : 0.f, v3 = i + 3 < n ? lds(ci + 12u) : 0.f;
+            sum += (v0 + v1) + (v2 + v3);
+          }
+          // sum / range: the hardware reciprocal and one remainder correction
+          const float range = q1 - q0, r = __fdividef(1.f, range), y = sum * r;
+          part += n == 0 ? c0 : fmaf(fmaf(-y, range, sum), r, y);
+        } else {
+          part += pair_direct(g, da, db, tg + ((int64_t)(s - s_base) * g.L + l0 + k) * cstep,
+                              bstep);
+        }
+      }
+      acc += part;
     }
   }
-  vg[v] = acc;
+  if (xi >= g.W || yi >= g.H || zi >= g.D) return;
+  float* dst = vg + (((size_t)b * g.D + zi) * g.H + yi) * g.W + xi;
+  if (accumulate) atomicAdd(dst, acc);
+  else *dst = acc;
 }
 
 }  // namespace vexh
@@ -172,6 +341,15 @@ int check_pts(const totri_array_t* a, const char* name, int64_t B, int64_t& n, v
   n = a->shape[2];
   p = vexh::Pts{static_cast<const float*>(a->data), a->strides[0], a->strides[1], a->strides[2]};
   return TOTRI_OK;
+}
+
+vexh::Geo make_geo(const totri_array_t* vol, int64_t S, int64_t L, int64_t T, const float* start,
+                   const float* end, float bw, float bo) {
+  vexh::Geo g{(int)vol->shape[1], (int)vol->shape[2], (int)vol->shape[3], (int)S, (int)L, (int)T,
+              start[0], start[1], start[2], end[0], end[1], end[2], bw, bo, 1.f / bw};
+  const float a = std::fabs(bw);
+  if (!(a > 1e-18f && a < 1e18f)) g.inv_bw = NAN;  // div_fixed's range
+  return g;
 }
 
 template <int LT>
@@ -219,9 +397,7 @@ int totri_volume_exhaustive_forward(const totri_array_t* vol, const totri_array_
   TOTRI_TRY(check_dim(transient, "transient", 2, S));
   TOTRI_TRY(check_dim(transient, "transient", 3, L));
   TOTRI_TRY(check_contiguous(transient, "transient"));
-  vexh::Geo g{(int)vol->shape[1], (int)vol->shape[2], (int)vol->shape[3], (int)S, (int)L,
-              (int)transient->shape[1], start[0], start[1], start[2], end[0], end[1], end[2],
-              bw, bo};
+  const vexh::Geo g = make_geo(vol, S, L, transient->shape[1], start, end, bw, bo);
   if (numel(transient) == 0) return TOTRI_OK;
   const int64_t nv = (int64_t)g.D * g.H * g.W;
   const size_t need = align_up(sizeof(uint32_t) * (nv + 64), 256);
@@ -246,9 +422,11 @@ int totri_volume_exhaustive_forward(const totri_array_t* vol, const totri_array_
       else TOTRI_TRY(launch_fwd<1>(g, b, vb, list, count, sp, lp, out, stream));
     } else if (want != 0) {
       return fail(TOTRI_ERR_INVALID_ARGUMENT, "laser tile must be 1, 8 or 32");
-    } else if ((size_t)g.T * 32 * 4 <= budget && L >= 32)
-      TOTRI_TRY(launch_fwd<32>(g, b, vb, list, count, sp, lp, out, stream));
-    else if ((size_t)g.T * 8 * 4 <= budget && L >= 8)
+    } else if ((size_t)g.T * 8 * 4 <= budget && L >= 4)
+      // 8 lasers: several CTAs per SM up to 1,600 bins or so, and whole 32-byte
+      // sectors of the output (36 lasers, 1,024 bins, 256 scan points x 2,150
+      // voxels: 0.25 ms; 32 lasers, one CTA per SM and a second tile of 4 lasers:
+      // 1.06 ms)
       TOTRI_TRY(launch_fwd<8>(g, b, vb, list, count, sp, lp, out, stream));
     else if ((size_t)g.T * 4 <= budget)
       TOTRI_TRY(launch_fwd<1>(g, b, vb, list, count, sp, lp, out, stream));
@@ -258,13 +436,18 @@ int totri_volume_exhaustive_forward(const totri_array_t* vol, const totri_array_
   return TOTRI_OK;
 }
 
-int totri_volume_exhaustive_grad_volume(const totri_array_t* tg,
-                                        const totri_array_t* scan_points,
-                                        const totri_array_t* laser_points,
-                                        const totri_array_t* scan_origin,
-                                        const totri_array_t* laser_origin,
-                                        const totri_array_t* vg, const float start[3],
-                                        const float end[3], float bw, float bo, void* stream_) {
+size_t totri_volume_exhaustive_grad_scratch(int64_t S, int64_t L, int64_t T) {
+  return mesh::exh_grad_scratch_bytes(S, L, T);
+}
+
+int totri_volume_exhaustive_grad_volume_ws(const totri_array_t* tg,
+                                           const totri_array_t* scan_points,
+                                           const totri_array_t* laser_points,
+                                           const totri_array_t* scan_origin,
+                                           const totri_array_t* laser_origin,
+                                           const totri_array_t* vg, const float start[3],
+                                           const float end[3], float bw, float bo, void* ws,
+                                           size_t ws_bytes, void* stream_) {
   (void)scan_origin;
   (void)laser_origin;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
@@ -280,15 +463,61 @@ int totri_volume_exhaustive_grad_volume(const totri_array_t* tg,
   TOTRI_TRY(check_dim(tg, "transient_grad", 2, S));
   TOTRI_TRY(check_dim(tg, "transient_grad", 3, L));
   TOTRI_TRY(check_contiguous(tg, "transient_grad"));
-  vexh::Geo g{(int)vg->shape[1], (int)vg->shape[2], (int)vg->shape[3], (int)S, (int)L,
-              (int)tg->shape[1], start[0], start[1], start[2], end[0], end[1], end[2], bw, bo};
+  const int64_t T = tg->shape[1];
+  const vexh::Geo g = make_geo(vg, S, L, T, start, end, bw, bo);
   const int64_t n = numel(vg);
   if (n == 0) return TOTRI_OK;
-  TOTRI_KERNEL("volume exhaustive adjoint", stream,
-               vexh::adjoint_kernel<<<(unsigned)ceil_div(n, 128), 128, 0, stream>>>(
-                   g, (int)B, sp, lp, static_cast<const float*>(tg->data),
-                   static_cast<float*>(vg->data)));
+  float* out = static_cast<float*>(vg->data);
+  if (S == 0 || L == 0 || T == 0) {
+    TOTRI_CUDA(cudaMemsetAsync(out, 0, sizeof(float) * n, stream));
+    return TOTRI_OK;
+  }
+  // Scan points per bins-last copy (all of them up to 2 GiB); 0: read in place.
+  // The copy costs one read and write of transient_grad, a pair's reads in place
+  // a sector per voxel and bin.
+  int64_t chunk = ws ? mesh::exh_grad_chunk_points(S, L, T) : 0;
+  if (ws_bytes < (size_t)chunk * L * T * sizeof(float)) chunk = 0;
+  const int64_t step = chunk > 0 ? chunk : S;
+  const int64_t blocks = ceil_div(g.W, 8) * ceil_div(g.H, 8) * ceil_div(g.D, 4);
+  // slices of the scan points until about 8 waves of CTAs (4 per SM), with at
+  // least 8 scan points each (a slice repeats the lasers' distances)
+  const int64_t slices = std::max<int64_t>(
+      1, std::min<int64_t>(ceil_div(32 * (int64_t)tune::sm_count(), blocks), step / 8));
+  const int per = (int)ceil_div(step, slices);
+  const int accumulate = ceil_div(step, per) > 1 || step < S;
+  if (accumulate) TOTRI_CUDA(cudaMemsetAsync(out, 0, sizeof(float) * n, stream));
+  const int64_t row = S * L;
+  for (int b = 0; b < (int)B; ++b) {
+    const float* tb = static_cast<const float*>(tg->data) + (int64_t)b * T * row;
+    for (int64_t sa = 0; sa < S; sa += step) {
+      const int64_t sb = std::min(S, sa + step);
+      const dim3 grid((unsigned)blocks, (unsigned)ceil_div(sb - sa, per));
+      if (chunk > 0) {
+        float* copy = static_cast<float*>(ws);
+        TOTRI_TRY(mesh::launch_bins_last(tb + sa * L, copy, (int)T, row, (sb - sa) * L, stream));
+        TOTRI_KERNEL("volume exhaustive adjoint", stream,
+                     vexh::adjoint_kernel<<<grid, 256, 0, stream>>>(
+                         g, b, sp, lp, (int)sa, (int)sb, per, copy, T, 1, out, accumulate));
+      } else {
+        TOTRI_KERNEL("volume exhaustive adjoint", stream,
+                     vexh::adjoint_kernel<<<grid, 256, 0, stream>>>(
+                         g, b, sp, lp, (int)sa, (int)sb, per, tb, 1, row, out, accumulate));
+      }
+    }
+  }
   return TOTRI_OK;
+}
+
+int totri_volume_exhaustive_grad_volume(const totri_array_t* tg,
+                                        const totri_array_t* scan_points,
+                                        const totri_array_t* laser_points,
+                                        const totri_array_t* scan_origin,
+                                        const totri_array_t* laser_origin,
+                                        const totri_array_t* vg, const float start[3],
+                                        const float end[3], float bw, float bo, void* stream) {
+  return totri_volume_exhaustive_grad_volume_ws(tg, scan_points, laser_points, scan_origin,
+                                                laser_origin, vg, start, end, bw, bo, nullptr, 0,
+                                                stream);
 }
 
 }  // extern "C"

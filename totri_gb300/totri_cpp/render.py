@@ -97,11 +97,11 @@ def mesh_exhaustive_grad_verts(verts, faces, material, scan_points, laser_points
                                        transient_grad.shape[1]))
 
 
-def _vol_call(name, tensors, a3, b3, bw, bo, device, voxels=None):
+def _vol_call(name, tensors, a3, b3, bw, bo, device, voxels=None, extra=()):
     """Calls a volume entry point; `voxels` (voxels per batch item) adds the
-    occupied-voxel scratch those entry points need."""
+    occupied-voxel scratch those entry points need, `extra` other workspace
+    arguments."""
     lib = _lib.load()
-    extra = ()
     if voxels is not None:
         n = int(lib.totri_volume_workspace(int(voxels)))
         ws = torch.empty(max(n, 1), dtype=torch.uint8, device=device)
@@ -181,10 +181,13 @@ def volume_render_exhaustive_grad_volume(transient_grad, scan_points, laser_poin
     _lib.require_cuda(transient_grad, scan_points, laser_points, scan_origin, laser_origin,
                       volume_grad)
     out = dense_out(volume_grad)
-    _vol_call("totri_volume_exhaustive_grad_volume",
+    n = int(_lib.load().totri_volume_exhaustive_grad_scratch(
+        int(scan_points.shape[2]), int(laser_points.shape[2]), int(transient_grad.shape[1])))
+    ws = torch.empty(n, dtype=torch.uint8, device=volume_grad.device) if n > 0 else None
+    _vol_call("totri_volume_exhaustive_grad_volume_ws",
               (transient_grad.contiguous(), scan_points, laser_points, scan_origin,
                laser_origin, out), volume_start, volume_end, bin_width, bin_offset,
-              volume_grad.device)
+              volume_grad.device, extra=ws_args(ws))
     finish_out(volume_grad, out)
 
 
