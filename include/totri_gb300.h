@@ -412,6 +412,21 @@ int totri_backprojection_exhaustive_velten_forward(
     const float volume_start[3], const float volume_end[3], float bin_width,
     float bin_offset, void* stream);
 
+/* The same with an optional workspace of
+ * totri_backprojection_exhaustive_velten_scratch(S, L, T) bytes (at most 2 GiB;
+ * smaller or null: the transient is read in place, more slowly), which holds
+ * bins-last copies of the transient, one batch item and range of scan points at
+ * a time. The results are the same up to FP32 summation order. */
+size_t totri_backprojection_exhaustive_velten_scratch(int64_t num_scan_points,
+                                                      int64_t num_laser_points,
+                                                      int64_t num_bins);
+int totri_backprojection_exhaustive_velten_forward_ws(
+    const totri_array_t* transient, const totri_array_t* scan_points,
+    const totri_array_t* laser_points, const totri_array_t* scan_origin,
+    const totri_array_t* laser_origin, const totri_array_t* volume,
+    const float volume_start[3], const float volume_end[3], float bin_width,
+    float bin_offset, void* workspace, size_t workspace_bytes, void* stream);
+
 /* Replaces totri_cpp.reconstruct.backprojection_exhaustive_arellano_forward
  * (src/reconstruct/backprojection.h:10-19, backprojection.cpp:8-20).
  * transient [B,T,S,L]; points [B,3,S] / [B,3,L]; volume [B,D,H,W]

@@ -149,3 +149,35 @@ def test_volume_pairs_edges(cuda_lib, shape, S, L, T, bw, bo):
         ref = oracle.volume_exhaustive_adjoint(tg[b], shape, sp.T, lp.T, st, en, bw, bo)
         assert rel(grad[b].cpu().numpy(), ref) < 1e-5
         assert rel(inplace[b].cpu().numpy(), ref) < 1e-5
+
+
+# (D, H, W), S, L, T, bin width, offset: voxel blocks of 8 x 8 x 16 and laser groups
+# of 8 with remainders, one to several slices of the scan points, more bins than
+# voxels (read in place), bins before and past [0, T), a single-voxel axis (no bin)
+VELTEN_PAIRS = [((2, 2, 2), 1, 1, 200, 0.02, 0.0), ((17, 9, 10), 9, 7, 300, 0.01, 0.0),
+                ((16, 8, 8), 5, 8, 64, 0.02, 1.9), ((33, 12, 7), 40, 17, 100, 0.02, 1.1),
+                ((12, 10, 8), 6, 9, 2000, 0.0017, 0.0), ((1, 9, 9), 3, 2, 100, 0.03, -0.2)]
+
+
+@pytest.mark.parametrize("shape,S,L,T,bw,bo", VELTEN_PAIRS)
+@pytest.mark.parametrize("origin", [False, True])
+def test_velten_pairs_edges(cuda_lib, shape, S, L, T, bw, bo, origin):
+    from totri_gb300 import _lib
+    g = np.random.default_rng(S + T)
+    sp, lp = points(g, S), points(g, L)
+    so, lo = (points(g, n, -0.3) if origin else None for n in (S, L))
+    st, en = (-0.5, -0.4, 0.5), (0.45, 0.5, 1.4)
+    tr = g.integers(0, 16, (2, T, S, L)).astype(np.float32)
+    pair = [cu(np.stack([p, p])) for p in (sp, lp)]
+    pair += [cu(np.stack([p, p])) if origin else torch.empty((2, 0, 3), device="cuda")
+             for p in (so, lo)]
+    out = torch.full((2,) + shape, 7.0, device="cuda")
+    K.backprojection_exhaustive_velten_forward(cu(tr), *pair, out, st, en, bw, bo)
+    inplace = torch.full((2,) + shape, 7.0, device="cuda")
+    _lib.check(cuda_lib.totri_backprojection_exhaustive_velten_forward(
+        *[_lib.array(t) for t in (cu(tr), *pair, inplace)], _lib.vec3(st), _lib.vec3(en), bw, bo,
+        _lib.stream_of(inplace.device)))
+    for b in range(2):
+        ref = oracle.bp_exhaustive_velten(tr[b], sp, lp, so, lo, shape, st, en, bw, bo)
+        assert np.array_equal(out[b].double().cpu().numpy(), ref)
+        assert np.array_equal(inplace[b].double().cpu().numpy(), ref)

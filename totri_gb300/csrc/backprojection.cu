@@ -13,6 +13,7 @@
 #include <string>
 
 #include "capi_common.cuh"
+#include "mesh_kernels.cuh"
 #include "tune.cuh"
 
 namespace totri {
@@ -587,6 +588,100 @@ __global__ void __launch_bounds__(128) velten_exhaustive_kernel(Grid g, int b, i
   vol[(size_t)b * nv + v] = value;
 }
 
+// Velten exhaustive over blocks of 8 x 8 x 16 voxels, four of a column per
+// thread. A path length is the sum of a scan and a laser distance, so a thread
+// keeps its voxels' distances to a group of kLG lasers in shared memory, takes
+// the distances to each scan point of its slice once per group, and a triple
+// costs two additions, the bin (exactly as nearest_bin rounds it: div_fixed and a
+// floor by an addition rounded down, two voxels per paired instruction) and one
+// read. Transient element (t, s, l) is tr[((s - s_base) L + l) cstep + t bstep]: in
+// bins-last order (kLast, bstep 1) the lanes' bins of a pair lie within a few
+// cache lines, in place every bin is another sector. What bounds it: the FP32
+// pipe (59%) and waits on the reads through L1, at 66% of issue slots.
+// 48^3 voxels x 256 scan points x 64 lasers, 1,024 bins: 7.9 ms (two correctly
+// rounded roots and a division per triple, in-place reads) -> 1.24 ms.
+constexpr int kLG = 8;
+template <bool kLast>
+__global__ void __launch_bounds__(256, 4) velten_pairs_kernel(
+    Grid g, int b, int T, int S, int L, Pts3 sp, Pts3 lp, Pts3 so, Pts3 lo, int has_so, int has_lo,
+    float bw, float bo, float inv_bw, int s_base, int s_end, int per_slice,
+    const float* __restrict__ tr, int64_t cstep, int64_t bstep, float* __restrict__ vol,
+    int accumulate) {
+  using u64 = unsigned long long;
+  __shared__ float4 laser[kLG][256];
+  __shared__ float lod[kLG];
+  const int nbx = (g.W + 7) >> 3, nby = (g.H + 7) >> 3;
+  const int x = (int)(blockIdx.x % nbx) * 8 + (threadIdx.x & 7);
+  const int y = (int)(blockIdx.x / nbx % nby) * 8 + ((threadIdx.x >> 3) & 7);
+  const int z0 = (int)(blockIdx.x / (nbx * nby)) * 16 + (threadIdx.x >> 6);
+  // voxels z0 + 4 v; those past the volume's edge work on a clamped position
+  fv3 p[4];
+#pragma unroll
+  for (int v = 0; v < 4; ++v)
+    p[v] = voxel_point(g, min(x, g.W - 1), min(y, g.H - 1), min(z0 + 4 * v, g.D - 1));
+  const u64 nbo = f2pack(-bo, -bo), nbw = f2pack(-bw, -bw), inv = f2pack(inv_bw, inv_bw);
+  const u64 half = f2pack(0.5f, 0.5f), big = f2pack(12582912.f, 12582912.f);  // 1.5 2^23
+  const int s0 = s_base + blockIdx.y * per_slice, s1 = min(s_end, s0 + per_slice);
+  u64 acc[2] = {0ull, 0ull};
+  for (int l0 = 0; l0 < L; l0 += kLG) {
+    const int nl = min(kLG, L - l0);
+    __syncthreads();  // the previous group's origin terms are consumed
+    if ((int)threadIdx.x < nl)
+      lod[threadIdx.x] =
+          has_lo ? xlen(xsub3(lp.at(b, l0 + threadIdx.x), lo.at(b, l0 + threadIdx.x))) : 0.f;
+#pragma unroll 1
+    for (int k = 0; k < nl; ++k) {
+      const fv3 q = lp.at(b, l0 + k);
+      laser[k][threadIdx.x] = make_float4(xlen(xsub3(q, p[0])), xlen(xsub3(q, p[1])),
+                                          xlen(xsub3(q, p[2])), xlen(xsub3(q, p[3])));
+    }
+    __syncthreads();
+    for (int s = s0; s < s1; ++s) {
+      const fv3 q = sp.at(b, s);
+      const float sod = has_so ? xlen(xsub3(q, so.at(b, s))) : 0.f;
+      u64 a[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        a[h] = f2pack(xadd(sod, xlen(xsub3(q, p[2 * h]))), xadd(sod, xlen(xsub3(q, p[2 * h + 1]))));
+      const float* col = tr + ((int64_t)(s - s_base) * L + l0) * cstep;
+      u64 part[2] = {0ull, 0ull};
+#pragma unroll 2
+      for (int k = 0; k < nl; ++k, col += cstep) {
+        const float4 d = laser[k][threadIdx.x];
+        const u64 o = f2pack(lod[k], lod[k]);
+        const u64 ld[2] = {f2pack(d.x, d.y), f2pack(d.z, d.w)};
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const u64 n = f2add(f2add(f2add(a[h], ld[h]), o), nbo);
+          u64 c = f2mul(n, inv);  // div_fixed
+          c = f2fma(f2fma(c, nbw, n), inv, c);
+          c = f2fma(f2fma(c, nbw, n), inv, c);
+          float xa, xb;
+          f2unpack(f2add_rm(f2add(c, half), big), xa, xb);
+          // (a bin outside [0, T), or a NaN, reads nothing)
+          const unsigned ta = __float_as_uint(xa) - 0x4B400000u;
+          const unsigned tb = __float_as_uint(xb) - 0x4B400000u;
+          const float va = ta < (unsigned)T ? __ldg(col + (kLast ? (int64_t)ta : ta * bstep)) : 0.f;
+          const float vb = tb < (unsigned)T ? __ldg(col + (kLast ? (int64_t)tb : tb * bstep)) : 0.f;
+          part[h] = f2add(part[h], f2pack(va, vb));
+        }
+      }
+      acc[0] = f2add(acc[0], part[0]);
+      acc[1] = f2add(acc[1], part[1]);
+    }
+  }
+  float val[4];
+  f2unpack(acc[0], val[0], val[1]);
+  f2unpack(acc[1], val[2], val[3]);
+#pragma unroll
+  for (int v = 0; v < 4; ++v) {
+    if (x >= g.W || y >= g.H || z0 + 4 * v >= g.D) continue;
+    float* dst = vol + (((size_t)b * g.D + z0 + 4 * v) * g.H + y) * g.W + x;
+    if (accumulate) atomicAdd(dst, val[v]);
+    else *dst = val[v];
+  }
+}
+
 struct Pts3T {  // [B, 3, n] with strides
   const float* p;
   int64_t sb, sc, sn;
@@ -828,11 +923,15 @@ int totri_backprojection_confocal_velten_adjoint(const totri_array_t* volume,
   return TOTRI_OK;
 }
 
-int totri_backprojection_exhaustive_velten_forward(
+size_t totri_backprojection_exhaustive_velten_scratch(int64_t S, int64_t L, int64_t T) {
+  return mesh::exh_grad_scratch_bytes(S, L, T);
+}
+
+int totri_backprojection_exhaustive_velten_forward_ws(
     const totri_array_t* transient, const totri_array_t* scan_points,
     const totri_array_t* laser_points, const totri_array_t* scan_origin,
     const totri_array_t* laser_origin, const totri_array_t* volume, const float start[3],
-    const float end[3], float bw, float bo, void* stream_) {
+    const float end[3], float bw, float bo, void* ws, size_t ws_bytes, void* stream_) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   bp::Grid g;
   int64_t B, S, L, So, Lo;
@@ -849,16 +948,68 @@ int totri_backprojection_exhaustive_velten_forward(
   TOTRI_TRY(check_dim(transient, "transient", 2, S));
   TOTRI_TRY(check_dim(transient, "transient", 3, L));
   TOTRI_TRY(check_contiguous(transient, "transient"));
-  const int T = (int)transient->shape[1];
+  const int64_t T = transient->shape[1];
   const int64_t nv = (int64_t)g.D * g.H * g.W;
   if (nv == 0) return TOTRI_OK;
+  const float* trp = static_cast<const float*>(transient->data);
+  float* volp = static_cast<float*>(volume->data);
+  // The blocked kernel takes its bins from div_fixed (bin widths within 1e-18 ..
+  // 1e18) and a rounding by addition (bins below 2^21); anything else goes one
+  // voxel per thread ("backprojection.velten.pairs" = 1: always).
+  const float abw = std::fabs(bw);
+  if (!(abw > 1e-18f && abw < 1e18f) || T > (1 << 21) || S == 0 || L == 0 || T == 0 ||
+      tune::get("backprojection.velten.pairs") == 1) {
+    for (int b = 0; b < (int)B; ++b)
+      TOTRI_KERNEL("backprojection velten exhaustive", stream,
+                   bp::velten_exhaustive_kernel<<<(unsigned)ceil_div(nv, 128), 128, 0, stream>>>(
+                       g, b, (int)T, (int)S, (int)L, sp, lp, so, lo, So > 0, Lo > 0, bw, bo, trp,
+                       volp));
+    return TOTRI_OK;
+  }
+  // Scan points per bins-last copy (all of them up to 2 GiB); 0: in place, also
+  // where a pair's column has more bins than the volume has voxels to read them.
+  int64_t chunk = ws && nv >= T ? mesh::exh_grad_chunk_points(S, L, T) : 0;
+  if (ws_bytes < (size_t)chunk * L * T * sizeof(float)) chunk = 0;
+  const int64_t step = chunk > 0 ? chunk : S;
+  const int64_t blocks = ceil_div(g.W, 8) * ceil_div(g.H, 8) * ceil_div(g.D, 16);
+  // slices of the scan points until about 4 waves of CTAs (4 per SM), with at
+  // least 4 scan points each (a slice repeats the lasers' distances)
+  const int64_t slices = std::max<int64_t>(
+      1, std::min<int64_t>(ceil_div(16 * (int64_t)tune::sm_count(), blocks), step / 4));
+  const int per = (int)ceil_div(step, slices);
+  const int accumulate = ceil_div(step, per) > 1 || step < S;
+  if (accumulate) TOTRI_CUDA(cudaMemsetAsync(volp, 0, sizeof(float) * B * nv, stream));
+  const int64_t row = S * L;
   for (int b = 0; b < (int)B; ++b)
-    TOTRI_KERNEL("backprojection velten exhaustive", stream,
-                 bp::velten_exhaustive_kernel<<<(unsigned)ceil_div(nv, 128), 128, 0, stream>>>(
-                     g, b, T, (int)S, (int)L, sp, lp, so, lo, So > 0, Lo > 0, bw, bo,
-                     static_cast<const float*>(transient->data),
-                     static_cast<float*>(volume->data)));
+    for (int64_t sa = 0; sa < S; sa += step) {
+      const int64_t sb = std::min(S, sa + step);
+      const dim3 grid((unsigned)blocks, (unsigned)ceil_div(sb - sa, per));
+      const float* tb = trp + (int64_t)b * T * row;
+      if (chunk > 0) {
+        float* copy = static_cast<float*>(ws);
+        TOTRI_TRY(mesh::launch_bins_last(tb + sa * L, copy, (int)T, row, (sb - sa) * L, stream));
+        TOTRI_KERNEL("backprojection velten exhaustive", stream,
+                     bp::velten_pairs_kernel<true><<<grid, 256, 0, stream>>>(
+                         g, b, (int)T, (int)S, (int)L, sp, lp, so, lo, So > 0, Lo > 0, bw, bo,
+                         1.f / bw, (int)sa, (int)sb, per, copy, T, 1, volp, accumulate));
+      } else {
+        TOTRI_KERNEL("backprojection velten exhaustive", stream,
+                     bp::velten_pairs_kernel<false><<<grid, 256, 0, stream>>>(
+                         g, b, (int)T, (int)S, (int)L, sp, lp, so, lo, So > 0, Lo > 0, bw, bo,
+                         1.f / bw, (int)sa, (int)sb, per, tb, 1, row, volp, accumulate));
+      }
+    }
   return TOTRI_OK;
+}
+
+int totri_backprojection_exhaustive_velten_forward(
+    const totri_array_t* transient, const totri_array_t* scan_points,
+    const totri_array_t* laser_points, const totri_array_t* scan_origin,
+    const totri_array_t* laser_origin, const totri_array_t* volume, const float start[3],
+    const float end[3], float bw, float bo, void* stream) {
+  return totri_backprojection_exhaustive_velten_forward_ws(
+      transient, scan_points, laser_points, scan_origin, laser_origin, volume, start, end, bw, bo,
+      nullptr, 0, stream);
 }
 
 int totri_backprojection_exhaustive_arellano_forward(

@@ -1,12 +1,14 @@
 """Drop-in for ``totri_cpp.reconstruct`` (reference src/totri.cpp:18-25)."""
+import torch
+
 from .. import _lib
-from ._common import dense_out, finish_out
+from ._common import dense_out, finish_out, ws_args
 
 
-def _call(name, tensors, a3, b3, bw, bo, device):
+def _call(name, tensors, a3, b3, bw, bo, device, extra=()):
     lib = _lib.load()
     st = getattr(lib, name)(*[_lib.array(t) for t in tensors], _lib.vec3(a3), _lib.vec3(b3),
-                            float(bw), float(bo), _lib.stream_of(device))
+                            float(bw), float(bo), *extra, _lib.stream_of(device))
     _lib.check(st)
 
 
@@ -56,7 +58,10 @@ def backprojection_exhaustive_velten_forward(transient, scan_points, laser_point
     (reference src/reconstruct/backprojection.cpp:36-49)."""
     _lib.require_cuda(transient, scan_points, laser_points, scan_origin, laser_origin, volume)
     out = dense_out(volume)
-    _call("totri_backprojection_exhaustive_velten_forward",
+    n = int(_lib.load().totri_backprojection_exhaustive_velten_scratch(
+        int(scan_points.shape[1]), int(laser_points.shape[1]), int(transient.shape[1])))
+    ws = torch.empty(n, dtype=torch.uint8, device=volume.device) if n > 0 else None
+    _call("totri_backprojection_exhaustive_velten_forward_ws",
           (transient.contiguous(), scan_points, laser_points, scan_origin, laser_origin, out),
-          volume_start, volume_end, bin_width, bin_offset, volume.device)
+          volume_start, volume_end, bin_width, bin_offset, volume.device, extra=ws_args(ws))
     finish_out(volume, out)
