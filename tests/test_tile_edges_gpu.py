@@ -181,3 +181,30 @@ def test_velten_pairs_edges(cuda_lib, shape, S, L, T, bw, bo, origin):
         ref = oracle.bp_exhaustive_velten(tr[b], sp, lp, so, lo, shape, st, en, bw, bo)
         assert np.array_equal(out[b].double().cpu().numpy(), ref)
         assert np.array_equal(inplace[b].double().cpu().numpy(), ref)
+
+
+# (D, H, W), Gaussians, attributes: bricks of 16 x 16 x 8 (or 4) and 8 x 8 x 8 with
+# remainders, single-voxel axes; Gaussian counts around the lane batches of 32,
+# the shares of a brick (32, 64, 128) and the tiles of 256; every attribute
+# specialisation (0-1, 2-4, 5-8)
+RBF = [((1, 1, 1), 1, 1), ((9, 17, 18), 31, 0), ((8, 16, 16), 33, 1), ((5, 3, 40), 65, 2),
+       ((12, 20, 9), 129, 4), ((17, 9, 33), 257, 1), ((7, 18, 15), 600, 5), ((11, 8, 8), 513, 8)]
+
+
+@pytest.mark.parametrize("shape,N,A", RBF)
+def test_rbf_edges(cuda_lib, shape, N, A):
+    """Forward 1e-5 and gradient 1e-4 of the FP64 oracle."""
+    from totri_gb300.totri_cpp import util as U
+    g = np.random.default_rng(N + A)
+    st, en = (-0.5, -0.5, 0.5), (0.5, 0.5, 1.5)
+    rbf = np.concatenate([g.uniform(-0.5, 0.5, (N, 3)) + np.array([0, 0, 1.0]),
+                          g.uniform(0.02, 0.3, (N, 1)), g.uniform(0.5, 1.5, (N, A))], 1)
+    rbf = rbf.astype(np.float32)
+    vol = torch.full((1, 1 + A) + shape, 7.0, device="cuda")
+    U.rbf2volume_gaussian_forward(cu(rbf[None]), vol, st, en)
+    ref = oracle.rbf2volume_forward(rbf, shape, st, en)
+    assert rel(vol[0].cpu().numpy(), ref) < 1e-5
+    vg = g.uniform(0.5, 1.5, (1 + A,) + shape).astype(np.float32)
+    out = torch.zeros((1, N, 4 + A), device="cuda")
+    U.rbf2volume_gaussian_grad(cu(rbf[None]), vol, cu(vg[None]), out, st, en)
+    assert rel(out[0].cpu().numpy(), oracle.rbf2volume_grad(rbf, ref, vg, st, en)) < 1e-4

@@ -39,9 +39,6 @@
 //                               thread (2, 4) / scan points per tile (8, 16, 32)
 //   "backprojection.velten.pairs" 1: one voxel per thread in the exhaustive Velten
 //   "rbf.cull"                  1: RBF kernels without the underflow cull
-//   "rbf.forward.vz"            1: one voxel per thread in the RBF forward (default two)
-//   "rbf.grad.pair"             2: one Gaussian per warp iteration in the RBF gradient
-//                               (default two)
 #pragma once
 
 #include <cuda_runtime.h>
