@@ -208,3 +208,33 @@ def test_rbf_edges(cuda_lib, shape, N, A):
     out = torch.zeros((1, N, 4 + A), device="cuda")
     U.rbf2volume_gaussian_grad(cu(rbf[None]), vol, cu(vg[None]), out, st, en)
     assert rel(out[0].cpu().numpy(), oracle.rbf2volume_grad(rbf, ref, vg, st, en)) < 1e-4
+
+
+# (X, Y, Z), N, T, bin width, offset: tiles of 16, 8 and 4 points (by the bins that
+# fit) with remainders, an odd bin count, one cell and two, slices of the voxels,
+# negative bin centres, rows too long for shared memory (gradient only)
+WALKS = [((1, 1, 1), 1, 900, 0.003, 0.0), ((3, 2, 2), 5, 901, 0.003, -0.2),
+         ((20, 21, 40), 33, 333, 0.008, 0.0), ((30, 40, 50), 17, 200, 0.013, 0.05),
+         ((4, 5, 9), 6, 4001, 0.0006, 0.0), ((4, 5, 9), 9, 6400, 0.0004, -0.1),
+         ((4, 5, 9), 3, 9600, 0.00027, 0.0)]
+
+
+@pytest.mark.parametrize("shape,N,T,bw,bo", WALKS)
+def test_volume_walk_edges(cuda_lib, shape, N, T, bw, bo):
+    """Forward 1e-5 and measurement-point gradient 1e-4 of the FP64 oracle (which
+    takes the same FP32 cells)."""
+    g = np.random.default_rng(N + T)
+    mp = np.stack([g.uniform(-1, 1, N), g.uniform(-1, 1, N), g.uniform(0, 0.7, N)])
+    mp = mp.astype(np.float32)
+    org, size = (-0.5, -0.5, 0.5), (1.0, 1.0, 1.0)
+    vol = g.uniform(0.5, 1.5, shape).astype(np.float32)
+    if T * 32 <= 200 * 1024:
+        ref = oracle.volume_confocal_forward(vol, mp, T, org, size, bw, bo)
+        out = torch.full((N, T), 7.0, device="cuda")
+        R.volume_confocal_forward(cu(vol), cu(mp), out, org, size, bw, bo)
+        assert rel(out.cpu().numpy(), ref) < 1e-5
+    y = g.uniform(0.5, 1.5, (N, T)).astype(np.float32)
+    gm = torch.full((3, N), 7.0, device="cuda")
+    R.volume_confocal_grad_measurement_points(gm, cu(vol), cu(mp), cu(y), org, size, bw, bo)
+    ref = oracle.volume_confocal_grad_mp(vol, mp, y, org, size, bw, bo)
+    assert rel(gm.cpu().numpy(), ref) < 1e-4

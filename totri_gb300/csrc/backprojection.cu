@@ -84,13 +84,6 @@ __device__ __forceinline__ int velten_bin(fv3 q, float od2, fv3 p, float bw, flo
   return nearest_bin(xadd(od2, xmul(2.f, xlen(xsub3(q, p)))), bw, bo);
 }
 
-// Square root within 2^-23 (the caller keeps x in the normal range).
-__device__ __forceinline__ float sqrt_approx(float x) {
-  float r;
-  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-
 // velten_bin for two voxels of a column at once with paired FP32 instructions,
 // the margin bounded once per box of voxels (box_bins) and the +1/2 of the bin
 // coordinate folded away. r2, the squared distance in x and y, is shared by

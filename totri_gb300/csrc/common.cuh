@@ -236,6 +236,13 @@ __device__ __forceinline__ float lds(uint32_t at) {
   return r;
 }
 
+// Square root within 2^-23 (the caller keeps x in the normal range).
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 // Minimum and maximum that give NaN when an operand is NaN.
 __device__ __forceinline__ float min_nan(float a, float b) {
   float r;

@@ -29,6 +29,8 @@
 //   "mesh.visibility.occupancy", ".chunks", ".seed", ".seed.steps", ".shaft.cap"
 //                               visibility launch shape and prefix (at its launcher)
 //   "volume.exact"              1: every volume sample takes the exact chain
+//   "volume.forward.points", ".slices" points per CTA (4, 8, 16, 32) and slices of the
+//                               voxels, forward and measurement-point gradient
 //   "volume.adjoint.mode"       0 lanes over 32 columns (default), 1 shared-memory
 //                               atomics, 2 lane-owned cells (up to 256 cells)
 //   "volume.adjoint.warps"      warps per CTA of the lanes-over-columns adjoint
