@@ -238,3 +238,52 @@ def test_volume_walk_edges(cuda_lib, shape, N, T, bw, bo):
     R.volume_confocal_grad_measurement_points(gm, cu(vol), cu(mp), cu(y), org, size, bw, bo)
     ref = oracle.volume_confocal_grad_mp(vol, mp, y, org, size, bw, bo)
     assert rel(gm.cpu().numpy(), ref) < 1e-4
+
+
+def _mesh(kind, faces, seed):
+    from totri_gb300 import scenes
+    if kind == "box":
+        v, f, _ = scenes.random_box(faces, seed)
+    elif kind == "sphere":
+        v, f, _ = scenes.uv_sphere(faces, seed)
+    else:  # a soup of large and tiny triangles, some degenerate
+        g = np.random.default_rng(seed)
+        c = g.uniform(-0.4, 0.4, (faces, 1, 3)) + np.array([0, 0, 1.0])
+        v = c + g.normal(size=(faces, 3, 3)) * g.choice([0.2, 0.02, 0.0], (faces, 1, 1))
+        v = torch.from_numpy(v.reshape(1, -1, 3).astype(np.float32))
+        f = torch.arange(3 * faces, dtype=torch.int32).reshape(1, -1, 3)
+    return v.cuda(), f.cuda()
+
+
+# (mesh, faces, wall points): one point to just past blocks of 32, one face to past
+# chunks of 32 and lists of 8
+LISTS = [("soup", 1, 1), ("soup", 2, 33), ("soup", 31, 31), ("soup", 33, 64), ("soup", 300, 100),
+         ("box", 300, 200), ("sphere", 700, 97), ("box", 3000, 300)]
+
+
+@pytest.mark.parametrize("kind,faces,P", LISTS)
+def test_visibility_lists_equal_brute_force(cuda_lib, kind, faces, P):
+    """The candidate-list kernels give the brute-force masks bit for bit: the
+    lists whole, capped so that groups and then single targets overflow to the
+    BVH, the surface walk off, a wall 40 m away, and two items in a batch."""
+    from totri_gb300 import autotune
+    v, f = _mesh(kind, faces, faces + P)
+    g = np.random.default_rng(P)
+    near = points(g, P)
+    far = points(g, P) * 20.0
+    far[:, 2] = -40.0
+    v2, f2 = torch.cat([v, v.flip(2)]), torch.cat([f, f])
+    for sp in (near, far):
+        pts = cu(np.stack([sp, sp]))
+        bf = R.mesh_visibility(v2, f2, pts, brute_force=True)
+        for cap, seed in ((0, 0), (40, 0), (1, 1)):
+            keys = {"mesh.visibility.list": 1, "mesh.visibility.list.cap": cap,
+                    "mesh.visibility.seed": seed}
+            try:
+                for k, x in keys.items():
+                    autotune.set_tile(k, x)
+                got = R.mesh_visibility(v2, f2, pts)
+            finally:
+                for k in keys:
+                    autotune.set_tile(k, 0)
+            assert torch.equal(got, bf), (cap, seed)

@@ -115,8 +115,8 @@ constexpr int kMaxPatchChunks = 16;
 // kWalk 0: target_visible_pp, 1: packet_visible, 2: target_visible_pp4, 3: shaft
 // search, 4: target_visible_pp's prefix and a 4-wide BVH search
 // (bvh_occluded_wide); kOcc: CTAs per SM that the register allocation must allow.
-template <int kWalk, int kOcc = 1>
-__global__ void __launch_bounds__(256, kOcc) visibility_patch_kernel(Scene sc, View3f pts, int P,
+template <int kWalk, int kOcc = 1, int kWarps = 8>
+__global__ void __launch_bounds__(32 * kWarps, kOcc) visibility_patch_kernel(Scene sc, View3f pts, int P,
                                                                int row0, int chunks,
                                                                int seed_mode, int seed_steps,
                                                                int shaft_cap) {
@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(256, kOcc) visibility_patch_kernel(Scene sc, V
   __shared__ int seeds[32];
   __shared__ int next_face;
   // per warp: two frontiers and the candidate list of the shaft search
-  __shared__ int shaft_buf[kWalk == 3 ? 8 * (2 * kShaftFrontier + kShaftCand) : 1];
+  __shared__ int shaft_buf[kWalk == 3 ? kWarps * (2 * kShaftFrontier + kShaftCand) : 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int b = blockIdx.z;
   const int ch0 = blockIdx.y * chunks;
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(256, kOcc) visibility_patch_kernel(Scene sc, V
   }
   __syncthreads();
   if (threadIdx.x < 32 && okp && (kWalk == 0 || kWalk == 3 || kWalk == 4)) gseeds[i] = seeds[lane];
-  for (int c = warp; c < nc; c += 8) {
+  for (int c = warp; c < nc; c += kWarps) {
     if (!okp) continue;
     uint32_t word = 0u;
 #pragma unroll
@@ -375,6 +375,227 @@ __global__ void __launch_bounds__(256, kOcc) visibility_queue_kernel(Scene sc, V
 #pragma unroll
     for (int j = 0; j < 32; ++j) word |= ((bits[c][j] >> lane) & 1u) << j;
     sc.mask[((size_t)b * sc.P + row0 + p) * sc.nch + ch0 + c] = word;
+  }
+}
+
+constexpr int kListWarps = 4, kListFaces = 8, kListFrontier = 256, kListCand = 512;
+
+// Warp minimum / maximum of a float (redux.sync on floats, sm_100a and later).
+__device__ __forceinline__ float warp_min_f(float x) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float warp_max_f(float x) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// Visibility over dense wall grids, in two kernels.
+//
+// visibility_walk_kernel decides the targets seen from behind as
+// visibility_patch_kernel does (surface walk from the last occluder, then the
+// BVH) and leaves the bits of front-facing targets set. A warp takes one block
+// of 32 wall points (one per lane) and a run of consecutive 32-face chunks from a
+// global queue, and keeps each point's last occluder in a register: a target's
+// neighbour in Morton order was decided just before by the same warp, so the
+// walks start closer than from seeds shared by eight warps on eight faces (3.5
+// -> 2.5 ms on the 20,480-face workload; runs of 2, 4 and 8 chunks 2.4, 2.5 and 2.5
+// ms there, but 3.1, 3.3, 3.7 and 5.2 ms for 1 to 8 chunks on a 12,288-face box).
+//
+// visibility_list_kernel then decides the front-facing targets without BVH
+// walks. A warp takes 32 wall points and kListFaces consecutive faces and
+// collects every face whose box meets the hull of the wall points and those
+// faces' hit boxes (shaft_candidates, about 100 of them). For each target the
+// lanes test that list, 32 boxes at a time, against the hull of the wall points
+// and the rays' own accepted hits on the target: an accepted occluder has t
+// in [0, tf], so its hit point lies on a segment from a wall point to such a
+// hit. That hull ends in a point for all but grazing targets, so a few
+// neighbours remain (8 on the 20,480-face workload, 18 on the box), and they get
+// the exact triangle test, all lanes on one face. When the list overflows, the
+// target's own hull is walked for its candidates; when those overflow too, or
+// fewer than two rays need it, the lanes search the BVH. Every accepted hit's
+// box is in the list and passes the second hull (both are padded beyond the
+// rounding, as make_shaft describes), so the bits are those of brute force.
+// What bounds them: instruction issue. Both together: 7.9 -> 4.6 ms on the
+// 20,480-face workload (4,096 points), 17.0 -> 7.5 ms on the box (6,767 points).
+// Lists for 4, 16 and 32 faces at a time took 2.4, 2.4 and 3.5 ms against 2.2 ms
+// on the 20,480-face workload, 4.9, 7.6 and 11.4 against 5.5 ms on the box.
+template <int kOcc>
+__global__ void __launch_bounds__(32 * kListWarps, kOcc) visibility_walk_kernel(
+    Scene sc, View3f pts, int P, int row0, uint32_t* next_unit, int seed_mode, int seed_steps) {
+  const int lane = threadIdx.x & 31;
+  const int patches = (P + 31) >> 5;
+  const unsigned units = (unsigned)patches * sc.nch * sc.B;
+  for (;;) {
+    unsigned unit = 0;
+    if (lane == 0) unit = atomicAdd(next_unit, 1u);
+    unit = __shfl_sync(0xffffffffu, unit, 0);
+    if (unit >= units) break;
+    const int ch = unit % sc.nch, pb = unit / sc.nch;
+    const int b = pb / patches, i = (pb - b * patches) * 32 + lane;
+    const int n = sc.meta[b].n;
+    const bool okp = i < P;
+    const uint32_t* order = sc.pscratch + 3 * (size_t)sc.B * P + (size_t)b * P;
+    int p = okp ? (int)order[i] : 0;
+    if (!TOTRI_INDEX_OK((unsigned)p < (unsigned)P, sc.status)) p = 0;
+    const fv3 o = okp ? mkv(pts.at(b, p, 0), pts.at(b, p, 1), pts.at(b, p, 2)) : mkv(0.f, 0.f, 0.f);
+    volatile int* gseeds = reinterpret_cast<int*>(sc.pscratch) + (size_t)b * P;
+    int seed = okp ? gseeds[i] : -1;
+    const int s0 = seed;
+    uint32_t word = 0u;
+    for (int j = 0; j < 32 && ch * 32 + j < n; ++j) {  // warp-uniform
+      const Target tg = load_target(sc, b, ch * 32 + j);
+      bool vis = false;
+      if (okp) {
+        fv3 dir;
+        float tmax, tf;
+        const fv3 nrm = cross(mkv(tg.a0.w, tg.a1.x, tg.a1.y), mkv(tg.a1.z, tg.a1.w, tg.a2.x));
+        if (n > 1 && !(dot(nrm, tg.c - o) > 0.f))
+          vis = true;  // left to visibility_list_kernel
+        else if (query_prefix(sc, b, n, tg, o, seed, seed_mode, seed_steps, dir, tmax, tf, vis))
+          vis = !bvh_occluded_wide(sc, b, n, tg.k, tg.f, o, dir, tmax, tf, sc.status, seed);
+      }
+      __syncwarp();
+      word |= (uint32_t)vis << j;
+    }
+    if (okp) sc.mask[((size_t)b * sc.P + row0 + p) * sc.nch + ch] = word;
+    if (okp && seed != s0) gseeds[i] = seed;
+  }
+}
+
+template <int kOcc>
+__global__ void __launch_bounds__(32 * kListWarps, kOcc) visibility_list_kernel(
+    Scene sc, View3f pts, int P, int row0, uint32_t* next_unit, int list_cap) {
+  __shared__ int buf[kListWarps][2 * kListFrontier + kListCand];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int* fr0 = buf[warp];
+  int* cand = fr0 + 2 * kListFrontier;
+  const int patches = (P + 31) >> 5, per_chunk = 32 / kListFaces;
+  const unsigned units = (unsigned)patches * sc.nch * per_chunk * sc.B;
+  for (;;) {
+    unsigned unit = 0;
+    if (lane == 0) unit = atomicAdd(next_unit, 1u);
+    unit = __shfl_sync(0xffffffffu, unit, 0);
+    if (unit >= units) break;
+    const int part = unit % per_chunk;
+    const unsigned r = unit / per_chunk;
+    const int ch = r % sc.nch, pb = r / sc.nch;
+    const int b = pb / patches, i = (pb - b * patches) * 32 + lane;
+    const int n = sc.meta[b].n;
+    const int k0 = ch * 32 + part * kListFaces;
+    if (k0 >= n || n == 1) continue;
+    const bool okp = i < P;
+    const uint32_t* order = sc.pscratch + 3 * (size_t)sc.B * P + (size_t)b * P;
+    int p = okp ? (int)order[i] : 0;
+    if (!TOTRI_INDEX_OK((unsigned)p < (unsigned)P, sc.status)) p = 0;
+    uint32_t* mrow = sc.mask + ((size_t)b * sc.P + row0 + p) * sc.nch + ch;
+    const uint32_t open0 = okp ? (*mrow >> (part * kListFaces)) & ((1u << kListFaces) - 1u) : 0u;
+    const uint32_t faces = __reduce_or_sync(0xffffffffu, open0);
+    if (faces == 0u) continue;
+    const fv3 o = okp ? mkv(pts.at(b, p, 0), pts.at(b, p, 1), pts.at(b, p, 2)) : mkv(0.f, 0.f, 0.f);
+    float plo[3], phi[3], pad = 0.f;  // the wall points' padded box
+    {
+      const float oc[3] = {o.x, o.y, o.z};
+      float mag = 0.f;
+      for (int a = 0; a < 3; ++a) {
+        plo[a] = warp_min_f(okp ? oc[a] : INFINITY);
+        phi[a] = warp_max_f(okp ? oc[a] : -INFINITY);
+        mag = fmaxf(mag, fmaxf(fabsf(plo[a]), fabsf(phi[a])));
+      }
+      pad = sc.meta[b].delta + ldexpf(isfinite(mag) ? mag : 0.f, -14);
+      for (int a = 0; a < 3; ++a) {
+        plo[a] -= pad;
+        phi[a] += pad;
+      }
+    }
+    uint32_t hidden = 0u;
+    int ncand = -2;  // -2: not collected yet, -1: overflow
+    for (uint32_t m = faces; m; m &= m - 1) {
+      const int j = __ffs(m) - 1, k = k0 + j;
+      const Target tg = load_target(sc, b, k);
+      const bool open = (open0 >> j) & 1u;
+      // the prefix's ray and own hit
+      const fv3 D = xsub3(tg.c, o);
+      const float dist = xlen(D);
+      const fv3 dir = mkv(xdiv(D.x, dist), xdiv(D.y, dist), xdiv(D.z, dist));
+      const float tmax = xadd(xmul(dist, 1.01f), 1e-3f);
+      float tf = 0.f;
+      const bool need =
+          open && dist >= 1e-6f && tri_hit(tg.a0, tg.a1, tg.a2, tg.a3, o, dir, tmax, tf);
+      const fv3 nrm = cross(mkv(tg.a0.w, tg.a1.x, tg.a1.y), mkv(tg.a1.z, tg.a1.w, tg.a2.x));
+      const bool front = need && !(dot(nrm, dir) > 0.f);
+      bool occ = false;
+      bool search = need;
+      if (__popc(__ballot_sync(0xffffffffu, front)) >= 2) {
+        if (ncand == -2) {
+          // the hull of the wall points and the open faces' hit boxes
+          float4 t2 = make_float4(0.f, INFINITY, INFINITY, INFINITY);
+          float4 t3 = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
+          if (lane < kListFaces && ((faces >> lane) & 1u)) {
+            const float4* q = tri_at(sc, b, k0 + lane);
+            t2 = __ldg(q + 2);
+            t3 = __ldg(q + 3);
+          }
+          const float clo[3] = {warp_min_f(t2.y) - pad, warp_min_f(t2.z) - pad,
+                                warp_min_f(t2.w) - pad};
+          const float chi[3] = {warp_max_f(t3.x) + pad, warp_max_f(t3.y) + pad,
+                                warp_max_f(t3.z) + pad};
+          ncand = shaft_candidates<kListFrontier, kListCand>(
+              sc, b, n, -1, make_shaft(plo, phi, clo, chi), fr0, fr0 + kListFrontier, cand, lane,
+              list_cap);
+        }
+        {
+          // the hull of the wall points and the rays' hits on the target
+          const float hx = fmaf(tf, dir.x, o.x), hy = fmaf(tf, dir.y, o.y);
+          const float hz = fmaf(tf, dir.z, o.z);
+          const float clo[3] = {warp_min_f(need ? hx : INFINITY) - pad,
+                                warp_min_f(need ? hy : INFINITY) - pad,
+                                warp_min_f(need ? hz : INFINITY) - pad};
+          const float chi[3] = {warp_max_f(need ? hx : -INFINITY) + pad,
+                                warp_max_f(need ? hy : -INFINITY) + pad,
+                                warp_max_f(need ? hz : -INFINITY) + pad};
+          const Shaft h = make_shaft(plo, phi, clo, chi);
+          int count = ncand;
+          if (ncand == -1)
+            count = shaft_candidates<kListFrontier, kListCand>(sc, b, n, k, h, fr0,
+                                                               fr0 + kListFrontier, cand, lane,
+                                                               list_cap);
+          for (int base = 0; base < count; base += 32) {
+            const int kk = base + lane < count ? cand[base + lane] : -1;
+            bool in = false;
+            if (kk >= 0 && kk != k) {
+              const float4* q = tri_at(sc, b, kk);
+              const float4 t2 = __ldg(q + 2), t3 = __ldg(q + 3);
+              in = shaft_box(h, t2.y, t2.z, t2.w, t3.x, t3.y, t3.z);
+            }
+            uint32_t mm = __ballot_sync(0xffffffffu, in);
+            while (mm) {
+              const int g = __shfl_sync(0xffffffffu, kk, __ffs(mm) - 1);
+              mm &= mm - 1;
+              if (search && !occ) {
+                const float4* q = tri_at(sc, b, g);
+                const float4 q0 = __ldg(q), q1 = __ldg(q + 1), q2 = __ldg(q + 2),
+                             q3 = __ldg(q + 3);
+                float tq;
+                if (tri_hit(q0, q1, q2, q3, o, dir, tmax, tq) &&
+                    (tq < tf || (tq == tf && __float_as_int(q3.w) < tg.f)))
+                  occ = true;
+              }
+            }
+          }
+          if (count >= 0) search = false;
+        }
+      }
+      if (search) {
+        int seed = -1;
+        occ = bvh_occluded_wide(sc, b, n, tg.k, tg.f, o, dir, tmax, tf, sc.status, seed);
+      }
+      __syncwarp();
+      hidden |= (uint32_t)(occ || (open && !need)) << j;
+    }
+    if (okp && hidden) atomicAnd(mrow, ~(hidden << (part * kListFaces)));
   }
 }
 
@@ -763,13 +984,15 @@ int launch_visibility(const Scene& sc, const View3f& pts, int P, int row0, bool 
     if (P >= (1 << 30) / 4) return fail(TOTRI_ERR_UNSUPPORTED, "too many wall points");
     const int st = launch_point_order(sc, pts, P, stream);
     if (st != TOTRI_OK) return st;
-    // Chunks per CTA: up to 8 while the grid keeps 8 CTAs per SM (20,480-face
-    // workload: 9.15 ms at 8, 9.3 at 4, 9.6 at 2, 10.4 at 1, 10.5 at 16).
+    // Chunks per CTA: up to 8 while the grid keeps 32 CTAs per SM (20,480 faces x
+    // 4,096 points: 9.15 ms at 8, 9.3 at 4, 9.6 at 2, 10.4 at 1, 10.5 at 16; 20,000
+    // faces x 400 and 144 points: 3.2 ms at the 6 and 2 that 8 CTAs per SM gave,
+    // 2.7 ms at 1).
+    const int64_t patches = ceil_div(P, 32);
     int chunks = tune::get("mesh.visibility.chunks");
-    if (chunks <= 0) {
-      const int64_t ctas = (int64_t)ceil_div(P, 32) * sc.nch * sc.B;
-      chunks = (int)std::max<int64_t>(1, std::min<int64_t>(8, ctas / (8 * tune::sm_count())));
-    }
+    if (chunks <= 0)
+      chunks = (int)std::max<int64_t>(
+          1, std::min<int64_t>(8, patches * sc.nch * sc.B / (32 * tune::sm_count())));
     if (chunks > kMaxPatchChunks)
       return fail(TOTRI_ERR_INVALID_ARGUMENT, "at most 16 face chunks per visibility block");
     const int seed_mode = tune::get("mesh.visibility.seed");
@@ -784,6 +1007,8 @@ int launch_visibility(const Scene& sc, const View3f& pts, int P, int row0, bool 
     const dim3 grid((unsigned)ceil_div(P, 32), (unsigned)ceil_div(sc.nch, chunks),
                     (unsigned)sc.B);
     const int mode = tune::get("mesh.visibility.mode");
+    const int list = tune::get("mesh.visibility.list");
+    const int64_t cta_count = (int64_t)grid.x * grid.y * grid.z;
     if (mode == kVisPatchPacket)
       TOTRI_KERNEL("mesh visibility", stream,
                    visibility_patch_kernel<1><<<grid, 256, 0, stream>>>(
@@ -796,6 +1021,34 @@ int launch_visibility(const Scene& sc, const View3f& pts, int P, int row0, bool 
       TOTRI_KERNEL("mesh visibility", stream,
                    visibility_patch_kernel<3><<<grid, 256, 0, stream>>>(
                        sc, pts, P, row0, chunks, seed_mode, seed_steps, shaft_cap));
+    // Dense wall grids (blocks of 32 points narrow enough for the hulls) with
+    // enough (block, chunk) units to feed the queues: from 2,048 points and 16,384
+    // units on the two kernels were faster on every mesh tried (1.02-1.11x on
+    // 20,000-face spheres at 48 x 48 and 101 x 23 points, 1.06x on 5,120 faces at 64 x
+    // 64, 2.2x on boxes there); below, 0.72-0.98x on spheres (5,120 faces at 40 x 40,
+    // 101 x 23 and 48 x 48 points, 20,000 at 40 x 40), though 1.3x on 20,480 faces at
+    // 32 x 32 and 1.3-1.6x on boxes. "mesh.visibility.list": 1 always, 2 never;
+    // ".list.cap" lowers the list's capacity.
+    else if (mode == 0 && tune::get("mesh.visibility.wide") != 2 &&
+             tune::get("mesh.visibility.queue") != 1 &&
+             tune::get("mesh.visibility.occupancy") == 0 &&
+             (list == 1 || (list == 0 && P >= 2048 && patches * sc.nch * sc.B >= 16384)) &&
+             patches * sc.nch * sc.B < ((int64_t)1 << 29)) {
+      int cap = tune::get("mesh.visibility.list.cap");
+      if (cap <= 0 || cap > kListCand) cap = kListCand;
+      // the queues' counters: the second quarter of the point scratch is free
+      // once the points are sorted (it holds at least one word)
+      uint32_t* next = sc.pscratch + (size_t)sc.B * P;
+      const unsigned ctas = 8u * (unsigned)tune::sm_count();
+      TOTRI_CUDA(cudaMemsetAsync(next, 0, sizeof(uint32_t), stream));
+      TOTRI_KERNEL("mesh visibility", stream,
+                   visibility_walk_kernel<8><<<ctas, 32 * kListWarps, 0, stream>>>(
+                       sc, pts, P, row0, next, seed_mode, seed_steps));
+      TOTRI_CUDA(cudaMemsetAsync(next, 0, sizeof(uint32_t), stream));
+      TOTRI_KERNEL("mesh visibility list", stream,
+                   visibility_list_kernel<8><<<ctas, 32 * kListWarps, 0, stream>>>(
+                       sc, pts, P, row0, next, cap));
+    }
     // The default: the surface-walk prefix, then the 4-wide BVH search
     // (bvh_occluded_wide) with registers for 4 CTAs per SM (60, no spills):
     // 8.81 ms against 9.19 ms for the binary search at 5 CTAs per SM (48
@@ -806,6 +1059,17 @@ int launch_visibility(const Scene& sc, const View3f& pts, int P, int row0, bool 
       if (tune::get("mesh.visibility.occupancy") == 5)
         TOTRI_KERNEL("mesh visibility", stream,
                      visibility_patch_kernel<4, 5><<<grid, 256, 0, stream>>>(
+                         sc, pts, P, row0, chunks, seed_mode, seed_steps, 0));
+      // Grids that fill less than a wave: more warps per CTA, fewer faces in a row
+      // per warp (768 faces x 143 and 35 points: 275 us with 8 warps, 190 with 16,
+      // 152 with 32; 320 faces x 1,024 points: 77, 65 and 74 us).
+      else if (cta_count <= tune::sm_count())
+        TOTRI_KERNEL("mesh visibility", stream,
+                     visibility_patch_kernel<4, 1, 32><<<grid, 1024, 0, stream>>>(
+                         sc, pts, P, row0, chunks, seed_mode, seed_steps, 0));
+      else if (cta_count <= 4 * tune::sm_count())
+        TOTRI_KERNEL("mesh visibility", stream,
+                     visibility_patch_kernel<4, 2, 16><<<grid, 512, 0, stream>>>(
                          sc, pts, P, row0, chunks, seed_mode, seed_steps, 0));
       else
         TOTRI_KERNEL("mesh visibility", stream,

@@ -24,6 +24,8 @@
 //   "mesh.visibility.mode"      1 per-lane BVH walk, 2 warp-packet walk, 7 one hull
 //                               per target (at its launcher)
 //   "mesh.visibility.queue"     1: queued BVH searches (visibility_queue_kernel)
+//   "mesh.visibility.list", ".list.cap" 1: front-facing targets over candidate lists always,
+//                               2: never (at its launcher) / most candidates in a list
 //   "mesh.visibility.wide"      2: binary BVH search after the surface-walk prefix
 //                               (the default is the 4-wide search)
 //   "mesh.visibility.occupancy", ".chunks", ".seed", ".seed.steps", ".shaft.cap"
