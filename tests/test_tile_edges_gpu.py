@@ -287,3 +287,53 @@ def test_visibility_lists_equal_brute_force(cuda_lib, kind, faces, P):
                 for k in keys:
                     autotune.set_tile(k, 0)
             assert torch.equal(got, bf), (cap, seed)
+
+
+@pytest.mark.parametrize("faces", [1, 2, 31, 33, 320, 1024, 1025, 1535, 1536, 1537])
+@pytest.mark.parametrize("P,B", [(1, 1), (33, 3), (2048, 1), (2049, 2)])
+def test_small_build_equals_the_general_one(cuda_lib, faces, P, B):
+    """Masks over the one-kernel build equal brute force over the general build:
+    whole lists, a list cut short by an invalid face, 64-bit indices and a
+    strided view, on both sides of the face limit and of the two point sorts."""
+    from totri_gb300 import autotune
+    g = np.random.default_rng(7 * faces + P)
+    V = faces // 2 + 3
+    verts = g.uniform(-1.0, 1.0, (B, V, 3)).astype(np.float32)
+    verts[..., 2] += 2.0
+    verts[:, V - 1] = verts[:, 0]  # a repeated vertex: equal Morton codes, degenerate faces
+    fac = g.integers(0, V, (B, faces, 3))
+    cut = fac.copy()
+    cut[B - 1, faces // 2, 1] = -1
+    pts = np.stack([points(g, P) for _ in range(B)])
+    wide = torch.zeros((B, 2 * P, 3), device="cuda")
+    wide[:, ::2] = cu(pts)
+    for f in (cu(fac.astype(np.int32)), cu(cut.astype(np.int64))):
+        v = cu(verts)
+        try:
+            autotune.set_tile("mesh.build.small", 2)
+            want = R.mesh_visibility(v, f, cu(pts), brute_force=True)
+        finally:
+            autotune.set_tile("mesh.build.small", 0)
+        assert torch.equal(R.mesh_visibility(v, f, cu(pts)), want)
+        assert torch.equal(R.mesh_visibility(v, f, wide[:, ::2]), want)
+        assert torch.equal(R.mesh_visibility(v, f, cu(pts), brute_force=True), want)
+
+
+@pytest.mark.parametrize("faces,S,L", [(300, 1, 1), (300, 33, 32), (60, 2100, 3), (60, 3, 65)])
+def test_joint_scan_and_laser_masks(cuda_lib, faces, S, L):
+    """Exhaustive renders whose scan and laser masks come from one launch, against
+    the oracle: sums of FP32 terms of one sign, a few per bin (the bound of the
+    other exhaustive renders)."""
+    g = np.random.default_rng(S + L)
+    v, f = _mesh("soup", faces, S)
+    m = torch.rand((1, v.shape[1], 1), device="cuda") + 0.5
+    sp, lp = points(g, S), points(g, L)
+    none = torch.empty((1, 0, 3), device="cuda")
+    out = torch.empty((1, 200, S, L), device="cuda")
+    R.mesh_exhaustive_forward(v, f, m, cu(sp[None]), cu(lp[None]), none, none, out, 0.05, 0.0, 0)
+    vn, fn = v[0].cpu().numpy(), f[0].cpu().numpy()
+    ref = oracle.mesh_exhaustive_forward(vn, fn, m[0].cpu().numpy(), sp, lp, None, None,
+                                         oracle.mesh_visibility(vn, fn, sp),
+                                         oracle.mesh_visibility(vn, fn, lp), 200, 0.05, 0.0)
+    assert np.linalg.norm(ref) > 0.0 or faces < 60
+    assert rel(out[0].cpu().numpy(), ref) < 1e-5

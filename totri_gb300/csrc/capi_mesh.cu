@@ -188,9 +188,11 @@ int confocal_grad_impl(const totri_array_t* verts, const totri_array_t* faces,
     sc = mesh::scene_from_workspace(ws, a.B, a.F, S);
   }
   if (!reuse && !masks) {
-    TOTRI_TRY(mesh::build_scene(sc, a.in, stream));
+    const mesh::WallSet wall{view3f(scan_points), (int)S, 0};
+    TOTRI_TRY(mesh::build_scene(sc, a.in, stream, &wall,
+                              occluded && mesh::orders_points(false) ? 1 : 0));
     if (occluded)
-      TOTRI_TRY(mesh::launch_visibility(sc, view3f(scan_points), (int)S, 0, false, stream));
+      TOTRI_TRY(mesh::launch_visibility(sc, &wall, 1, false, false, stream));
     else
       TOTRI_TRY(all_visible(sc, S, stream));
   }
@@ -228,6 +230,15 @@ int check_exhaustive(const totri_array_t* verts, const totri_array_t* faces,
   return TOTRI_OK;
 }
 
+// The BVH and the masks of the scan points (rows 0 .. S - 1) and laser points.
+int exhaustive_masks(const mesh::Scene& sc, const ExhArgs& e, const totri_array_t* scan_points,
+                     const totri_array_t* laser_points, cudaStream_t stream) {
+  const mesh::WallSet walls[2] = {{view3f(scan_points), (int)e.S, 0},
+                                  {view3f(laser_points), (int)e.L, (int)e.S}};
+  TOTRI_TRY(mesh::build_scene(sc, e.m.in, stream, walls, mesh::orders_points(false) ? 2 : 0));
+  return mesh::launch_visibility(sc, walls, 2, false, false, stream);
+}
+
 int exhaustive_grad_impl(const totri_array_t* verts, const totri_array_t* faces,
                          const totri_array_t* material, const totri_array_t* scan_points,
                          const totri_array_t* laser_points, const totri_array_t* scan_origin,
@@ -250,10 +261,7 @@ int exhaustive_grad_impl(const totri_array_t* verts, const totri_array_t* faces,
   TOTRI_TRY(check_workspace(ws, ws_bytes, base));
   const mesh::Scene sc = mesh::scene_from_workspace(ws, e.m.B, e.m.F, P);
   if (!reuse) {
-    TOTRI_TRY(mesh::build_scene(sc, e.m.in, stream));
-    TOTRI_TRY(mesh::launch_visibility(sc, view3f(scan_points), (int)e.S, 0, false, stream));
-    TOTRI_TRY(
-        mesh::launch_visibility(sc, view3f(laser_points), (int)e.L, (int)e.S, false, stream));
+    TOTRI_TRY(exhaustive_masks(sc, e, scan_points, laser_points, stream));
   }
   // the bytes past the mesh layout (256-aligned) are the optional scratch
   void* scratch = ws_bytes > base ? static_cast<char*>(ws) + base : nullptr;
@@ -316,9 +324,11 @@ static int confocal_forward_impl(const totri_array_t* verts, const totri_array_t
   const mesh::Layout L = mesh::layout(a.B, a.F, S);
   TOTRI_TRY(check_workspace(ws, ws_bytes, L.total));
   const mesh::Scene sc = mesh::scene_from_workspace(ws, a.B, a.F, S);
-  TOTRI_TRY(mesh::build_scene(sc, a.in, stream));
+  const mesh::WallSet wall{view3f(scan_points), (int)S, 0};
+  TOTRI_TRY(mesh::build_scene(sc, a.in, stream, &wall,
+                              occluded && mesh::orders_points(false) ? 1 : 0));
   if (occluded)
-    TOTRI_TRY(mesh::launch_visibility(sc, view3f(scan_points), (int)S, 0, false, stream));
+    TOTRI_TRY(mesh::launch_visibility(sc, &wall, 1, false, false, stream));
   else
     TOTRI_TRY(all_visible(sc, S, stream));
   return mesh::launch_confocal_splat(sc, view3f(scan_points), view3f(scan_origin), has_origin,
@@ -414,9 +424,7 @@ int totri_mesh_exhaustive_forward(const totri_array_t* verts, const totri_array_
   const int64_t P = e.S + e.L;
   TOTRI_TRY(check_workspace(ws, ws_bytes, mesh::layout(e.m.B, e.m.F, P).total));
   const mesh::Scene sc = mesh::scene_from_workspace(ws, e.m.B, e.m.F, P);
-  TOTRI_TRY(mesh::build_scene(sc, e.m.in, stream));
-  TOTRI_TRY(mesh::launch_visibility(sc, view3f(scan_points), (int)e.S, 0, false, stream));
-  TOTRI_TRY(mesh::launch_visibility(sc, view3f(laser_points), (int)e.L, (int)e.S, false, stream));
+  TOTRI_TRY(exhaustive_masks(sc, e, scan_points, laser_points, stream));
   return mesh::launch_exhaustive_splat(sc, view3f(scan_points), view3f(laser_points), e.org,
                                        (int)e.S, (int)e.L, static_cast<float*>(transient->data),
                                        (int)e.T, bw, bo, stream);
@@ -483,8 +491,10 @@ int totri_mesh_visibility(const totri_array_t* verts, const totri_array_t* faces
   const mesh::Layout L = mesh::layout(a.B, a.F, P);
   TOTRI_TRY(check_workspace(ws, ws_bytes, L.total));
   const mesh::Scene sc = mesh::scene_from_workspace(ws, a.B, a.F, P);
-  TOTRI_TRY(mesh::build_scene(sc, a.in, stream));
-  TOTRI_TRY(mesh::launch_visibility(sc, view3f(points), (int)P, 0, brute_force != 0, stream));
+  const mesh::WallSet wall{view3f(points), (int)P, 0};
+  TOTRI_TRY(mesh::build_scene(sc, a.in, stream, &wall,
+                              mesh::orders_points(brute_force != 0) ? 1 : 0));
+  TOTRI_TRY(mesh::launch_visibility(sc, &wall, 1, brute_force != 0, false, stream));
   return mesh::launch_mask_unsort(sc, (int)P, static_cast<uint32_t*>(mask->data), stream);
 }
 
@@ -517,7 +527,8 @@ int totri_mesh_prepared_visibility(const totri_array_t* verts, const totri_array
   TOTRI_TRY(check_workspace(const_cast<void*>(ws), ws_bytes, mesh::layout(a.B, a.F, 0).total));
   TOTRI_TRY(check_masks(masks, masks_bytes, a.B, a.F, P));
   const mesh::Scene sc = mesh::scene_with_masks(const_cast<void*>(ws), a.B, a.F, masks, P);
-  return mesh::launch_visibility(sc, view3f(points), (int)P, 0, false, stream);
+  const mesh::WallSet wall{view3f(points), (int)P, 0};
+  return mesh::launch_visibility(sc, &wall, 1, false, true, stream);
 }
 
 int totri_mesh_prepared_confocal_forward(const totri_array_t* verts, const totri_array_t* faces,

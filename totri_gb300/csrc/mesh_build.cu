@@ -12,7 +12,10 @@
 //   6. records   sorted TriRec / ShadeRec
 //   7. hierarchy Karras 2012 internal nodes, parent links
 //   8. refit     bottom-up boxes (second arrival at a node merges its children)
+// Small meshes go through all stages in one kernel (build_small_kernel).
+#include "capi_common.cuh"
 #include "mesh.cuh"
+#include "mesh_kernels.cuh"
 #include "tune.cuh"
 
 namespace totri {
@@ -25,29 +28,23 @@ constexpr int kSortBits = 10;
 constexpr int kSortDigits = 1 << kSortBits;
 constexpr int kSortUnroll = 4;  // batches of 32 keys loaded ahead per warp
 
-__global__ void init_kernel(Scene sc, int F) {
-  const int b = blockIdx.y;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < sc.F) sc.counter[(size_t)b * sc.F + i] = 0;
-  if (i == 0) {
-    Meta& m = sc.meta[b];
-    m.n = F;
-    m.term_neg = 0;
-    m.scale = 0.f;
-    m.delta = 0.f;
-    for (int a = 0; a < 3; ++a) {
-      m.cmin[a] = ford(3.0e38f);
-      m.cmax[a] = ford(-3.0e38f);
-    }
-  }
-  if (b == 0 && i == 0 && blockIdx.x == 0) {
-    // status word is cleared by the host with a memset
+__device__ __forceinline__ void init_meta(Meta& m, int F) {
+  m.n = F;
+  m.term_neg = 0;
+  m.scale = 0.f;
+  m.delta = 0.f;
+  for (int a = 0; a < 3; ++a) {
+    m.cmin[a] = ford(3.0e38f);
+    m.cmax[a] = ford(-3.0e38f);
   }
 }
 
-__global__ void faces_kernel(Scene sc, BuildInputs in) {
-  const int b = blockIdx.y;
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void init_item(const Scene& sc, int F, int b, int i) {
+  if (i < sc.F) sc.counter[(size_t)b * sc.F + i] = 0;
+  if (i == 0) init_meta(sc.meta[b], F);
+}
+
+__device__ __forceinline__ void faces_item(const Scene& sc, const BuildInputs& in, int b, int f) {
   if (f >= in.F) return;
   bool bad = false;
   for (int k = 0; k < 3; ++k) {
@@ -69,9 +66,7 @@ __device__ __forceinline__ void face_verts(const BuildInputs& in, int b, int f, 
   }
 }
 
-__global__ void bounds_kernel(Scene sc, BuildInputs in) {
-  const int b = blockIdx.y;
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void bounds_item(const Scene& sc, const BuildInputs& in, int b, int f) {
   const int n = sc.meta[b].n;
   float scale = 0.f;
   float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
@@ -104,7 +99,7 @@ __global__ void bounds_kernel(Scene sc, BuildInputs in) {
       hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], off));
     }
   }
-  if ((threadIdx.x & 31) == 0 && blockIdx.x * blockDim.x + (threadIdx.x & ~31) < n) {
+  if ((threadIdx.x & 31) == 0 && f < n) {  // (f: the warp's first face)
     Meta& m = sc.meta[b];
     atomicMax(reinterpret_cast<int*>(&m.scale), __float_as_int(scale));
     for (int a = 0; a < 3; ++a) {
@@ -123,9 +118,7 @@ __device__ __forceinline__ uint32_t spread10(uint32_t x) {
   return x;
 }
 
-__global__ void morton_kernel(Scene sc, BuildInputs in) {
-  const int b = blockIdx.y;
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void morton_item(const Scene& sc, const BuildInputs& in, int b, int f) {
   const int n = sc.meta[b].n;
   if (f >= n) return;
   fv3 v[3];
@@ -148,6 +141,42 @@ __global__ void morton_kernel(Scene sc, BuildInputs in) {
   sc.vals[base + f] = (uint32_t)f;
 }
 
+// The same sort for at most kBitonicKeys keys: a bitonic network over
+// (key, position) words in shared memory, unique and so in the stable order. One
+// thread per pair; a warp's 32 pairs lie in its own 64 words at strides up to 32,
+// where a warp barrier is enough.
+constexpr int kBitonicKeys = 2048;
+__device__ __forceinline__ void cta_bitonic_sort(const uint32_t* k0, const uint32_t* v0,
+                                                uint32_t* k1, uint32_t* v1, int n,
+                                                unsigned long long* w) {
+  const int tid = threadIdx.x;
+  int m = 64;
+  while (m < n) m <<= 1;
+  for (int i = tid; i < m; i += kSortThreads)
+    w[i] = i < n ? ((unsigned long long)k0[i] << 32) | (unsigned)i : ~0ull;
+  __syncthreads();
+  for (int k = 2; k <= m; k <<= 1)
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      if (tid < (m >> 1)) {
+        const int i = 2 * tid - (tid & (j - 1));
+        const unsigned long long a = w[i], c = w[i + j];
+        if ((a > c) == ((i & k) == 0)) {
+          w[i] = c;
+          w[i + j] = a;
+        }
+      }
+      // (the next stride: j / 2, or k after the last one)
+      if (j > 32 || (j == 1 && k > 32)) __syncthreads(); else __syncwarp();
+    }
+  __syncthreads();
+  for (int i = tid; i < n; i += kSortThreads) {
+    const unsigned long long a = w[i];
+    k1[i] = (uint32_t)(a >> 32);
+    v1[i] = v0[(uint32_t)a];
+  }
+  __syncthreads();
+}
+
 // One-CTA stable LSD radix sort of n 30-bit keys with their values: three
 // 10-bit passes k0/v0 -> k1/v1 -> k0/v0 -> k1/v1, so the sorted pairs end in
 // k1/v1. Warp w owns the w-th of 32 contiguous chunks of the input. A pass
@@ -163,6 +192,12 @@ __device__ void cta_radix_sort30(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint3
   uint32_t* offset = smem + 32 * kSortDigits;  // [1024] first position of each digit
   uint32_t* total = offset + kSortDigits;      // [1024] digit totals; [32] scan partials
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // (a radix pass costs 5 us however few the keys: 320 faces' whole build took 66 us
+  // with the radix sort and a global edge table, 40 us with this and a shared one)
+  if (n <= kBitonicKeys) {
+    cta_bitonic_sort(k0, v0, k1, v1, n, reinterpret_cast<unsigned long long*>(smem));
+    return;
+  }
   const uint32_t lt = (1u << lane) - 1u;
   const int chunk = (((n + 31) / 32) + 31) & ~31;
   const int lo = min(n, warp * chunk), hi = min(n, lo + chunk);
@@ -248,24 +283,19 @@ __device__ void cta_radix_sort30(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint3
   }
 }
 
-__global__ void __launch_bounds__(kSortThreads) sort_kernel(Scene sc) {
-  extern __shared__ uint32_t smem[];
-  const int b = blockIdx.x;
+__device__ __forceinline__ void sort_item(const Scene& sc, int b, uint32_t* smem) {
   uint32_t* k0 = sc.keys + (size_t)b * 2 * sc.F;
   uint32_t* v0 = sc.vals + (size_t)b * 2 * sc.F;
   cta_radix_sort30(k0, v0, k0 + sc.F, v0 + sc.F, sc.meta[b].n, smem);
 }
 
-// Morton order of P wall points, one CTA per batch item: bounding box, 30-bit
+// Morton order of P wall points by one CTA: bounding box, 30-bit
 // codes over it, radix sort. scr is [4][B][P] (keys, values, keys, values);
 // the permutation (point indices in Morton order) ends in the fourth quarter,
 // and the first quarter is then set to -1: the visibility kernel keeps each
 // point's last occluder there (by Morton position of the point).
-__global__ void __launch_bounds__(kSortThreads) point_order_kernel(View3f pts, int P, int B,
-                                                                  uint32_t* scr) {
-  extern __shared__ uint32_t smem[];
-  __shared__ int box[6];
-  const int b = blockIdx.x;
+__device__ __forceinline__ void point_order_item(const View3f& pts, int P, int B, int b,
+                                                 uint32_t* scr, uint32_t* smem, int* box) {
   const size_t BP = (size_t)B * P;
   uint32_t* k0 = scr + (size_t)b * P;
   uint32_t* v0 = scr + BP + (size_t)b * P;
@@ -306,9 +336,7 @@ __global__ void __launch_bounds__(kSortThreads) point_order_kernel(View3f pts, i
   for (int i = threadIdx.x; i < P; i += blockDim.x) k0[i] = ~0u;
 }
 
-__global__ void records_kernel(Scene sc, BuildInputs in) {
-  const int b = blockIdx.y;
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void records_item(const Scene& sc, const BuildInputs& in, int b, int k) {
   const Meta& m = sc.meta[b];
   const int n = m.n;
   if (k >= n) return;
@@ -352,9 +380,7 @@ __device__ __forceinline__ int kdelta(const uint32_t* keys, int n, int i, int j)
   return __clz(a ^ c);
 }
 
-__global__ void hierarchy_kernel(Scene sc) {
-  const int b = blockIdx.y;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void hierarchy_item(const Scene& sc, int b, int i) {
   const int n = sc.meta[b].n;
   if (i >= n - 1) return;
   const uint32_t* keys = sc.keys + (size_t)b * 2 * sc.F + (size_t)sc.sorted_buf * sc.F;
@@ -384,9 +410,10 @@ __global__ void hierarchy_kernel(Scene sc) {
   if (i == 0) sc.iparent[base] = -1;
 }
 
-__global__ void refit_kernel(Scene sc) {
-  const int b = blockIdx.y;
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+// kCta: the mesh's threads are one CTA, counter its arrival counts in shared
+// memory.
+template <bool kCta>
+__device__ __forceinline__ void refit_item(const Scene& sc, int b, int k, int* counter) {
   const int n = sc.meta[b].n;
   if (k >= n || n < 2) return;
   const float delta = sc.meta[b].delta;
@@ -406,9 +433,9 @@ __global__ void refit_kernel(Scene sc) {
       nd[node_plane(side, 0, a)] = lo[a];
       nd[node_plane(side, 1, a)] = hi[a];
     }
-    __threadfence();
-    if (atomicAdd(&sc.counter[base + node], 1) == 0) return;
-    __threadfence();
+    if (kCta) __threadfence_block(); else __threadfence();
+    if (atomicAdd(&counter[node], 1) == 0) return;
+    if (kCta) __threadfence_block(); else __threadfence();
     const volatile float* vn = nd;
     for (int a = 0; a < 3; ++a) {
       lo[a] = fminf(vn[node_plane(0, 0, a)], vn[node_plane(1, 0, a)]);
@@ -425,9 +452,7 @@ __global__ void refit_kernel(Scene sc) {
 // boxes are replaced by its grandchildren's (a leaf child keeps its own box and
 // slot), read after the refit has finished every box. Slots 0 and 1 are always
 // filled; an unused slot carries the code kWideEmpty (traversals skip it).
-__global__ void widen_kernel(Scene sc) {
-  const int b = blockIdx.y;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void widen_item(const Scene& sc, int b, int i) {
   const int n = sc.meta[b].n;
   if (i >= n - 1) return;
   const size_t base = (size_t)b * sc.F;
@@ -484,14 +509,11 @@ __device__ __forceinline__ void face_vertex_ids(const Scene& sc, int b, int k, u
   vi[2] = (uint32_t)__float_as_int(s[3].w);
 }
 
-__global__ void edge_insert_kernel(Scene sc) {
-  const int b = blockIdx.y;
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void edge_insert_item(const Scene& sc, int b, int k, unsigned long long* keys,
+                                                int2* vals) {
   if (k >= sc.meta[b].n) return;
   uint32_t vi[3];
   face_vertex_ids(sc, b, k, vi);
-  unsigned long long* keys = sc.ekeys + (size_t)b * sc.ecap;
-  int2* vals = sc.evals + (size_t)b * sc.ecap;
   for (int e = 0; e < 3; ++e) {
     const uint32_t a = vi[(e + 1) % 3], c = vi[(e + 2) % 3];
     if (a == c) continue;
@@ -508,14 +530,11 @@ __global__ void edge_insert_kernel(Scene sc) {
   }
 }
 
-__global__ void edge_link_kernel(Scene sc) {
-  const int b = blockIdx.y;
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void edge_link_item(const Scene& sc, int b, int k, const unsigned long long* keys,
+                                                const int2* vals) {
   if (k >= sc.meta[b].n) return;
   uint32_t vi[3];
   face_vertex_ids(sc, b, k, vi);
-  const unsigned long long* keys = sc.ekeys + (size_t)b * sc.ecap;
-  const int2* vals = sc.evals + (size_t)b * sc.ecap;
   int nb[3];
   for (int e = 0; e < 3; ++e) {
     nb[e] = -1;
@@ -538,18 +557,170 @@ __global__ void edge_link_kernel(Scene sc) {
   sc.adj[(size_t)b * sc.F + k] = make_int4(nb[0], nb[1], nb[2], 0);
 }
 
-int launch_point_order(const Scene& sc, const View3f& pts, int P, cudaStream_t stream) {
-  const size_t smem = sizeof(uint32_t) * (32 * kSortDigits + 2 * kSortDigits);
-  TOTRI_CUDA(tune::ensure_dynamic_smem(
-      reinterpret_cast<const void*>(point_order_kernel), smem));
-  TOTRI_KERNEL("mesh point order", stream,
-               point_order_kernel<<<sc.B, kSortThreads, smem, stream>>>(pts, P, sc.B,
-                                                                         sc.pscratch));
+// One thread per face (or node) and batch item.
+__global__ void init_kernel(Scene sc, int F) {
+  init_item(sc, F, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x);
+}
+__global__ void faces_kernel(Scene sc, BuildInputs in) {
+  faces_item(sc, in, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x);
+}
+__global__ void bounds_kernel(Scene sc, BuildInputs in) {
+  bounds_item(sc, in, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x);
+}
+__global__ void morton_kernel(Scene sc, BuildInputs in) {
+  morton_item(sc, in, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x);
+}
+__global__ void records_kernel(Scene sc, BuildInputs in) {
+  records_item(sc, in, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x);
+}
+__global__ void hierarchy_kernel(Scene sc) {
+  hierarchy_item(sc, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x);
+}
+__global__ void refit_kernel(Scene sc) {
+  const int b = blockIdx.y;
+  refit_item<false>(sc, b, blockIdx.x * blockDim.x + threadIdx.x, sc.counter + (size_t)b * sc.F);
+}
+__global__ void widen_kernel(Scene sc) {
+  widen_item(sc, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x);
+}
+__global__ void edge_insert_kernel(Scene sc) {
+  const int b = blockIdx.y;
+  edge_insert_item(sc, b, blockIdx.x * blockDim.x + threadIdx.x, sc.ekeys + (size_t)b * sc.ecap,
+              sc.evals + (size_t)b * sc.ecap);
+}
+__global__ void edge_link_kernel(Scene sc) {
+  const int b = blockIdx.y;
+  edge_link_item(sc, b, blockIdx.x * blockDim.x + threadIdx.x, sc.ekeys + (size_t)b * sc.ecap,
+              sc.evals + (size_t)b * sc.ecap);
+}
+
+// Morton order of one wall-point set per CTA: sets x batch items.
+__global__ void __launch_bounds__(kSortThreads) point_order_kernel(WallPoints w0, WallPoints w1,
+                                                                  int B) {
+  extern __shared__ uint32_t smem[];
+  __shared__ int box[6];
+  const WallPoints& w = blockIdx.y ? w1 : w0;
+  point_order_item(w.pts, w.P, B, blockIdx.x, w.scratch, smem, box);
+}
+
+// One CTA per mesh (blockIdx.y = 0) and, beside it, per wall-point set.
+__global__ void __launch_bounds__(kSortThreads) sort_kernel(Scene sc, WallPoints w0,
+                                                           WallPoints w1) {
+  extern __shared__ uint32_t smem[];
+  __shared__ int box[6];
+  const int b = blockIdx.x;
+  if (blockIdx.y > 0) {
+    const WallPoints& w = blockIdx.y == 1 ? w0 : w1;
+    point_order_item(w.pts, w.P, sc.B, b, w.scratch, smem, box);
+    return;
+  }
+  sort_item(sc, b, smem);
+}
+
+// The whole build of one small mesh by one CTA, a barrier between the stages
+// instead of a kernel each, the edge table and the refit's counters in shared
+// memory, and the wall points' order by further CTAs of the same launch
+// (blockIdx.y = 1, 2). Latency bounds it: a stage is a few dependent loads. The
+// 11 kernels and 3 memsets of the general build took 110 us at 320 faces and 144
+// points and 132 us at 1,536 faces; this takes 41 and 107 us (22 us at one face),
+// and the call loses another 15 us of gaps. It was the faster one for every batch
+// tried at 33, 320 and 1,536 faces (1 to 600 meshes: 249 against 316 us at 600 x
+// 320 faces); at 2,048 faces the two are level (122 and 132 us of kernels, calls
+// 0.98-1.00x). "mesh.build.small" = 2 turns it off.
+constexpr int kSmallFaces = 1536;
+constexpr int kSortWords = 32 * kSortDigits + 2 * kSortDigits;
+static_assert(17 * kSmallFaces <= kSortWords, "edge table and counters fit the sort's memory");
+__global__ void __launch_bounds__(kSortThreads) build_small_kernel(Scene sc, BuildInputs in,
+                                                                  WallPoints w0, WallPoints w1) {
+  extern __shared__ uint32_t smem[];
+  __shared__ int box[6];
+  const int b = blockIdx.x, tid = threadIdx.x;
+  if (blockIdx.y > 0) {
+    const WallPoints& w = blockIdx.y == 1 ? w0 : w1;
+    point_order_item(w.pts, w.P, sc.B, b, w.scratch, smem, box);
+    return;
+  }
+  if (sc.B == 1 && tid == 0) *sc.status = 0u;
+  const int F = in.F, F32 = (F + 31) & ~31;
+  if (tid == 0) init_meta(sc.meta[b], F);
+  __syncthreads();
+  for (int i = tid; i < F; i += kSortThreads) faces_item(sc, in, b, i);
+  __syncthreads();
+  for (int i = tid; i < F32; i += kSortThreads) bounds_item(sc, in, b, i);  // (whole warps)
+  __syncthreads();
+  for (int i = tid; i < F; i += kSortThreads) morton_item(sc, in, b, i);
+  __syncthreads();
+  sort_item(sc, b, smem);
+  __syncthreads();
+  // from here on the sort's memory holds the edge table and the refit's counters
+  unsigned long long* ekeys = reinterpret_cast<unsigned long long*>(smem);  // [4 F]
+  int2* evals = reinterpret_cast<int2*>(ekeys + sc.ecap);                   // [4 F]
+  int* counter = reinterpret_cast<int*>(evals + sc.ecap);                   // [F]
+  for (int i = tid; i < sc.ecap; i += kSortThreads) {
+    ekeys[i] = kEdgeEmpty;
+    evals[i] = make_int2(-1, -1);
+  }
+  for (int i = tid; i < F; i += kSortThreads) counter[i] = 0;
+  for (int i = tid; i < F; i += kSortThreads) {
+    records_item(sc, in, b, i);
+    hierarchy_item(sc, b, i);  // (needs the sorted keys only)
+  }
+  __syncthreads();
+  for (int i = tid; i < F; i += kSortThreads) {
+    edge_insert_item(sc, b, i, ekeys, evals);
+    refit_item<true>(sc, b, i, counter);
+  }
+  __syncthreads();
+  for (int i = tid; i < F; i += kSortThreads) {
+    edge_link_item(sc, b, i, ekeys, evals);
+    widen_item(sc, b, i);
+  }
+}
+
+namespace {
+
+WallPoints wall_points(const Scene& sc, const WallSet& w) {
+  return WallPoints{w.pts, w.P, sc.pscratch + 4 * (size_t)sc.B * w.row0};
+}
+
+int check_walls(const WallSet* sets, int nsets) {
+  for (int j = 0; j < nsets; ++j)
+    if (sets[j].P >= (1 << 30) / 4) return fail(TOTRI_ERR_UNSUPPORTED, "too many wall points");
   return TOTRI_OK;
 }
 
-int build_scene(const Scene& sc, const BuildInputs& in, cudaStream_t stream) {
+const size_t kSortSmem = sizeof(uint32_t) * kSortWords;
+
+}  // namespace
+
+int launch_point_order(const Scene& sc, const WallSet* sets, int nsets, cudaStream_t stream) {
+  if (nsets == 0) return TOTRI_OK;
+  TOTRI_TRY(check_walls(sets, nsets));
+  TOTRI_CUDA(tune::ensure_dynamic_smem(
+      reinterpret_cast<const void*>(point_order_kernel), kSortSmem));
+  TOTRI_KERNEL("mesh point order", stream,
+               point_order_kernel<<<dim3((unsigned)sc.B, (unsigned)nsets), kSortThreads, kSortSmem,
+                                    stream>>>(wall_points(sc, sets[0]),
+                                              wall_points(sc, sets[nsets - 1]), sc.B));
+  return TOTRI_OK;
+}
+
+int build_scene(const Scene& sc, const BuildInputs& in, cudaStream_t stream, const WallSet* sets,
+                int nsets) {
   const int B = sc.B;
+  TOTRI_TRY(check_walls(sets, nsets));
+  const WallPoints w0 = nsets > 0 ? wall_points(sc, sets[0]) : WallPoints{};
+  const WallPoints w1 = nsets > 1 ? wall_points(sc, sets[1]) : WallPoints{};
+  const dim3 gridS((unsigned)B, 1u + (unsigned)nsets);
+  if (in.F > 0 && in.F <= kSmallFaces && tune::get("mesh.build.small") != 2) {
+    if (B > 1) TOTRI_CUDA(cudaMemsetAsync(sc.status, 0, sizeof(uint32_t), stream));
+    TOTRI_CUDA(tune::ensure_dynamic_smem(
+        reinterpret_cast<const void*>(build_small_kernel), kSortSmem));
+    TOTRI_KERNEL("mesh build", stream,
+                 build_small_kernel<<<gridS, kSortThreads, kSortSmem, stream>>>(sc, in, w0, w1));
+    return TOTRI_OK;
+  }
+  if (in.F == 0) TOTRI_TRY(launch_point_order(sc, sets, nsets, stream));
   const dim3 blk(256);
   const dim3 gridF((unsigned)ceil_div(sc.F, 256), (unsigned)B);
   TOTRI_CUDA(cudaMemsetAsync(sc.status, 0, sizeof(uint32_t), stream));
@@ -558,10 +729,9 @@ int build_scene(const Scene& sc, const BuildInputs& in, cudaStream_t stream) {
     TOTRI_KERNEL("mesh faces", stream, faces_kernel<<<gridF, blk, 0, stream>>>(sc, in));
     TOTRI_KERNEL("mesh bounds", stream, bounds_kernel<<<gridF, blk, 0, stream>>>(sc, in));
     TOTRI_KERNEL("mesh morton", stream, morton_kernel<<<gridF, blk, 0, stream>>>(sc, in));
-    const size_t smem = sizeof(uint32_t) * (32 * kSortDigits + 2 * kSortDigits);
-    TOTRI_CUDA(tune::ensure_dynamic_smem(
-        reinterpret_cast<const void*>(sort_kernel), smem));
-    TOTRI_KERNEL("mesh sort", stream, sort_kernel<<<B, kSortThreads, smem, stream>>>(sc));
+    TOTRI_CUDA(tune::ensure_dynamic_smem(reinterpret_cast<const void*>(sort_kernel), kSortSmem));
+    TOTRI_KERNEL("mesh sort", stream,
+                 sort_kernel<<<gridS, kSortThreads, kSortSmem, stream>>>(sc, w0, w1));
     TOTRI_KERNEL("mesh records", stream, records_kernel<<<gridF, blk, 0, stream>>>(sc, in));
     TOTRI_CUDA(cudaMemsetAsync(sc.ekeys, 0xff, sizeof(unsigned long long) * B * sc.ecap, stream));
     TOTRI_CUDA(cudaMemsetAsync(sc.evals, 0xff, sizeof(int2) * B * sc.ecap, stream));

@@ -112,12 +112,20 @@ __global__ void __launch_bounds__(256) visibility_kernel(Scene sc, View3f pts, i
 // one mask word per point and chunk. This is the default visibility kernel.
 constexpr int kMaxPatchChunks = 16;
 
+// The wall-point sets of one launch: blocks of 32 points, set 0 in blocks
+// [0, blocks0), set 1 (if any) after them.
+struct Walls {
+  View3f pts0, pts1;
+  int P0, P1, row0, row1;
+  unsigned blocks0;
+};
+
 // kWalk 0: target_visible_pp, 1: packet_visible, 2: target_visible_pp4, 3: shaft
 // search, 4: target_visible_pp's prefix and a 4-wide BVH search
 // (bvh_occluded_wide); kOcc: CTAs per SM that the register allocation must allow.
 template <int kWalk, int kOcc = 1, int kWarps = 8>
-__global__ void __launch_bounds__(32 * kWarps, kOcc) visibility_patch_kernel(Scene sc, View3f pts, int P,
-                                                               int row0, int chunks,
+__global__ void __launch_bounds__(32 * kWarps, kOcc) visibility_patch_kernel(Scene sc, Walls walls,
+                                                               int chunks,
                                                                int seed_mode, int seed_steps,
                                                                int shaft_cap) {
   __shared__ uint32_t bits[kMaxPatchChunks][32];  // [chunk][face j]: visible from point lane
@@ -128,15 +136,21 @@ __global__ void __launch_bounds__(32 * kWarps, kOcc) visibility_patch_kernel(Sce
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int b = blockIdx.z;
   const int ch0 = blockIdx.y * chunks;
-  const int i = blockIdx.x * 32 + lane;  // position in Morton order
+  // one or two sets of wall points, the blocks of the second after the first's
+  const bool second = blockIdx.x >= walls.blocks0;
+  const View3f pts = second ? walls.pts1 : walls.pts0;
+  const int P = second ? walls.P1 : walls.P0, row0 = second ? walls.row1 : walls.row0;
+  uint32_t* scratch = sc.pscratch + 4 * (size_t)sc.B * row0;
+  // position in Morton order
+  const int i = (int)(blockIdx.x - (second ? walls.blocks0 : 0u)) * 32 + lane;
   const int n = sc.meta[b].n;
   const bool okp = i < P;
-  const uint32_t* order = sc.pscratch + 3 * (size_t)sc.B * P + (size_t)b * P;
+  const uint32_t* order = scratch + 3 * (size_t)sc.B * P + (size_t)b * P;
   int p = okp ? (int)order[i] : 0;
   if (!TOTRI_INDEX_OK((unsigned)p < (unsigned)P, sc.status)) p = 0;
   const fv3 o = okp ? mkv(pts.at(b, p, 0), pts.at(b, p, 1), pts.at(b, p, 2)) : mkv(0.f, 0.f, 0.f);
   volatile int* vseeds = seeds;
-  volatile int* gseeds = reinterpret_cast<int*>(sc.pscratch) + (size_t)b * P;
+  volatile int* gseeds = reinterpret_cast<int*>(scratch) + (size_t)b * P;
   if (threadIdx.x < 32) seeds[lane] = okp ? gseeds[i] : -1;
   if (threadIdx.x == 0) next_face = 0;
   __syncthreads();
@@ -962,8 +976,38 @@ int launch_mask_unsort(const Scene& sc, int P, uint32_t* out, cudaStream_t strea
   return TOTRI_OK;
 }
 
-int launch_visibility(const Scene& sc, const View3f& pts, int P, int row0, bool brute,
-                      cudaStream_t stream) {
+// Dense wall grids (blocks of 32 points narrow enough for the hulls) with
+// enough (block, chunk) units to feed the queues: from 2,048 points and 16,384
+// units on the two kernels were faster on every mesh tried (1.02-1.11x on
+// 20,000-face spheres at 48 x 48 and 101 x 23 points, 1.06x on 5,120 faces at 64 x
+// 64, 2.2x on boxes there); below, 0.72-0.98x on spheres (5,120 faces at 40 x 40,
+// 101 x 23 and 48 x 48 points, 20,000 at 40 x 40), though 1.3x on 20,480 faces at
+// 32 x 32 and 1.3-1.6x on boxes. "mesh.visibility.list": 1 always, 2 never;
+// ".list.cap" lowers the list's capacity.
+static bool list_rule(const Scene& sc, int P) {
+  const int list = tune::get("mesh.visibility.list");
+  const int64_t units = ceil_div(P, 32) * sc.nch * sc.B;
+  return tune::get("mesh.visibility.mode") == 0 && tune::get("mesh.visibility.wide") != 2 &&
+         tune::get("mesh.visibility.queue") != 1 && tune::get("mesh.visibility.occupancy") == 0 &&
+         (list == 1 || (list == 0 && P >= 2048 && units >= 16384)) && units < ((int64_t)1 << 29);
+}
+
+bool orders_points(bool brute) {
+  const int mode = tune::get("mesh.visibility.mode");
+  return !brute && mode != kVisRay && mode != kVisPacket && mode != kVisRayPostponed;
+}
+
+static int launch_visibility_sets(const Scene& sc0, const WallSet* sets, int nsets, bool brute,
+                                  cudaStream_t stream) {
+  // (the kernels over one set find its scratch at sc.pscratch)
+  const View3f& pts = sets[0].pts;
+  const int row0 = sets[0].row0;
+  const int P = sets[0].P;
+  Scene sc = sc0;
+  sc.pscratch += 4 * (size_t)sc.B * row0;
+  const int P2 = nsets > 1 ? sets[1].P : 0;
+  const Walls walls{pts, nsets > 1 ? sets[1].pts : pts, P, P2, row0, nsets > 1 ? sets[1].row0 : 0,
+                    (unsigned)ceil_div(P, 32)};
   const int64_t units = (int64_t)sc.B * P * sc.nch;
   if (units == 0) return TOTRI_OK;
   const unsigned blocks = (unsigned)ceil_div(units * 32, 256);
@@ -981,14 +1025,11 @@ int launch_visibility(const Scene& sc, const View3f& pts, int P, int row0, bool 
                  visibility_kernel<kVisRayPostponed><<<blocks, 256, 0, stream>>>(sc, pts, P,
                                                                                   row0));
   } else {
-    if (P >= (1 << 30) / 4) return fail(TOTRI_ERR_UNSUPPORTED, "too many wall points");
-    const int st = launch_point_order(sc, pts, P, stream);
-    if (st != TOTRI_OK) return st;
     // Chunks per CTA: up to 8 while the grid keeps 32 CTAs per SM (20,480 faces x
     // 4,096 points: 9.15 ms at 8, 9.3 at 4, 9.6 at 2, 10.4 at 1, 10.5 at 16; 20,000
     // faces x 400 and 144 points: 3.2 ms at the 6 and 2 that 8 CTAs per SM gave,
     // 2.7 ms at 1).
-    const int64_t patches = ceil_div(P, 32);
+    const int64_t patches = ceil_div(P, 32) + ceil_div(P2, 32);
     int chunks = tune::get("mesh.visibility.chunks");
     if (chunks <= 0)
       chunks = (int)std::max<int64_t>(
@@ -1004,36 +1045,23 @@ int launch_visibility(const Scene& sc, const View3f& pts, int P, int row0, bool 
     // per-lane search)
     int shaft_cap = tune::get("mesh.visibility.shaft.cap");
     if (shaft_cap <= 0 || shaft_cap > kShaftCand) shaft_cap = kShaftCand;
-    const dim3 grid((unsigned)ceil_div(P, 32), (unsigned)ceil_div(sc.nch, chunks),
+    const dim3 grid((unsigned)patches, (unsigned)ceil_div(sc.nch, chunks),
                     (unsigned)sc.B);
     const int mode = tune::get("mesh.visibility.mode");
-    const int list = tune::get("mesh.visibility.list");
     const int64_t cta_count = (int64_t)grid.x * grid.y * grid.z;
     if (mode == kVisPatchPacket)
       TOTRI_KERNEL("mesh visibility", stream,
                    visibility_patch_kernel<1><<<grid, 256, 0, stream>>>(
-                       sc, pts, P, row0, chunks, kSeedOff, 0, 0));
+                       sc0, walls, chunks, kSeedOff, 0, 0));
     else if (mode == kVisPatchWide)
       TOTRI_KERNEL("mesh visibility", stream,
                    visibility_patch_kernel<2><<<grid, 256, 0, stream>>>(
-                       sc, pts, P, row0, chunks, kSeedOff, 0, 0));
+                       sc0, walls, chunks, kSeedOff, 0, 0));
     else if (mode == kVisPatchShaft)
       TOTRI_KERNEL("mesh visibility", stream,
                    visibility_patch_kernel<3><<<grid, 256, 0, stream>>>(
-                       sc, pts, P, row0, chunks, seed_mode, seed_steps, shaft_cap));
-    // Dense wall grids (blocks of 32 points narrow enough for the hulls) with
-    // enough (block, chunk) units to feed the queues: from 2,048 points and 16,384
-    // units on the two kernels were faster on every mesh tried (1.02-1.11x on
-    // 20,000-face spheres at 48 x 48 and 101 x 23 points, 1.06x on 5,120 faces at 64 x
-    // 64, 2.2x on boxes there); below, 0.72-0.98x on spheres (5,120 faces at 40 x 40,
-    // 101 x 23 and 48 x 48 points, 20,000 at 40 x 40), though 1.3x on 20,480 faces at
-    // 32 x 32 and 1.3-1.6x on boxes. "mesh.visibility.list": 1 always, 2 never;
-    // ".list.cap" lowers the list's capacity.
-    else if (mode == 0 && tune::get("mesh.visibility.wide") != 2 &&
-             tune::get("mesh.visibility.queue") != 1 &&
-             tune::get("mesh.visibility.occupancy") == 0 &&
-             (list == 1 || (list == 0 && P >= 2048 && patches * sc.nch * sc.B >= 16384)) &&
-             patches * sc.nch * sc.B < ((int64_t)1 << 29)) {
+                       sc0, walls, chunks, seed_mode, seed_steps, shaft_cap));
+    else if (nsets == 1 && list_rule(sc, P)) {
       int cap = tune::get("mesh.visibility.list.cap");
       if (cap <= 0 || cap > kListCand) cap = kListCand;
       // the queues' counters: the second quarter of the point scratch is free
@@ -1059,22 +1087,22 @@ int launch_visibility(const Scene& sc, const View3f& pts, int P, int row0, bool 
       if (tune::get("mesh.visibility.occupancy") == 5)
         TOTRI_KERNEL("mesh visibility", stream,
                      visibility_patch_kernel<4, 5><<<grid, 256, 0, stream>>>(
-                         sc, pts, P, row0, chunks, seed_mode, seed_steps, 0));
+                         sc0, walls, chunks, seed_mode, seed_steps, 0));
       // Grids that fill less than a wave: more warps per CTA, fewer faces in a row
       // per warp (768 faces x 143 and 35 points: 275 us with 8 warps, 190 with 16,
       // 152 with 32; 320 faces x 1,024 points: 77, 65 and 74 us).
       else if (cta_count <= tune::sm_count())
         TOTRI_KERNEL("mesh visibility", stream,
                      visibility_patch_kernel<4, 1, 32><<<grid, 1024, 0, stream>>>(
-                         sc, pts, P, row0, chunks, seed_mode, seed_steps, 0));
+                         sc0, walls, chunks, seed_mode, seed_steps, 0));
       else if (cta_count <= 4 * tune::sm_count())
         TOTRI_KERNEL("mesh visibility", stream,
                      visibility_patch_kernel<4, 2, 16><<<grid, 512, 0, stream>>>(
-                         sc, pts, P, row0, chunks, seed_mode, seed_steps, 0));
+                         sc0, walls, chunks, seed_mode, seed_steps, 0));
       else
         TOTRI_KERNEL("mesh visibility", stream,
                      visibility_patch_kernel<4, 4><<<grid, 256, 0, stream>>>(
-                         sc, pts, P, row0, chunks, seed_mode, seed_steps, 0));
+                         sc0, walls, chunks, seed_mode, seed_steps, 0));
     }
     // The queued BVH searches (visibility_queue_kernel) when
     // "mesh.visibility.queue" = 1; queue entries pack the target's Morton
@@ -1095,19 +1123,38 @@ int launch_visibility(const Scene& sc, const View3f& pts, int P, int row0, bool 
     else if (tune::get("mesh.visibility.occupancy") == 1)
       TOTRI_KERNEL("mesh visibility", stream,
                    visibility_patch_kernel<0, 1><<<grid, 256, 0, stream>>>(
-                       sc, pts, P, row0, chunks, seed_mode, seed_steps, 0));
+                       sc0, walls, chunks, seed_mode, seed_steps, 0));
     else if (tune::get("mesh.visibility.occupancy") == 4)
       TOTRI_KERNEL("mesh visibility", stream,
                    visibility_patch_kernel<0, 4><<<grid, 256, 0, stream>>>(
-                       sc, pts, P, row0, chunks, seed_mode, seed_steps, 0));
+                       sc0, walls, chunks, seed_mode, seed_steps, 0));
     else if (tune::get("mesh.visibility.occupancy") == 6)
       TOTRI_KERNEL("mesh visibility", stream,
                    visibility_patch_kernel<0, 6><<<grid, 256, 0, stream>>>(
-                       sc, pts, P, row0, chunks, seed_mode, seed_steps, 0));
+                       sc0, walls, chunks, seed_mode, seed_steps, 0));
     else
       TOTRI_KERNEL("mesh visibility", stream,
                    visibility_patch_kernel<0, 5><<<grid, 256, 0, stream>>>(
-                       sc, pts, P, row0, chunks, seed_mode, seed_steps, 0));
+                       sc0, walls, chunks, seed_mode, seed_steps, 0));
+  }
+  return TOTRI_OK;
+}
+
+int launch_visibility(const Scene& sc, const WallSet* sets, int nsets, bool brute, bool order,
+                      cudaStream_t stream) {
+  if (order && orders_points(brute)) {
+    const int st = launch_point_order(sc, sets, nsets, stream);
+    if (st != TOTRI_OK) return st;
+  }
+  // Two sets go in one launch of visibility_patch_kernel where that is the
+  // kernel for both (no key selects another one, neither set takes the lists).
+  const bool one = nsets == 2 && !brute && tune::get("mesh.visibility.mode") == 0 &&
+                   tune::get("mesh.visibility.queue") != 1 && sets[0].P > 0 && sets[1].P > 0 &&
+                   !list_rule(sc, sets[0].P) && !list_rule(sc, sets[1].P);
+  if (one) return launch_visibility_sets(sc, sets, 2, brute, stream);
+  for (int j = 0; j < nsets; ++j) {
+    const int st = launch_visibility_sets(sc, sets + j, 1, brute, stream);
+    if (st != TOTRI_OK) return st;
   }
   return TOTRI_OK;
 }

@@ -326,10 +326,25 @@ __device__ __forceinline__ void scatter_face_grad(const GradOut& out, int b, flo
 }
 
 // Host launchers.
-int launch_visibility(const Scene& sc, const View3f& pts, int P, int row0, bool brute,
+// A set of P wall points whose mask rows start at row0; its sort scratch is the
+// [4][B][P] words of sc.pscratch from 4 B row0 on (order in the last quarter).
+struct WallSet {
+  View3f pts;
+  int P, row0;
+};
+struct WallPoints {  // the same on the device
+  View3f pts;
+  int P;
+  uint32_t* scratch;
+};
+// Whether launch_visibility reads the points in Morton order.
+bool orders_points(bool brute);
+// Masks of one or two wall-point sets, already ordered (build_scene) unless
+// order is set.
+int launch_visibility(const Scene& sc, const WallSet* sets, int nsets, bool brute, bool order,
                       cudaStream_t stream);
-// Morton order of P wall points into sc.pscratch ([4][B][P]; order in the last quarter).
-int launch_point_order(const Scene& sc, const View3f& pts, int P, cudaStream_t stream);
+// Morton orders of one or two wall-point sets.
+int launch_point_order(const Scene& sc, const WallSet* sets, int nsets, cudaStream_t stream);
 // Wall-to-origin terms of the exhaustive renderer (detector and laser).
 struct Origins {
   View3f so, lo;
@@ -359,7 +374,9 @@ int launch_confocal_grad(const Scene& sc, const View3f& sp, const View3f& so, in
                          const float* tgrad, int T, int S, float bw, float bo, const GradOut& out,
                          cudaStream_t stream);
 
-int build_scene(const Scene& sc, const BuildInputs& in, cudaStream_t stream);
+// Builds the scene and orders up to two sets of wall points.
+int build_scene(const Scene& sc, const BuildInputs& in, cudaStream_t stream,
+                const WallSet* sets = nullptr, int nsets = 0);
 
 }  // namespace mesh
 }  // namespace totri

@@ -26,6 +26,7 @@
 //   "mesh.visibility.queue"     1: queued BVH searches (visibility_queue_kernel)
 //   "mesh.visibility.list", ".list.cap" 1: front-facing targets over candidate lists always,
 //                               2: never (at its launcher) / most candidates in a list
+//   "mesh.build.small"          2: small meshes take the build of large ones too
 //   "mesh.visibility.wide"      2: binary BVH search after the surface-walk prefix
 //                               (the default is the 4-wide search)
 //   "mesh.visibility.occupancy", ".chunks", ".seed", ".seed.steps", ".shaft.cap"
