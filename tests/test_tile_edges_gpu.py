@@ -337,3 +337,71 @@ def test_joint_scan_and_laser_masks(cuda_lib, faces, S, L):
                                          oracle.mesh_visibility(vn, fn, lp), 200, 0.05, 0.0)
     assert np.linalg.norm(ref) > 0.0 or faces < 60
     assert rel(out[0].cpu().numpy(), ref) < 1e-5
+
+
+# S, L, bins, bin width, bin offset, origins: one point to just past tiles of 8 and
+# 32 columns, fewer lasers than a tile has columns (many scan points in a tile),
+# bins to just past windows, an odd bin count (padded rows), a first bin inside
+# the mesh's returns (corners before bin 0) and a last one inside them
+EXHAUSTIVE = [(1, 1, 1, 6.0, 0.0, False), (3, 11, 97, 0.06, 0.0, False),
+              (33, 1, 64, 0.1, 0.0, True), (1, 40, 301, 0.012, 2.3, False),
+              (7, 33, 60, 0.02, 1.9, True), (40, 6, 500, 0.011, 0.0, True),
+              (36, 32, 1021, 0.0051, 0.3, False)]
+
+
+def _exhaustive(shape, seed):
+    S, L, T, bw, bo, origin = shape
+    g = np.random.default_rng(seed)
+    v, f = _mesh("soup", 90, seed)
+    m = torch.rand((1, v.shape[1], 1), device="cuda") + 0.5
+    sp, lp = points(g, S), points(g, L)
+    so, lo = (points(g, S, -0.4), points(g, L, -0.6)) if origin else (None, None)
+    n = [x[0].cpu().numpy() for x in (v, f, m)]
+    vis = [oracle.mesh_visibility(n[0], n[1], p) for p in (sp, lp)]
+    none = torch.empty((1, 0, 3), device="cuda")
+    dev = [v, f, m, cu(sp[None]), cu(lp[None]), cu(so[None]) if origin else none,
+           cu(lo[None]) if origin else none]
+    return dev, (*n, sp, lp, so, lo, *vis, T, bw, bo)
+
+
+@pytest.mark.parametrize("shape", EXHAUSTIVE)
+@pytest.mark.parametrize("layout", [0, 2])
+def test_exhaustive_grad_edges(cuda_lib, shape, layout):
+    """Either side in the lanes, bins-last rows and the caller's order; the bound
+    of the other exhaustive gradients."""
+    from totri_gb300 import autotune
+    S, L, T, bw, bo, _ = shape
+    dev, ref = _exhaustive(shape, S + L)
+    tg = np.random.default_rng(T).standard_normal((T, S, L)).astype(np.float32)
+    vg, mg = torch.empty_like(dev[0]), torch.empty_like(dev[2])
+    try:
+        autotune.set_tile("mesh.exhaustive.grad.layout", layout)
+        R.mesh_exhaustive_grad_verts(*dev, cu(tg[None]), vg, mg, bw, bo, 0)
+    finally:
+        autotune.set_tile("mesh.exhaustive.grad.layout", 0)
+    rv, rm = oracle.mesh_exhaustive_grad(*ref, tg)
+    assert rel(vg[0].cpu().numpy(), rv) < 1e-5
+    assert rel(mg[0].cpu().numpy(), rm) < 1e-5
+
+
+def test_exhaustive_grad_follows_the_decided_bins(cuda_lib):
+    """Slivers with corners within rounding of a bin edge: the gradient splits each
+    tent where the decided bins say (one that did not moved two vertices by 5e-4,
+    the whole by 2.6e-5). FP32 sums over some 100 pairs per vertex: 2e-6."""
+    from totri_gb300 import scenes
+    v, f, m = [x.cuda() for x in scenes.uv_sphere(20000, 8, center=(0.03, -0.05, 1.0))]
+    m = m.reshape(1, -1, 1)
+    sp, lp = scenes.wall_grid(5)[0].numpy(), scenes.wall_grid(4)[0].numpy()
+    T, bw = 2048, 0.0025
+    tg = torch.randn((1, T, 25, 16), generator=torch.Generator().manual_seed(3))
+    none = torch.empty((1, 0, 3), device="cuda")
+    vg, mg = torch.empty_like(v), torch.empty_like(m)
+    R.mesh_exhaustive_grad_verts(v, f, m, cu(sp[None]), cu(lp[None]), none, none, tg.cuda(), vg,
+                                 mg, bw, 0.0, 0)
+    vn, fn, mn = v[0].cpu().numpy(), f[0].cpu().numpy(), m[0].cpu().numpy()
+    rv, rm = oracle.mesh_exhaustive_grad(vn, fn, mn, sp, lp, None, None,
+                                         oracle.mesh_visibility(vn, fn, sp),
+                                         oracle.mesh_visibility(vn, fn, lp), T, bw, 0.0,
+                                         tg[0].numpy())
+    assert rel(vg[0].cpu().numpy(), rv) < 2e-6
+    assert rel(mg[0].cpu().numpy(), rm) < 2e-6

@@ -980,7 +980,8 @@ int totri_backprojection_exhaustive_velten_forward_ws(
       const float* tb = trp + (int64_t)b * T * row;
       if (chunk > 0) {
         float* copy = static_cast<float*>(ws);
-        TOTRI_TRY(mesh::launch_bins_last(tb + sa * L, copy, (int)T, row, (sb - sa) * L, stream));
+        TOTRI_TRY(mesh::launch_bins_last(tb + sa * L, copy, (int)T, (int)T, row, (sb - sa) * L,
+                                         stream));
         TOTRI_KERNEL("backprojection velten exhaustive", stream,
                      bp::velten_pairs_kernel<true><<<grid, 256, 0, stream>>>(
                          g, b, (int)T, (int)S, (int)L, sp, lp, so, lo, So > 0, Lo > 0, bw, bo,

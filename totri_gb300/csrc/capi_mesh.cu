@@ -292,7 +292,7 @@ size_t totri_mesh_workspace(int64_t batch, int64_t num_verts, int64_t num_faces,
 
 size_t totri_mesh_exhaustive_grad_scratch(int64_t num_scan_points, int64_t num_laser_points,
                                           int64_t num_bins) {
-  return mesh::exh_grad_scratch_bytes(num_scan_points, num_laser_points, num_bins);
+  return mesh::mesh_grad_scratch_bytes(num_scan_points, num_laser_points, num_bins);
 }
 
 static int confocal_forward_impl(const totri_array_t* verts, const totri_array_t* faces,

@@ -502,44 +502,56 @@ __global__ void __launch_bounds__(256) exh_grad_compact_kernel(
 //     enters through the normal's Jacobian (AlphaExhaustiveGradVerts,
 //     mesh_common.h:549-630);
 //   - the unit vectors u_m = (v_m - p)/|v_m - p| that make up d c_k / d v.
-// A triple then only combines two records: the alpha gradient is taken in the
-// face's own vertex order (the formula is the same in any order), and only
-// the tent terms follow the sorted order. A CTA takes its faces one at a time
+// A triple then only needs its two factors P = alpha area-weighted gradient and Q_m
+// = alpha times the tent's weight of vertex m: the vertex gradients are linear in
+// the two records, sum P (cm_s + cm_l), sum P (wv_s + wv_l) and sum Q_m (u_s + u_l),
+// the alpha gradient being taken in the face's own vertex order (the formula is
+// the same in any order). A lane therefore keeps one point's record while its warp
+// walks the other points: it adds the other point's part triple by triple, 16
+// multiply-adds, and its own part once at the end, times the sums of P and Q; the
+// normal's Jacobian is applied to the face's sum. The lanes stand for the scan or
+// the laser points, whichever fill 32 better. A CTA takes its faces one at a time
 // over a slice of at most kFaceSlice scan points and the lasers in chunks of
-// kFaceSlice; its 256 threads share each face's (s, l) pairs. The decisions
-// (vertex order, bins) are those of exh_pair.
+// kFaceSlice. The decisions (vertex order, bins) are those of exh_pair.
+// 20,000 faces x 400 x 144 points, 2,048 bins: 8.2 ms (71% of the issue slots, the
+// ALU pipe 70% busy with selects and compares) against 11.9 ms when each of
+// a pair's 48 record fields was read per triple, the tent's three parts were walked
+// apart and bins were read one by one; 768 faces x 143 x 35 points: 76 against 458
+// us, of which one face per CTA instead of 8 gave 368 (96 CTAs before).
 constexpr int kFaceSlice = 256;
-constexpr int kFacesPerCta = 8;
+constexpr int kFacesPerCta = 1;
 // Most bytes of one bins-last copy of transient_grad (a range of scan points
 // of one batch item; launch_exhaustive_grad).
 constexpr size_t kGradChunkBytes = size_t(2) << 30;
-constexpr int kRec = 24;  // floats per point record (fields below)
+constexpr int kRec = 28;  // floats per point record (fields below; 28 keeps 16-byte reads of
+                          // 8 neighbouring records on distinct banks)
 enum : int {
   kRecD = 0,     // [3] exact FP32 lengths
-  kRecDlo = 3,   // [3] their low parts
-  kRecOd = 6,    // origin term, FP32
-  kRecOdlo = 7,  // its low part
-  kRecA = 8,     // alpha factor
-  kRecCm = 9,    // [3]
-  kRecWv = 12,   // [3]
-  kRecU = 15,    // [9] unit vectors u_m
+  kRecA = 3,     // alpha factor
+  kRecDlo = 4,   // [3] the lengths' low parts
+  kRecOdlo = 7,  // the origin term's low part
+  kRecCm = 8,    // [3]
+  kRecWv = 11,   // [3]
+  kRecU = 14,    // [9] unit vectors u_m
+  kRecOd = 23,   // origin term, FP32
+  kRecAt = 24,   // the point's index (int)
 };
 
 // Fills the record of point p (origin o if has_o) for the face (v, c, n);
-// rec[f * stride] is field f.
+// rec[f] is field f.
 __device__ __forceinline__ void exh_point_record(const fv3 v[3], fv3 c, fv3 n, fv3 p, bool has_o,
-                                                 fv3 o, float* rec, int stride) {
+                                                 fv3 o, float* rec) {
 #pragma unroll
   for (int m = 0; m < 3; ++m) {
     const float d = xlen(xsub3(v[m], p));
     const DFloat df = len_df(v[m], p);
-    rec[(kRecD + m) * stride] = d;
-    rec[(kRecDlo + m) * stride] = (df.hi - d) + df.lo;
+    rec[kRecD + m] = d;
+    rec[kRecDlo + m] = (df.hi - d) + df.lo;
     const float inv = vdiv(1.f, d);
     const fv3 u = inv * (v[m] - p);
-    rec[(kRecU + 3 * m) * stride] = u.x;
-    rec[(kRecU + 3 * m + 1) * stride] = u.y;
-    rec[(kRecU + 3 * m + 2) * stride] = u.z;
+    rec[kRecU + 3 * m] = u.x;
+    rec[kRecU + 3 * m + 1] = u.y;
+    rec[kRecU + 3 * m + 2] = u.z;
   }
   float od = 0.f, odlo = 0.f;
   if (has_o) {
@@ -547,20 +559,20 @@ __device__ __forceinline__ void exh_point_record(const fv3 v[3], fv3 c, fv3 n, f
     const DFloat df = len_df(p, o);
     odlo = (df.hi - od) + df.lo;
   }
-  rec[kRecOd * stride] = od;
-  rec[kRecOdlo * stride] = odlo;
+  rec[kRecOd] = od;
+  rec[kRecOdlo] = odlo;
   const fv3 r = c - p;
   const float rr = dot(r, r), nr = dot(n, r);
   const bool front = r.z > 0.f;
-  rec[kRecA * stride] = front ? vdiv(r.z * fabsf(nr), rr * rr) : 0.f;
+  rec[kRecA] = front ? vdiv(r.z * fabsf(nr), rr * rr) : 0.f;
   const float kr = vdiv(-4.f, 3.f * rr), knr = vdiv(1.f, nr), kw = vdiv(1.f, 3.f * r.z);
   const fv3 cm = kr * r + (knr * (1.f / 3.f)) * n + mkv(0.f, 0.f, front ? kw : 0.f);
-  rec[kRecCm * stride] = cm.x;
-  rec[(kRecCm + 1) * stride] = cm.y;
-  rec[(kRecCm + 2) * stride] = cm.z;
-  rec[kRecWv * stride] = knr * r.x;
-  rec[(kRecWv + 1) * stride] = knr * r.y;
-  rec[(kRecWv + 2) * stride] = knr * r.z;
+  rec[kRecCm] = cm.x;
+  rec[kRecCm + 1] = cm.y;
+  rec[kRecCm + 2] = cm.z;
+  rec[kRecWv] = knr * r.x;
+  rec[kRecWv + 1] = knr * r.y;
+  rec[kRecWv + 2] = knr * r.z;
 }
 
 // Block-wide compaction: returns this thread's slot among the threads whose
@@ -580,22 +592,108 @@ __device__ __forceinline__ int block_slot(bool flag, int* warp_counts, int* tota
   return flag ? base + __popc(bal & ((1u << lane) - 1u)) : -1;
 }
 
-template <int kOcc>
+// tent_grad and the vertices' tent weights {part0, gs0, gs1, gs2} from sums over
+// the bins: with t the distance of a bin's edges from the first foot, cut to the
+// rising side, W1 = sum g (t1 - t0) and M1 = sum g (t1^2 - t0^2), and W2, M2
+// likewise from the second foot. At a bin's edges the area of a side moves with
+// its foot and slope alone; the moves of the peak within its bin cancel between
+// the sides. Coordinates truncate toward zero, so bin 0 reaches back to a corner
+// in (-1, 0), and where the first foot is in a bin below 0 the sides are cut at 0,
+// each if its peak is (tent_grad's terms).
+// kLast: the column's bins lie side by side (bstep 1) in rows of a multiple of 4
+// bins on 16-byte boundaries, read four at a time: 32 columns are 32 cache lines,
+// and an access costs the same for one bin or four.
+template <bool kLast>
+__device__ __forceinline__ float4 tent_weights(const float* __restrict__ col, int64_t stride,
+                                               int T, float x0, float x1, float x2, int b0,
+                                               int b1, int b2, float inv_bw) {
+  const float d1 = x1 - x0, d2 = x2 - x1;
+  const unsigned long long feet = f2pack(-x0, x2);
+  const int first = max(b0, 0), last = min(b2, T - 1);
+  // the lower edge of the first bin, clamped to the sides
+  const float e0 = (float)(first - b0);
+  unsigned long long from =
+      f2pack(b0 >= 0 ? 0.f : (b1 < 0 ? d1 : e0 - x0), b1 < 0 ? x2 - e0 : d2);
+  const int start = kLast ? first & ~3 : first;
+  const float es = (float)(start - b0);
+  unsigned long long edge = f2pack(es, -es), W = 0ull, M = 0ull;
+  auto four = [&](const float g[4], int i, int skip) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      edge = f2add(edge, f2pack(1.f, -1.f));
+      float t, u;
+      f2unpack(f2add(edge, feet), t, u);
+      // (the decided bins say where a side ends: a corner rounded across an edge
+      // stays in its bin)
+      const bool past = i + k >= b1;
+      const unsigned long long to =
+          f2pack(past ? d1 : t, past ? (i + k >= b2 ? 0.f : u) : d2);
+      if (kLast && k < 3 && k < skip) continue;  // (before the first bin)
+      // (t1 - t0, u1 - u0: the falling side's sums come out negated)
+      const unsigned long long gw = f2mul(f2pack(g[k], g[k]), f2sub(to, from));
+      W = f2add(W, gw);
+      M = f2fma(gw, f2add(to, from), M);
+      from = to;
+    }
+  };
+  auto load = [&](int i, float g[4]) {  // bins i .. i + 3, zero past the last one
+    if (kLast) {
+      const float4 q = __ldg(reinterpret_cast<const float4*>(col + i));
+      g[0] = i <= last ? q.x : 0.f;
+      g[1] = i + 1 <= last ? q.y : 0.f;
+      g[2] = i + 2 <= last ? q.z : 0.f;
+      g[3] = i + 3 <= last ? q.w : 0.f;
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        g[k] = i + k <= last ? __ldg(col + (int64_t)(i + k) * stride) : 0.f;
+    }
+  };
+  float g[4];
+  load(start, g);
+  int skip = first - start;
+  for (int i = start;;) {
+    float next[4] = {0.f, 0.f, 0.f, 0.f};
+    const bool more = i + 4 <= last;
+    if (more) load(i + 4, next);  // in flight over the four bins at hand
+    four(g, i, skip);
+    if (!more) break;
+    i += 4;
+    skip = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) g[k] = next[k];
+  }
+  float W1, W2, M1, M2;
+  f2unpack(W, W1, W2);
+  f2unpack(M, M1, M2);
+  const float is = vdiv(1.f, x2 - x0), i1 = vdiv(1.f, d1), i2 = vdiv(1.f, d2);
+  float f1 = W1 * i1, h1 = 0.5f * M1 * i1, e1 = h1 * i1;
+  float f2 = -W2 * i2, h2 = -0.5f * M2 * i2, e2 = h2 * i2;
+  const bool no1 = !(fabsf(d1) > 1e-15f), no2 = !(fabsf(d2) > 1e-15f);
+  if (no1 || no2) {  // a side of no width: all in the peak's bin
+    const float gp = b1 >= 0 && b1 < T ? __ldg(col + (int64_t)b1 * stride) : 0.f;
+    if (no1) f1 = gp, h1 = 0.f, e1 = 0.5f * gp;
+    if (no2) f2 = gp, h2 = 0.f, e2 = 0.5f * gp;
+  }
+  const float S = h1 + h2, yc = 2.f * is, k = yc * inv_bw;
+  return make_float4(yc * S, k * ((e1 - f1) + S * is), k * (e2 - e1), k * ((f2 - e2) - S * is));
+}
+
+template <int kOcc, bool kLast>
 __global__ void __launch_bounds__(256, kOcc) exh_grad_face_kernel(
     Scene sc, View3f sp, View3f lp, Origins org, int S, int L, const float* __restrict__ tgrad,
-    int T, float bw, float bo, GradOut out, int faces_per_cta, int lchunk, int sslice, int b0,
-    int s_base, int s_end, int64_t bstride, int64_t cstep, int64_t bstep) {
+    int T, float bw, float bo, int fixed, GradOut out, int faces_per_cta, int lchunk, int sslice,
+    int b0, int s_base, int s_end, int64_t bstride, int64_t cstep, int64_t bstep) {
   // Batch item b0 + blockIdx.y, scan points [s_base, s_end); transient_grad
   // element (t, s, l) of item b is tgrad[(b - b0) bstride + ((s - s_base) L +
   // l) cstep + t bstep]: the caller's [B, T, S, L] tensor (b0 = s_base = 0,
   // bstride = T S L, cstep = 1, bstep = S L) or one item's bins-last copy of
   // a range of scan points (cstep = T, bstep = 1).
-  extern __shared__ float recs[];        // scan-point then laser-point records, SoA
-  float* srec = recs;
-  float* lrec = recs + kRec * kFaceSlice;
-  __shared__ short sidx[kFaceSlice], lidx[kFaceSlice];
+  extern __shared__ float4 recs4[];  // scan-point then laser-point records
+  float* srec = reinterpret_cast<float*>(recs4);
+  float* lrec = srec + kRec * kFaceSlice;
   __shared__ int counts[2][8];
-  __shared__ float red[8][10];
+  __shared__ float red[8][16], tot[16];
   const int b = b0 + blockIdx.y;
   const int n = sc.meta[b].n;
   const int nlc = (L + lchunk - 1) / lchunk;
@@ -604,10 +702,10 @@ __global__ void __launch_bounds__(256, kOcc) exh_grad_face_kernel(
   const int la = (blockIdx.z % nlc) * lchunk, lb = min(L, la + lchunk);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float* tgb = tgrad + (int64_t)(b - b0) * bstride;
-  const int64_t stride = bstep;
   const float4* shade = sc.shade + (size_t)b * sc.F * 4;
   const uint32_t* mrows = sc.mask + (size_t)b * sc.P * sc.nch;
   const float inv_bw = __frcp_rn(bw);
+  const bool plain = !org.has_so && !org.has_lo && bo == 0.f;  // nothing added to a path
   for (int fi = 0; fi < faces_per_cta; ++fi) {
     const int k = blockIdx.x * faces_per_cta + fi;
     if (k >= n) break;  // CTA-uniform
@@ -615,12 +713,9 @@ __global__ void __launch_bounds__(256, kOcc) exh_grad_face_kernel(
     const float4 s2r = __ldg(shade + 4 * k + 2), s3r = __ldg(shade + 4 * k + 3);
     const fv3 v[3] = {mkv(s0r.x, s0r.y, s0r.z), mkv(s1r.x, s1r.y, s1r.z), mkv(s2r.x, s2r.y, s2r.z)};
     const fv3 c = mkv(s3r.x, s3r.y, s3r.z);
-    const fv3 e1 = v[1] - v[0], e2 = v[2] - v[0];
-    const fv3 nrm = cross(e1, e2);
+    const fv3 nrm = cross(v[1] - v[0], v[2] - v[0]);
     const float nn = dot(nrm, nrm);
-    const float rho = s0r.w;
-    const float kf = 100.f * rho * rsqrtf(nn);
-    const fv3 wf = vdiv(-1.f, nn) * nrm;
+    const float kf = 100.f * s0r.w * rsqrtf(nn);
     const int ch = k >> 5;
     const uint32_t bit = 1u << (k & 31);
     // the face's scan-point records over this slice
@@ -633,13 +728,14 @@ __global__ void __launch_bounds__(256, kOcc) exh_grad_face_kernel(
         const fv3 p = mkv(sp.at(b, s, 0), sp.at(b, s, 1), sp.at(b, s, 2));
         const fv3 o = org.has_so ? mkv(org.so.at(b, s, 0), org.so.at(b, s, 1), org.so.at(b, s, 2))
                                  : mkv(0.f, 0.f, 0.f);
-        exh_point_record(v, c, nrm, p, org.has_so, o, srec + at, kFaceSlice);
-        sidx[at] = (short)tid;
+        exh_point_record(v, c, nrm, p, org.has_so, o, srec + at * kRec);
+        srec[at * kRec + kRecAt] = __int_as_float(s - s_base);
       }
     }
-    float acc[10];
+    // pairs of sum P cm [3], sum P wv [3], sum Q_m u_m [9], sum P
+    unsigned long long acc[8];
 #pragma unroll
-    for (int q = 0; q < 10; ++q) acc[q] = 0.f;
+    for (int q = 0; q < 8; ++q) acc[q] = 0ull;
     for (int l0 = la; l0 < lb && ns > 0; l0 += kFaceSlice) {
       int nl;
       {
@@ -651,137 +747,196 @@ __global__ void __launch_bounds__(256, kOcc) exh_grad_face_kernel(
           const fv3 p = mkv(lp.at(b, l, 0), lp.at(b, l, 1), lp.at(b, l, 2));
           const fv3 o = org.has_lo ? mkv(org.lo.at(b, l, 0), org.lo.at(b, l, 1), org.lo.at(b, l, 2))
                                    : mkv(0.f, 0.f, 0.f);
-          exh_point_record(v, c, nrm, p, org.has_lo, o, lrec + at, kFaceSlice);
-          lidx[at] = (short)tid;
+          exh_point_record(v, c, nrm, p, org.has_lo, o, lrec + at * kRec);
+          lrec[at * kRec + kRecAt] = __int_as_float(l);
         }
       }
       __syncthreads();
-      const int pairs = ns * nl;
-      // pair index tid + 256 t walks (si, li) with li fastest
-      int si = nl > 0 ? tid / nl : 0, li = nl > 0 ? tid - si * nl : 0;
-      const int dq = nl > 0 ? 256 / nl : 0, dr = nl > 0 ? 256 - dq * nl : 0;
-      for (int pi = tid; pi < pairs; pi += 256) {
-        const float* rs = srec + si;
-        const float* rl = lrec + li;
-        const int s = s0 + sidx[si], l = l0 + lidx[li];
-        li += dr;
-        si += dq;
-        if (li >= nl) {
-          li -= nl;
-          ++si;
-        }
-        const float as = rs[kRecA * kFaceSlice], al = rl[kRecA * kFaceSlice];
-        const float alpha = kf * as * al;
-        if (!(alpha > 0.f)) continue;
-        float d[3];
-#pragma unroll
-        for (int m = 0; m < 3; ++m)
-          d[m] = xadd(rs[(kRecD + m) * kFaceSlice], rl[(kRecD + m) * kFaceSlice]);
-        // the vertex order of exh_sort (stable compare-swaps on the path length)
-        int p0 = 0, p1 = 1, p2 = 2;
-        float d0 = d[0], d1 = d[1], d2 = d[2];
-        if (d0 > d1) { float t = d0; d0 = d1; d1 = t; int u = p0; p0 = p1; p1 = u; }
-        if (d1 > d2) { float t = d1; d1 = d2; d2 = t; int u = p1; p1 = p2; p2 = u; }
-        if (d0 > d1) { float t = d0; d0 = d1; d1 = t; int u = p0; p0 = p1; p1 = u; }
-        const float ods = rs[kRecOd * kFaceSlice], odl = rl[kRecOd * kFaceSlice];
-        const float od = xadd(ods, odl);
-        int bin[3];
-        bin[0] = bin_of(xdiv(xsub(xadd(d0, od), bo), bw));
-        bin[1] = bin_of(xdiv(xsub(xadd(d1, od), bo), bw));
-        bin[2] = bin_of(xdiv(xsub(xadd(d2, od), bo), bw));
-        if (bin[0] >= T || bin[2] < 0) continue;
-        const float* col = tgb + ((int64_t)(s - s_base) * L + l) * cstep;
-        fv3 da[3];
-        {
-          const fv3 w = wf + mkv(rs[kRecWv * kFaceSlice], rs[(kRecWv + 1) * kFaceSlice],
-                                 rs[(kRecWv + 2) * kFaceSlice]) +
-                        mkv(rl[kRecWv * kFaceSlice], rl[(kRecWv + 1) * kFaceSlice],
-                            rl[(kRecWv + 2) * kFaceSlice]);
-          const fv3 cm = mkv(rs[kRecCm * kFaceSlice] + rl[kRecCm * kFaceSlice],
-                             rs[(kRecCm + 1) * kFaceSlice] + rl[(kRecCm + 1) * kFaceSlice],
-                             rs[(kRecCm + 2) * kFaceSlice] + rl[(kRecCm + 2) * kFaceSlice]);
-          const fv3 g1 = cross(e2, w), g2 = cross(w, e1);
-          da[0] = alpha * (cm - g1 - g2);
-          da[1] = alpha * (cm + g1);
-          da[2] = alpha * (cm + g2);
-        }
-        const float dadm = vdiv(alpha, rho);
-        if (bin[0] == bin[2]) {
-          const float g = __ldg(col + (int64_t)bin[0] * stride);
-#pragma unroll
-          for (int m = 0; m < 3; ++m) {
-            acc[3 * m] += g * da[m].x;
-            acc[3 * m + 1] += g * da[m].y;
-            acc[3 * m + 2] += g * da[m].z;
+      // The lanes take the points that fill the last warp row better; laser points
+      // unless that is a third worse where their bins lie side by side.
+      const int gs = (ns + 31) >> 5, gl = (nl + 31) >> 5;
+      const bool over_s = kLast ? ns * gl >= nl * gs : 3 * ns * gl > 4 * nl * gs;
+      const float* mine = over_s ? srec : lrec;
+      const float* other = over_s ? lrec : srec;
+      const int nm = over_s ? ns : nl, no = over_s ? nl : ns, gm = over_s ? gs : gl;
+      const int64_t mstep = (over_s ? (int64_t)L : 1) * cstep;
+      const int64_t ostep = (over_s ? 1 : (int64_t)L) * cstep;
+      // rows (32 points of one side, one point of the other), split over the warps
+      int r = (int)((int64_t)warp * gm * no / 8);
+      const int r_end = (int)((int64_t)(warp + 1) * gm * no / 8);
+      while (r < r_end) {
+        const int grp = r / no;
+        int j = r - grp * no;
+        const int j_end = min(no, j + r_end - r);
+        r += j_end - j;
+        const int i = grp * 32 + lane;
+        const float* rm = mine + min(i, nm - 1) * kRec;
+        const float4 m0 = *reinterpret_cast<const float4*>(rm);      // D, A
+        const float4 m1 = *reinterpret_cast<const float4*>(rm + 4);  // Dlo, odlo
+        const float mod = rm[kRecOd];
+        const float am = i < nm ? m0.w * kf : 0.f;
+        const float* colm = tgb + __float_as_int(rm[kRecAt]) * mstep;
+        float gP = 0.f, gQ0 = 0.f, gQ1 = 0.f, gQ2 = 0.f;
+        bool used = false;
+        for (; j < j_end; ++j) {
+          const float* ro = other + j * kRec;
+          const float4 o0 = *reinterpret_cast<const float4*>(ro);
+          const float alpha = am * o0.w;
+          if (!(alpha > 0.f)) continue;
+          const float4 o1 = *reinterpret_cast<const float4*>(ro + 4);
+          // path lengths: hi is the FP32 chain's sum, lo what it rounds off
+          DFloat e0 = two_sum(m0.x, o0.x), e1 = two_sum(m0.y, o0.y), e2 = two_sum(m0.z, o0.z);
+          e0.lo += m1.x + o1.x;
+          e1.lo += m1.y + o1.y;
+          e2.lo += m1.z + o1.z;
+          // the vertex order of exh_sort (stable compare-swaps on the path length)
+          auto swap_if = [](bool y, DFloat& a, DFloat& z) {
+            const DFloat t = a;
+            a.hi = y ? z.hi : a.hi;
+            a.lo = y ? z.lo : a.lo;
+            z.hi = y ? t.hi : z.hi;
+            z.lo = y ? t.lo : z.lo;
+          };
+          const bool y0 = e0.hi > e1.hi;
+          swap_if(y0, e0, e1);
+          const bool y1 = e1.hi > e2.hi;
+          swap_if(y1, e1, e2);
+          const bool y2 = e0.hi > e1.hi;
+          swap_if(y2, e0, e1);
+          if (!plain) {
+            const float ood = ro[kRecOd];
+            const DFloat od = df_add(DFloat{mod, m1.w}, DFloat{ood, o1.w});
+            auto add = [&](DFloat& e) {
+              e = df_add(e, od);
+              const DFloat f = two_sum(e.hi, -bo);
+              e.hi = f.hi;
+              e.lo += f.lo;
+            };
+            add(e0);
+            add(e1);
+            add(e2);
           }
-          acc[9] += g * dadm;
-          continue;
+          float c0, c1, c2;
+          if (fixed) {
+            c0 = div_fixed(e0.hi, bw, inv_bw);
+            c1 = div_fixed(e1.hi, bw, inv_bw);
+            c2 = div_fixed(e2.hi, bw, inv_bw);
+          } else {
+            c0 = xdiv(e0.hi, bw);
+            c1 = xdiv(e1.hi, bw);
+            c2 = xdiv(e2.hi, bw);
+          }
+          auto bin = [](float x) { return __float2int_rz(fminf(fmaxf(x, -1.0e9f), 1.0e9f)); };
+          const int b0c = bin(c0), b1c = bin(c1), b2c = bin(c2);
+          if (b0c >= T || b2c < 0) continue;
+          const float* col = colm + __float_as_int(ro[kRecAt]) * ostep;
+          float4 w;  // area, weights of the sorted vertices
+          if (b0c == b2c) {
+            w = make_float4(__ldg(col + (int64_t)b0c * bstep), 0.f, 0.f, 0.f);
+          } else {
+            // corners relative to the first bin (bin_offset)
+            const float base = (float)b0c;
+            auto rel = [&](float cc, DFloat e) {
+              return fmaf(__fmaf_rn(-cc, bw, e.hi) + e.lo, inv_bw, cc - base);
+            };
+            const float x0 = rel(c0, e0), x1 = rel(c1, e1), x2 = rel(c2, e2);
+            w = tent_weights<kLast>(col, bstep, T, x0, x1, x2, b0c, b1c, b2c, inv_bw);
+          }
+          // back to the face's own order
+          auto swap_back = [](bool y, float& a, float& z) {
+            const float t = a;
+            a = y ? z : a;
+            z = y ? t : z;
+          };
+          swap_back(y2, w.y, w.z);
+          swap_back(y1, w.z, w.w);
+          swap_back(y0, w.y, w.z);
+          const float P = alpha * w.x, Q0 = alpha * w.y, Q1 = alpha * w.z, Q2 = alpha * w.w;
+          used = true;
+          gP += P;
+          gQ0 += Q0;
+          gQ1 += Q1;
+          gQ2 += Q2;
+          const ulonglong2 o2 = *reinterpret_cast<const ulonglong2*>(ro + 8);   // cm, wv
+          const ulonglong2 o3 = *reinterpret_cast<const ulonglong2*>(ro + 12);  // wv, u
+          const ulonglong2 o4 = *reinterpret_cast<const ulonglong2*>(ro + 16);
+          const ulonglong2 o5 = *reinterpret_cast<const ulonglong2*>(ro + 20);  // u, od
+          const unsigned long long PP = f2pack(P, P), Q00 = f2pack(Q0, Q0), Q11 = f2pack(Q1, Q1);
+          const unsigned long long Q22 = f2pack(Q2, Q2);
+          acc[0] = f2fma(PP, o2.x, acc[0]);
+          acc[1] = f2fma(PP, o2.y, acc[1]);
+          acc[2] = f2fma(PP, o3.x, acc[2]);
+          acc[3] = f2fma(Q00, o3.y, acc[3]);
+          acc[4] = f2fma(f2pack(Q0, Q1), o4.x, acc[4]);
+          acc[5] = f2fma(Q11, o4.y, acc[5]);
+          acc[6] = f2fma(Q22, o5.x, acc[6]);
+          float u8, ood;
+          f2unpack(o5.y, u8, ood);
+          acc[7] = f2fma(f2pack(Q2, P), f2pack(u8, 1.f), acc[7]);
         }
-        // double-float path lengths of the three vertices, then the corners
-        // of the sorted ones relative to bin[0]
-        const DFloat odf = df_add(DFloat{ods, rs[kRecOdlo * kFaceSlice]},
-                                  DFloat{odl, rl[kRecOdlo * kFaceSlice]});
-        float xo[3];
-#pragma unroll
-        for (int m = 0; m < 3; ++m) {
-          const DFloat path =
-              df_add(df_add(DFloat{rs[(kRecD + m) * kFaceSlice], rs[(kRecDlo + m) * kFaceSlice]},
-                            DFloat{rl[(kRecD + m) * kFaceSlice], rl[(kRecDlo + m) * kFaceSlice]}),
-                     odf);
-          xo[m] = bin_offset(path, bo, bw, inv_bw, bin[0]);
+        if (used) {  // this lane's own point
+          const unsigned long long PP = f2pack(gP, gP);
+          const ulonglong2* q = reinterpret_cast<const ulonglong2*>(rm + 8);
+          acc[0] = f2fma(PP, q[0].x, acc[0]);
+          acc[1] = f2fma(PP, q[0].y, acc[1]);
+          acc[2] = f2fma(PP, q[1].x, acc[2]);
+          acc[3] = f2fma(f2pack(gQ0, gQ0), q[1].y, acc[3]);
+          acc[4] = f2fma(f2pack(gQ0, gQ1), q[2].x, acc[4]);
+          acc[5] = f2fma(f2pack(gQ1, gQ1), q[2].y, acc[5]);
+          acc[6] = f2fma(f2pack(gQ2, gQ2), q[3].x, acc[6]);
+          acc[7] = f2fma(f2pack(gQ2, 0.f), f2pack(rm[kRecU + 8], 0.f), acc[7]);
         }
-        auto pick = [](const float a[3], int i) { return i == 0 ? a[0] : (i == 1 ? a[1] : a[2]); };
-        const float x[3] = {pick(xo, p0), pick(xo, p1), pick(xo, p2)};
-        TentGrad tgr;
-        tent_grad(col, stride, T, x, bin, tgr);
-        const float span = x[2] - x[0];
-        const float kk = vdiv(-2.f, bw * span * span);
-        // tent terms per sorted position: gamma_k u_(perm k), u = u_s + u_l
-        const float gs0 = vdiv(tgr.a0, bw) - tgr.ayc * kk, gs1 = vdiv(tgr.a1, bw);
-        const float gs2 = vdiv(tgr.a2, bw) + tgr.ayc * kk;
-#pragma unroll
-        for (int m = 0; m < 3; ++m) {
-          const float gm = m == p0 ? gs0 : (m == p1 ? gs1 : gs2);
-          const float ag = alpha * gm;
-          const fv3 u = mkv(rs[(kRecU + 3 * m) * kFaceSlice] + rl[(kRecU + 3 * m) * kFaceSlice],
-                            rs[(kRecU + 3 * m + 1) * kFaceSlice] +
-                                rl[(kRecU + 3 * m + 1) * kFaceSlice],
-                            rs[(kRecU + 3 * m + 2) * kFaceSlice] +
-                                rl[(kRecU + 3 * m + 2) * kFaceSlice]);
-          acc[3 * m] += tgr.part0 * da[m].x + ag * u.x;
-          acc[3 * m + 1] += tgr.part0 * da[m].y + ag * u.y;
-          acc[3 * m + 2] += tgr.part0 * da[m].z + ag * u.z;
-        }
-        acc[9] += dadm * tgr.part0;
       }
       __syncthreads();  // records are rewritten for the next laser chunk / face
     }
-    // the face's gradient: warp sums, then one thread per vertex component
+    if (ns > 0) {  // CTA-uniform
+      // the face's sums, then one thread per vertex component
 #pragma unroll
-    for (int q = 0; q < 10; ++q) {
-      const float t = warp_sum(acc[q]);
-      if (lane == 0) red[warp][q] = t;
-    }
-    __syncthreads();
-    if (tid < 10 && ns > 0) {
-      float t = 0.f;
-      for (int w = 0; w < 8; ++w) t += red[w][tid];
+      for (int q = 0; q < 8; ++q) {
+        float x, y;
+        f2unpack(acc[q], x, y);
+        x = warp_sum(x);
+        y = warp_sum(y);
+        if (lane == 0) {
+          red[warp][2 * q] = x;
+          red[warp][2 * q + 1] = y;
+        }
+      }
+      __syncthreads();
+      if (tid < 16) {
+        float t = 0.f;
+        for (int w = 0; w < 8; ++w) t += red[w][tid];
+        tot[tid] = t;
+      }
+      __syncthreads();
       const int vi[3] = {__float_as_int(s1r.w), __float_as_int(s2r.w), __float_as_int(s3r.w)};
       if (tid < 9) {
         const int m = tid / 3, a = tid - 3 * m;
+        // d alpha: w = sum P (wf + wv), wf = -n / |n|^2, through the normal's Jacobian
+        const fv3 w = (vdiv(-1.f, nn) * tot[15]) * nrm + mkv(tot[3], tot[4], tot[5]);
+        const fv3 g1 = cross(v[2] - v[0], w), g2 = cross(w, v[1] - v[0]);
+        const fv3 g = m == 0 ? -(g1 + g2) : (m == 1 ? g1 : g2);
+        const float t = tot[a] + (a == 0 ? g.x : (a == 1 ? g.y : g.z)) + tot[6 + tid];
         if (vi[m] < 0 || vi[m] >= out.V) {
           atomicOr(sc.status, kStatusFaceIndexRange);
         } else if (out.vg) {
           atomicAdd(out.vg + b * out.vsb + vi[m] * out.vsv + a * out.vsc, t);
         }
-      } else if (out.mg) {
+      } else if (tid == 9 && out.mg) {
+        const float t = vdiv(tot[15], s0r.w);
         for (int m = 0; m < 3; ++m)
           if (vi[m] >= 0 && vi[m] < out.V)
             atomicAdd(out.mg + b * out.msb + vi[m] * out.msv, (1.f / 3.f) * t);
       }
+      __syncthreads();
     }
-    __syncthreads();
   }
+}
+
+// Whether bin coordinates may take div_fixed: any path length then either has a
+// coordinate in its range or an alpha of zero.
+static bool fixed_division(float bw, float bo) {
+  return bw >= 0x1p-60f && bw <= 0x1p60f && std::fabs(bo) <= 0x1p60f;
 }
 
 template <int LT>
@@ -880,11 +1035,11 @@ int launch_exhaustive_splat(const Scene& sc, const View3f& sp, const View3f& lp,
   return fail(TOTRI_ERR_UNSUPPORTED, "number of bins too large for the shared-memory tile");
 }
 
-// out[c][t] = in[t row + c] for c < n, t < T: a [T][n] block of rows of
-// length `row` into bins-last order, through 32 x 32 tiles in shared memory
+// out[c Tp + t] = in[t row + c] for c < n, t < T: a [T][n] block of rows of
+// length `row` into bins-last order (rows of Tp >= T), through 32 x 32 tiles in shared memory
 // (coalesced reads and writes).
 __global__ void __launch_bounds__(256) bins_last_kernel(const float* __restrict__ in,
-                                                        float* __restrict__ out, int T,
+                                                        float* __restrict__ out, int T, int Tp,
                                                         int64_t row, int64_t n) {
   __shared__ float tile[32][33];
   const int64_t c0 = (int64_t)blockIdx.x * 32;
@@ -900,15 +1055,15 @@ __global__ void __launch_bounds__(256) bins_last_kernel(const float* __restrict_
   for (int r = threadIdx.y; r < 32; r += 8) {
     const int64_t c = c0 + r;
     const int t = t0 + threadIdx.x;
-    if (t < T && c < n) dst[c * T + t] = tile[threadIdx.x][r];
+    if (t < T && c < n) dst[c * Tp + t] = tile[threadIdx.x][r];
   }
 }
 
-int launch_bins_last(const float* in, float* out, int T, int64_t row, int64_t n,
+int launch_bins_last(const float* in, float* out, int T, int Tp, int64_t row, int64_t n,
                      cudaStream_t stream) {
   TOTRI_KERNEL("mesh grad layout", stream,
                bins_last_kernel<<<dim3((unsigned)ceil_div(n, 32), (unsigned)ceil_div(T, 32)),
-                                  dim3(32, 8), 0, stream>>>(in, out, T, row, n));
+                                  dim3(32, 8), 0, stream>>>(in, out, T, Tp, row, n));
   return TOTRI_OK;
 }
 
@@ -923,6 +1078,12 @@ int64_t exh_grad_chunk_points(int64_t S, int64_t L, int64_t T) {
 size_t exh_grad_scratch_bytes(int64_t S, int64_t L, int64_t T) {
   const int64_t c = exh_grad_chunk_points(S, L, T);
   return c > 0 ? align_up((size_t)c * (size_t)L * (size_t)T * sizeof(float), 256) : 0;
+}
+
+// The mesh gradient's copies have rows of a multiple of 4 bins.
+static int64_t padded_bins(int64_t T) { return (T + 3) & ~(int64_t)3; }
+size_t mesh_grad_scratch_bytes(int64_t S, int64_t L, int64_t T) {
+  return exh_grad_scratch_bytes(S, L, padded_bins(T));
 }
 
 int launch_exhaustive_grad(const Scene& sc, const View3f& sp, const View3f& lp,
@@ -945,32 +1106,28 @@ int launch_exhaustive_grad(const Scene& sc, const View3f& sp, const View3f& lp,
   // 32-mesh batch).
   const int mode = tune::get("mesh.exhaustive.grad.mode");
   if (mode != 1 && mode != 2) {
-    // "mesh.exhaustive.grad.faces": faces per CTA (default 8);
+    // "mesh.exhaustive.grad.faces": faces per CTA (default 1: within 2% of 2 and 8
+    // on 20,000 faces, 1.8 to 5 times faster than 8 on 500 and 1,500);
     // "mesh.exhaustive.grad.occupancy" = 4: registers capped for 4 CTAs per SM
     // (64, with spills) instead of 3 (80); "mesh.exhaustive.grad.sslice" /
     // ".lchunk": scan points / lasers per CTA.
     const int fpc = tune::get("mesh.exhaustive.grad.faces") > 0
                         ? (int)tune::get("mesh.exhaustive.grad.faces")
                         : kFacesPerCta;
+    const int fixed = fixed_division(bw, bo);
     const bool occ4 = tune::get("mesh.exhaustive.grad.occupancy") == 4;
-    const void* fn = occ4 ? reinterpret_cast<const void*>(exh_grad_face_kernel<4>)
-                          : reinterpret_cast<const void*>(exh_grad_face_kernel<3>);
     const size_t smem = sizeof(float) * 2 * kRec * kFaceSlice;
-    TOTRI_CUDA(tune::ensure_dynamic_smem(fn, smem));
     auto launch = [&](const float* tg, int lchunk, int sslice, int b0, int nb, int sa, int sb,
-                      int64_t bstride, int64_t cstep, int64_t bstep) -> int {
+                      int64_t bstride, int64_t cstep, int64_t bstep, bool last) -> int {
       const dim3 grid((unsigned)ceil_div(sc.F, fpc), (unsigned)nb,
                       (unsigned)(ceil_div(sb - sa, sslice) * ceil_div(L, lchunk)));
-      if (occ4)
-        TOTRI_KERNEL("mesh exhaustive grad", stream,
-                     exh_grad_face_kernel<4><<<grid, 256, smem, stream>>>(
-                         sc, sp, lp, org, S, L, tg, T, bw, bo, out, fpc, lchunk, sslice, b0, sa,
-                         sb, bstride, cstep, bstep));
-      else
-        TOTRI_KERNEL("mesh exhaustive grad", stream,
-                     exh_grad_face_kernel<3><<<grid, 256, smem, stream>>>(
-                         sc, sp, lp, org, S, L, tg, T, bw, bo, out, fpc, lchunk, sslice, b0, sa,
-                         sb, bstride, cstep, bstep));
+      auto* kern = last ? (occ4 ? exh_grad_face_kernel<4, true> : exh_grad_face_kernel<3, true>)
+                        : (occ4 ? exh_grad_face_kernel<4, false> : exh_grad_face_kernel<3, false>);
+      TOTRI_CUDA(tune::ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
+      TOTRI_KERNEL("mesh exhaustive grad", stream,
+                   kern<<<grid, 256, smem, stream>>>(sc, sp, lp, org, S, L, tg, T, bw, bo, fixed,
+                                                     out, fpc, lchunk, sslice, b0, sa, sb, bstride,
+                                                     cstep, bstep));
       return TOTRI_OK;
     };
     int lchunk = tune::get("mesh.exhaustive.grad.lchunk");
@@ -985,22 +1142,22 @@ int launch_exhaustive_grad(const Scene& sc, const View3f& sp, const View3f& lp,
     // 51.0 ms at 32x32 (copies included), with whole 256 x 256 tiles.
     // "mesh.exhaustive.grad.layout" = 2 reads transient_grad in place;
     // "mesh.exhaustive.grad.chunk" caps the scan points per copy.
-    int64_t cpts = exh_grad_chunk_points(S, L, T);
+    int64_t cpts = exh_grad_chunk_points(S, L, padded_bins(T));
     const int64_t cap = tune::get("mesh.exhaustive.grad.chunk");
     if (cap > 0) cpts = std::min(cpts, cap);
     if (tune::get("mesh.exhaustive.grad.layout") != 2 && cpts > 0 && scratch &&
-        scratch_bytes >= (size_t)cpts * L * T * sizeof(float)) {
+        scratch_bytes >= (size_t)cpts * L * padded_bins(T) * sizeof(float)) {
       if (lchunk <= 0 || lchunk > kFaceSlice) lchunk = kFaceSlice;
       if (sslice <= 0 || sslice > kFaceSlice) sslice = kFaceSlice;
       sslice = (int)std::min<int64_t>(sslice, cpts);
       float* copy = static_cast<float*>(scratch);
-      const int64_t row = (int64_t)S * L;
+      const int64_t row = (int64_t)S * L, Tp = padded_bins(T);
       for (int b = 0; b < sc.B; ++b)
         for (int64_t sa = 0; sa < S; sa += cpts) {
           const int64_t sb = std::min<int64_t>(S, sa + cpts), n = (sb - sa) * L;
-          TOTRI_TRY(launch_bins_last(tgrad + ((int64_t)b * T) * row + sa * L, copy, T, row, n,
+          TOTRI_TRY(launch_bins_last(tgrad + ((int64_t)b * T) * row + sa * L, copy, T, (int)Tp, row, n,
                                      stream));
-          TOTRI_TRY(launch(copy, lchunk, sslice, b, 1, (int)sa, (int)sb, 0, T, 1));
+          TOTRI_TRY(launch(copy, lchunk, sslice, b, 1, (int)sa, (int)sb, 0, Tp, 1, true));
         }
       return TOTRI_OK;
     }
@@ -1015,7 +1172,8 @@ int launch_exhaustive_grad(const Scene& sc, const View3f& sp, const View3f& lp,
     const bool wide_rows = (int64_t)S * L >= (int64_t)1 << 19;
     if (lchunk <= 0 || lchunk > kFaceSlice) lchunk = wide_rows ? 32 : kFaceSlice;
     if (sslice <= 0 || sslice > kFaceSlice) sslice = wide_rows ? 128 : kFaceSlice;
-    return launch(tgrad, lchunk, sslice, 0, sc.B, 0, S, (int64_t)T * S * L, 1, (int64_t)S * L);
+    return launch(tgrad, lchunk, sslice, 0, sc.B, 0, S, (int64_t)T * S * L, 1, (int64_t)S * L,
+                  false);
   }
   if (mode == 1) {
     const size_t smem = sizeof(uint32_t) * (size_t)(S + L);

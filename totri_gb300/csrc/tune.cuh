@@ -12,7 +12,7 @@
 //   "mesh.exhaustive.exact"     1: every exhaustive sample takes the exact chain
 //   "mesh.exhaustive.grad.mode" 1 per-lane mask tests, 2 compacted triples
 //                               (default: per-face point records)
-//   "mesh.exhaustive.grad.faces" faces per CTA of the point-record gradient (8)
+//   "mesh.exhaustive.grad.faces" faces per CTA of the point-record gradient (1)
 //   "mesh.exhaustive.grad.occupancy" 4: that kernel capped for 4 CTAs/SM (64
 //                               registers) instead of 3
 //   "mesh.exhaustive.grad.lchunk", ".sslice" lasers / scan points per CTA of the

@@ -494,7 +494,8 @@ int totri_volume_exhaustive_grad_volume_ws(const totri_array_t* tg,
       const dim3 grid((unsigned)blocks, (unsigned)ceil_div(sb - sa, per));
       if (chunk > 0) {
         float* copy = static_cast<float*>(ws);
-        TOTRI_TRY(mesh::launch_bins_last(tb + sa * L, copy, (int)T, row, (sb - sa) * L, stream));
+        TOTRI_TRY(mesh::launch_bins_last(tb + sa * L, copy, (int)T, (int)T, row, (sb - sa) * L,
+                                         stream));
         TOTRI_KERNEL("volume exhaustive adjoint", stream,
                      vexh::adjoint_kernel<<<grid, 256, 0, stream>>>(
                          g, b, sp, lp, (int)sa, (int)sb, per, copy, T, 1, out, accumulate));
