@@ -365,6 +365,25 @@ def _exhaustive(shape, seed):
 
 
 @pytest.mark.parametrize("shape", EXHAUSTIVE)
+@pytest.mark.parametrize("cols,window", [(8, 0), (8, 50), (32, 0), (32, 37), (32, 700)])
+def test_exhaustive_columns_edges(cuda_lib, shape, cols, window):
+    """Sums of a few FP32 terms of one sign per bin, as in the other exhaustive
+    renders, whose bound this is."""
+    from totri_gb300 import autotune
+    S, L, T, bw, bo, _ = shape
+    dev, ref = _exhaustive(shape, S + L)
+    out = torch.full((1, T, S, L), 5.0, device="cuda")
+    try:
+        autotune.set_tile("mesh.exhaustive.splat.columns", cols)
+        autotune.set_tile("mesh.exhaustive.splat.window", window)
+        R.mesh_exhaustive_forward(*dev, out, bw, bo, 0)
+    finally:
+        autotune.set_tile("mesh.exhaustive.splat.columns", 0)
+        autotune.set_tile("mesh.exhaustive.splat.window", 0)
+    assert rel(out[0].cpu().numpy(), oracle.mesh_exhaustive_forward(*ref)) < 1e-5
+
+
+@pytest.mark.parametrize("shape", EXHAUSTIVE)
 @pytest.mark.parametrize("layout", [0, 2])
 def test_exhaustive_grad_edges(cuda_lib, shape, layout):
     """Either side in the lanes, bins-last rows and the caller's order; the bound

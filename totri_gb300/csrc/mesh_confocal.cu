@@ -394,18 +394,6 @@ __global__ void __launch_bounds__(256, kOcc) visibility_queue_kernel(Scene sc, V
 
 constexpr int kListWarps = 4, kListFaces = 8, kListFrontier = 256, kListCand = 512;
 
-// Warp minimum / maximum of a float (redux.sync on floats, sm_100a and later).
-__device__ __forceinline__ float warp_min_f(float x) {
-  float r;
-  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ float warp_max_f(float x) {
-  float r;
-  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
-  return r;
-}
-
 // Visibility over dense wall grids, in two kernels.
 //
 // visibility_walk_kernel decides the targets seen from behind as

@@ -933,6 +933,287 @@ __global__ void __launch_bounds__(256, kOcc) exh_grad_face_kernel(
   }
 }
 
+// The bins [w0, w1) of one output column in shared memory: bin b at h[(b - w0) CT].
+template <int CT>
+struct Window {
+  float* h;
+  int w0, w1;
+  __device__ __forceinline__ int lo() const { return w0; }
+  __device__ __forceinline__ int hi() const { return w1; }
+  __device__ __forceinline__ bool in(int b) const { return b >= w0 && b < w1; }
+  __device__ __forceinline__ void add(int b, float v) const { atomicAdd(h + (b - w0) * CT, v); }
+};
+
+// splat_tent with one sum per bin: the rising and the falling side over the
+// bin's interval, relative to the tent's feet. Coordinates truncate toward zero:
+// bin 0 reaches back to a corner in (-1, 0), and where the first foot is in a bin
+// below 0 the sides are cut at 0, each if its peak is (splat_segment's terms).
+template <int CT>
+__device__ __forceinline__ void splat_tent_columns(const Window<CT>& w, float c0, float c1,
+                                                   float c2, float alpha) {
+  // (a NaN coordinate: a path length of NaN, in bin -1e9 as in bin_of's
+  // -2147483647 on no transient)
+  const int b0 = __float2int_rz(fminf(fmaxf(c0, -1.0e9f), 1.0e9f));
+  const int b2 = __float2int_rz(fminf(fmaxf(c2, -1.0e9f), 1.0e9f));
+  if (b0 >= w.w1 || b2 < w.w0) return;
+  if (b0 == b2) {
+    w.add(b0, alpha);
+    return;
+  }
+  const float d1 = c1 - c0, d2 = c2 - c1, span = c2 - c0;
+  // half slopes; a side narrower than 1e-12 bin has no area to speak of
+  const float hs1 = d1 > 1e-12f ? vdiv(alpha, span * d1) : 0.f;
+  const float hs2 = d2 > 1e-12f ? vdiv(-alpha, span * d2) : 0.f;
+  const int first = max(b0, w.w0), last = min(b2, w.w1 - 1);
+  const float e0 = (float)first;
+  // the bin's lower edge from the feet, clamped to the sides
+  const bool in1 = c1 > -1.f;  // the peak's bin is not below 0
+  unsigned long long from =
+      first > b0 && (b0 >= 0 || first > 0)
+          ? f2pack(fminf(e0 - c0, d1), fminf(fmaxf(c2 - e0, 0.f), d2))
+          : f2pack(b0 >= 0 ? 0.f : (in1 ? e0 - c0 : d1), in1 ? d2 : c2 - e0);
+  const unsigned long long feet = f2pack(-c0, c2);
+  unsigned long long edge = f2pack(e0, -e0);
+  float* at = w.h + (first - w.w0) * CT;
+  for (int i = first; i <= last; ++i, at += CT) {
+    edge = f2add(edge, f2pack(1.f, -1.f));
+    float t, u, up, down;
+    f2unpack(f2add(edge, feet), t, u);
+    const unsigned long long to = f2pack(fminf(t, d1), fminf(fmaxf(u, 0.f), d2));
+    // (the falling side's difference is negative, and so is its half slope)
+    f2unpack(f2mul(f2sub(to, from), f2add(to, from)), up, down);
+    atomicAdd(at, fmaf(up, hs1, down * hs2));
+    from = to;
+  }
+}
+
+// What a face adds to every pair of one wall point p: the squared distances of its
+// vertices and the point's factor of alpha, |n.r| r.z / |r|^4 with r = c - p.
+__device__ __forceinline__ float4 splat_record(fv3 v0, fv3 v1, fv3 v2, fv3 c, fv3 n, fv3 p) {
+  const fv3 r = c - p;
+  const float rr = dot(r, r);
+  const float a = r.z > 0.f ? vdiv(r.z * fabsf(dot(n, r)), rr * rr) : 0.f;
+  return make_float4(xlen2(v0 - p), xlen2(v1 - p), xlen2(v2 - p), a);
+}
+
+// Forward over CT output columns (s, l) per CTA: column = s L + l, the order of the
+// output's rows. A lane owns a column (with CT = 8, four lanes do), so the
+// adds of a warp never meet in a word; a warp walks its 32-face chunks, prepares
+// the faces that some column sees (vertices, centroid, normal, 100 rho / |n|) and,
+// for tiles over at most two scan points, those points' records, one face per
+// lane, and then takes the faces one by one with all lanes (four by four with CT =
+// 8). The columns' bins are a window [w0, w0 + W) of the T, W rows of shared
+// memory: where T > W the CTA first bounds each column's path lengths over the
+// chunks it sees, and walks the faces again for every further W bins.
+// Instruction issue bounds it (72% of the slots at 26 warps per SM): of 8.8 ms for
+// 20,000 faces x 400 x 144 points and 2,048 bins with 16 warps, the tents took 4.0
+// (1.1 of it the compare-and-swap of a float add in shared memory), the laser
+// records 1.9, the corners 0.9 and the rest 2.2), as it did the CTA per scan point
+// and 4 lasers (10.3 ms), whose lanes met in the same bins and computed both
+// points' lengths for every pair. 32 warps over one window of 1,024 bins (one CTA
+// per SM) take 7.8 ms, as fewer columns need a second pass. The coordinates are
+// exh_pair_filtered's, bit for bit; exact ones from a square root per length and
+// a fixed division were 0.5 ms faster, but moved single bins by 1e-3.
+constexpr int kColScan = 2;  // scan points with records prepared per face
+constexpr int kColStage = 32 * (16 + 4 * kColScan);  // floats per warp
+template <int CT, int kColWarps>
+__global__ void __launch_bounds__(32 * kColWarps, 32 / kColWarps) exh_splat_columns_kernel(
+    Scene sc, View3f sp, View3f lp, Origins org, int S, int L, float* __restrict__ out, int T,
+    float bw, float bo, FastBins fb, int W) {
+  extern __shared__ float4 smem4[];
+  __shared__ int range[2][CT];
+  __shared__ float spts[kColScan][3];
+  constexpr int G = 32 / CT;  // faces taken together
+  const int b = blockIdx.y;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int cl = lane & (CT - 1), grp = lane / CT;
+  const int64_t C = (int64_t)S * L;
+  const int64_t col0 = (int64_t)blockIdx.x * CT;
+  const bool ok = col0 + cl < C;
+  const int64_t col = ok ? col0 + cl : col0;
+  const int s_first = (int)(col0 / L);
+  const int s = (int)(col / L), l = (int)(col - (int64_t)s * L);
+  const bool tab = (int)((min(col0 + CT, C) - 1) / L) - s_first < kColScan;  // CTA-uniform
+  float4* stage = smem4 + warp * (kColStage / 4);
+  float* hist = reinterpret_cast<float*>(smem4 + kColWarps * (kColStage / 4));
+  const fv3 p = mkv(sp.at(b, s, 0), sp.at(b, s, 1), sp.at(b, s, 2));
+  const fv3 q = mkv(lp.at(b, l, 0), lp.at(b, l, 1), lp.at(b, l, 2));
+  const float od = origin_term(org, b, s, l, p, q);
+  if (threadIdx.x < kColScan) {
+    const int si = min(s_first + (int)threadIdx.x, S - 1);
+    for (int a = 0; a < 3; ++a) spts[threadIdx.x][a] = sp.at(b, si, a);
+  }
+  if (threadIdx.x < CT) {
+    range[0][threadIdx.x] = T;
+    range[1][threadIdx.x] = -1;
+  }
+  const int n = sc.meta[b].n;
+  const int nchu = (n + 31) >> 5;
+  const uint32_t* ms = sc.mask + ((size_t)b * sc.P + s) * sc.nch;
+  const uint32_t* ml = sc.mask + ((size_t)b * sc.P + S + l) * sc.nch;
+  const float4* shade = sc.shade + (size_t)b * sc.F * 4;
+  auto seen = [&](int ch) {  // the column's faces of a chunk
+    const uint32_t m = ok ? __ldg(ms + ch) & __ldg(ml + ch) : 0u;
+    return n - ch * 32 >= 32 ? m : m & ((1u << (n - ch * 32)) - 1u);
+  };
+  __syncthreads();
+  int w0 = 0, passes = 1;
+  if (T > W) {
+    int lo = T, hi = -1;
+    for (int ch = warp; ch < nchu; ch += kColWarps) {
+      const uint32_t bits = seen(ch);
+      if (!__any_sync(0xffffffffu, bits != 0u)) continue;
+      const int k = min(ch * 32 + lane, n - 1);
+      const float4 s0r = __ldg(shade + 4 * k), s1r = __ldg(shade + 4 * k + 1);
+      const float4 s2r = __ldg(shade + 4 * k + 2);
+      // the chunk's box (a face with a NaN coordinate adds nothing)
+      const float bx0 = warp_min_f(fminf(fminf(s0r.x, s1r.x), s2r.x));
+      const float by0 = warp_min_f(fminf(fminf(s0r.y, s1r.y), s2r.y));
+      const float bz0 = warp_min_f(fminf(fminf(s0r.z, s1r.z), s2r.z));
+      const float bx1 = warp_max_f(fmaxf(fmaxf(s0r.x, s1r.x), s2r.x));
+      const float by1 = warp_max_f(fmaxf(fmaxf(s0r.y, s1r.y), s2r.y));
+      const float bz1 = warp_max_f(fmaxf(fmaxf(s0r.z, s1r.z), s2r.z));
+      if (bits == 0u) continue;
+      auto near = [&](fv3 o) {
+        const float x = fmaxf(fmaxf(bx0 - o.x, o.x - bx1), 0.f);
+        const float y = fmaxf(fmaxf(by0 - o.y, o.y - by1), 0.f);
+        const float z = fmaxf(fmaxf(bz0 - o.z, o.z - bz1), 0.f);
+        return sqrtf(fmaf(x, x, fmaf(y, y, z * z)));
+      };
+      auto far = [&](fv3 o) {
+        const float x = fmaxf(bx1 - o.x, o.x - bx0), y = fmaxf(by1 - o.y, o.y - by0);
+        const float z = fmaxf(bz1 - o.z, o.z - bz0);
+        return sqrtf(fmaf(x, x, fmaf(y, y, z * z)));
+      };
+      // Each length and sum of the exact chain and of this one is within a few
+      // roundings of its value: 4e-6 of the terms and two bins cover them.
+      const float dn = near(p) + near(q), df = far(p) + far(q);
+      const float inv_bw = fb.inv_bw;
+      const float m = fmaf(4e-6f * inv_bw, df + od + fabsf(bo), 2.f);
+      const float clo = (dn + od - bo) * inv_bw - m, chi = (df + od - bo) * inv_bw + m;
+      // (NaN or infinite bounds: the whole range)
+      lo = min(lo, clo > 0.f ? (clo < (float)T ? (int)clo : T) : 0);
+      hi = max(hi, chi < (float)T ? (chi >= 0.f ? (int)chi : -1) : T - 1);
+    }
+    atomicMin(&range[0][cl], lo);
+    atomicMax(&range[1][cl], hi);
+    __syncthreads();
+    for (int i = 0; i < CT; ++i) {
+      const int bins = range[1][i] - range[0][i] + 1;
+      passes = max(passes, (bins + W - 1) / W);
+    }
+    w0 = range[0][cl];
+  }
+  for (int pass = 0; pass < passes; ++pass, w0 += W) {
+    for (int i = threadIdx.x; i < W * CT; i += blockDim.x) hist[i] = 0.f;
+    __syncthreads();
+    const Window<CT> win{hist + cl, w0, min(w0 + W, T)};
+    for (int ch = warp; ch < nchu; ch += kColWarps) {
+      const uint32_t bits = seen(ch);
+      uint32_t any = __reduce_or_sync(0xffffffffu, bits);
+      if (any == 0u) continue;
+      __syncwarp();  // the last chunk's stage has been read
+      if ((any >> lane) & 1u) {
+        const int k = ch * 32 + lane;
+        const float4 s0r = __ldg(shade + 4 * k), s1r = __ldg(shade + 4 * k + 1);
+        const float4 s2r = __ldg(shade + 4 * k + 2), s3r = __ldg(shade + 4 * k + 3);
+        const fv3 v0 = mkv(s0r.x, s0r.y, s0r.z), v1 = mkv(s1r.x, s1r.y, s1r.z);
+        const fv3 v2 = mkv(s2r.x, s2r.y, s2r.z), c = mkv(s3r.x, s3r.y, s3r.z);
+        const fv3 nn = cross(v1 - v0, v2 - v0);
+        stage[lane] = make_float4(v0.x, v0.y, v0.z, v1.x);
+        stage[32 + lane] = make_float4(v1.y, v1.z, v2.x, v2.y);
+        stage[64 + lane] = make_float4(v2.z, c.x, c.y, c.z);
+        stage[96 + lane] = make_float4(nn.x, nn.y, nn.z, 100.f * s0r.w * rsqrtf(dot(nn, nn)));
+        if (tab)
+#pragma unroll
+          for (int i = 0; i < kColScan; ++i)
+            stage[128 + 32 * i + lane] =
+                splat_record(v0, v1, v2, c, nn, mkv(spts[i][0], spts[i][1], spts[i][2]));
+      }
+      __syncwarp();
+      while (any) {
+        uint32_t mine = any;
+        if (G > 1) {
+#pragma unroll
+          for (int i = 1; i < G; ++i) mine = grp >= i ? mine & (mine - 1u) : mine;
+        }
+        const int j = __ffs(mine) - 1;
+#pragma unroll
+        for (int i = 0; i < G; ++i) any &= any - 1u;
+        if (j < 0 || !((bits >> j) & 1u)) continue;
+        const float4 a0 = stage[j], a1 = stage[32 + j], a2 = stage[64 + j], a3 = stage[96 + j];
+        const fv3 v0 = mkv(a0.x, a0.y, a0.z), v1 = mkv(a0.w, a1.x, a1.y);
+        const fv3 v2 = mkv(a1.z, a1.w, a2.x), c = mkv(a2.y, a2.z, a2.w);
+        const fv3 nn = mkv(a3.x, a3.y, a3.z);
+        const float4 rl = splat_record(v0, v1, v2, c, nn, q);
+        const float4 rs = tab ? stage[128 + 32 * (s - s_first) + j]
+                              : splat_record(v0, v1, v2, c, nn, p);
+        const float alpha = rs.w * rl.w * a3.w;
+        if (!(alpha > 0.f)) continue;
+        // exh_pair_filtered's coordinates and tests, on the sorted lengths alone
+        // (the sum of two lengths contracted as there; NaN for a length of zero)
+        auto sum = [](float ds2, float dl2) {
+          return fmaf(ds2, rsqrt_approx(ds2), dl2 * rsqrt_approx(dl2));
+        };
+        float d[3] = {sum(rs.x, rl.x), sum(rs.y, rl.y), sum(rs.z, rl.z)}, c3[3];
+        auto sort = [&]() {
+          const float m01 = fminf(d[0], d[1]), x01 = fmaxf(d[0], d[1]), m12 = fminf(x01, d[2]);
+          d[2] = fmaxf(x01, d[2]);
+          d[0] = fminf(m01, m12);
+          d[1] = fmaxf(m01, m12);
+        };
+        sort();
+        const float u = 5.9604645e-8f;
+        bool sure = d[1] - d[0] > 16.f * u * d[2] && d[2] - d[1] > 16.f * u * d[2];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const float x = d[k] + od, cc = fmaf(x, fb.inv_bw, fb.nbo);
+          const float m = fmaf(fb.kc, x, fb.kb) + 8.f * u * fabsf(cc);
+          sure = sure && fabsf(cc - rintf(cc)) > m && fabsf(cc) < 1.0e9f;
+          c3[k] = cc;
+        }
+        if (!sure) {
+          auto both = [&](fv3 v) { return xadd(xlen(xsub3(v, p)), xlen(xsub3(v, q))); };
+          d[0] = both(v0);
+          d[1] = both(v1);
+          d[2] = both(v2);
+          sort();
+#pragma unroll
+          for (int k = 0; k < 3; ++k) c3[k] = xdiv(xsub(xadd(d[k], od), bo), bw);
+        }
+        splat_tent_columns<CT>(win, c3[0], c3[1], c3[2], alpha);
+      }
+    }
+    __syncthreads();
+    // rows out[b][t][col0 .. col0 + CT): a pass writes its window, the first
+    // one also what lies before, the last one what lies after
+    if (ok) {
+      float* ob = out + (size_t)b * T * C + col;
+      const int ta = pass == 0 ? 0 : w0, tb = pass == passes - 1 ? T : min(w0 + W, T);
+      for (int t = warp * G + grp; t < T; t += kColWarps * G) {
+        if (t < ta || t >= tb) continue;
+        ob[(size_t)t * C] = win.in(t) ? hist[(t - w0) * CT + cl] : 0.f;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+template <int CT, int kColWarps>
+static int launch_exh_columns(const Scene& sc, const View3f& sp, const View3f& lp,
+                              const Origins& org, int S, int L, float* out, int T, float bw,
+                              float bo, int W, cudaStream_t stream) {
+  const FastBins fast = make_fast_bins(bw, bo, tune::get("mesh.exhaustive.exact") != 1);
+  const size_t smem = sizeof(float) * ((size_t)kColWarps * kColStage + (size_t)W * CT);
+  const dim3 grid((unsigned)ceil_div((int64_t)S * L, CT), (unsigned)sc.B);
+  auto* kern = exh_splat_columns_kernel<CT, kColWarps>;
+  TOTRI_CUDA(tune::ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
+  TOTRI_KERNEL("mesh exhaustive splat", stream,
+               kern<<<grid, 32 * kColWarps, smem, stream>>>(sc, sp, lp, org, S, L, out, T, bw, bo,
+                                                            fast, W));
+  return TOTRI_OK;
+}
+
 // Whether bin coordinates may take div_fixed: any path length then either has a
 // coordinate in its range or an alpha of zero.
 static bool fixed_division(float bw, float bo) {
@@ -1018,6 +1299,47 @@ int launch_exhaustive_splat(const Scene& sc, const View3f& sp, const View3f& lp,
       case 32: return launch_exh_splat<32>(sc, sp, lp, org, S, L, out, T, bw, bo, stream);
       default: return fail(TOTRI_ERR_INVALID_ARGUMENT, "laser tile must be 1, 4, 8, 16 or 32");
     }
+  }
+  // Columns (exh_splat_columns_kernel) up to the 2,048 bins that were measured, from
+  // 1,024 columns on (ms, the tiles below against 8 and 32 columns; 400 x 144, 64 x
+  // 144, 169 x 36 and 64 x 16 points):
+  //   20,000 faces, 1,024 bins  8.30 / 6.85 / 5.86   1.68 / 1.21 / 1.07
+  //                             1.39 / 0.94 / 1.18   0.68 / 0.30 / 0.83
+  //   20,000 faces, 2,048 bins 10.27 / 9.31 / 7.80   1.88 / 1.66 / 1.44
+  //                             1.61 / 1.26 / 1.87   0.52 / 0.41 / 1.32
+  //   5,000 faces, 1,024 bins   2.61 / 2.60 / 2.26   0.54 / 0.47 / 0.44
+  //                             0.45 / 0.37 / 0.43   0.23 / 0.13 / 0.34
+  //   1,500 faces, 1,024 bins   1.08 / 1.43 / 1.16   0.24 / 0.27 / 0.25
+  //                             0.19 / 0.21 / 0.25   0.12 / 0.09 / 0.22
+  //   500 faces, 1,024 bins     0.58 / 0.92 / 0.65   0.13 / 0.17 / 0.14
+  //                             0.10 / 0.13 / 0.15   0.06 / 0.05 / 0.12
+  // Small meshes spend the time on the rows, not on the faces: they take 8 columns
+  // only where the tiles leave SMs idle (up to 16 columns per SM and 1,024 bins, or
+  // 48 with two faces per bin: 0.16 against 0.15 ms for 1,500 faces, 512 bins, 169 x
+  // 36 points). A window of 496 bins leaves room for two CTAs per SM; a mesh whose
+  // paths span more than half of 2,048 bins needs a second pass over its faces.
+  // "mesh.exhaustive.splat.columns" = 1 turns the kernel off, 8 and 32 select a
+  // tile, ".window" its bins.
+  const int cols = tune::get("mesh.exhaustive.splat.columns");
+  if (cols != 1 && tune::get("mesh.exhaustive.splat.mode") != 1 && (size_t)T * 4 <= budget) {
+    const int64_t all = (int64_t)S * L * sc.B;
+    const int sms = tune::sm_count();
+    const bool many = sc.F >= 4096;
+    const bool few = all <= 16 * sms && T <= 1024;
+    const int ct = cols > 0 ? cols
+                   : all < 1024 || T > 2048 || !(many || few || (all <= 48 * sms && sc.F >= 2 * T)) ? 0
+                   : many && all >= 48 * sms ? 32
+                                                          : 8;
+    int W = tune::get("mesh.exhaustive.splat.window");
+    if (W <= 0) W = ct == 32 ? (T <= 496 ? 496 : 1024) : 1984;
+    const bool full = W > 496;  // 32 warps share one window
+    W = std::min(W, T);
+    if (ct == 32 && full)
+      return launch_exh_columns<32, 32>(sc, sp, lp, org, S, L, out, T, bw, bo, W, stream);
+    if (ct == 32)
+      return launch_exh_columns<32, 16>(sc, sp, lp, org, S, L, out, T, bw, bo, W, stream);
+    if (ct == 8)
+      return launch_exh_columns<8, 16>(sc, sp, lp, org, S, L, out, T, bw, bo, W, stream);
   }
   // Built-in choice: the widest laser tile whose histogram stays within 40 KB,
   // so several CTAs share an SM (2048 bins x 64x64 x 16x16, 32 meshes: 4.4 s

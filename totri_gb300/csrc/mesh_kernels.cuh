@@ -25,12 +25,26 @@ __device__ __forceinline__ void sort3(Q& q) {
   if (q.d[0] > q.d[1]) sw(0, 1);
 }
 
+// Warp minimum / maximum of a float (redux.sync on floats, sm_100a and later).
+__device__ __forceinline__ float warp_min_f(float x) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float warp_max_f(float x) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 // One wall column of a shared-memory histogram [T][TS].
 template <int TS>
 struct Hist {
   float* h;
   int sl;
   int T;
+  __device__ __forceinline__ int lo() const { return 0; }
+  __device__ __forceinline__ int hi() const { return T; }
   __device__ __forceinline__ bool in(int b) const { return b >= 0 && b < T; }
   __device__ __forceinline__ void add(int b, float v) const { atomicAdd(h + b * TS + sl, v); }
 };
@@ -56,7 +70,7 @@ __device__ __forceinline__ void splat_segment(const H& h, float ca, int ba, floa
     const float w = (float)(ba + 1) - ca;
     h.add(ba, w * (ya + 0.5f * w * slope));
   }
-  const int lo = max(ba + 1, 0), hi = min(bb, h.T);
+  const int lo = max(ba + 1, h.lo()), hi = min(bb, h.hi());
   for (int i = lo; i < hi; ++i) h.add(i, ya + (((float)i + 0.5f) - ca) * slope);
   if (h.in(bb)) {
     const float w = cb - (float)bb;
@@ -69,7 +83,7 @@ __device__ __forceinline__ void splat_segment(const H& h, float ca, int ba, floa
 template <class H>
 __device__ __forceinline__ void splat_tent(const H& h, const float c[3], const int bin[3],
                                            float alpha) {
-  if (bin[0] >= h.T || bin[2] < 0) return;
+  if (bin[0] >= h.hi() || bin[2] < h.lo()) return;
   if (bin[0] == bin[2]) {
     h.add(bin[0], alpha);
     return;
