@@ -424,3 +424,29 @@ def test_exhaustive_grad_follows_the_decided_bins(cuda_lib):
                                          tg[0].numpy())
     assert rel(vg[0].cpu().numpy(), rv) < 2e-6
     assert rel(mg[0].cpu().numpy(), rm) < 2e-6
+
+
+# S, T, bin width, bin offset, origin, mesh: corners before bin 0 and after the last,
+# one point, tents of one bin and of many, slivers with corners at bin edges
+@pytest.mark.parametrize("S,T,bw,bo,origin,kind", [
+    (1, 1, 6.0, 0.0, False, "soup"), (33, 40, 0.02, 1.9, False, "soup"),
+    (64, 97, 0.06, 0.0, True, "soup"), (31, 900, 0.004, 0.3, True, "soup"),
+    (36, 2048, 0.0025, 0.0, False, "sphere")])
+def test_confocal_grad_edges(cuda_lib, S, T, bw, bo, origin, kind):
+    """FP32 sums over a vertex's few hundred pairs, as in the exhaustive gradients,
+    whose bound this is."""
+    g = np.random.default_rng(S + T)
+    v, f = _mesh(kind, 20000 if kind == "sphere" else 90, S)
+    m = torch.rand((1, v.shape[1], 1), device="cuda") + 0.5
+    sp = points(g, S)
+    so = points(g, S, -0.4) if origin else None
+    none = torch.empty((1, 0, 3), device="cuda")
+    tg = g.standard_normal((T, S)).astype(np.float32)
+    vg, mg = torch.empty_like(v), torch.empty_like(m)
+    R.mesh_confocal_grad_verts(v, f, m, cu(sp[None]), cu(so[None]) if origin else none,
+                               cu(tg[None]), vg, mg, bw, bo, 0)
+    vn, fn, mn = v[0].cpu().numpy(), f[0].cpu().numpy(), m[0].cpu().numpy()
+    rv, rm = oracle.mesh_confocal_grad(vn, fn, mn, sp, so, oracle.mesh_visibility(vn, fn, sp), T,
+                                       bw, bo, tg)
+    assert rel(vg[0].cpu().numpy(), rv) < 1e-5
+    assert rel(mg[0].cpu().numpy(), rm) < 1e-5

@@ -797,79 +797,44 @@ __global__ void __launch_bounds__(256, 2) splat_compact_kernel(Scene sc, View3f 
   flush_tile<TS>(hist, transient + (size_t)b * T * S, T, S, s0);
 }
 
-// The tent corners of a pair relative to its first bin, from double-float
-// path lengths 2 |v_k - p| + od (bin_offset); od is the double-float origin
-// term 2 |p - o| (zero without origins).
-__device__ __forceinline__ void confocal_corners(const ConfocalPair& q, fv3 p, DFloat od, float bw,
-                                                 float inv_bw, float bo, float x[3]) {
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const DFloat d = len_df(q.v[k], p);
-    x[k] = bin_offset(df_add(DFloat{2.f * d.hi, 2.f * d.lo}, od), bo, bw, inv_bw, q.bin[0]);
-  }
+// The gradient of a face over its visible scan points, following
+// mesh_confocal_grad_verts_optix.cu:248-314 and AlphaConfocalGradVerts
+// (mesh_common.h:429-463), as sums that are linear in the pair's two factors: P =
+// alpha times the gradient over the tent's area, and Q_m = alpha times the tent's
+// weight of vertex m (pair_weights). With r = c - p,
+//   d log(alpha) / d v_k = J_n^T (kn n + knr r) + kr r + (knr/3) n + kw n_w
+// and d path / d v_m = 2 u_m, u_m the unit vector from the point, so a pair adds
+// P kr r, P knr r, P knr, P kw, P and 2 Q_m u_m; the normal and its Jacobian follow
+// once per face.
+struct FaceSums {
+  unsigned long long a[9];  // pairs: kr r and knr r (x y, z x, y z), (knr, kw), (P, u0 x), ...
+};
+
+// |v - p| as the FP32 chain's length and its low part (len_df's sums, with the
+// Newton step taken from the chain's square root).
+__device__ __forceinline__ DFloat len_exact(fv3 v, fv3 p, float& inv) {
+  const DFloat dx = two_sum(v.x, -p.x), dy = two_sum(v.y, -p.y), dz = two_sum(v.z, -p.z);
+  const float d = xlen(mkv(dx.hi, dy.hi, dz.hi));
+  const float hx = __fmul_rn(dx.hi, dx.hi), hy = __fmul_rn(dy.hi, dy.hi);
+  const float hz = __fmul_rn(dz.hi, dz.hi);
+  const float lx = __fmaf_rn(dx.hi, dx.hi, -hx), ly = __fmaf_rn(dy.hi, dy.hi, -hy);
+  const float lz = __fmaf_rn(dz.hi, dz.hi, -hz);
+  const DFloat s1 = two_sum(hx, hy);
+  const DFloat s2 = two_sum(s1.hi, hz);
+  const float lo = (s1.lo + s2.lo) + (lx + ly + lz) +
+                   2.f * (dx.hi * dx.lo + dy.hi * dy.lo + dz.hi * dz.lo);
+  inv = vdiv(1.f, d);
+  return DFloat{d, d > 0.f ? (__fmaf_rn(-d, d, s2.hi) + lo) * (0.5f * inv) : 0.f};
 }
 
-// Gradient of one visible pair with respect to the three (sorted) vertices and
-// the albedo, following mesh_confocal_grad_verts_optix.cu:248-314 and
-// AlphaConfocalGradVerts (mesh_common.h:429-463), with the tent corners x taken
-// relative to bin[0] (confocal_corners). Returns false when the pair
-// contributes nothing.
-__device__ __forceinline__ bool pair_grad_confocal(const ConfocalPair& q, const float x[3], fv3 c,
-                                                   fv3 p, float rho, float bw,
-                                                   const float* __restrict__ tg_col, int T, int S,
-                                                   fv3 dv[3], float& dmat) {
-  const float alpha = alpha_confocal(q, c, p, rho);
-  if (!(alpha > 0.f)) return false;
-  if (q.bin[0] >= T || q.bin[2] < 0) return false;
-  const fv3 e1 = q.v[1] - q.v[0], e2 = q.v[2] - q.v[0];
-  const fv3 n = cross(e1, e2);
-  const fv3 r = c - p;
-  // d log(alpha) / d v_k = J_n^T (kn n + knr r) + kr r + (knr/3) n + kw n_w
-  const float kn = vdiv(-1.f, dot(n, n));
-  const float kr = vdiv(-8.f, 3.f * dot(r, r));
-  const float kw = vdiv(2.f, 3.f * r.z);
-  const float knr = vdiv(2.f, dot(n, r));
-  const fv3 w = kn * n + knr * r;
-  const fv3 g1 = cross(e2, w), g2 = cross(w, e1);
-  const fv3 common = kr * r + (knr * (1.f / 3.f)) * n + mkv(0.f, 0.f, kw);
-  const fv3 da0 = alpha * (common - g1 - g2);
-  const fv3 da1 = alpha * (common + g1);
-  const fv3 da2 = alpha * (common + g2);
-  const float dadm = vdiv(alpha, rho);
-  if (q.bin[0] == q.bin[2]) {
-    const float g = __ldg(tg_col + (size_t)q.bin[0] * S);
-    dv[0] = g * da0;
-    dv[1] = g * da1;
-    dv[2] = g * da2;
-    dmat = g * dadm;
-    return true;
-  }
-  TentGrad tgr;
-  tent_grad(tg_col, S, T, x, q.bin, tgr);
-  // part1 = Ayc * dyc + A0 * dc0 + A1 * dc1 + A2 * dc2 (see TentGrad)
-  const float span = x[2] - x[0];
-  const float kk = vdiv(-4.f, bw * span * span);
-  const fv3 r0 = q.v[0] - p, r1 = q.v[1] - p, r2 = q.v[2] - p;
-  const fv3 dc0 = vdiv(2.f, bw * q.d[0]) * r0;
-  const fv3 dc1 = vdiv(2.f, bw * q.d[1]) * r1;
-  const fv3 dc2 = vdiv(2.f, bw * q.d[2]) * r2;
-  const fv3 dyc0 = vdiv(kk, -q.d[0]) * r0;
-  const fv3 dyc2 = vdiv(kk, q.d[2]) * r2;
-  const fv3 p1_0 = tgr.ayc * dyc0 + tgr.a0 * dc0;
-  const fv3 p1_1 = tgr.a1 * dc1;
-  const fv3 p1_2 = tgr.ayc * dyc2 + tgr.a2 * dc2;
-  dv[0] = tgr.part0 * da0 + alpha * p1_0;
-  dv[1] = tgr.part0 * da1 + alpha * p1_1;
-  dv[2] = tgr.part0 * da2 + alpha * p1_2;
-  dmat = dadm * tgr.part0;
-  return true;
-}
-
-// Three CTAs per SM (80 registers, a few spills): 1.46 ms against 1.51 ms at
-// 128 registers and two CTAs on the differentiable step.
-__global__ void __launch_bounds__(256, 3) grad_kernel(Scene sc, View3f sp, View3f so, int has_origin,
+// Instruction issue bounds it (75% of the slots). 20,480 faces x 4,096 points, 1,024
+// bins: 1.44 ms when each pair built the vertices' gradients, took every length
+// twice (chain and double-float) and walked the tent's three parts apart (1,200
+// instructions per 32 visible pairs), 1.03 ms now; 320 faces x 1,024 points: 46 and
+// 37 us. Two CTAs per SM (no spills) against 1.05 ms and 40 us with three.
+__global__ void __launch_bounds__(256, 2) grad_kernel(Scene sc, View3f sp, View3f so, int has_origin,
                                                    const float* __restrict__ tgrad, int T, int S,
-                                                   float bw, float bo, GradOut out) {
+                                                   float bw, float bo, int fixed, GradOut out) {
   extern __shared__ uint32_t mcol[];  // [slice] mask words of this 32-face chunk
   __shared__ int gq[8][64];           // per-warp queue of visible scan points
   const int b = blockIdx.y;
@@ -886,34 +851,66 @@ __global__ void __launch_bounds__(256, 3) grad_kernel(Scene sc, View3f sp, View3
   const float* tgb = tgrad + (size_t)b * T * S;
   const float4* shade = sc.shade + (size_t)b * sc.F * 4;
   const float inv_bw = __frcp_rn(bw);
+  const bool plain = !has_origin && bo == 0.f;  // nothing added to a path
   for (int j = warp; j < 32; j += nw) {
     const int k = ch * 32 + j;
     if (k >= n) break;
     const float4 s0r = __ldg(shade + 4 * k), s1r = __ldg(shade + 4 * k + 1);
     const float4 s2r = __ldg(shade + 4 * k + 2), s3r = __ldg(shade + 4 * k + 3);
     const fv3 c = mkv(s3r.x, s3r.y, s3r.z);
-    fv3 acc[3] = {mkv(0.f, 0.f, 0.f), mkv(0.f, 0.f, 0.f), mkv(0.f, 0.f, 0.f)};
-    float accm = 0.f;
+    const fv3 v0 = mkv(s0r.x, s0r.y, s0r.z), v1 = mkv(s1r.x, s1r.y, s1r.z);
+    const fv3 v2 = mkv(s2r.x, s2r.y, s2r.z);
+    const fv3 e1 = v1 - v0, e2 = v2 - v0;
+    const fv3 nrm = cross(e1, e2);
+    const float nn = dot(nrm, nrm);
+    const float kf = xdiv(100.f * s0r.w, xsqrt(nn));
+    FaceSums sums;
+    bool used = false;
+#pragma unroll
+    for (int i = 0; i < 9; ++i) sums.a[i] = 0ull;
     auto run = [&](int s) {
       const fv3 p = mkv(sp.at(b, s, 0), sp.at(b, s, 1), sp.at(b, s, 2));
-      float od = 0.f;
-      DFloat odf{0.f, 0.f};
-      if (has_origin) {
-        const fv3 o = mkv(so.at(b, s, 0), so.at(b, s, 1), so.at(b, s, 2));
-        od = xmul(2.f, xlen(xsub3(p, o)));
-        const DFloat d = len_df(p, o);
-        odf = DFloat{2.f * d.hi, 2.f * d.lo};
+      const fv3 r = c - p;
+      if (!(r.z > 0.f)) return;
+      const float nr = dot(nrm, r), rr = dot(r, r), rr2 = rr * rr;
+      const float alpha = vdiv(kf * (r.z * r.z) * (nr * nr), rr2 * rr2);
+      if (!(alpha > 0.f)) return;
+      float i0, i1, i2;  // 1 / |v_m - p|
+      auto path = [&](fv3 v, float& inv) {
+        const DFloat d = len_exact(v, p, inv);
+        return DFloat{2.f * d.hi, 2.f * d.lo};
+      };
+      DFloat d0 = path(v0, i0), d1 = path(v1, i1), d2 = path(v2, i2);
+      const PathOrder order = sort_paths(d0, d1, d2);
+      if (!plain) {
+        DFloat od{0.f, 0.f};
+        if (has_origin) {
+          const fv3 o = mkv(so.at(b, s, 0), so.at(b, s, 1), so.at(b, s, 2));
+          float unused;
+          const DFloat d = len_exact(p, o, unused);
+          od = DFloat{2.f * d.hi, 2.f * d.lo};
+        }
+        d0 = path_offset(d0, od, bo);
+        d1 = path_offset(d1, od, bo);
+        d2 = path_offset(d2, od, bo);
       }
-      ConfocalPair q;
-      confocal_pair(s0r, s1r, s2r, p, od, bw, bo, q);
-      if (q.bin[0] >= T || q.bin[2] < 0) return;
-      float x[3];
-      confocal_corners(q, p, odf, bw, inv_bw, bo, x);
-      fv3 dv[3];
-      float dm;
-      if (!pair_grad_confocal(q, x, c, p, s0r.w, bw, tgb + s, T, S, dv, dm)) return;
-      add_permuted(acc, dv, q.perm);
-      accm += dm;
+      float4 w;
+      if (!pair_weights<false>(tgb + s, S, T, d0, d1, d2, bw, inv_bw, fixed, order, w)) return;
+      const float P = alpha * w.x, knr = vdiv(2.f, nr), kw = vdiv(2.f, 3.f * r.z);
+      const float pr = P * vdiv(-8.f, 3.f * rr), pn = P * knr;
+      const float q0 = 2.f * alpha * w.y * i0, q1 = 2.f * alpha * w.z * i1;
+      const float q2 = 2.f * alpha * w.w * i2;
+      const fv3 r0 = v0 - p, r1 = v1 - p, r2 = v2 - p;
+      used = true;
+      sums.a[0] = f2fma(f2pack(pr, pr), f2pack(r.x, r.y), sums.a[0]);
+      sums.a[1] = f2fma(f2pack(pr, pn), f2pack(r.z, r.x), sums.a[1]);
+      sums.a[2] = f2fma(f2pack(pn, pn), f2pack(r.y, r.z), sums.a[2]);
+      sums.a[3] = f2fma(f2pack(P, P), f2pack(knr, kw), sums.a[3]);
+      sums.a[4] = f2fma(f2pack(P, q0), f2pack(1.f, r0.x), sums.a[4]);
+      sums.a[5] = f2fma(f2pack(q0, q0), f2pack(r0.y, r0.z), sums.a[5]);
+      sums.a[6] = f2fma(f2pack(q1, q1), f2pack(r1.x, r1.y), sums.a[6]);
+      sums.a[7] = f2fma(f2pack(q1, q2), f2pack(r1.z, r2.x), sums.a[7]);
+      sums.a[8] = f2fma(f2pack(q2, q2), f2pack(r2.y, r2.z), sums.a[8]);
     };
     // visible scan points are queued and evaluated 32 at a time, one per lane
     int* qw = gq[warp];
@@ -937,6 +934,22 @@ __global__ void __launch_bounds__(256, 3) grad_kernel(Scene sc, View3f sp, View3
     __syncwarp();
     if (lane < cnt) run(qw[lane]);
     __syncwarp();
+    float t[18];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) f2unpack(sums.a[i], t[2 * i], t[2 * i + 1]);
+    const float sP = t[8];
+    // (a lane without a pair leaves zeros: the face's normal may be anything)
+    fv3 acc[3] = {mkv(0.f, 0.f, 0.f), mkv(0.f, 0.f, 0.f), mkv(0.f, 0.f, 0.f)};
+    float accm = 0.f;
+    if (used) {
+      const fv3 jw = (vdiv(-1.f, nn) * sP) * nrm + mkv(t[3], t[4], t[5]);
+      const fv3 g1 = cross(e2, jw), g2 = cross(jw, e1);
+      const fv3 common = mkv(t[0], t[1], t[2]) + (t[6] * (1.f / 3.f)) * nrm + mkv(0.f, 0.f, t[7]);
+      acc[0] = common - g1 - g2 + mkv(t[9], t[10], t[11]);
+      acc[1] = common + g1 + mkv(t[12], t[13], t[14]);
+      acc[2] = common + g2 + mkv(t[15], t[16], t[17]);
+      accm = xdiv(sP, s0r.w);
+    }
     scatter_face_grad(out, b, s1r, s2r, s3r, acc, accm, sc.status);
   }
 }
@@ -1214,7 +1227,7 @@ int launch_confocal_grad(const Scene& sc, const View3f& sp, const View3f& so, in
   const dim3 grid((unsigned)sc.nch, (unsigned)sc.B, (unsigned)split);
   TOTRI_KERNEL("mesh confocal grad", stream,
                grad_kernel<<<grid, 256, smem, stream>>>(sc, sp, so, has_origin, tgrad, T, S, bw,
-                                                        bo, out));
+                                                        bo, fixed_division(bw, bo), out));
   return TOTRI_OK;
 }
 

@@ -592,93 +592,6 @@ __device__ __forceinline__ int block_slot(bool flag, int* warp_counts, int* tota
   return flag ? base + __popc(bal & ((1u << lane) - 1u)) : -1;
 }
 
-// tent_grad and the vertices' tent weights {part0, gs0, gs1, gs2} from sums over
-// the bins: with t the distance of a bin's edges from the first foot, cut to the
-// rising side, W1 = sum g (t1 - t0) and M1 = sum g (t1^2 - t0^2), and W2, M2
-// likewise from the second foot. At a bin's edges the area of a side moves with
-// its foot and slope alone; the moves of the peak within its bin cancel between
-// the sides. Coordinates truncate toward zero, so bin 0 reaches back to a corner
-// in (-1, 0), and where the first foot is in a bin below 0 the sides are cut at 0,
-// each if its peak is (tent_grad's terms).
-// kLast: the column's bins lie side by side (bstep 1) in rows of a multiple of 4
-// bins on 16-byte boundaries, read four at a time: 32 columns are 32 cache lines,
-// and an access costs the same for one bin or four.
-template <bool kLast>
-__device__ __forceinline__ float4 tent_weights(const float* __restrict__ col, int64_t stride,
-                                               int T, float x0, float x1, float x2, int b0,
-                                               int b1, int b2, float inv_bw) {
-  const float d1 = x1 - x0, d2 = x2 - x1;
-  const unsigned long long feet = f2pack(-x0, x2);
-  const int first = max(b0, 0), last = min(b2, T - 1);
-  // the lower edge of the first bin, clamped to the sides
-  const float e0 = (float)(first - b0);
-  unsigned long long from =
-      f2pack(b0 >= 0 ? 0.f : (b1 < 0 ? d1 : e0 - x0), b1 < 0 ? x2 - e0 : d2);
-  const int start = kLast ? first & ~3 : first;
-  const float es = (float)(start - b0);
-  unsigned long long edge = f2pack(es, -es), W = 0ull, M = 0ull;
-  auto four = [&](const float g[4], int i, int skip) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      edge = f2add(edge, f2pack(1.f, -1.f));
-      float t, u;
-      f2unpack(f2add(edge, feet), t, u);
-      // (the decided bins say where a side ends: a corner rounded across an edge
-      // stays in its bin)
-      const bool past = i + k >= b1;
-      const unsigned long long to =
-          f2pack(past ? d1 : t, past ? (i + k >= b2 ? 0.f : u) : d2);
-      if (kLast && k < 3 && k < skip) continue;  // (before the first bin)
-      // (t1 - t0, u1 - u0: the falling side's sums come out negated)
-      const unsigned long long gw = f2mul(f2pack(g[k], g[k]), f2sub(to, from));
-      W = f2add(W, gw);
-      M = f2fma(gw, f2add(to, from), M);
-      from = to;
-    }
-  };
-  auto load = [&](int i, float g[4]) {  // bins i .. i + 3, zero past the last one
-    if (kLast) {
-      const float4 q = __ldg(reinterpret_cast<const float4*>(col + i));
-      g[0] = i <= last ? q.x : 0.f;
-      g[1] = i + 1 <= last ? q.y : 0.f;
-      g[2] = i + 2 <= last ? q.z : 0.f;
-      g[3] = i + 3 <= last ? q.w : 0.f;
-    } else {
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        g[k] = i + k <= last ? __ldg(col + (int64_t)(i + k) * stride) : 0.f;
-    }
-  };
-  float g[4];
-  load(start, g);
-  int skip = first - start;
-  for (int i = start;;) {
-    float next[4] = {0.f, 0.f, 0.f, 0.f};
-    const bool more = i + 4 <= last;
-    if (more) load(i + 4, next);  // in flight over the four bins at hand
-    four(g, i, skip);
-    if (!more) break;
-    i += 4;
-    skip = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) g[k] = next[k];
-  }
-  float W1, W2, M1, M2;
-  f2unpack(W, W1, W2);
-  f2unpack(M, M1, M2);
-  const float is = vdiv(1.f, x2 - x0), i1 = vdiv(1.f, d1), i2 = vdiv(1.f, d2);
-  float f1 = W1 * i1, h1 = 0.5f * M1 * i1, e1 = h1 * i1;
-  float f2 = -W2 * i2, h2 = -0.5f * M2 * i2, e2 = h2 * i2;
-  const bool no1 = !(fabsf(d1) > 1e-15f), no2 = !(fabsf(d2) > 1e-15f);
-  if (no1 || no2) {  // a side of no width: all in the peak's bin
-    const float gp = b1 >= 0 && b1 < T ? __ldg(col + (int64_t)b1 * stride) : 0.f;
-    if (no1) f1 = gp, h1 = 0.f, e1 = 0.5f * gp;
-    if (no2) f2 = gp, h2 = 0.f, e2 = 0.5f * gp;
-  }
-  const float S = h1 + h2, yc = 2.f * is, k = yc * inv_bw;
-  return make_float4(yc * S, k * ((e1 - f1) + S * is), k * (e2 - e1), k * ((f2 - e2) - S * is));
-}
-
 template <int kOcc, bool kLast>
 __global__ void __launch_bounds__(256, kOcc) exh_grad_face_kernel(
     Scene sc, View3f sp, View3f lp, Origins org, int S, int L, const float* __restrict__ tgrad,
@@ -715,7 +628,7 @@ __global__ void __launch_bounds__(256, kOcc) exh_grad_face_kernel(
     const fv3 c = mkv(s3r.x, s3r.y, s3r.z);
     const fv3 nrm = cross(v[1] - v[0], v[2] - v[0]);
     const float nn = dot(nrm, nrm);
-    const float kf = 100.f * s0r.w * rsqrtf(nn);
+    const float kf = xdiv(100.f * s0r.w, xsqrt(nn));
     const int ch = k >> 5;
     const uint32_t bit = 1u << (k & 31);
     // the face's scan-point records over this slice
@@ -790,67 +703,17 @@ __global__ void __launch_bounds__(256, kOcc) exh_grad_face_kernel(
           e1.lo += m1.y + o1.y;
           e2.lo += m1.z + o1.z;
           // the vertex order of exh_sort (stable compare-swaps on the path length)
-          auto swap_if = [](bool y, DFloat& a, DFloat& z) {
-            const DFloat t = a;
-            a.hi = y ? z.hi : a.hi;
-            a.lo = y ? z.lo : a.lo;
-            z.hi = y ? t.hi : z.hi;
-            z.lo = y ? t.lo : z.lo;
-          };
-          const bool y0 = e0.hi > e1.hi;
-          swap_if(y0, e0, e1);
-          const bool y1 = e1.hi > e2.hi;
-          swap_if(y1, e1, e2);
-          const bool y2 = e0.hi > e1.hi;
-          swap_if(y2, e0, e1);
+          const PathOrder order = sort_paths(e0, e1, e2);
           if (!plain) {
             const float ood = ro[kRecOd];
             const DFloat od = df_add(DFloat{mod, m1.w}, DFloat{ood, o1.w});
-            auto add = [&](DFloat& e) {
-              e = df_add(e, od);
-              const DFloat f = two_sum(e.hi, -bo);
-              e.hi = f.hi;
-              e.lo += f.lo;
-            };
-            add(e0);
-            add(e1);
-            add(e2);
+            e0 = path_offset(e0, od, bo);
+            e1 = path_offset(e1, od, bo);
+            e2 = path_offset(e2, od, bo);
           }
-          float c0, c1, c2;
-          if (fixed) {
-            c0 = div_fixed(e0.hi, bw, inv_bw);
-            c1 = div_fixed(e1.hi, bw, inv_bw);
-            c2 = div_fixed(e2.hi, bw, inv_bw);
-          } else {
-            c0 = xdiv(e0.hi, bw);
-            c1 = xdiv(e1.hi, bw);
-            c2 = xdiv(e2.hi, bw);
-          }
-          auto bin = [](float x) { return __float2int_rz(fminf(fmaxf(x, -1.0e9f), 1.0e9f)); };
-          const int b0c = bin(c0), b1c = bin(c1), b2c = bin(c2);
-          if (b0c >= T || b2c < 0) continue;
           const float* col = colm + __float_as_int(ro[kRecAt]) * ostep;
-          float4 w;  // area, weights of the sorted vertices
-          if (b0c == b2c) {
-            w = make_float4(__ldg(col + (int64_t)b0c * bstep), 0.f, 0.f, 0.f);
-          } else {
-            // corners relative to the first bin (bin_offset)
-            const float base = (float)b0c;
-            auto rel = [&](float cc, DFloat e) {
-              return fmaf(__fmaf_rn(-cc, bw, e.hi) + e.lo, inv_bw, cc - base);
-            };
-            const float x0 = rel(c0, e0), x1 = rel(c1, e1), x2 = rel(c2, e2);
-            w = tent_weights<kLast>(col, bstep, T, x0, x1, x2, b0c, b1c, b2c, inv_bw);
-          }
-          // back to the face's own order
-          auto swap_back = [](bool y, float& a, float& z) {
-            const float t = a;
-            a = y ? z : a;
-            z = y ? t : z;
-          };
-          swap_back(y2, w.y, w.z);
-          swap_back(y1, w.z, w.w);
-          swap_back(y0, w.y, w.z);
+          float4 w;  // area, weights of the vertices
+          if (!pair_weights<kLast>(col, bstep, T, e0, e1, e2, bw, inv_bw, fixed, order, w)) continue;
           const float P = alpha * w.x, Q0 = alpha * w.y, Q1 = alpha * w.z, Q2 = alpha * w.w;
           used = true;
           gP += P;
@@ -923,7 +786,7 @@ __global__ void __launch_bounds__(256, kOcc) exh_grad_face_kernel(
           atomicAdd(out.vg + b * out.vsb + vi[m] * out.vsv + a * out.vsc, t);
         }
       } else if (tid == 9 && out.mg) {
-        const float t = vdiv(tot[15], s0r.w);
+        const float t = xdiv(tot[15], s0r.w);
         for (int m = 0; m < 3; ++m)
           if (vi[m] >= 0 && vi[m] < out.V)
             atomicAdd(out.mg + b * out.msb + vi[m] * out.msv, (1.f / 3.f) * t);
@@ -1212,12 +1075,6 @@ static int launch_exh_columns(const Scene& sc, const View3f& sp, const View3f& l
                kern<<<grid, 32 * kColWarps, smem, stream>>>(sc, sp, lp, org, S, L, out, T, bw, bo,
                                                             fast, W));
   return TOTRI_OK;
-}
-
-// Whether bin coordinates may take div_fixed: any path length then either has a
-// coordinate in its range or an alpha of zero.
-static bool fixed_division(float bw, float bo) {
-  return bw >= 0x1p-60f && bw <= 0x1p60f && std::fabs(bo) <= 0x1p60f;
 }
 
 template <int LT>
