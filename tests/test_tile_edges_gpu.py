@@ -450,3 +450,32 @@ def test_confocal_grad_edges(cuda_lib, S, T, bw, bo, origin, kind):
                                        bw, bo, tg)
     assert rel(vg[0].cpu().numpy(), rv) < 1e-5
     assert rel(mg[0].cpu().numpy(), rm) < 1e-5
+
+
+@pytest.mark.parametrize("S,T,bw,bo,origin", [
+    (1, 1, 6.0, 0.0, False), (9, 40, 0.02, 1.9, False), (33, 97, 0.06, 0.0, True),
+    (64, 1021, 0.0051, 0.3, True), (31, 301, 0.012, 2.3, False)])
+@pytest.mark.parametrize("cols,window", [(8, 0), (8, 50), (32, 0), (32, 37), (32, 700)])
+def test_confocal_columns_edges(cuda_lib, S, T, bw, bo, origin, cols, window):
+    """Sums of a few FP32 terms of one sign per bin, as in the other renders, whose
+    bound this is."""
+    from totri_gb300 import autotune
+    g = np.random.default_rng(S + T)
+    v, f = _mesh("soup", 300, S)
+    m = torch.rand((1, v.shape[1], 1), device="cuda") + 0.5
+    sp = points(g, S)
+    so = points(g, S, -0.4) if origin else None
+    none = torch.empty((1, 0, 3), device="cuda")
+    out = torch.full((1, T, S), 5.0, device="cuda")
+    try:
+        autotune.set_tile("mesh.confocal.splat.columns", cols)
+        autotune.set_tile("mesh.confocal.splat.window", window)
+        R.mesh_confocal_forward(v, f, m, cu(sp[None]), cu(so[None]) if origin else none, out, bw,
+                                bo, 0)
+    finally:
+        autotune.set_tile("mesh.confocal.splat.columns", 0)
+        autotune.set_tile("mesh.confocal.splat.window", 0)
+    vn, fn, mn = v[0].cpu().numpy(), f[0].cpu().numpy(), m[0].cpu().numpy()
+    ref = oracle.mesh_confocal_forward(vn, fn, mn, sp, so, oracle.mesh_visibility(vn, fn, sp), T,
+                                       bw, bo)
+    assert rel(out[0].cpu().numpy(), ref) < 1e-5

@@ -23,7 +23,7 @@ CANDIDATES = {
     # Morton-ordered wall-point patches (the built-in choice), 5 the same warps
     # walking as one packet, 6 the same warps over the 4-wide tree
     "mesh.visibility.mode": (3, 4, 6),
-    "mesh.confocal.splat.ts": (1, 2, 4, 8, 16),
+    "mesh.confocal.splat.ts": (0, 1, 2, 4, 8, 16),
     "mesh.exhaustive.splat.lt": (0, 1, 4, 8, 16, 32),
 }
 

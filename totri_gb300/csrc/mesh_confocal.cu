@@ -1201,6 +1201,25 @@ int launch_confocal_splat(const Scene& sc, const View3f& sp, const View3f& so, i
       default: return fail(TOTRI_ERR_INVALID_ARGUMENT, "scan tile must be 1, 2, 4, 8 or 16");
     }
   }
+  // Columns (splat_columns_kernel with 8 scan points per tile) for large meshes and
+  // for middling ones over few points, from 1,024 points on (us, the tiles below
+  // against it; 1,024, 2,304 and 4,096 points):
+  //   20,480 faces, 1,024 bins  335/232  586/296  761/544; 2,048: 434/343 527/423 1025/788
+  //   12,288 faces (a box), 2,048 bins, 6,767 points  936/867
+  //   5,000 faces, 1,024 bins   140/123  228/142  268/249; 2,048: 195/193 234/220 419/391
+  //   1,500 faces, 1,024 bins    68/66   104/74   124/131; 2,048: 104/113 121/124 216/216
+  //   700 faces, 512 bins        39/41    58/44    63/74
+  // Below 1,024 points its tiles leave SMs idle (20,480 faces, 256 points: 123/262),
+  // and small meshes spend the time on the rows. With 32 points per tile: 670, 669
+  // and 574 us in the first row. "mesh.confocal.splat.columns" = 1 turns it off, 8
+  // and 32 select a tile, ".window" its bins.
+  const int cols = tune::get("mesh.confocal.splat.columns");
+  const int64_t all = (int64_t)S * sc.B;
+  const bool large = sc.F >= 12288 ? T <= 2048 : sc.F >= 4096 && T <= 1024;
+  const bool few = sc.F >= 1024 && all <= 16 * tune::sm_count() && T <= 1024;
+  const int ct = cols > 0 ? cols : all >= 1024 && (large || few) ? 8 : 0;
+  if (ct > 1 && (size_t)T * 4 <= budget && tune::get("mesh.confocal.splat.mode") != 1)
+    return launch_confocal_columns(sc, sp, so, has_origin, ct, transient, T, S, bw, bo, stream);
   // Built-in choice: the widest scan tile that keeps the histogram within
   // 40 KB (several CTAs per SM) and still gives every SM tiles to work on.
   const size_t kTileBytes = 40 * 1024;

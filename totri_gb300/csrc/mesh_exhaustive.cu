@@ -879,8 +879,11 @@ __device__ __forceinline__ float4 splat_record(fv3 v0, fv3 v1, fv3 v2, fv3 c, fv
 // a fixed division were 0.5 ms faster, but moved single bins by 1e-3.
 constexpr int kColScan = 2;  // scan points with records prepared per face
 constexpr int kColStage = 32 * (16 + 4 * kColScan);  // floats per warp
-template <int CT, int kColWarps>
-__global__ void __launch_bounds__(32 * kColWarps, 32 / kColWarps) exh_splat_columns_kernel(
+// kConfocal: a column is a scan point, its path twice one length (L = 1, lp unused).
+// 20,480 faces x 4,096 points, 1,024 bins: 0.76 ms with blocks of 8 points whose
+// lanes met in the same bins, 0.54 ms.
+template <int CT, int kColWarps, bool kConfocal>
+__global__ void __launch_bounds__(32 * kColWarps, 32 / kColWarps) splat_columns_kernel(
     Scene sc, View3f sp, View3f lp, Origins org, int S, int L, float* __restrict__ out, int T,
     float bw, float bo, FastBins fb, int W) {
   extern __shared__ float4 smem4[];
@@ -896,13 +899,15 @@ __global__ void __launch_bounds__(32 * kColWarps, 32 / kColWarps) exh_splat_colu
   const int64_t col = ok ? col0 + cl : col0;
   const int s_first = (int)(col0 / L);
   const int s = (int)(col / L), l = (int)(col - (int64_t)s * L);
-  const bool tab = (int)((min(col0 + CT, C) - 1) / L) - s_first < kColScan;  // CTA-uniform
+  // (CTA-uniform)
+  const bool tab = !kConfocal && (int)((min(col0 + CT, C) - 1) / L) - s_first < kColScan;
   float4* stage = smem4 + warp * (kColStage / 4);
   float* hist = reinterpret_cast<float*>(smem4 + kColWarps * (kColStage / 4));
   const fv3 p = mkv(sp.at(b, s, 0), sp.at(b, s, 1), sp.at(b, s, 2));
-  const fv3 q = mkv(lp.at(b, l, 0), lp.at(b, l, 1), lp.at(b, l, 2));
-  const float od = origin_term(org, b, s, l, p, q);
-  if (threadIdx.x < kColScan) {
+  const fv3 q = kConfocal ? p : mkv(lp.at(b, l, 0), lp.at(b, l, 1), lp.at(b, l, 2));
+  float od = origin_term(org, b, s, l, p, q);
+  if (kConfocal) od = xmul(2.f, od);
+  if (!kConfocal && threadIdx.x < kColScan) {
     const int si = min(s_first + (int)threadIdx.x, S - 1);
     for (int a = 0; a < 3; ++a) spts[threadIdx.x][a] = sp.at(b, si, a);
   }
@@ -916,7 +921,7 @@ __global__ void __launch_bounds__(32 * kColWarps, 32 / kColWarps) exh_splat_colu
   const uint32_t* ml = sc.mask + ((size_t)b * sc.P + S + l) * sc.nch;
   const float4* shade = sc.shade + (size_t)b * sc.F * 4;
   auto seen = [&](int ch) {  // the column's faces of a chunk
-    const uint32_t m = ok ? __ldg(ms + ch) & __ldg(ml + ch) : 0u;
+    const uint32_t m = ok ? (kConfocal ? __ldg(ms + ch) : __ldg(ms + ch) & __ldg(ml + ch)) : 0u;
     return n - ch * 32 >= 32 ? m : m & ((1u << (n - ch * 32)) - 1u);
   };
   __syncthreads();
@@ -1009,14 +1014,17 @@ __global__ void __launch_bounds__(32 * kColWarps, 32 / kColWarps) exh_splat_colu
         const fv3 v2 = mkv(a1.z, a1.w, a2.x), c = mkv(a2.y, a2.z, a2.w);
         const fv3 nn = mkv(a3.x, a3.y, a3.z);
         const float4 rl = splat_record(v0, v1, v2, c, nn, q);
-        const float4 rs = tab ? stage[128 + 32 * (s - s_first) + j]
-                              : splat_record(v0, v1, v2, c, nn, p);
+        const float4 rs = kConfocal ? rl
+                          : tab     ? stage[128 + 32 * (s - s_first) + j]
+                                    : splat_record(v0, v1, v2, c, nn, p);
         const float alpha = rs.w * rl.w * a3.w;
         if (!(alpha > 0.f)) continue;
-        // exh_pair_filtered's coordinates and tests, on the sorted lengths alone
-        // (the sum of two lengths contracted as there; NaN for a length of zero)
+        // exh_pair_filtered's (confocal_pair_filtered's) coordinates and tests, on the
+        // sorted lengths alone (the sum of two lengths contracted as there; NaN for a
+        // length of zero)
         auto sum = [](float ds2, float dl2) {
-          return fmaf(ds2, rsqrt_approx(ds2), dl2 * rsqrt_approx(dl2));
+          const float dl = dl2 * rsqrt_approx(dl2);
+          return kConfocal ? dl : fmaf(ds2, rsqrt_approx(ds2), dl);
         };
         float d[3] = {sum(rs.x, rl.x), sum(rs.y, rl.y), sum(rs.z, rl.z)}, c3[3];
         auto sort = [&]() {
@@ -1030,13 +1038,17 @@ __global__ void __launch_bounds__(32 * kColWarps, 32 / kColWarps) exh_splat_colu
         bool sure = d[1] - d[0] > 16.f * u * d[2] && d[2] - d[1] > 16.f * u * d[2];
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-          const float x = d[k] + od, cc = fmaf(x, fb.inv_bw, fb.nbo);
+          const float x = kConfocal ? fmaf(2.f, d[k], od) : d[k] + od;
+          const float cc = fmaf(x, fb.inv_bw, fb.nbo);
           const float m = fmaf(fb.kc, x, fb.kb) + 8.f * u * fabsf(cc);
           sure = sure && fabsf(cc - rintf(cc)) > m && fabsf(cc) < 1.0e9f;
           c3[k] = cc;
         }
         if (!sure) {
-          auto both = [&](fv3 v) { return xadd(xlen(xsub3(v, p)), xlen(xsub3(v, q))); };
+          auto both = [&](fv3 v) {
+            const float dl = xlen(xsub3(v, q));
+            return kConfocal ? xmul(2.f, dl) : xadd(xlen(xsub3(v, p)), dl);
+          };
           d[0] = both(v0);
           d[1] = both(v1);
           d[2] = both(v2);
@@ -1062,16 +1074,17 @@ __global__ void __launch_bounds__(32 * kColWarps, 32 / kColWarps) exh_splat_colu
   }
 }
 
-template <int CT, int kColWarps>
-static int launch_exh_columns(const Scene& sc, const View3f& sp, const View3f& lp,
-                              const Origins& org, int S, int L, float* out, int T, float bw,
-                              float bo, int W, cudaStream_t stream) {
-  const FastBins fast = make_fast_bins(bw, bo, tune::get("mesh.exhaustive.exact") != 1);
+template <int CT, int kColWarps, bool kConfocal>
+static int launch_columns(const Scene& sc, const View3f& sp, const View3f& lp,
+                          const Origins& org, int S, int L, float* out, int T, float bw, float bo,
+                          int W, cudaStream_t stream) {
+  const FastBins fast = make_fast_bins(
+      bw, bo, tune::get(kConfocal ? "mesh.confocal.exact" : "mesh.exhaustive.exact") != 1);
   const size_t smem = sizeof(float) * ((size_t)kColWarps * kColStage + (size_t)W * CT);
   const dim3 grid((unsigned)ceil_div((int64_t)S * L, CT), (unsigned)sc.B);
-  auto* kern = exh_splat_columns_kernel<CT, kColWarps>;
+  auto* kern = splat_columns_kernel<CT, kColWarps, kConfocal>;
   TOTRI_CUDA(tune::ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
-  TOTRI_KERNEL("mesh exhaustive splat", stream,
+  TOTRI_KERNEL(kConfocal ? "mesh confocal splat" : "mesh exhaustive splat", stream,
                kern<<<grid, 32 * kColWarps, smem, stream>>>(sc, sp, lp, org, S, L, out, T, bw, bo,
                                                             fast, W));
   return TOTRI_OK;
@@ -1140,6 +1153,31 @@ static int launch_exh_splat(const Scene& sc, const View3f& sp, const View3f& lp,
   return TOTRI_OK;
 }
 
+// The tile's kernel: windows of W bins (0: as many as fit, two CTAs per SM up to 496
+// bins of 32 columns, else 32 warps over one window).
+template <bool kConfocal>
+static int launch_tile(int ct, const Scene& sc, const View3f& sp, const View3f& lp,
+                       const Origins& org, int S, int L, float* out, int T, float bw, float bo,
+                       int W, cudaStream_t stream) {
+  if (W <= 0) W = ct == 32 ? (T <= 496 ? 496 : 1024) : 1984;
+  const bool full = W > 496;
+  W = std::min(W, T);
+  if (ct == 32 && full)
+    return launch_columns<32, 32, kConfocal>(sc, sp, lp, org, S, L, out, T, bw, bo, W, stream);
+  if (ct == 32)
+    return launch_columns<32, 16, kConfocal>(sc, sp, lp, org, S, L, out, T, bw, bo, W, stream);
+  if (ct == 8)
+    return launch_columns<8, 16, kConfocal>(sc, sp, lp, org, S, L, out, T, bw, bo, W, stream);
+  return fail(TOTRI_ERR_INVALID_ARGUMENT, "column tile must be 8 or 32");
+}
+
+int launch_confocal_columns(const Scene& sc, const View3f& sp, const View3f& so, int has_origin,
+                            int ct, float* transient, int T, int S, float bw, float bo,
+                            cudaStream_t stream) {
+  return launch_tile<true>(ct, sc, sp, sp, Origins{so, so, has_origin, 0}, S, 1, transient, T, bw,
+                           bo, tune::get("mesh.confocal.splat.window"), stream);
+}
+
 int launch_exhaustive_splat(const Scene& sc, const View3f& sp, const View3f& lp,
                             const Origins& org, int S, int L, float* out, int T, float bw,
                             float bo, cudaStream_t stream) {
@@ -1157,7 +1195,7 @@ int launch_exhaustive_splat(const Scene& sc, const View3f& sp, const View3f& lp,
       default: return fail(TOTRI_ERR_INVALID_ARGUMENT, "laser tile must be 1, 4, 8, 16 or 32");
     }
   }
-  // Columns (exh_splat_columns_kernel) up to the 2,048 bins that were measured, from
+  // Columns (splat_columns_kernel) up to the 2,048 bins that were measured, from
   // 1,024 columns on (ms, the tiles below against 8 and 32 columns; 400 x 144, 64 x
   // 144, 169 x 36 and 64 x 16 points):
   //   20,000 faces, 1,024 bins  8.30 / 6.85 / 5.86   1.68 / 1.21 / 1.07
@@ -1183,20 +1221,12 @@ int launch_exhaustive_splat(const Scene& sc, const View3f& sp, const View3f& lp,
     const int sms = tune::sm_count();
     const bool many = sc.F >= 4096;
     const bool few = all <= 16 * sms && T <= 1024;
-    const int ct = cols > 0 ? cols
+    const int ct = cols > 1 ? cols
                    : all < 1024 || T > 2048 || !(many || few || (all <= 48 * sms && sc.F >= 2 * T)) ? 0
                    : many && all >= 48 * sms ? 32
                                                           : 8;
-    int W = tune::get("mesh.exhaustive.splat.window");
-    if (W <= 0) W = ct == 32 ? (T <= 496 ? 496 : 1024) : 1984;
-    const bool full = W > 496;  // 32 warps share one window
-    W = std::min(W, T);
-    if (ct == 32 && full)
-      return launch_exh_columns<32, 32>(sc, sp, lp, org, S, L, out, T, bw, bo, W, stream);
-    if (ct == 32)
-      return launch_exh_columns<32, 16>(sc, sp, lp, org, S, L, out, T, bw, bo, W, stream);
-    if (ct == 8)
-      return launch_exh_columns<8, 16>(sc, sp, lp, org, S, L, out, T, bw, bo, W, stream);
+    const int W = tune::get("mesh.exhaustive.splat.window");
+    if (ct != 0) return launch_tile<false>(ct, sc, sp, lp, org, S, L, out, T, bw, bo, W, stream);
   }
   // Built-in choice: the widest laser tile whose histogram stays within 40 KB,
   // so several CTAs share an SM (2048 bins x 64x64 x 16x16, 32 meshes: 4.4 s

@@ -530,6 +530,10 @@ struct Origins {
   int has_so, has_lo;
 };
 
+// The confocal splat over tiles of ct = 8 or 32 scan points (splat_columns_kernel).
+int launch_confocal_columns(const Scene& sc, const View3f& sp, const View3f& so, int has_origin,
+                            int ct, float* transient, int T, int S, float bw, float bo,
+                            cudaStream_t stream);
 int launch_exhaustive_splat(const Scene& sc, const View3f& sp, const View3f& lp,
                             const Origins& org, int S, int L, float* out, int T, float bw,
                             float bo, cudaStream_t stream);

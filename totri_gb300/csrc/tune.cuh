@@ -12,6 +12,7 @@
 //   "mesh.exhaustive.exact"     1: every exhaustive sample takes the exact chain
 //   "mesh.exhaustive.grad.mode" 1 per-lane mask tests, 2 compacted triples
 //                               (default: per-face point records)
+//   "mesh.confocal.splat.columns", ".window",
 //   "mesh.exhaustive.splat.columns", ".window" 1: never the columns kernel, 8 or 32:
 //                               its tile / bins per pass (at its launcher)
 //   "mesh.exhaustive.grad.faces" faces per CTA of the point-record gradient (1)
