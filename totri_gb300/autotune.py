@@ -18,11 +18,12 @@ import torch
 from . import _lib
 
 CANDIDATES = {
-    # 1 per-lane BVH walk, 2 warp-packet walk, 3 per-lane with postponed leaf tests
-    # (point-major warps), 4 postponed leaf tests with face-major warps over
-    # Morton-ordered wall-point patches (the built-in choice), 5 the same warps
-    # walking as one packet, 6 the same warps over the 4-wide tree
-    "mesh.visibility.mode": (3, 4, 6),
+    # 0 the built-in choice (candidate lists on dense walls, else face-major warps
+    # over Morton-ordered wall-point patches and the 4-wide tree), 1 per-lane BVH
+    # walk, 2 warp-packet walk, 3 per-lane with postponed leaf tests (point-major
+    # warps), 4 postponed leaf tests with face-major warps over the patches, 5 the
+    # same warps walking as one packet, 6 the same warps over the 4-wide tree
+    "mesh.visibility.mode": (0, 3, 4, 6),
     "mesh.confocal.splat.ts": (0, 1, 2, 4, 8, 16),
     "mesh.exhaustive.splat.lt": (0, 1, 4, 8, 16, 32),
 }
