@@ -479,3 +479,35 @@ def test_confocal_columns_edges(cuda_lib, S, T, bw, bo, origin, cols, window):
     ref = oracle.mesh_confocal_forward(vn, fn, mn, sp, so, oracle.mesh_visibility(vn, fn, sp), T,
                                        bw, bo)
     assert rel(out[0].cpu().numpy(), ref) < 1e-5
+
+
+@pytest.mark.parametrize("kind,faces,P", LISTS)
+@pytest.mark.parametrize("wall", ["plane", "tilted", "line", "space"])
+def test_walk_runs_and_point_orders(cuda_lib, kind, faces, P, wall):
+    """Masks are the brute-force ones whatever the runs of the walk kernel and the
+    order of the points: a wall along two axes, one across all three, points on a
+    line and in space, with repeated points."""
+    from totri_gb300 import autotune
+    v, f = _mesh(kind, faces, faces + P)
+    g = np.random.default_rng(faces)
+    pts = points(g, P)
+    if wall == "tilted":
+        pts[:, 2] = 0.7 * pts[:, 0] - 0.4 * pts[:, 1] - 0.5
+    elif wall == "line":
+        pts[:, 1:] = 0.0
+    elif wall == "space":
+        pts[:, 2] = g.uniform(-2.0, 0.0, P).astype(np.float32)
+    pts[P // 2] = pts[0]
+    pts = cu(pts[None])
+    bf = R.mesh_visibility(v, f, pts, brute_force=True)
+    for parts, morton, lists in ((1, 0, 1), (4, 0, 1), (4, 1, 1), (0, 0, 2)):
+        keys = {"mesh.visibility.list": lists, "mesh.visibility.list.parts": parts,
+                "mesh.visibility.morton": morton}
+        try:
+            for k, x in keys.items():
+                autotune.set_tile(k, x)
+            got = R.mesh_visibility(v, f, pts)
+        finally:
+            for k in keys:
+                autotune.set_tile(k, 0)
+        assert torch.equal(got, bf), keys

@@ -426,16 +426,19 @@ constexpr int kListWarps = 4, kListFaces = 8, kListFrontier = 256, kListCand = 5
 // on the 20,480-face workload, 4.9, 7.6 and 11.4 against 5.5 ms on the box.
 template <int kOcc>
 __global__ void __launch_bounds__(32 * kListWarps, kOcc) visibility_walk_kernel(
-    Scene sc, View3f pts, int P, int row0, uint32_t* next_unit, int seed_mode, int seed_steps) {
+    Scene sc, View3f pts, int P, int row0, uint32_t* next_unit, int parts, int seed_mode,
+    int seed_steps) {
   const int lane = threadIdx.x & 31;
   const int patches = (P + 31) >> 5;
-  const unsigned units = (unsigned)patches * sc.nch * sc.B;
+  const unsigned units = (unsigned)patches * sc.nch * sc.B * parts;
+  const int run = 32 / parts;
   for (;;) {
     unsigned unit = 0;
     if (lane == 0) unit = atomicAdd(next_unit, 1u);
     unit = __shfl_sync(0xffffffffu, unit, 0);
     if (unit >= units) break;
-    const int ch = unit % sc.nch, pb = unit / sc.nch;
+    const int j0 = (int)(unit % parts) * run, up = unit / parts;
+    const int ch = up % sc.nch, pb = up / sc.nch;
     const int b = pb / patches, i = (pb - b * patches) * 32 + lane;
     const int n = sc.meta[b].n;
     const bool okp = i < P;
@@ -447,7 +450,7 @@ __global__ void __launch_bounds__(32 * kListWarps, kOcc) visibility_walk_kernel(
     int seed = okp ? gseeds[i] : -1;
     const int s0 = seed;
     uint32_t word = 0u;
-    for (int j = 0; j < 32 && ch * 32 + j < n; ++j) {  // warp-uniform
+    for (int j = j0; j < j0 + run && ch * 32 + j < n; ++j) {  // warp-uniform
       const Target tg = load_target(sc, b, ch * 32 + j);
       bool vis = false;
       if (okp) {
@@ -462,7 +465,10 @@ __global__ void __launch_bounds__(32 * kListWarps, kOcc) visibility_walk_kernel(
       __syncwarp();
       word |= (uint32_t)vis << j;
     }
-    if (okp) sc.mask[((size_t)b * sc.P + row0 + p) * sc.nch + ch] = word;
+    uint32_t* mw = sc.mask + ((size_t)b * sc.P + row0 + p) * sc.nch + ch;
+    if (okp && parts == 1) *mw = word;
+    // (a run of 8 faces is a byte of the word)
+    if (okp && parts == 4) reinterpret_cast<uint8_t*>(mw)[j0 >> 3] = (uint8_t)(word >> j0);
     if (okp && seed != s0) gseeds[i] = seed;
   }
 }
@@ -978,19 +984,19 @@ int launch_mask_unsort(const Scene& sc, int P, uint32_t* out, cudaStream_t strea
 }
 
 // Dense wall grids (blocks of 32 points narrow enough for the hulls) with
-// enough (block, chunk) units to feed the queues: from 2,048 points and 16,384
-// units on the two kernels were faster on every mesh tried (1.02-1.11x on
-// 20,000-face spheres at 48 x 48 and 101 x 23 points, 1.06x on 5,120 faces at 64 x
-// 64, 2.2x on boxes there); below, 0.72-0.98x on spheres (5,120 faces at 40 x 40,
-// 101 x 23 and 48 x 48 points, 20,000 at 40 x 40), though 1.3x on 20,480 faces at
-// 32 x 32 and 1.3-1.6x on boxes. "mesh.visibility.list": 1 always, 2 never;
-// ".list.cap" lowers the list's capacity.
+// enough (block, chunk) units to feed the queues: from 1,024 points and 5,000 units
+// on the two kernels took 0.50-0.99x of the patch kernel's time on spheres, boxes
+// and displaced icospheres of 1,280 to 20,480 faces at 1,024 to 10,201 points (us:
+// 20,480 faces, 4,096 points 4,540 against 7,966; 8,000, 3,136 points 1,736 against
+// 2,444, a box 2,751 against 5,842; 1,280, 4,096 points 324 against 361). Below,
+// 1.0-1.3x, and 1.1-1.4x at 576 points (20,000 faces 2,333 against 2,067).
+// "mesh.visibility.list": 1 always, 2 never; ".list.cap" lowers the list's capacity.
 static bool list_rule(const Scene& sc, int P) {
   const int list = tune::get("mesh.visibility.list");
   const int64_t units = ceil_div(P, 32) * sc.nch * sc.B;
   return tune::get("mesh.visibility.mode") == 0 && tune::get("mesh.visibility.wide") != 2 &&
          tune::get("mesh.visibility.queue") != 1 && tune::get("mesh.visibility.occupancy") == 0 &&
-         (list == 1 || (list == 0 && P >= 2048 && units >= 16384)) && units < ((int64_t)1 << 29);
+         (list == 1 || (list == 0 && P >= 1024 && units >= 5000)) && units < ((int64_t)1 << 29);
 }
 
 bool orders_points(bool brute) {
@@ -1069,10 +1075,15 @@ static int launch_visibility_sets(const Scene& sc0, const WallSet* sets, int nse
       // once the points are sorted (it holds at least one word)
       uint32_t* next = sc.pscratch + (size_t)sc.B * P;
       const unsigned ctas = 8u * (unsigned)tune::sm_count();
+      // Walks in runs of 8 faces where whole chunks are few for 4,864 warps (5,000
+      // faces, 2,304 points: 0.84 against 0.98 of the patch kernel's time), of 32 else
+      // (a run's faces seed each other: 20,480 faces, 4,096 points 2.5 against 3.7 ms).
+      int parts = tune::get("mesh.visibility.list.parts");
+      if (parts != 1 && parts != 4) parts = ceil_div(P, 32) * sc.nch * sc.B < 24576 ? 4 : 1;
       TOTRI_CUDA(cudaMemsetAsync(next, 0, sizeof(uint32_t), stream));
       TOTRI_KERNEL("mesh visibility", stream,
                    visibility_walk_kernel<8><<<ctas, 32 * kListWarps, 0, stream>>>(
-                       sc, pts, P, row0, next, seed_mode, seed_steps));
+                       sc, pts, P, row0, next, parts, seed_mode, seed_steps));
       TOTRI_CUDA(cudaMemsetAsync(next, 0, sizeof(uint32_t), stream));
       TOTRI_KERNEL("mesh visibility list", stream,
                    visibility_list_kernel<8><<<ctas, 32 * kListWarps, 0, stream>>>(

@@ -515,6 +515,7 @@ struct WallPoints {  // the same on the device
   View3f pts;
   int P;
   uint32_t* scratch;
+  bool morton;  // the Morton order always
 };
 // Whether launch_visibility reads the points in Morton order.
 bool orders_points(bool brute);

@@ -29,6 +29,8 @@
 //   "mesh.visibility.queue"     1: queued BVH searches (visibility_queue_kernel)
 //   "mesh.visibility.list", ".list.cap" 1: front-facing targets over candidate lists always,
 //                               2: never (at its launcher) / most candidates in a list
+//   "mesh.visibility.list.parts" runs of a face chunk in its walk kernel (1, 4)
+//   "mesh.visibility.morton"    1: wall points in Morton order always
 //   "mesh.build.small"          2: small meshes take the build of large ones too
 //   "mesh.visibility.wide"      2: binary BVH search after the surface-walk prefix
 //                               (the default is the 4-wide search)
