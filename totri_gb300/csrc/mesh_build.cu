@@ -318,8 +318,10 @@ __device__ __forceinline__ uint32_t hilbert2(uint32_t x, uint32_t y) {
 // Points near a plane along two axes follow a Hilbert curve, whose runs of 32 stay
 // together on grids of any size: visibility of 20,480 faces from 56 x 56 points
 // took 5.2 ms over blocks in Morton order, which jumps inside a block there, and
-// 3.9 ms now; from 40 x 40, 4.1 and 2.8 ms; from 64 x 64, 4.6 and 4.5. Other points
-// take the Morton order, as all do with "mesh.visibility.morton" = 1. scr is
+// 3.9 ms now; from 40 x 40, 4.1 and 2.8 ms. Other points take the Morton order, as
+// all do with "mesh.visibility.morton" = 1, and so do 2^k points, whose grids' blocks
+// are whole in it (five meshes at 64 x 64 points: 5.13 ms in the mean, 5.27 along
+// the curve). scr is
 // [4][B][P] (keys, values, keys, values); the permutation (point indices in that
 // order) ends in the fourth quarter, and the first quarter is then set to -1: the
 // visibility kernel keeps each point's last occluder there (by the point's place).
@@ -353,7 +355,7 @@ __device__ __forceinline__ void point_order_item(const View3f& pts, int P, int B
   for (int a = 0; a < 3; ++a) ext[a] = iord(box[3 + a]) - iord(box[a]);
   const int thin = ext[0] <= ext[1] ? (ext[0] <= ext[2] ? 0 : 2) : (ext[1] <= ext[2] ? 1 : 2);
   const int ax = thin == 0 ? 1 : 0, ay = thin == 2 ? 1 : 2;
-  const bool flat = ext[thin] <= 0.25f * fminf(ext[ax], ext[ay]) && !morton;
+  const bool flat = ext[thin] <= 0.25f * fminf(ext[ax], ext[ay]) && (P & (P - 1)) != 0 && !morton;
   auto cell = [&](int i, int a, float cells) {
     float u = ext[a] > 0.f ? (pts.at(b, i, a) - iord(box[a])) / ext[a] : 0.f;
     u = fminf(fmaxf(u, 0.f), 1.f);
@@ -545,8 +547,8 @@ __device__ __forceinline__ void face_vertex_ids(const Scene& sc, int b, int k, u
   vi[2] = (uint32_t)__float_as_int(s[3].w);
 }
 
-__device__ __forceinline__ void edge_insert_item(const Scene& sc, int b, int k, unsigned long long* keys,
-                                                int2* vals) {
+__device__ __forceinline__ void edge_insert_item(const Scene& sc, int b, int k,
+                                                unsigned long long* keys, int2* vals) {
   if (k >= sc.meta[b].n) return;
   uint32_t vi[3];
   face_vertex_ids(sc, b, k, vi);
@@ -566,8 +568,9 @@ __device__ __forceinline__ void edge_insert_item(const Scene& sc, int b, int k, 
   }
 }
 
-__device__ __forceinline__ void edge_link_item(const Scene& sc, int b, int k, const unsigned long long* keys,
-                                                const int2* vals) {
+__device__ __forceinline__ void edge_link_item(const Scene& sc, int b, int k,
+                                              const unsigned long long* keys,
+                                              const int2* vals) {
   if (k >= sc.meta[b].n) return;
   uint32_t vi[3];
   face_vertex_ids(sc, b, k, vi);
@@ -630,7 +633,7 @@ __global__ void edge_link_kernel(Scene sc) {
               sc.evals + (size_t)b * sc.ecap);
 }
 
-// Morton order of one wall-point set per CTA: sets x batch items.
+// Order of one wall-point set per CTA: sets x batch items.
 __global__ void __launch_bounds__(kSortThreads) point_order_kernel(WallPoints w0, WallPoints w1,
                                                                   int B) {
   extern __shared__ uint32_t smem[];

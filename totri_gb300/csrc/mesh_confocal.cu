@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(256) visibility_kernel(Scene sc, View3f pts, i
   if (lane == 0) sc.mask[((size_t)b * sc.P + row0 + p) * sc.nch + ch] = word;
 }
 
-// One CTA per (block of 32 wall points in Morton order, run of `chunks`
+// One CTA per (block of 32 wall points in their order, run of `chunks`
 // 32-face chunks): each warp takes one face of the run at a time and its 32
 // lanes cast the rays from the 32 points, which lie on a compact patch of
 // the wall and end on the same centroid, so the lanes walk nearly the same BVH
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(32 * kWarps, kOcc) visibility_patch_kernel(Sce
   const View3f pts = second ? walls.pts1 : walls.pts0;
   const int P = second ? walls.P1 : walls.P0, row0 = second ? walls.row1 : walls.row0;
   uint32_t* scratch = sc.pscratch + 4 * (size_t)sc.B * row0;
-  // position in Morton order
+  // position in the order
   const int i = (int)(blockIdx.x - (second ? walls.blocks0 : 0u)) * 32 + lane;
   const int n = sc.meta[b].n;
   const bool okp = i < P;
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(256, kOcc) visibility_queue_kernel(Scene sc, V
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int b = blockIdx.z;
   const int ch0 = blockIdx.y * chunks;
-  const int i = blockIdx.x * 32 + lane;  // position in Morton order
+  const int i = blockIdx.x * 32 + lane;  // position in the order
   const int n = sc.meta[b].n;
   const bool okp = i < P;
   const uint32_t* order = sc.pscratch + 3 * (size_t)sc.B * P + (size_t)b * P;

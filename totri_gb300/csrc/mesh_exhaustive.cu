@@ -713,7 +713,8 @@ __global__ void __launch_bounds__(256, kOcc) exh_grad_face_kernel(
           }
           const float* col = colm + __float_as_int(ro[kRecAt]) * ostep;
           float4 w;  // area, weights of the vertices
-          if (!pair_weights<kLast>(col, bstep, T, e0, e1, e2, bw, inv_bw, fixed, order, w)) continue;
+          if (!pair_weights<kLast>(col, bstep, T, e0, e1, e2, bw, inv_bw, fixed, order, w))
+            continue;
           const float P = alpha * w.x, Q0 = alpha * w.y, Q1 = alpha * w.z, Q2 = alpha * w.w;
           used = true;
           gP += P;
@@ -1221,10 +1222,11 @@ int launch_exhaustive_splat(const Scene& sc, const View3f& sp, const View3f& lp,
     const int sms = tune::sm_count();
     const bool many = sc.F >= 4096;
     const bool few = all <= 16 * sms && T <= 1024;
+    const bool middling = all <= 48 * sms && sc.F >= 2 * T;
     const int ct = cols > 1 ? cols
-                   : all < 1024 || T > 2048 || !(many || few || (all <= 48 * sms && sc.F >= 2 * T)) ? 0
-                   : many && all >= 48 * sms ? 32
-                                                          : 8;
+                   : all < 1024 || T > 2048 || !(many || few || middling) ? 0
+                   : many && all >= 48 * sms                              ? 32
+                                                                          : 8;
     const int W = tune::get("mesh.exhaustive.splat.window");
     if (ct != 0) return launch_tile<false>(ct, sc, sp, lp, org, S, L, out, T, bw, bo, W, stream);
   }

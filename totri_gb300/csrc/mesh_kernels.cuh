@@ -517,13 +517,13 @@ struct WallPoints {  // the same on the device
   uint32_t* scratch;
   bool morton;  // the Morton order always
 };
-// Whether launch_visibility reads the points in Morton order.
+// Whether launch_visibility reads the points in order.
 bool orders_points(bool brute);
 // Masks of one or two wall-point sets, already ordered (build_scene) unless
 // order is set.
 int launch_visibility(const Scene& sc, const WallSet* sets, int nsets, bool brute, bool order,
                       cudaStream_t stream);
-// Morton orders of one or two wall-point sets.
+// Orders of one or two wall-point sets.
 int launch_point_order(const Scene& sc, const WallSet* sets, int nsets, cudaStream_t stream);
 // Wall-to-origin terms of the exhaustive renderer (detector and laser).
 struct Origins {
