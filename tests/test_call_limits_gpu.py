@@ -1,0 +1,74 @@
+"""Calls at the limits of what the entry points take: units, widths, counts and
+values far from an ordinary scan's, repeated calls, several faces per block."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from totri_gb300 import _lib, autotune, scenes
+from totri_gb300.totri_cpp import reconstruct as K
+from totri_gb300.totri_cpp import render as R
+
+pytestmark = pytest.mark.gpu
+
+START, END = (-0.5, -0.4, 0.5), (0.45, 0.5, 1.4)
+
+
+def cu(a):
+    return torch.as_tensor(np.ascontiguousarray(a)).cuda()
+
+
+def points(g, n, z=0.0):
+    return np.stack([g.uniform(-1, 1, n), g.uniform(-1, 1, n), np.full(n, z)], 1).astype(np.float32)
+
+
+def rel(a, b):
+    a = np.asarray(a, np.float64)
+    return float(np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-300))
+
+
+class tuned:
+    """Tuning keys set for a block."""
+
+    def __init__(self, keys):
+        self.keys = keys
+
+    def __enter__(self):
+        for k, v in self.keys.items():
+            autotune.set_tile(k, v)
+
+    def __exit__(self, *_):
+        for k in self.keys:
+            autotune.set_tile(k, 0)
+
+
+def sphere(faces, seed):
+    """A sphere in front of the wall: half of its faces are seen from behind."""
+    v, f, m = scenes.uv_sphere(faces, seed, center=(0.03, -0.05, 1.0))
+    return v.cuda(), f.cuda(), m.reshape(1, -1, 1).cuda()
+
+
+def mesh_masks(v, f, *walls):
+    vn, fn = v[0].cpu().numpy(), f[0].cpu().numpy()
+    return [oracle.mesh_visibility(vn, fn, p) for p in walls]
+
+
+@pytest.mark.parametrize("faces_per_block", [1, 2, 5, 32])
+def test_exhaustive_gradient_of_unseen_faces(cuda_lib, faces_per_block):
+    """Several faces per block, runs of them seen by no scan point (FP32 sums of a
+    vertex's few hundred pairs: 1e-5, as in the other exhaustive gradients)."""
+    g = np.random.default_rng(3)
+    v, f, m = sphere(2000, 8)
+    sp, lp = points(g, 40), points(g, 9)
+    none = torch.empty((1, 0, 3), device="cuda")
+    T, bw = 300, 0.02
+    tg = g.standard_normal((T, 40, 9)).astype(np.float32)
+    vn, fn, mn = (x[0].cpu().numpy() for x in (v, f, m))
+    rv, rm = oracle.mesh_exhaustive_grad(vn, fn, mn, sp, lp, None, None,
+                                         *mesh_masks(v, f, sp, lp), T, bw, 0.0, tg)
+    vg, mg = torch.empty_like(v), torch.empty_like(m)
+    with tuned({"mesh.exhaustive.grad.faces": faces_per_block}):
+        R.mesh_exhaustive_grad_verts(v, f, m, cu(sp[None]), cu(lp[None]), none, none,
+                                     cu(tg[None]), vg, mg, bw, 0.0, 0)
+    assert rel(vg[0].cpu().numpy(), rv) < 1e-5
+    assert rel(mg[0].cpu().numpy(), rm) < 1e-5

@@ -792,8 +792,10 @@ __global__ void __launch_bounds__(256, kOcc) exh_grad_face_kernel(
           if (vi[m] >= 0 && vi[m] < out.V)
             atomicAdd(out.mg + b * out.msb + vi[m] * out.msv, (1.f / 3.f) * t);
       }
-      __syncthreads();
     }
+    // the face's counts, records and sums have been read (a face that no scan point
+    // sees has come here past one barrier only)
+    __syncthreads();
   }
 }
 
