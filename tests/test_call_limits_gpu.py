@@ -72,3 +72,39 @@ def test_exhaustive_gradient_of_unseen_faces(cuda_lib, faces_per_block):
                                      cu(tg[None]), vg, mg, bw, 0.0, 0)
     assert rel(vg[0].cpu().numpy(), rv) < 1e-5
     assert rel(mg[0].cpu().numpy(), rm) < 1e-5
+
+
+def test_visibility_keys_changed_by_another_thread(cuda_lib):
+    """A call takes its visibility keys once: masks of one wall (mesh_visibility) and of
+    two (the exhaustive render, whose sums are those of the same pairs: 1e-5) while
+    another thread cycles the kernels that do and do not read the points in order."""
+    import threading
+    g = np.random.default_rng(5)
+    v, f, m = sphere(1700, 4)
+    sp, lp = cu(points(g, 200)[None]), cu(points(g, 35)[None])
+    none = torch.empty((1, 0, 3), device="cuda")
+    want = R.mesh_visibility(v, f, sp, brute_force=True)
+    ref = torch.empty((1, 200, 200, 35), device="cuda")
+    R.mesh_exhaustive_forward(v, f, m, sp, lp, none, none, ref, 0.03, 0.0, 0)
+    stop = threading.Event()
+
+    def cycle():
+        while not stop.is_set():
+            for mode in (3, 4, 1, 0):
+                autotune.set_tile("mesh.visibility.mode", mode)
+            for queue in (1, 0):
+                autotune.set_tile("mesh.visibility.queue", queue)
+
+    other = threading.Thread(target=cycle)
+    other.start()
+    try:
+        for _ in range(200):
+            assert torch.equal(R.mesh_visibility(v, f, sp), want)
+            out = torch.full_like(ref, 7.0)
+            R.mesh_exhaustive_forward(v, f, m, sp, lp, none, none, out, 0.03, 0.0, 0)
+            assert float((out - ref).norm() / ref.norm()) < 1e-5
+    finally:
+        stop.set()
+        other.join()
+        autotune.set_tile("mesh.visibility.mode", 0)
+        autotune.set_tile("mesh.visibility.queue", 0)

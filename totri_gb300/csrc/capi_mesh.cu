@@ -189,10 +189,11 @@ int confocal_grad_impl(const totri_array_t* verts, const totri_array_t* faces,
   }
   if (!reuse && !masks) {
     const mesh::WallSet wall{view3f(scan_points), (int)S, 0};
-    TOTRI_TRY(mesh::build_scene(sc, a.in, stream, &wall,
-                              occluded && mesh::orders_points(false) ? 1 : 0));
+    const mesh::VisKeys keys = mesh::visibility_keys(false);
+    TOTRI_TRY(
+        mesh::build_scene(sc, a.in, stream, &wall, occluded && keys.ordered() ? 1 : 0));
     if (occluded)
-      TOTRI_TRY(mesh::launch_visibility(sc, &wall, 1, false, false, stream));
+      TOTRI_TRY(mesh::launch_visibility(sc, &wall, 1, keys, false, stream));
     else
       TOTRI_TRY(all_visible(sc, S, stream));
   }
@@ -235,8 +236,9 @@ int exhaustive_masks(const mesh::Scene& sc, const ExhArgs& e, const totri_array_
                      const totri_array_t* laser_points, cudaStream_t stream) {
   const mesh::WallSet walls[2] = {{view3f(scan_points), (int)e.S, 0},
                                   {view3f(laser_points), (int)e.L, (int)e.S}};
-  TOTRI_TRY(mesh::build_scene(sc, e.m.in, stream, walls, mesh::orders_points(false) ? 2 : 0));
-  return mesh::launch_visibility(sc, walls, 2, false, false, stream);
+  const mesh::VisKeys keys = mesh::visibility_keys(false);
+  TOTRI_TRY(mesh::build_scene(sc, e.m.in, stream, walls, keys.ordered() ? 2 : 0));
+  return mesh::launch_visibility(sc, walls, 2, keys, false, stream);
 }
 
 int exhaustive_grad_impl(const totri_array_t* verts, const totri_array_t* faces,
@@ -325,10 +327,11 @@ static int confocal_forward_impl(const totri_array_t* verts, const totri_array_t
   TOTRI_TRY(check_workspace(ws, ws_bytes, L.total));
   const mesh::Scene sc = mesh::scene_from_workspace(ws, a.B, a.F, S);
   const mesh::WallSet wall{view3f(scan_points), (int)S, 0};
-  TOTRI_TRY(mesh::build_scene(sc, a.in, stream, &wall,
-                              occluded && mesh::orders_points(false) ? 1 : 0));
+  const mesh::VisKeys keys = mesh::visibility_keys(false);
+  TOTRI_TRY(
+      mesh::build_scene(sc, a.in, stream, &wall, occluded && keys.ordered() ? 1 : 0));
   if (occluded)
-    TOTRI_TRY(mesh::launch_visibility(sc, &wall, 1, false, false, stream));
+    TOTRI_TRY(mesh::launch_visibility(sc, &wall, 1, keys, false, stream));
   else
     TOTRI_TRY(all_visible(sc, S, stream));
   return mesh::launch_confocal_splat(sc, view3f(scan_points), view3f(scan_origin), has_origin,
@@ -492,9 +495,9 @@ int totri_mesh_visibility(const totri_array_t* verts, const totri_array_t* faces
   TOTRI_TRY(check_workspace(ws, ws_bytes, L.total));
   const mesh::Scene sc = mesh::scene_from_workspace(ws, a.B, a.F, P);
   const mesh::WallSet wall{view3f(points), (int)P, 0};
-  TOTRI_TRY(mesh::build_scene(sc, a.in, stream, &wall,
-                              mesh::orders_points(brute_force != 0) ? 1 : 0));
-  TOTRI_TRY(mesh::launch_visibility(sc, &wall, 1, brute_force != 0, false, stream));
+  const mesh::VisKeys keys = mesh::visibility_keys(brute_force != 0);
+  TOTRI_TRY(mesh::build_scene(sc, a.in, stream, &wall, keys.ordered() ? 1 : 0));
+  TOTRI_TRY(mesh::launch_visibility(sc, &wall, 1, keys, false, stream));
   return mesh::launch_mask_unsort(sc, (int)P, static_cast<uint32_t*>(mask->data), stream);
 }
 
@@ -528,7 +531,7 @@ int totri_mesh_prepared_visibility(const totri_array_t* verts, const totri_array
   TOTRI_TRY(check_masks(masks, masks_bytes, a.B, a.F, P));
   const mesh::Scene sc = mesh::scene_with_masks(const_cast<void*>(ws), a.B, a.F, masks, P);
   const mesh::WallSet wall{view3f(points), (int)P, 0};
-  return mesh::launch_visibility(sc, &wall, 1, false, true, stream);
+  return mesh::launch_visibility(sc, &wall, 1, mesh::visibility_keys(false), true, stream);
 }
 
 int totri_mesh_prepared_confocal_forward(const totri_array_t* verts, const totri_array_t* faces,

@@ -991,21 +991,28 @@ int launch_mask_unsort(const Scene& sc, int P, uint32_t* out, cudaStream_t strea
 // 2,444, a box 2,751 against 5,842; 1,280, 4,096 points 324 against 361). Below,
 // 1.0-1.3x, and 1.1-1.4x at 576 points (20,000 faces 2,333 against 2,067).
 // "mesh.visibility.list": 1 always, 2 never; ".list.cap" lowers the list's capacity.
-static bool list_rule(const Scene& sc, int P) {
-  const int list = tune::get("mesh.visibility.list");
+static bool list_rule(const Scene& sc, int P, const VisKeys& keys) {
   const int64_t units = ceil_div(P, 32) * sc.nch * sc.B;
-  return tune::get("mesh.visibility.mode") == 0 && tune::get("mesh.visibility.wide") != 2 &&
-         tune::get("mesh.visibility.queue") != 1 && tune::get("mesh.visibility.occupancy") == 0 &&
-         (list == 1 || (list == 0 && P >= 1024 && units >= 5000)) && units < ((int64_t)1 << 29);
+  return keys.mode == 0 && keys.wide != 2 && keys.queue != 1 && keys.occupancy == 0 &&
+         (keys.list == 1 || (keys.list == 0 && P >= 1024 && units >= 5000)) &&
+         units < ((int64_t)1 << 29);
 }
 
-bool orders_points(bool brute) {
-  const int mode = tune::get("mesh.visibility.mode");
+VisKeys visibility_keys(bool brute) {
+  return VisKeys{brute,
+                 tune::get("mesh.visibility.mode"),
+                 tune::get("mesh.visibility.queue"),
+                 tune::get("mesh.visibility.list"),
+                 tune::get("mesh.visibility.wide"),
+                 tune::get("mesh.visibility.occupancy")};
+}
+
+bool VisKeys::ordered() const {
   return !brute && mode != kVisRay && mode != kVisPacket && mode != kVisRayPostponed;
 }
 
-static int launch_visibility_sets(const Scene& sc0, const WallSet* sets, int nsets, bool brute,
-                                  cudaStream_t stream) {
+static int launch_visibility_sets(const Scene& sc0, const WallSet* sets, int nsets,
+                                  const VisKeys& keys, cudaStream_t stream) {
   // (the kernels over one set find its scratch at sc.pscratch)
   const View3f& pts = sets[0].pts;
   const int row0 = sets[0].row0;
@@ -1018,16 +1025,16 @@ static int launch_visibility_sets(const Scene& sc0, const WallSet* sets, int nse
   const int64_t units = (int64_t)sc.B * P * sc.nch;
   if (units == 0) return TOTRI_OK;
   const unsigned blocks = (unsigned)ceil_div(units * 32, 256);
-  if (brute) {
+  if (keys.brute) {
     TOTRI_KERNEL("mesh visibility brute", stream,
                  visibility_kernel<kVisBrute><<<blocks, 256, 0, stream>>>(sc, pts, P, row0));
-  } else if (tune::get("mesh.visibility.mode") == kVisRay) {
+  } else if (keys.mode == kVisRay) {
     TOTRI_KERNEL("mesh visibility", stream,
                  visibility_kernel<kVisRay><<<blocks, 256, 0, stream>>>(sc, pts, P, row0));
-  } else if (tune::get("mesh.visibility.mode") == kVisPacket) {
+  } else if (keys.mode == kVisPacket) {
     TOTRI_KERNEL("mesh visibility", stream,
                  visibility_kernel<kVisPacket><<<blocks, 256, 0, stream>>>(sc, pts, P, row0));
-  } else if (tune::get("mesh.visibility.mode") == kVisRayPostponed) {
+  } else if (keys.mode == kVisRayPostponed) {
     TOTRI_KERNEL("mesh visibility", stream,
                  visibility_kernel<kVisRayPostponed><<<blocks, 256, 0, stream>>>(sc, pts, P,
                                                                                   row0));
@@ -1054,21 +1061,20 @@ static int launch_visibility_sets(const Scene& sc0, const WallSet* sets, int nse
     if (shaft_cap <= 0 || shaft_cap > kShaftCand) shaft_cap = kShaftCand;
     const dim3 grid((unsigned)patches, (unsigned)ceil_div(sc.nch, chunks),
                     (unsigned)sc.B);
-    const int mode = tune::get("mesh.visibility.mode");
     const int64_t cta_count = (int64_t)grid.x * grid.y * grid.z;
-    if (mode == kVisPatchPacket)
+    if (keys.mode == kVisPatchPacket)
       TOTRI_KERNEL("mesh visibility", stream,
                    visibility_patch_kernel<1><<<grid, 256, 0, stream>>>(
                        sc0, walls, chunks, kSeedOff, 0, 0));
-    else if (mode == kVisPatchWide)
+    else if (keys.mode == kVisPatchWide)
       TOTRI_KERNEL("mesh visibility", stream,
                    visibility_patch_kernel<2><<<grid, 256, 0, stream>>>(
                        sc0, walls, chunks, kSeedOff, 0, 0));
-    else if (mode == kVisPatchShaft)
+    else if (keys.mode == kVisPatchShaft)
       TOTRI_KERNEL("mesh visibility", stream,
                    visibility_patch_kernel<3><<<grid, 256, 0, stream>>>(
                        sc0, walls, chunks, seed_mode, seed_steps, shaft_cap));
-    else if (nsets == 1 && list_rule(sc, P)) {
+    else if (nsets == 1 && list_rule(sc, P, keys)) {
       int cap = tune::get("mesh.visibility.list.cap");
       if (cap <= 0 || cap > kListCand) cap = kListCand;
       // the queues' counters: the second quarter of the point scratch is free
@@ -1095,8 +1101,8 @@ static int launch_visibility_sets(const Scene& sc0, const WallSet* sets, int nse
     // registers, spilling) and 9.26 ms for the 4-wide search capped at 5, per
     // mesh_visibility call on the differentiable workload (build included).
     // "mesh.visibility.wide" = 2 selects the binary search.
-    else if (tune::get("mesh.visibility.wide") != 2 && tune::get("mesh.visibility.queue") != 1) {
-      if (tune::get("mesh.visibility.occupancy") == 5)
+    else if (keys.wide != 2 && keys.queue != 1) {
+      if (keys.occupancy == 5)
         TOTRI_KERNEL("mesh visibility", stream,
                      visibility_patch_kernel<4, 5><<<grid, 256, 0, stream>>>(
                          sc0, walls, chunks, seed_mode, seed_steps, 0));
@@ -1119,8 +1125,8 @@ static int launch_visibility_sets(const Scene& sc0, const WallSet* sets, int nse
     // The queued BVH searches (visibility_queue_kernel) when
     // "mesh.visibility.queue" = 1; queue entries pack the target's Morton
     // position in 26 bits.
-    else if (tune::get("mesh.visibility.queue") == 1 && sc.F < (1 << 26)) {
-      if (tune::get("mesh.visibility.occupancy") == 4)
+    else if (keys.queue == 1 && sc.F < (1 << 26)) {
+      if (keys.occupancy == 4)
         TOTRI_KERNEL("mesh visibility", stream,
                      visibility_queue_kernel<4><<<grid, 256, 0, stream>>>(
                          sc, pts, P, row0, chunks, seed_mode, seed_steps));
@@ -1132,15 +1138,15 @@ static int launch_visibility_sets(const Scene& sc0, const WallSet* sets, int nse
     // Registers capped for 5 CTAs per SM (48 a thread, 28 bytes of spills):
     // 8.84 ms against 9.33 ms uncapped (60 registers, 4 CTAs) and 9.03 ms at
     // 6 CTAs (40 registers) inside the differentiable 20,480-face step.
-    else if (tune::get("mesh.visibility.occupancy") == 1)
+    else if (keys.occupancy == 1)
       TOTRI_KERNEL("mesh visibility", stream,
                    visibility_patch_kernel<0, 1><<<grid, 256, 0, stream>>>(
                        sc0, walls, chunks, seed_mode, seed_steps, 0));
-    else if (tune::get("mesh.visibility.occupancy") == 4)
+    else if (keys.occupancy == 4)
       TOTRI_KERNEL("mesh visibility", stream,
                    visibility_patch_kernel<0, 4><<<grid, 256, 0, stream>>>(
                        sc0, walls, chunks, seed_mode, seed_steps, 0));
-    else if (tune::get("mesh.visibility.occupancy") == 6)
+    else if (keys.occupancy == 6)
       TOTRI_KERNEL("mesh visibility", stream,
                    visibility_patch_kernel<0, 6><<<grid, 256, 0, stream>>>(
                        sc0, walls, chunks, seed_mode, seed_steps, 0));
@@ -1152,20 +1158,20 @@ static int launch_visibility_sets(const Scene& sc0, const WallSet* sets, int nse
   return TOTRI_OK;
 }
 
-int launch_visibility(const Scene& sc, const WallSet* sets, int nsets, bool brute, bool order,
-                      cudaStream_t stream) {
-  if (order && orders_points(brute)) {
+int launch_visibility(const Scene& sc, const WallSet* sets, int nsets, const VisKeys& keys,
+                      bool order, cudaStream_t stream) {
+  if (order && keys.ordered()) {
     const int st = launch_point_order(sc, sets, nsets, stream);
     if (st != TOTRI_OK) return st;
   }
   // Two sets go in one launch of visibility_patch_kernel where that is the
   // kernel for both (no key selects another one, neither set takes the lists).
-  const bool one = nsets == 2 && !brute && tune::get("mesh.visibility.mode") == 0 &&
-                   tune::get("mesh.visibility.queue") != 1 && sets[0].P > 0 && sets[1].P > 0 &&
-                   !list_rule(sc, sets[0].P) && !list_rule(sc, sets[1].P);
-  if (one) return launch_visibility_sets(sc, sets, 2, brute, stream);
+  const bool one = nsets == 2 && !keys.brute && keys.mode == 0 && keys.queue != 1 &&
+                   sets[0].P > 0 && sets[1].P > 0 && !list_rule(sc, sets[0].P, keys) &&
+                   !list_rule(sc, sets[1].P, keys);
+  if (one) return launch_visibility_sets(sc, sets, 2, keys, stream);
   for (int j = 0; j < nsets; ++j) {
-    const int st = launch_visibility_sets(sc, sets + j, 1, brute, stream);
+    const int st = launch_visibility_sets(sc, sets + j, 1, keys, stream);
     if (st != TOTRI_OK) return st;
   }
   return TOTRI_OK;

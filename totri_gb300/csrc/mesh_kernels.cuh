@@ -517,12 +517,19 @@ struct WallPoints {  // the same on the device
   uint32_t* scratch;
   bool morton;  // the Morton order always
 };
-// Whether launch_visibility reads the points in order.
-bool orders_points(bool brute);
+// The tuning keys that choose among the visibility kernels, read once per call:
+// whether the build orders the points and which kernel reads them must agree when
+// another thread changes a key in between.
+struct VisKeys {
+  bool brute;
+  int mode, queue, list, wide, occupancy;
+  bool ordered() const;  // whether the kernel reads the points in order
+};
+VisKeys visibility_keys(bool brute);
 // Masks of one or two wall-point sets, already ordered (build_scene) unless
 // order is set.
-int launch_visibility(const Scene& sc, const WallSet* sets, int nsets, bool brute, bool order,
-                      cudaStream_t stream);
+int launch_visibility(const Scene& sc, const WallSet* sets, int nsets, const VisKeys& keys,
+                      bool order, cudaStream_t stream);
 // Orders of one or two wall-point sets.
 int launch_point_order(const Scene& sc, const WallSet* sets, int nsets, cudaStream_t stream);
 // Wall-to-origin terms of the exhaustive renderer (detector and laser).
