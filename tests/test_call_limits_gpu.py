@@ -108,3 +108,24 @@ def test_visibility_keys_changed_by_another_thread(cuda_lib):
         other.join()
         autotune.set_tile("mesh.visibility.mode", 0)
         autotune.set_tile("mesh.visibility.queue", 0)
+
+
+@pytest.mark.parametrize("seed", [1, 3, 7])
+def test_volume_pairs_whose_offset_takes_most_of_the_path(cuda_lib, seed):
+    """Bins of 2e-8 at a path of 2.26 less an offset of 2.26: the lengths' roundings are
+    several bins, so a block's bins have no sound bounds. FP32 fractions of the
+    oracle's bins: 1e-5, as in the other gradients."""
+    g = np.random.default_rng(seed)
+    a, b, r, q = g.uniform(0, 6.28, 24), g.uniform(0, 6.28, 9), 0.6, 0.45
+    sp = np.stack([r * np.cos(a), r * np.sin(a), 0 * a], 1).astype(np.float32)
+    lp = np.stack([q * np.cos(b), q * np.sin(b), 0 * b], 1).astype(np.float32)
+    st, en = (0.0, 0.0, 1.0), (1e-6, 1e-6, 1.000001)
+    T, bw, bo = 12000, 2e-8, float(np.sqrt(1 + r * r) + np.sqrt(1 + q * q) - 1e-4)
+    tg = g.uniform(0.5, 1.5, (T, 24, 9)).astype(np.float32)
+    none = torch.empty((1, 3, 0), device="cuda")
+    out = torch.empty((1, 4, 4, 4), device="cuda")
+    R.volume_render_exhaustive_grad_volume(cu(tg[None]), cu(sp.T[None]), cu(lp.T[None]), none,
+                                           none, out, st, en, bw, bo)
+    ref = oracle.volume_exhaustive_adjoint(tg, (4, 4, 4), sp.T, lp.T, st, en, bw, bo)
+    assert np.linalg.norm(ref) > 0.0
+    assert rel(out[0].cpu().numpy(), ref) < 1e-5
