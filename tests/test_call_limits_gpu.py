@@ -129,3 +129,25 @@ def test_volume_pairs_whose_offset_takes_most_of_the_path(cuda_lib, seed):
     ref = oracle.volume_exhaustive_adjoint(tg, (4, 4, 4), sp.T, lp.T, st, en, bw, bo)
     assert np.linalg.norm(ref) > 0.0
     assert rel(out[0].cpu().numpy(), ref) < 1e-5
+
+
+@pytest.mark.parametrize("bo", [2.5, 3.2, 6.5])
+def test_volume_pairs_with_a_negative_bin_width(cuda_lib, bo):
+    """Time running backwards, with voxels whose later end is past [0, T) and whose
+    earlier one is inside: such a voxel adds nothing, in the forward and in the
+    gradient alike (the two are adjoint: 1e-5 of the product of the norms)."""
+    g = np.random.default_rng(11)
+    shape, S, L, T = (6, 7, 9), 5, 9, 100
+    sp, lp = (cu(points(g, n).T[None]) for n in (S, L))
+    none = torch.empty((1, 3, 0), device="cuda")
+    vol = cu(g.uniform(0.5, 1.5, (1,) + shape).astype(np.float32))
+    y = cu(g.uniform(0.5, 1.5, (1, T, S, L)).astype(np.float32))
+    out = torch.empty_like(y)
+    R.volume_render_exhaustive_forward(vol, sp, lp, none, none, out, START, END, -0.04, bo)
+    grad = torch.empty_like(vol)
+    R.volume_render_exhaustive_grad_volume(y, sp, lp, none, none, grad, START, END, -0.04, bo)
+    out, grad, vol, y = (t.double() for t in (out, grad, vol, y))
+    assert bool(torch.isfinite(out).all()) and bool(torch.isfinite(grad).all())
+    scale = float(out.norm() * y.norm() + grad.norm() * vol.norm())
+    assert scale > 0.0
+    assert abs(float((out * y).sum() - (grad * vol).sum())) < 1e-5 * scale

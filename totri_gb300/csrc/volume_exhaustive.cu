@@ -90,6 +90,7 @@ __device__ __forceinline__ Interval interval(const Geo& g, float d0, float d1) {
     bf1 = (float)(g.T - 1);
     last = g.T - 1;
   }
+  if (first >= g.T || last < 0) return r;  // (a negative bin width: first is the later one)
   r.ok = true;
   r.first = first;
   r.last = last;
