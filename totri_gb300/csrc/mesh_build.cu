@@ -636,7 +636,7 @@ __global__ void edge_link_kernel(Scene sc) {
 // Order of one wall-point set per CTA: sets x batch items.
 __global__ void __launch_bounds__(kSortThreads) point_order_kernel(WallPoints w0, WallPoints w1,
                                                                   int B) {
-  extern __shared__ uint32_t smem[];
+  extern __shared__ __align__(16) uint32_t smem[];
   __shared__ int box[6];
   const WallPoints& w = blockIdx.y ? w1 : w0;
   point_order_item(w.pts, w.P, B, blockIdx.x, w.scratch, smem, box, w.morton);
@@ -645,7 +645,7 @@ __global__ void __launch_bounds__(kSortThreads) point_order_kernel(WallPoints w0
 // One CTA per mesh (blockIdx.y = 0) and, beside it, per wall-point set.
 __global__ void __launch_bounds__(kSortThreads) sort_kernel(Scene sc, WallPoints w0,
                                                            WallPoints w1) {
-  extern __shared__ uint32_t smem[];
+  extern __shared__ __align__(16) uint32_t smem[];
   __shared__ int box[6];
   const int b = blockIdx.x;
   if (blockIdx.y > 0) {
@@ -671,7 +671,7 @@ constexpr int kSortWords = 32 * kSortDigits + 2 * kSortDigits;
 static_assert(17 * kSmallFaces <= kSortWords, "edge table and counters fit the sort's memory");
 __global__ void __launch_bounds__(kSortThreads) build_small_kernel(Scene sc, BuildInputs in,
                                                                   WallPoints w0, WallPoints w1) {
-  extern __shared__ uint32_t smem[];
+  extern __shared__ __align__(16) uint32_t smem[];
   __shared__ int box[6];
   const int b = blockIdx.x, tid = threadIdx.x;
   if (blockIdx.y > 0) {

@@ -884,7 +884,8 @@ __global__ void __launch_bounds__(256, 3) confocal_adjoint_columns_kernel(
   // cell za + slab, the next slab's first)
   const int za = blockIdx.z * slab, zb = min(g.Z, za + slab), zn = min(zb, g.Z - 1) - za;
   const int rows = slab + 1;
-  extern __shared__ float acc[];  // [warp][rows][32], [warp][32] bin values, the bin table
+  // [warp][rows][32], [warp][32] bin values, the bin table
+  extern __shared__ __align__(16) float acc[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   float4* vbuf = reinterpret_cast<float4*>(acc + (size_t)nw * rows * 32 + warp * 32);
   float4* tab = reinterpret_cast<float4*>(acc + (size_t)nw * (rows + 1) * 32);
