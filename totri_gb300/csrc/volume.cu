@@ -41,7 +41,7 @@ __device__ __forceinline__ float centre(float o, float s, int n, int i) {
 struct Sample {
   bool ok;
   int zi;
-  float alpha, f2;
+  float alpha, f1, f2;  // f1 = (depth / tc^2)^2, f2 = f1^2
 };
 
 // The reference's sample at (point w, bin t, column x/y) (volume_cuda.cu:23-57):
@@ -49,7 +49,7 @@ struct Sample {
 // rounding per operation; alpha and f2 are values.
 __device__ __forceinline__ Sample sample(const Geo& g, float wx, float wy, float wz, int t,
                                          float x, float y) {
-  Sample s{false, 0, 0.f, 0.f};
+  Sample s{false, 0, 0.f, 0.f, 0.f};
   const float tc = xadd(xmul((float)t, g.bw), g.bo);
   const float dx = xsub(wx, x), dy = xsub(wy, y);
   const float d2 = xsub(xsub(xmul(tc, tc), xmul(dx, dx)), xmul(dy, dy));
@@ -63,7 +63,8 @@ __device__ __forceinline__ Sample sample(const Geo& g, float wx, float wy, float
   s.zi = (int)fl;
   s.alpha = zh - fl;
   const float q = __fdividef(depth, tc * tc);  // a value: the hardware reciprocal (2 ulp)
-  s.f2 = (q * q) * (q * q);
+  s.f1 = q * q;
+  s.f2 = s.f1 * s.f1;
   return s;
 }
 
@@ -81,7 +82,7 @@ __device__ __forceinline__ Sample sample(const Geo& g, float wx, float wy, float
 __device__ __forceinline__ Sample sample_filtered(const Geo& g, float wx, float wy, float wz,
                                                   int t, float x, float y) {
   if (g.exact) return sample(g, wx, wy, wz, t, x, y);
-  Sample s{false, 0, 0.f, 0.f};
+  Sample s{false, 0, 0.f, 0.f, 0.f};
   const float tc = xadd(xmul((float)t, g.bw), g.bo);
   const float dx = xsub(wx, x), dy = xsub(wy, y);
   const float d2 = xsub(xsub(xmul(tc, tc), xmul(dx, dx)), xmul(dy, dy));
@@ -100,7 +101,8 @@ __device__ __forceinline__ Sample sample_filtered(const Geo& g, float wx, float 
   s.zi = (int)fl;
   s.alpha = fr;
   const float q = __fdividef(depth, tc * tc);
-  s.f2 = (q * q) * (q * q);
+  s.f1 = q * q;
+  s.f2 = s.f1 * s.f1;
   return s;
 }
 
@@ -211,8 +213,10 @@ __global__ void compact_kernel(Geo g, const float* __restrict__ vol, int64_t n, 
 
 constexpr int kPT = 8;  // points per CTA of grad_mp_wide_kernel
 
-// Table entries of two bins each: (tc^2, tc^2, 1 / tc^8, 1 / tc^8) of bins 2 i
-// and 2 i + 1, padded to a multiple of four bins.
+// Table entries of two bins each: (tc^2, tc^2, 1 / tc^4, 1 / tc^4) of bins 2 i
+// and 2 i + 1, padded to a multiple of four bins. A sample's f2 = (depth / tc^2)^4 is
+// (d2 / tc^4)^2: 1 / tc^8 and d2^2, whose product it is too, leave the FP32 range at tc
+// of 4e5 and 1e-5 (a scene of a metre in micrometres, or in light microseconds).
 __host__ __device__ constexpr int bin_table(int T) { return 2 * ((T + 3) / 4); }
 
 // One measurement point's constants for the walks over occupied voxels.
@@ -238,12 +242,12 @@ __device__ __forceinline__ WalkPoint walk_point(const Geo& g, float wx, float wy
   return p;
 }
 
-// Calls f(t, lower, fr, d2, i8, depth) for every sample of the point in the
+// Calls f(t, lower, fr, a, b, depth), f2 = (a b)^2, for every sample of the point in the
 // interpolation cells of an occupied voxel (column centre x, y, cell k): lower
 // is true for cell k (the voxel is its lower node, weight 1 - fr) and false for
 // cell k - 1 (weight fr). The bins come from inverting the column geometry,
 // widened by span_eps, two at a time from an even one with paired FP32
-// instructions; tab holds (tc^2, tc^2, 1 / tc^8, 1 / tc^8) of each two. The depth
+// instructions; tab holds (tc^2, tc^2, 1 / tc^4, 1 / tc^4) of each two. The depth
 // is the hardware reciprocal square root's with one remainder correction
 // (within an ulp of the correctly rounded root), the cell coordinate the
 // exact chain's operations on it; where its fraction lies within the margin of a
@@ -279,7 +283,7 @@ __device__ __forceinline__ void walk_voxel(const Geo& g, const float4* tab, cons
     for (int t = t0 & ~1; t <= t1; t += 2) {
       const float4 tb = tab[t >> 1];
       const u64 d2 = f2add(f2add(f2pack(tb.x, tb.y), ndx), ndy);
-      float d[2], z[2], fr[2], off[2], depth[2];
+      float d[2], z[2], fr[2], off[2], depth[2], i4[2] = {tb.z, tb.w};
       f2unpack(d2, d[0], d[1]);
       const float r0 = rsqrt_approx(d[0]), r1 = rsqrt_approx(d[1]);
       u64 q = f2mul(d2, f2pack(r0, r1));
@@ -300,9 +304,11 @@ __device__ __forceinline__ void walk_voxel(const Geo& g, const float4* tab, cons
           const Sample sm = sample(g, p.wx, p.wy, p.wz, t + h, x, y);
           cell = sm.ok ? 0x4B400000 + sm.zi : -1;
           fr[h] = sm.alpha;
+          d[h] = sm.f1;
+          i4[h] = 1.f;
         }
         if (cell == lower || cell == upper)
-          f(t + h, cell == lower, fr[h], d[h], h ? tb.w : tb.z, depth[h]);
+          f(t + h, cell == lower, fr[h], d[h], i4[h], depth[h]);
       }
     }
   }
@@ -311,16 +317,16 @@ __device__ __forceinline__ void walk_voxel(const Geo& g, const float4* tab, cons
 // The bin table of walk_voxel, in shared memory; all threads of the CTA.
 __device__ __forceinline__ void fill_bin_table(const Geo& g, float4* tab) {
   for (int i = threadIdx.x; i < bin_table(g.T); i += blockDim.x) {
-    float tc2[2], i8[2];
+    float tc2[2], i4[2];
     for (int h = 0; h < 2; ++h) {
       const int t = 2 * i + h;
       const float tc = xadd(xmul((float)t, g.bw), g.bo);
       tc2[h] = xmul(tc, tc);
       const float i2 = __fdividef(1.f, tc2[h]);
-      i8[h] = (i2 * i2) * (i2 * i2);
-      if (t >= g.T) tc2[h] = -INFINITY, i8[h] = 0.f;  // padding: no sample
+      i4[h] = i2 * i2;
+      if (t >= g.T) tc2[h] = -INFINITY, i4[h] = 0.f;  // padding: no sample
     }
-    tab[i] = make_float4(tc2[0], tc2[1], i8[0], i8[1]);
+    tab[i] = make_float4(tc2[0], tc2[1], i4[0], i4[1]);
   }
 }
 
@@ -354,9 +360,9 @@ __global__ void __launch_bounds__(32 * PT > 256 ? 32 * PT : 256) confocal_forwar
     for (uint32_t v = v0 + threadIdx.x / PT; v < v1; v += blockDim.x / PT) {
       const float4 rec = __ldg(recs + v);
       walk_voxel<kSigned>(g, tab, p, tz, rec.x, rec.y, __float_as_int(rec.w),
-                          [&](int t, bool lower, float fr, float d2, float i8, float) {
-                            const float w = lower ? 1.f - fr : fr;
-                            atomicAdd(col + t * PT, rec.z * w * ((d2 * d2) * i8));
+                          [&](int t, bool lower, float fr, float a, float b, float) {
+                            const float w = lower ? 1.f - fr : fr, f1 = a * b;
+                            atomicAdd(col + t * PT, rec.z * w * (f1 * f1));
                           });
     }
   }
@@ -406,18 +412,19 @@ __global__ void __launch_bounds__(32 * PT > 256 ? 32 * PT : 256) grad_mp_kernel(
       const float4 rec = __ldg(recs + v);
       // with f2 = (depth / tc^2)^4 and w the interpolation weight, d(w f2) / d depth
       // = w 4 f2 / depth +- scale f2, and d depth / d(wx, wy) = -(wx - x, wy - y) / depth
+      // (lengths of the quotient in slices, so that it keeps the range of the result)
       float radial = 0.f, axial = 0.f;
       walk_voxel<kSigned>(g, tab, p, tz, rec.x, rec.y, __float_as_int(rec.w),
-                          [&](int t, bool lower, float fr, float d2, float i8, float depth) {
-                            const float w = lower ? 1.f - fr : fr;
-                            const float df2 = col[t * PT] * ((d2 * d2) * i8);
+                          [&](int t, bool lower, float fr, float a, float b, float depth) {
+                            const float w = lower ? 1.f - fr : fr, f1 = a * b;
+                            const float df2 = col[t * PT] * (f1 * f1);
                             const float slope = lower ? -g.scale * df2 : g.scale * df2;
                             const float inv = __fdividef(1.f, depth);
-                            radial += fmaf(4.f * w * df2, inv, slope) * inv;
+                            radial += fmaf(4.f * w * df2, inv, slope) * (inv * g.dz);
                             axial += slope;
                           });
-      gx -= rec.z * (p.wx - rec.x) * radial;
-      gy -= rec.z * (p.wy - rec.y) * radial;
+      gx -= rec.z * ((p.wx - rec.x) * g.scale) * radial;
+      gy -= rec.z * ((p.wy - rec.y) * g.scale) * radial;
       gz += rec.z * axial;
     }
   }
@@ -778,9 +785,9 @@ struct AdjPoint {
 // boundary go through the exact chain. The step may touch up to three bins on
 // each side of [t0, t1]: without kCheck (no negative bin centres) those are real
 // bins, rejected unless they hold a sample, or table padding (tc^2 = -inf); with
-// kCheck they belong to the other walk and are skipped. Each sample's values
-// are those of sample_filtered or, near a boundary, of the exact chain, bit
-// for bit.
+// kCheck they belong to the other walk and are skipped. A sample's cell is the exact
+// chain's; its fraction and f2 are values of the paired arithmetic or, near a
+// boundary, of the exact chain.
 template <bool kCheck>
 __device__ __forceinline__ void adj_walk(const Geo& g, const float4* __restrict__ tab,
                                          float4* vbuf, const float* __restrict__ row,
@@ -820,8 +827,8 @@ __device__ __forceinline__ void adj_walk(const Geo& g, const float4* __restrict_
         const u64 fr = f2sub(zh, f2sub(fx, big));
         f2unpack(fx, xa, xb);
         f2unpack(f2add(fr, half), off[2 * h], off[2 * h + 1]);
-        const u64 v = f2mul(f2mul(f2mul(d2, d2), f2pack(tb.z, tb.w)),
-                            h ? f2pack(v4.z, v4.w) : f2pack(v4.x, v4.y));
+        const u64 fall = f2mul(d2, f2pack(tb.z, tb.w));
+        const u64 v = f2mul(fall, f2mul(fall, h ? f2pack(v4.z, v4.w) : f2pack(v4.x, v4.y)));
         const u64 upper = f2mul(fr, v);
         f2unpack(upper, w1[2 * h], w1[2 * h + 1]);
         f2unpack(f2sub(v, upper), w0[2 * h], w0[2 * h + 1]);
@@ -853,8 +860,8 @@ __device__ __forceinline__ void adj_walk(const Geo& g, const float4* __restrict_
 // voxel columns (an 8 x 4 tile: y fastest) and all lanes on one point and one
 // bin at a time. The point's transient row is then read once per warp (32 bins
 // per coalesced load), and the bin's tc^2 (the sample chain's FP32 value) and
-// 1 / tc^8 come from a per-CTA table in shared memory (broadcast reads), so f2 =
-// (depth / tc^2)^4 = d2^2 / tc^8 needs no second special-function op. A CTA
+// 1 / tc^4 come from a per-CTA table in shared memory (broadcast reads), so f2 =
+// (depth / tc^2)^4 = (d2 / tc^4)^2 needs no second special-function op. A CTA
 // takes one slab of the columns' cells (the samples whose cell pair starts
 // there; the pair's second cell may be the next slab's first, one extra row),
 // and each lane owns its column's cells of the slab in shared memory
