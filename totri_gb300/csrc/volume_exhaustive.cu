@@ -24,6 +24,12 @@ struct Geo {
   int D, H, W, S, L, T;
   float sx, sy, sz, ex, ey, ez, bw, bo;
   float inv_bw;  // 1 / bw for div_fixed; NaN where it does not apply (every pair is exact)
+  // The farthest path whose bins have sound bounds in adjoint_kernel. With u = 2^-24
+  // the exact chain's lengths and the bounds' each lie within 8 u far of the true ones,
+  // and the offset adds u |bo| to either difference: a window's extra bin each side
+  // holds them while 16 u (far + |bo|) is below half a bin width. (At a bin width of
+  // 2e-8, a path of 2.26 less an offset of 2.26 missed one bin in 2,000 by more.)
+  float window_far;
 };
 
 struct Pts {  // [B, 3, n] with strides
@@ -257,13 +263,7 @@ __global__ void __launch_bounds__(256, 4) adjoint_kernel(Geo g, int b, Pts sp, P
       const float far = __shfl_sync(0xffffffffu, sfar, (s - s0) & 31) + lfar;
       const float c0 = (near - g.bo) / g.bw, c1 = (far - g.bo) / g.bw;
       int2 w = make_int2(0, 0);
-      // With u = 2^-24 the exact chain's lengths and these bounds each lie within 8 u
-      // far of the true ones, and the offset adds u |bo| to either difference: the
-      // window's extra bin each side holds them while 16 u (far + |bo|) is below half
-      // a bin. (A bin width of 2e-8 at a path of 2.26 less an offset of 2.26 missed one
-      // bin in 2,000 by more.) NaN: no window.
-      const bool sound = 9.5367432e-7f * (far + fabsf(g.bo)) < 0.5f * g.bw;
-      if (sound && c0 > -262144.f && c1 < 262144.f) {
+      if (far < g.window_far && c0 > -262144.f && c1 < 262144.f) {  // (NaN: no window)
         w.x = max((int)floorf(c0) - 1, 0);
         w.y = min((int)floorf(c1) + 1, g.T - 1) - w.x + 1;
         if (w.y > kRows || w.y < 0) w.y = 0;
@@ -353,7 +353,8 @@ int check_pts(const totri_array_t* a, const char* name, int64_t B, int64_t& n, v
 vexh::Geo make_geo(const totri_array_t* vol, int64_t S, int64_t L, int64_t T, const float* start,
                    const float* end, float bw, float bo) {
   vexh::Geo g{(int)vol->shape[1], (int)vol->shape[2], (int)vol->shape[3], (int)S, (int)L, (int)T,
-              start[0], start[1], start[2], end[0], end[1], end[2], bw, bo, 1.f / bw};
+              start[0], start[1], start[2], end[0], end[1], end[2], bw, bo, 1.f / bw,
+               std::fma(524288.f, bw, -std::fabs(bo))};
   const float a = std::fabs(bw);
   if (!(a > 1e-18f && a < 1e18f)) g.inv_bw = NAN;  // div_fixed's range
   return g;
