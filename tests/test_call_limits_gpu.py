@@ -178,3 +178,25 @@ def test_volume_render_in_other_units(cuda_lib, unit, exact):
     ref = oracle.volume_confocal_grad_mp(vol, mp, y, org, size, bw, 0.0)
     if np.abs(ref).max() < 1e37 and np.abs(ref).max() > 1e-33:
         assert rel(gm.cpu().numpy(), ref) < 1e-4
+
+
+def test_volume_pairs_gradient_of_infinite_elements(cuda_lib):
+    """Infinite elements of transient_grad give the infinities (and the NaN where both
+    signs meet) of the oracle, with the workspace and without."""
+    g = np.random.default_rng(2)
+    shape, S, L, T = (5, 6, 7), 4, 3, 200
+    sp, lp = points(g, S), points(g, L)
+    tg = g.uniform(0.5, 1.5, (T, S, L)).astype(np.float32)
+    tg[120, 1, 1], tg[130, 2, 0] = np.inf, -np.inf
+    ref = oracle.volume_exhaustive_adjoint(tg, shape, sp.T, lp.T, START, END, 0.02, 0.0)
+    assert np.isposinf(ref).any() and np.isneginf(ref).any() and np.isfinite(ref).any()
+    none = torch.empty((1, 3, 0), device="cuda")
+    args = [cu(tg[None]), cu(sp.T[None]), cu(lp.T[None]), none, none]
+    out, inplace = (torch.empty((1,) + shape, device="cuda") for _ in range(2))
+    R.volume_render_exhaustive_grad_volume(*args, out, START, END, 0.02, 0.0)
+    _lib.check(cuda_lib.totri_volume_exhaustive_grad_volume(
+        *[_lib.array(t) for t in (*args, inplace)], _lib.vec3(START), _lib.vec3(END), 0.02, 0.0,
+        _lib.stream_of(out.device)))
+    for got in (out[0].cpu().numpy(), inplace[0].cpu().numpy()):
+        for kind in (np.isnan, np.isposinf, np.isneginf):
+            assert np.array_equal(kind(got), kind(ref))

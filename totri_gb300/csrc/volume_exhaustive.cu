@@ -177,6 +177,13 @@ __global__ void __launch_bounds__(256) forward_kernel(Geo g, int b, const float*
   }
 }
 
+// x held within the finite range, sign kept; a NaN gives a finite value.
+__device__ __forceinline__ float clamp_finite(float x) {
+  float r;
+  asm("min.xorsign.abs.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(3.4028235e38f));
+  return r;
+}
+
 // d loss / d volume: per voxel, the forward weights against transient_grad. A
 // CTA takes a block of 8 x 8 x 4 voxels, one per thread, and the scan points of
 // its slice; a thread holds the distances of its voxel's ends to kLC lasers in
@@ -320,9 +327,10 @@ __global__ void __launch_bounds__(256, 4) adjoint_kernel(Geo g, int b, Pts sp, P
             const float v2 = i + 2 < n ? lds(ci + 8u) : 0.f, v3 = i + 3 < n ? lds(ci + 12u) : 0.f;
             sum += (v0 + v1) + (v2 + v3);
           }
-          // sum / range: the hardware reciprocal and one remainder correction
+          // sum / range: the hardware reciprocal and one remainder correction (a finite
+          // one: an infinite quotient stays)
           const float range = q1 - q0, r = __fdividef(1.f, range), y = sum * r;
-          part += n == 0 ? c0 : fmaf(fmaf(-y, range, sum), r, y);
+          part += n == 0 ? c0 : fmaf(clamp_finite(fmaf(-y, range, sum)), r, y);
         } else {
           part += pair_direct(g, da, db, tg + ((int64_t)(s - s_base) * g.L + l0 + k) * cstep,
                               bstep);
