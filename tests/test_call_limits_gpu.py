@@ -200,3 +200,30 @@ def test_volume_pairs_gradient_of_infinite_elements(cuda_lib):
     for got in (out[0].cpu().numpy(), inplace[0].cpu().numpy()):
         for kind in (np.isnan, np.isposinf, np.isneginf):
             assert np.array_equal(kind(got), kind(ref))
+
+
+def test_exhaustive_calls_of_two_million_bins(cuda_lib):
+    """More tiles of 32 bins than a grid has rows: the exhaustive Velten backprojection
+    equals its one-voxel-per-thread kernel bit for bit (one pair: each voxel is one
+    bin), the volume gradient its in-place reads (1e-5)."""
+    T, none = 1 << 21, torch.empty((1, 0, 3), device="cuda")
+    p = cu(np.array([[[0.1, -0.2, 0.0]]], np.float32))
+    tr = torch.rand((1, T, 1, 1), device="cuda")
+    shape = (1, 128, 128, 128)  # as many voxels as bins: the layout copy is used
+    got, want = torch.empty(shape, device="cuda"), torch.empty(shape, device="cuda")
+    K.backprojection_exhaustive_velten_forward(tr, p, p, none, none, got, START, END, 2e-6, 0.0)
+    with tuned({"backprojection.velten.pairs": 1}):
+        K.backprojection_exhaustive_velten_forward(tr, p, p, none, none, want, START, END, 2e-6,
+                                                   0.0)
+    assert float(want.abs().sum()) > 0.0
+    assert torch.equal(got, want)
+    T = 2100000
+    tg = torch.rand((1, T, 1, 1), device="cuda")
+    q, none = p.transpose(1, 2).contiguous(), torch.empty((1, 3, 0), device="cuda")
+    grad, inplace = (torch.empty((1, 4, 4, 4), device="cuda") for _ in range(2))
+    R.volume_render_exhaustive_grad_volume(tg, q, q, none, none, grad, START, END, 2e-6, 0.0)
+    _lib.check(cuda_lib.totri_volume_exhaustive_grad_volume(
+        *[_lib.array(t) for t in (tg, q, q, none, none, inplace)], _lib.vec3(START),
+        _lib.vec3(END), 2e-6, 0.0, _lib.stream_of(grad.device)))
+    assert float(inplace.abs().sum()) > 0.0
+    assert float((grad - inplace).norm() / inplace.norm()) < 1e-5

@@ -1274,9 +1274,14 @@ __global__ void __launch_bounds__(256) bins_last_kernel(const float* __restrict_
 
 int launch_bins_last(const float* in, float* out, int T, int Tp, int64_t row, int64_t n,
                      cudaStream_t stream) {
-  TOTRI_KERNEL("mesh grad layout", stream,
-               bins_last_kernel<<<dim3((unsigned)ceil_div(n, 32), (unsigned)ceil_div(T, 32)),
-                                  dim3(32, 8), 0, stream>>>(in, out, T, Tp, row, n));
+  constexpr int kBins = 65535 * 32;  // a grid has 65,535 rows of tiles
+  for (int64_t t0 = 0; t0 < T; t0 += kBins) {
+    const int bins = (int)std::min<int64_t>(T - t0, kBins);
+    TOTRI_KERNEL("mesh grad layout", stream,
+                 bins_last_kernel<<<dim3((unsigned)ceil_div(n, 32), (unsigned)ceil_div(bins, 32)),
+                                    dim3(32, 8), 0, stream>>>(in + t0 * row, out + t0, bins, Tp,
+                                                              row, n));
+  }
   return TOTRI_OK;
 }
 
