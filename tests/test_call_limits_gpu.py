@@ -227,3 +227,29 @@ def test_exhaustive_calls_of_two_million_bins(cuda_lib):
         _lib.vec3(END), 2e-6, 0.0, _lib.stream_of(grad.device)))
     assert float(inplace.abs().sum()) > 0.0
     assert float((grad - inplace).norm() / inplace.norm()) < 1e-5
+
+
+def test_exhaustive_gradient_of_black_and_degenerate_faces(cuda_lib):
+    """Faces of albedo zero and negative, and faces whose squared area is below the FP32
+    range: they add nothing to the oracle's gradient and nothing (no NaN) here."""
+    g = np.random.default_rng(4)
+    v, f, m = sphere(300, 2)
+    half = m.shape[1] // 2
+    m[:, half:] = 0.0
+    m[:, -20:] = -0.5
+    tiny = torch.tensor([[[0.0, 0.0, 0.4], [1e-12, 0.0, 0.4], [0.0, 1e-12, 0.4]]]).cuda()
+    tri = torch.arange(3, device="cuda", dtype=f.dtype).reshape(1, 1, 3) + v.shape[1]
+    v, f = torch.cat([v, tiny], 1), torch.cat([f, tri, tri.flip(2)], 1)
+    m = torch.cat([m, torch.ones((1, 3, 1), device="cuda")], 1)
+    sp, lp = points(g, 20), points(g, 7)
+    none = torch.empty((1, 0, 3), device="cuda")
+    tg = g.standard_normal((200, 20, 7)).astype(np.float32)
+    vn, fn, mn = (x[0].cpu().numpy() for x in (v, f, m))
+    rv, rm = oracle.mesh_exhaustive_grad(vn, fn, mn, sp, lp, None, None,
+                                         *mesh_masks(v, f, sp, lp), 200, 0.03, 0.0, tg)
+    assert np.isfinite(rv).all() and np.isfinite(rm).all()
+    vg, mg = torch.empty_like(v), torch.empty_like(m)
+    R.mesh_exhaustive_grad_verts(v, f, m, cu(sp[None]), cu(lp[None]), none, none, cu(tg[None]),
+                                 vg, mg, 0.03, 0.0, 0)
+    assert rel(vg[0].cpu().numpy(), rv) < 1e-5
+    assert rel(mg[0].cpu().numpy(), rm) < 1e-5

@@ -777,7 +777,10 @@ __global__ void __launch_bounds__(256, kOcc) exh_grad_face_kernel(
       if (tid < 9) {
         const int m = tid / 3, a = tid - 3 * m;
         // d alpha: w = sum P (wf + wv), wf = -n / |n|^2, through the normal's Jacobian
-        const fv3 w = (vdiv(-1.f, nn) * tot[15]) * nrm + mkv(tot[3], tot[4], tot[5]);
+        // (a face without a pair adds zeros, whatever its normal and albedo)
+        const float wf = tot[15] != 0.f ? vdiv(-1.f, nn) * tot[15] : 0.f;
+        fv3 w = mkv(tot[3], tot[4], tot[5]);
+        if (wf != 0.f) w = wf * nrm + w;
         const fv3 g1 = cross(v[2] - v[0], w), g2 = cross(w, v[1] - v[0]);
         const fv3 g = m == 0 ? -(g1 + g2) : (m == 1 ? g1 : g2);
         const float t = tot[a] + (a == 0 ? g.x : (a == 1 ? g.y : g.z)) + tot[6 + tid];
@@ -787,7 +790,7 @@ __global__ void __launch_bounds__(256, kOcc) exh_grad_face_kernel(
           atomicAdd(out.vg + b * out.vsb + vi[m] * out.vsv + a * out.vsc, t);
         }
       } else if (tid == 9 && out.mg) {
-        const float t = xdiv(tot[15], s0r.w);
+        const float t = tot[15] != 0.f ? xdiv(tot[15], s0r.w) : 0.f;
         for (int m = 0; m < 3; ++m)
           if (vi[m] >= 0 && vi[m] < out.V)
             atomicAdd(out.mg + b * out.msb + vi[m] * out.msv, (1.f / 3.f) * t);
