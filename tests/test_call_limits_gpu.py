@@ -253,3 +253,49 @@ def test_exhaustive_gradient_of_black_and_degenerate_faces(cuda_lib):
                                  vg, mg, 0.03, 0.0, 0)
     assert rel(vg[0].cpu().numpy(), rv) < 1e-5
     assert rel(mg[0].cpu().numpy(), rm) < 1e-5
+
+
+@pytest.mark.parametrize("bw,bo", [(-0.02, 5.0), (-0.3, 5.0), (-2.0, 8.0), (0.02, 0.0)])
+def test_mesh_gradients_with_a_negative_bin_width(cuda_lib, bw, bo):
+    """Time running backwards: both gradients against the oracle (1e-5, as forwards)."""
+    g = np.random.default_rng(6)
+    v, f, m = sphere(2000, 8)
+    sp, lp = points(g, 40), points(g, 5)
+    none, T = torch.empty((1, 0, 3), device="cuda"), 300
+    vn, fn, mn = (x[0].cpu().numpy() for x in (v, f, m))
+    vs, vl = mesh_masks(v, f, sp, lp)
+    vg, mg = torch.empty_like(v), torch.empty_like(m)
+    tg = g.standard_normal((T, 40)).astype(np.float32)
+    R.mesh_confocal_grad_verts(v, f, m, cu(sp[None]), none, cu(tg[None]), vg, mg, bw, bo, 0)
+    rv, rm = oracle.mesh_confocal_grad(vn, fn, mn, sp, None, vs, T, bw, bo, tg)
+    assert np.linalg.norm(rv) > 0.0
+    assert rel(vg[0].cpu().numpy(), rv) < 1e-5
+    assert rel(mg[0].cpu().numpy(), rm) < 1e-5
+    tg = g.standard_normal((T, 40, 5)).astype(np.float32)
+    rv, rm = oracle.mesh_exhaustive_grad(vn, fn, mn, sp, lp, None, None, vs, vl, T, bw, bo, tg)
+    for layout in (0, 2):
+        with tuned({"mesh.exhaustive.grad.layout": layout}):
+            R.mesh_exhaustive_grad_verts(v, f, m, cu(sp[None]), cu(lp[None]), none, none,
+                                         cu(tg[None]), vg, mg, bw, bo, 0)
+        assert rel(vg[0].cpu().numpy(), rv) < 1e-5
+        assert rel(mg[0].cpu().numpy(), rm) < 1e-5
+
+
+@pytest.mark.parametrize("T", [300, 2048])
+def test_large_mesh_renders_with_a_negative_bin_width(cuda_lib, T):
+    """A mesh large enough for the columns kernel is rendered by the tiles: equal to
+    them but for the order of the adds (terms of both signs: 1e-4)."""
+    g = np.random.default_rng(6)
+    v, f, m = sphere(20000, 8)
+    sp = cu(points(g, 1100)[None])
+    none = torch.empty((1, 0, 3), device="cuda")
+    calls = [((1, T, 1100), lambda out: R.mesh_confocal_forward(v, f, m, sp, none, out, -0.3, 5.0, 0)),
+             ((1, T, 40, 30), lambda out: R.mesh_exhaustive_forward(
+                 v, f, m, sp[:, :40], sp[:, :30], none, none, out, -0.3, 5.0, 0))]
+    for shape, call in calls:
+        got, want = torch.empty(shape, device="cuda"), torch.empty(shape, device="cuda")
+        call(got)
+        with tuned({"mesh.confocal.splat.columns": 1, "mesh.exhaustive.splat.columns": 1}):
+            call(want)
+        assert float(want.abs().sum()) > 0.0
+        assert float((got - want).norm() / want.norm()) < 1e-4

@@ -838,6 +838,8 @@ __device__ __forceinline__ DFloat len_exact(fv3 v, fv3 p, float& inv) {
 // twice (chain and double-float) and walked the tent's three parts apart (1,200
 // instructions per 32 visible pairs), 1.03 ms now; 320 faces x 1,024 points: 46 and
 // 37 us. Two CTAs per SM (no spills) against 1.05 ms and 40 us with three.
+// kForward: the bin width is positive.
+template <bool kForward>
 __global__ void __launch_bounds__(256, 2) grad_kernel(Scene sc, View3f sp, View3f so, int has_origin,
                                                    const float* __restrict__ tgrad, int T, int S,
                                                    float bw, float bo, int fixed, GradOut out) {
@@ -901,7 +903,7 @@ __global__ void __launch_bounds__(256, 2) grad_kernel(Scene sc, View3f sp, View3
         d2 = path_offset(d2, od, bo);
       }
       float4 w;
-      if (!pair_weights<false>(tgb + s, S, T, d0, d1, d2, bw, inv_bw, fixed, order, w)) return;
+      if (!pair_weights<false, kForward>(tgb + s, S, T, d0, d1, d2, bw, inv_bw, fixed, order, w)) return;
       const float P = alpha * w.x, knr = vdiv(2.f, nr), kw = vdiv(2.f, 3.f * r.z);
       const float pr = P * vdiv(-8.f, 3.f * rr), pn = P * knr;
       const float q0 = 2.f * alpha * w.y * i0, q1 = 2.f * alpha * w.z * i1;
@@ -1235,7 +1237,8 @@ int launch_confocal_splat(const Scene& sc, const View3f& sp, const View3f& so, i
   const bool large = sc.F >= 12288 ? T <= 2048 : sc.F >= 4096 && T <= 1024;
   const bool few = sc.F >= 1024 && all <= 16 * tune::sm_count() && T <= 1024;
   const int ct = cols > 0 ? cols : all >= 1024 && (large || few) ? 8 : 0;
-  if (ct > 1 && (size_t)T * 4 <= budget && tune::get("mesh.confocal.splat.mode") != 1)
+  // (its sides and windows run forwards in time)
+  if (ct > 1 && bw > 0.f && (size_t)T * 4 <= budget && tune::get("mesh.confocal.splat.mode") != 1)
     return launch_confocal_columns(sc, sp, so, has_origin, ct, transient, T, S, bw, bo, stream);
   // Built-in choice: the widest scan tile that keeps the histogram within
   // 40 KB (several CTAs per SM) and still gives every SM tiles to work on.
@@ -1258,12 +1261,12 @@ int launch_confocal_grad(const Scene& sc, const View3f& sp, const View3f& so, in
   const int split =
       tune::grad_split("mesh.confocal.grad.split", (int64_t)sc.nch * sc.B, S, kMaxSlice);
   const size_t smem = sizeof(uint32_t) * (size_t)ceil_div(S, split);
-  TOTRI_CUDA(tune::ensure_dynamic_smem(
-      reinterpret_cast<const void*>(grad_kernel), smem));
+  const auto kernel = bw > 0.f ? grad_kernel<true> : grad_kernel<false>;
+  TOTRI_CUDA(tune::ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem));
   const dim3 grid((unsigned)sc.nch, (unsigned)sc.B, (unsigned)split);
   TOTRI_KERNEL("mesh confocal grad", stream,
-               grad_kernel<<<grid, 256, smem, stream>>>(sc, sp, so, has_origin, tgrad, T, S, bw,
-                                                        bo, fixed_division(bw, bo), out));
+               kernel<<<grid, 256, smem, stream>>>(sc, sp, so, has_origin, tgrad, T, S, bw, bo,
+                                                   fixed_division(bw, bo), out));
   return TOTRI_OK;
 }
 

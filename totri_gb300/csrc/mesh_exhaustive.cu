@@ -592,7 +592,8 @@ __device__ __forceinline__ int block_slot(bool flag, int* warp_counts, int* tota
   return flag ? base + __popc(bal & ((1u << lane) - 1u)) : -1;
 }
 
-template <int kOcc, bool kLast>
+// kForward: the bin width is positive.
+template <int kOcc, bool kLast, bool kForward>
 __global__ void __launch_bounds__(256, kOcc) exh_grad_face_kernel(
     Scene sc, View3f sp, View3f lp, Origins org, int S, int L, const float* __restrict__ tgrad,
     int T, float bw, float bo, int fixed, GradOut out, int faces_per_cta, int lchunk, int sslice,
@@ -713,7 +714,7 @@ __global__ void __launch_bounds__(256, kOcc) exh_grad_face_kernel(
           }
           const float* col = colm + __float_as_int(ro[kRecAt]) * ostep;
           float4 w;  // area, weights of the vertices
-          if (!pair_weights<kLast>(col, bstep, T, e0, e1, e2, bw, inv_bw, fixed, order, w))
+          if (!pair_weights<kLast, kForward>(col, bstep, T, e0, e1, e2, bw, inv_bw, fixed, order, w))
             continue;
           const float P = alpha * w.x, Q0 = alpha * w.y, Q1 = alpha * w.z, Q2 = alpha * w.w;
           used = true;
@@ -1222,7 +1223,9 @@ int launch_exhaustive_splat(const Scene& sc, const View3f& sp, const View3f& lp,
   // "mesh.exhaustive.splat.columns" = 1 turns the kernel off, 8 and 32 select a
   // tile, ".window" its bins.
   const int cols = tune::get("mesh.exhaustive.splat.columns");
-  if (cols != 1 && tune::get("mesh.exhaustive.splat.mode") != 1 && (size_t)T * 4 <= budget) {
+  // Its sides and windows run forwards in time: the tiles take negative bin widths.
+  if (cols != 1 && bw > 0.f && tune::get("mesh.exhaustive.splat.mode") != 1 &&
+      (size_t)T * 4 <= budget) {
     const int64_t all = (int64_t)S * L * sc.B;
     const int sms = tune::sm_count();
     const bool many = sc.F >= 4096;
@@ -1342,8 +1345,12 @@ int launch_exhaustive_grad(const Scene& sc, const View3f& sp, const View3f& lp,
                       int64_t bstride, int64_t cstep, int64_t bstep, bool last) -> int {
       const dim3 grid((unsigned)ceil_div(sc.F, fpc), (unsigned)nb,
                       (unsigned)(ceil_div(sb - sa, sslice) * ceil_div(L, lchunk)));
-      auto* kern = last ? (occ4 ? exh_grad_face_kernel<4, true> : exh_grad_face_kernel<3, true>)
-                        : (occ4 ? exh_grad_face_kernel<4, false> : exh_grad_face_kernel<3, false>);
+      auto* kern = last ? (occ4 ? exh_grad_face_kernel<4, true, true>
+                                : exh_grad_face_kernel<3, true, true>)
+                        : (occ4 ? exh_grad_face_kernel<4, false, true>
+                                : exh_grad_face_kernel<3, false, true>);
+      if (!(bw > 0.f))
+        kern = last ? exh_grad_face_kernel<3, true, false> : exh_grad_face_kernel<3, false, false>;
       TOTRI_CUDA(tune::ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
       TOTRI_KERNEL("mesh exhaustive grad", stream,
                    kern<<<grid, 256, smem, stream>>>(sc, sp, lp, org, S, L, tg, T, bw, bo, fixed,

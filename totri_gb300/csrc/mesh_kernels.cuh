@@ -378,10 +378,26 @@ __device__ __forceinline__ DFloat path_offset(DFloat e, DFloat od, float bo) {
   return DFloat{f.hi, e.lo + f.lo};
 }
 
+// The same of a tent whose bins run backwards (a negative bin width) from
+// tent_grad's sums: the weight of a vertex is the move of the area with its foot or
+// peak, and for the first and the last one with the tent's height too.
+__device__ __forceinline__ float4 reversed_weights(const float* __restrict__ col, int64_t stride,
+                                                   int T, float x0, float x1, float x2, int b0,
+                                                   int b1, int b2, float bw) {
+  const float x[3] = {x0, x1, x2};
+  const int bin[3] = {b0, b1, b2};
+  TentGrad g;
+  tent_grad(col, stride, T, x, bin, g);
+  const float span = x2 - x0, height = vdiv(2.f, bw * span * span) * g.ayc;
+  return make_float4(g.part0, vdiv(g.a0, bw) + height, vdiv(g.a1, bw), vdiv(g.a2, bw) - height);
+}
+
 // tent_weights of a pair from its sorted paths (path_offset), in the vertices' own
 // order; false if no bin of the transient is touched. The coordinates of the FP32
 // chain decide the bins; the corners are relative to the first one (bin_offset).
-template <bool kLast>
+// kForward: the bin width is positive (a test in the other kernels' inner loop took 1
+// and 2% of the two gradients).
+template <bool kLast, bool kForward>
 __device__ __forceinline__ bool pair_weights(const float* __restrict__ col, int64_t stride, int T,
                                              DFloat e0, DFloat e1, DFloat e2, float bw,
                                              float inv_bw, int fixed, const PathOrder& order,
@@ -407,8 +423,11 @@ __device__ __forceinline__ bool pair_weights(const float* __restrict__ col, int6
   auto rel = [&](float c, DFloat e) {
     return fmaf(__fmaf_rn(-c, bw, e.hi) + e.lo, inv_bw, c - base);
   };
-  w = tent_weights<kLast>(col, stride, T, rel(c0, e0), rel(c1, e1), rel(c2, e2), b0, b1, b2,
-                          inv_bw);
+  const float x0 = rel(c0, e0), x1 = rel(c1, e1), x2 = rel(c2, e2);
+  if (!kForward && b0 > b2)
+    w = reversed_weights(col, stride, T, x0, x1, x2, b0, b1, b2, bw);
+  else
+    w = tent_weights<kLast>(col, stride, T, x0, x1, x2, b0, b1, b2, inv_bw);
   auto swap_back = [](bool y, float& a, float& z) {
     const float t = a;
     a = y ? z : a;
