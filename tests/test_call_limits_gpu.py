@@ -299,3 +299,23 @@ def test_large_mesh_renders_with_a_negative_bin_width(cuda_lib, T):
             call(want)
         assert float(want.abs().sum()) > 0.0
         assert float((got - want).norm() / want.norm()) < 1e-4
+
+
+@pytest.mark.parametrize("want", [1, 2, 3, 5])
+def test_volume_walks_with_other_point_counts(cuda_lib, want):
+    """"volume.forward.points" below 4 leaves the built-in choice, a count in between
+    takes the next lower tile (it divided by zero points): the oracle's values."""
+    g = np.random.default_rng(9)
+    shape, N, T, bw = (5, 6, 7), 21, 90, 0.02
+    mp = np.stack([g.uniform(-1, 1, N), g.uniform(-1, 1, N), np.zeros(N)]).astype(np.float32)
+    vol = g.uniform(0.5, 1.5, shape).astype(np.float32)
+    y = g.uniform(0.5, 1.5, (N, T)).astype(np.float32)
+    org, size = (-0.5, -0.5, 0.5), (1.0, 1.0, 1.0)
+    out, gm = torch.full((N, T), 7.0, device="cuda"), torch.full((3, N), 7.0, device="cuda")
+    with tuned({"volume.forward.points": want}):
+        R.volume_confocal_forward(cu(vol), cu(mp), out, org, size, bw, 0.0)
+        R.volume_confocal_grad_measurement_points(gm, cu(vol), cu(mp), cu(y), org, size, bw, 0.0)
+    ref = oracle.volume_confocal_forward(vol, mp, T, org, size, bw, 0.0)
+    assert rel(out.cpu().numpy(), ref) < 1e-5
+    ref = oracle.volume_confocal_grad_mp(vol, mp, y, org, size, bw, 0.0)
+    assert rel(gm.cpu().numpy(), ref) < 1e-4

@@ -1335,9 +1335,8 @@ int launch_exhaustive_grad(const Scene& sc, const View3f& sp, const View3f& lp,
     // "mesh.exhaustive.grad.occupancy" = 4: registers capped for 4 CTAs per SM
     // (64, with spills) instead of 3 (80); "mesh.exhaustive.grad.sslice" /
     // ".lchunk": scan points / lasers per CTA.
-    const int fpc = tune::get("mesh.exhaustive.grad.faces") > 0
-                        ? (int)tune::get("mesh.exhaustive.grad.faces")
-                        : kFacesPerCta;
+    int fpc = tune::get("mesh.exhaustive.grad.faces");
+    if (fpc <= 0) fpc = kFacesPerCta;
     const int fixed = fixed_division(bw, bo);
     const bool occ4 = tune::get("mesh.exhaustive.grad.occupancy") == 4;
     const size_t smem = sizeof(float) * 2 * kRec * kFaceSlice;

@@ -1117,7 +1117,8 @@ WalkTile walk_tile(int64_t N, int T, int64_t voxels) {
   // 128^3 voxels, 16,384 points, 1,024 bins: 16 points 6.1 ms alone, 5.6 in 2
   // slices, 5.4 in 8; 8 points 6.3 / 5.9 / 5.6 ms, 32 points 7.1 / 6.4 / 6.4 ms.
   // 41 x 37 x 53 x 899 points, 500 bins: 16 points 0.43 ms alone, 0.11 in 8.
-  const int want = tune::get("volume.forward.points");
+  int want = tune::get("volume.forward.points");
+  if (want < 4) want = 0;  // (fewer than 4 points: the built-in choice)
   for (const int pt : {32, 16, 8, 4}) {
     if (bytes(pt) > budget || pt > (want > 0 ? want : 16)) continue;
     w.points = pt;
