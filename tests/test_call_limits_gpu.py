@@ -319,3 +319,30 @@ def test_volume_walks_with_other_point_counts(cuda_lib, want):
     assert rel(out.cpu().numpy(), ref) < 1e-5
     ref = oracle.volume_confocal_grad_mp(vol, mp, y, org, size, bw, 0.0)
     assert rel(gm.cpu().numpy(), ref) < 1e-4
+
+
+def repeats(call, times=8):
+    """Whether `call` gives the same bits each time."""
+    first = call()
+    return all(torch.equal(call(), first) for _ in range(times - 1))
+
+
+@pytest.mark.parametrize("N", [20, 200, 256, 500, 512])
+@pytest.mark.parametrize("shape", [(20, 21, 22), (9, 10, 65)])
+def test_volume_adjoint_of_few_points_repeats(cuda_lib, N, shape):
+    """Up to 512 points the adjoint's sums have a fixed order; against the FP64 oracle
+    1e-5, as with more points."""
+    g = np.random.default_rng(N)
+    mp = np.stack([g.uniform(-1, 1, N), g.uniform(-1, 1, N), np.zeros(N)]).astype(np.float32)
+    y = g.uniform(0.5, 1.5, (N, 150)).astype(np.float32)
+    org, size = (-0.5, -0.5, 0.5), (1.0, 1.0, 1.0)
+    mpc, yc = cu(mp), cu(y)
+
+    def call():
+        out = torch.full(shape, 7.0, device="cuda")
+        R.volume_confocal_adjoint(out, mpc, yc, org, size, 0.02, 0.0)
+        return out
+
+    assert repeats(call)
+    ref = oracle.volume_confocal_adjoint(y, shape, mp, org, size, 0.02, 0.0)
+    assert rel(call().cpu().numpy(), ref) < 1e-5

@@ -9,6 +9,8 @@
 // (voxel, point), found by inverting the sphere/column geometry and then
 // re-deciding each bin with the reference's FP32 sample arithmetic. Each CTA
 // owns a tile of points and keeps their transient rows in shared memory.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -21,6 +23,8 @@
 
 namespace totri {
 namespace volume {
+
+namespace cg = cooperative_groups;
 
 struct Geo {
   int X, Y, Z;
@@ -856,6 +860,33 @@ __device__ __forceinline__ void adj_walk(const Geo& g, const float4* __restrict_
   }
 }
 
+// The end of confocal_adjoint_columns_kernel in a cluster of point groups: a cell's sum
+// over the warps' copies of all groups, in order, so that the result does not depend
+// on which group ends first (two slabs share a cell, but two terms added to zero
+// commute).
+__device__ __forceinline__ void add_cluster_columns(const Geo& g, float* acc, int nw, int rows,
+                                                    int tx, int ty, int za, float* vol,
+                                                    int accumulate) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int peers = (int)cluster.num_blocks();
+  cluster.sync();  // every group has its copies
+  for (int jj = cluster.block_rank() * blockDim.x + threadIdx.x; jj < rows * 32;
+       jj += peers * blockDim.x) {
+    const int r = jj >> 5, l = jj & 31, z = za + r;
+    const int cy = ty + (l & 7), cx = tx + (l >> 3);
+    if (cx >= g.X || cy >= g.Y || z >= g.Z) continue;
+    float sum = 0.f;
+    for (int c = 0; c < peers; ++c) {
+      const float* copies = cluster.map_shared_rank(acc, c);
+      for (int w = 0; w < nw; ++w) sum += copies[((size_t)w * rows + r) * 32 + l];
+    }
+    float* dst = vol + ((size_t)cx * g.Y + cy) * g.Z + z;
+    if (accumulate) atomicAdd(dst, sum);
+    else *dst = sum;
+  }
+  cluster.sync();  // no group leaves while another reads its copies
+}
+
 // Exact adjoint of the forward with the lanes of a warp over 32 neighbouring
 // voxel columns (an 8 x 4 tile: y fastest) and all lanes on one point and one
 // bin at a time. The point's transient row is then read once per warp (32 bins
@@ -881,8 +912,9 @@ __device__ __forceinline__ void adj_walk(const Geo& g, const float4* __restrict_
 // points x 1,024 bins: 62.8 -> 39.5 ms, at
 // 73% of the shared-memory pipe's wavefronts.
 // kSigned: there may be negative bin centres (a negative bin offset), whose bins
-// are a second walk of a point.
-template <bool kSigned>
+// are a second walk of a point. kCluster: the point groups form a cluster
+// (add_cluster_columns).
+template <bool kSigned, bool kCluster>
 __global__ void __launch_bounds__(256, 3) confocal_adjoint_columns_kernel(
     Geo g, Points mp, int N, int points_per_group, int run, const float* __restrict__ tr,
     float* __restrict__ vol, int accumulate, int slab) {
@@ -978,6 +1010,10 @@ __global__ void __launch_bounds__(256, 3) confocal_adjoint_columns_kernel(
                          x, y, za, zn);
       }
     }
+  }
+  if constexpr (kCluster) {
+    add_cluster_columns(g, acc, nw, rows, tx, ty, za, vol, accumulate);
+    return;
   }
   __syncthreads();
   // cell za + r of column l: the sum over the warps' copies (l fastest: no
@@ -1257,15 +1293,36 @@ int totri_volume_confocal_adjoint(const totri_array_t* vol, const totri_array_t*
         (int)std::max<int64_t>(1, std::min<int64_t>(want, ceil_div(N, (int64_t)run * warps)));
     const int per = (int)(ceil_div(ceil_div(N, groups), run) * run);
     const int used = (int)ceil_div(N, per);
-    const int accumulate = used > 1 || nslab > 1;
+    // up to 8 groups form a cluster, which sums them in order: the result repeats bit
+    // for bit (more groups add in the order in which they end)
+    const int peers = used <= 8 ? used : 1;
+    const int accumulate = used > peers || nslab > 1;
     if (accumulate) TOTRI_CUDA(cudaMemsetAsync(vd, 0, sizeof(float) * numel(vol), stream));
     const dim3 grid3((unsigned)tiles, (unsigned)used, (unsigned)nslab);
-    const auto kernel = g.bo < 0.f && !g.all_bins ? volume::confocal_adjoint_columns_kernel<true>
-                                                  : volume::confocal_adjoint_columns_kernel<false>;
+    const bool negative = g.bo < 0.f && !g.all_bins;
+    const auto kernel =
+        peers > 1 ? (negative ? volume::confocal_adjoint_columns_kernel<true, true>
+                              : volume::confocal_adjoint_columns_kernel<false, true>)
+                  : (negative ? volume::confocal_adjoint_columns_kernel<true, false>
+                              : volume::confocal_adjoint_columns_kernel<false, false>);
     TOTRI_CUDA(tune::ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem));
+    cudaLaunchAttribute cluster[1];
+    cluster[0].id = cudaLaunchAttributeClusterDimension;
+    cluster[0].val.clusterDim.x = 1;
+    cluster[0].val.clusterDim.y = (unsigned)peers;
+    cluster[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid3;
+    cfg.blockDim = dim3(warps * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = cluster;
+    cfg.numAttrs = peers > 1 ? 1 : 0;
+    cudaError_t le = cudaSuccess;
     TOTRI_KERNEL("volume confocal adjoint", stream,
-                 kernel<<<grid3, warps * 32, smem, stream>>>(g, pts, N, per, run, trd, vd,
-                                                             accumulate, slab));
+                 le = cudaLaunchKernelEx(&cfg, kernel, g, pts, N, per, run, trd, vd, accumulate,
+                                         slab));
+    TOTRI_CUDA(le);
     return TOTRI_OK;
   }
   if (Z <= 256 && mode == 2) {
