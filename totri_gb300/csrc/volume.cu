@@ -832,7 +832,7 @@ __device__ __forceinline__ void adj_walk(const Geo& g, const float4* __restrict_
         f2unpack(fx, xa, xb);
         f2unpack(f2add(fr, half), off[2 * h], off[2 * h + 1]);
         const u64 fall = f2mul(d2, f2pack(tb.z, tb.w));
-        const u64 v = f2mul(fall, f2mul(fall, h ? f2pack(v4.z, v4.w) : f2pack(v4.x, v4.y)));
+        const u64 v = f2mul(f2mul(fall, fall), h ? f2pack(v4.z, v4.w) : f2pack(v4.x, v4.y));
         const u64 upper = f2mul(fr, v);
         f2unpack(upper, w1[2 * h], w1[2 * h + 1]);
         f2unpack(f2sub(v, upper), w0[2 * h], w0[2 * h + 1]);
