@@ -413,13 +413,21 @@ int totri_backprojection_exhaustive_velten_forward(
     float bin_offset, void* stream);
 
 /* The same with an optional workspace of
- * totri_backprojection_exhaustive_velten_scratch(S, L, T) bytes (at most 2 GiB;
- * smaller or null: the transient is read in place, more slowly), which holds
- * bins-last copies of the transient, one batch item and range of scan points at
- * a time. The results are the same up to FP32 summation order. */
+ * totri_backprojection_exhaustive_velten_scratch(S, L, T) bytes, which is enough for
+ * any volume (at most 2 GiB and some 20 MB), or of the bytes that a call with the
+ * volume [D, H, W] and this bin width uses (..._workspace). It holds bins-last copies
+ * of the transient, one batch item and range of scan points at a time, and the
+ * partial sums of a launch. With less room or null the transient is read in place and
+ * a launch is not split: more slowly, the results the same up to FP32 summation
+ * order. A call repeats bit for bit with the same workspace size. */
 size_t totri_backprojection_exhaustive_velten_scratch(int64_t num_scan_points,
                                                       int64_t num_laser_points,
                                                       int64_t num_bins);
+size_t totri_backprojection_exhaustive_velten_workspace(int64_t num_scan_points,
+                                                        int64_t num_laser_points,
+                                                        int64_t num_bins, int64_t depth,
+                                                        int64_t height, int64_t width,
+                                                        float bin_width);
 int totri_backprojection_exhaustive_velten_forward_ws(
     const totri_array_t* transient, const totri_array_t* scan_points,
     const totri_array_t* laser_points, const totri_array_t* scan_origin,

@@ -346,3 +346,23 @@ def test_volume_adjoint_of_few_points_repeats(cuda_lib, N, shape):
     assert repeats(call)
     ref = oracle.volume_confocal_adjoint(y, shape, mp, org, size, 0.02, 0.0)
     assert rel(call().cpu().numpy(), ref) < 1e-5
+
+
+@pytest.mark.parametrize("shape,S,L,T", [((24, 24, 24), 256, 36, 300), ((5, 9, 3), 41, 7, 400)])
+def test_exhaustive_velten_repeats(cuda_lib, shape, S, L, T):
+    """The slices of a launch are added in order; bins-last copies and in place."""
+    g = np.random.default_rng(S)
+    sp, lp = cu(points(g, S)[None]), cu(points(g, L)[None])
+    none = torch.empty((1, 0, 3), device="cuda")
+    tr = cu(g.uniform(0.5, 1.5, (1, T, S, L)).astype(np.float32))
+
+    def call():
+        out = torch.full((1,) + shape, 7.0, device="cuda")
+        K.backprojection_exhaustive_velten_forward(tr, sp, lp, none, none, out, START, END, 0.02,
+                                                   0.0)
+        return out
+
+    assert repeats(call)
+    ref = oracle.bp_exhaustive_velten(tr[0].cpu().numpy(), sp[0].cpu().numpy(),
+                                      lp[0].cpu().numpy(), None, None, shape, START, END, 0.02, 0.0)
+    assert rel(call()[0].cpu().numpy(), ref) < 1e-5

@@ -598,8 +598,7 @@ template <bool kLast>
 __global__ void __launch_bounds__(256, 4) velten_pairs_kernel(
     Grid g, int b, int T, int S, int L, Pts3 sp, Pts3 lp, Pts3 so, Pts3 lo, int has_so, int has_lo,
     float bw, float bo, float inv_bw, int s_base, int s_end, int per_slice,
-    const float* __restrict__ tr, int64_t cstep, int64_t bstep, float* __restrict__ vol,
-    int accumulate) {
+    const float* __restrict__ tr, int64_t cstep, int64_t bstep, float* __restrict__ vol, int add) {
   using u64 = unsigned long long;
   __shared__ float4 laser[kLG][256];
   __shared__ float lod[kLG];
@@ -669,9 +668,9 @@ __global__ void __launch_bounds__(256, 4) velten_pairs_kernel(
 #pragma unroll
   for (int v = 0; v < 4; ++v) {
     if (x >= g.W || y >= g.H || z0 + 4 * v >= g.D) continue;
-    float* dst = vol + (((size_t)b * g.D + z0 + 4 * v) * g.H + y) * g.W + x;
-    if (accumulate) atomicAdd(dst, val[v]);
-    else *dst = val[v];
+    // (a slice's volume is its own)
+    float* dst = vol + (((size_t)blockIdx.y * g.D + z0 + 4 * v) * g.H + y) * g.W + x;
+    *dst = add ? *dst + val[v] : val[v];
   }
 }
 
@@ -916,8 +915,36 @@ int totri_backprojection_confocal_velten_adjoint(const totri_array_t* volume,
   return TOTRI_OK;
 }
 
+// The blocked kernel takes its bins from div_fixed (bin widths within 1e-18 .. 1e18)
+// and a rounding by addition (bins below 2^21); anything else goes one voxel per
+// thread ("backprojection.velten.pairs" = 1: always).
+static bool velten_blocked(int64_t S, int64_t L, int64_t T, float bw) {
+  const float abw = std::fabs(bw);
+  return abw > 1e-18f && abw < 1e18f && T <= (1 << 21) && S > 0 && L > 0 && T > 0 &&
+         tune::get("backprojection.velten.pairs") != 1;
+}
+
+// Bins-last copies but where a pair's column has more bins than the volume has voxels
+// to read them; slices of the scan points until about 4 waves of CTAs (4 per SM), with
+// at least 4 scan points each (a slice repeats the lasers' distances).
+static mesh::PairPlan velten_plan(int64_t S, int64_t L, int64_t T, int64_t D, int64_t H, int64_t W,
+                                  size_t ws_bytes) {
+  const int64_t blocks = ceil_div(W, 8) * ceil_div(H, 8) * ceil_div(D, 16);
+  return mesh::pair_plan(S, L, T, D * H * W, blocks, 16 * (int64_t)tune::sm_count(), 4,
+                         D * H * W >= T, ws_bytes);
+}
+
 size_t totri_backprojection_exhaustive_velten_scratch(int64_t S, int64_t L, int64_t T) {
-  return mesh::exh_grad_scratch_bytes(S, L, T);
+  // Partial sums of a launch: slices of at most 1,024 voxels per CTA, fewer than
+  // 2 x 16 CTAs per SM where there is more than one.
+  const size_t partial = S < 8 ? 0 : sizeof(float) * 1024 * 32 * (size_t)tune::sm_count();
+  return S > 0 && L > 0 && T > 0 ? mesh::exh_grad_scratch_bytes(S, L, T) + partial : 0;
+}
+
+size_t totri_backprojection_exhaustive_velten_workspace(int64_t S, int64_t L, int64_t T, int64_t D,
+                                                        int64_t H, int64_t W, float bw) {
+  if (D <= 0 || H <= 0 || W <= 0 || !velten_blocked(S, L, T, bw)) return 0;
+  return velten_plan(S, L, T, D, H, W, SIZE_MAX).bytes;
 }
 
 int totri_backprojection_exhaustive_velten_forward_ws(
@@ -946,12 +973,7 @@ int totri_backprojection_exhaustive_velten_forward_ws(
   if (nv == 0) return TOTRI_OK;
   const float* trp = static_cast<const float*>(transient->data);
   float* volp = static_cast<float*>(volume->data);
-  // The blocked kernel takes its bins from div_fixed (bin widths within 1e-18 ..
-  // 1e18) and a rounding by addition (bins below 2^21); anything else goes one
-  // voxel per thread ("backprojection.velten.pairs" = 1: always).
-  const float abw = std::fabs(bw);
-  if (!(abw > 1e-18f && abw < 1e18f) || T > (1 << 21) || S == 0 || L == 0 || T == 0 ||
-      tune::get("backprojection.velten.pairs") == 1) {
+  if (!velten_blocked(S, L, T, bw)) {
     for (int b = 0; b < (int)B; ++b)
       TOTRI_KERNEL("backprojection velten exhaustive", stream,
                    bp::velten_exhaustive_kernel<<<(unsigned)ceil_div(nv, 128), 128, 0, stream>>>(
@@ -959,39 +981,35 @@ int totri_backprojection_exhaustive_velten_forward_ws(
                        volp));
     return TOTRI_OK;
   }
-  // Scan points per bins-last copy (all of them up to 2 GiB); 0: in place, also
-  // where a pair's column has more bins than the volume has voxels to read them.
-  int64_t chunk = ws && nv >= T ? mesh::exh_grad_chunk_points(S, L, T) : 0;
-  if (ws_bytes < (size_t)chunk * L * T * sizeof(float)) chunk = 0;
-  const int64_t step = chunk > 0 ? chunk : S;
+  const mesh::PairPlan plan = velten_plan(S, L, T, g.D, g.H, g.W, ws ? ws_bytes : 0);
   const int64_t blocks = ceil_div(g.W, 8) * ceil_div(g.H, 8) * ceil_div(g.D, 16);
-  // slices of the scan points until about 4 waves of CTAs (4 per SM), with at
-  // least 4 scan points each (a slice repeats the lasers' distances)
-  const int64_t slices = std::max<int64_t>(
-      1, std::min<int64_t>(ceil_div(16 * (int64_t)tune::sm_count(), blocks), step / 4));
-  const int per = (int)ceil_div(step, slices);
-  const int accumulate = ceil_div(step, per) > 1 || step < S;
-  if (accumulate) TOTRI_CUDA(cudaMemsetAsync(volp, 0, sizeof(float) * B * nv, stream));
   const int64_t row = S * L;
+  float* copy = static_cast<float*>(ws);
+  float* part = reinterpret_cast<float*>(static_cast<char*>(ws) + plan.part_at);
   for (int b = 0; b < (int)B; ++b)
-    for (int64_t sa = 0; sa < S; sa += step) {
-      const int64_t sb = std::min(S, sa + step);
-      const dim3 grid((unsigned)blocks, (unsigned)ceil_div(sb - sa, per));
+    for (int64_t sa = 0; sa < S; sa += plan.step) {
+      const int64_t sb = std::min(S, sa + plan.step);
+      const int slices = (int)ceil_div(sb - sa, plan.per);
+      const dim3 grid((unsigned)blocks, (unsigned)slices);
       const float* tb = trp + (int64_t)b * T * row;
-      if (chunk > 0) {
-        float* copy = static_cast<float*>(ws);
+      float* out = volp + (int64_t)b * nv;
+      float* dst = slices > 1 ? part : out;
+      const int add = slices == 1 && sa > 0;
+      if (plan.chunk > 0) {
         TOTRI_TRY(mesh::launch_bins_last(tb + sa * L, copy, (int)T, (int)T, row, (sb - sa) * L,
                                          stream));
         TOTRI_KERNEL("backprojection velten exhaustive", stream,
                      bp::velten_pairs_kernel<true><<<grid, 256, 0, stream>>>(
                          g, b, (int)T, (int)S, (int)L, sp, lp, so, lo, So > 0, Lo > 0, bw, bo,
-                         1.f / bw, (int)sa, (int)sb, per, copy, T, 1, volp, accumulate));
+                         1.f / bw, (int)sa, (int)sb, plan.per, copy, T, 1, dst, add));
       } else {
         TOTRI_KERNEL("backprojection velten exhaustive", stream,
                      bp::velten_pairs_kernel<false><<<grid, 256, 0, stream>>>(
                          g, b, (int)T, (int)S, (int)L, sp, lp, so, lo, So > 0, Lo > 0, bw, bo,
-                         1.f / bw, (int)sa, (int)sb, per, tb, 1, row, volp, accumulate));
+                         1.f / bw, (int)sa, (int)sb, plan.per, tb, 1, row, dst, add));
       }
+      if (slices > 1)
+        TOTRI_TRY(mesh::launch_sum_slices(part, slices, nv, out, sa > 0, stream));
     }
   return TOTRI_OK;
 }

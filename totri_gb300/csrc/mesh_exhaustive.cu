@@ -1304,6 +1304,43 @@ size_t exh_grad_scratch_bytes(int64_t S, int64_t L, int64_t T) {
   return c > 0 ? align_up((size_t)c * (size_t)L * (size_t)T * sizeof(float), 256) : 0;
 }
 
+PairPlan pair_plan(int64_t S, int64_t L, int64_t T, int64_t voxels, int64_t blocks, int64_t ctas,
+                   int64_t least, bool copies, size_t ws_bytes) {
+  PairPlan p{};
+  p.chunk = copies ? exh_grad_chunk_points(S, L, T) : 0;
+  size_t copy = (size_t)p.chunk * (size_t)L * (size_t)T * sizeof(float);
+  if (copy > ws_bytes) p.chunk = 0, copy = 0;
+  p.part_at = align_up(copy, 256);
+  p.step = p.chunk > 0 ? p.chunk : S;
+  const int64_t volume = voxels * (int64_t)sizeof(float);
+  const int64_t room = ws_bytes > p.part_at && volume > 0
+                           ? (int64_t)((ws_bytes - p.part_at) / (size_t)volume) : 0;
+  const int64_t slices = std::max<int64_t>(
+      1, std::min({ceil_div(ctas, blocks), p.step / least, room}));
+  p.per = (int)ceil_div(p.step, slices);
+  p.slices = (int)ceil_div(p.step, p.per);
+  p.bytes = p.slices > 1 ? p.part_at + (size_t)(p.slices * volume) : copy;
+  return p;
+}
+
+__global__ void __launch_bounds__(256) sum_slices_kernel(const float* __restrict__ part, int slices,
+                                                         int64_t n, float* __restrict__ out,
+                                                         int add) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  float sum = add ? out[i] : 0.f;
+  for (int s = 0; s < slices; ++s) sum += __ldg(part + s * n + i);
+  out[i] = sum;
+}
+
+int launch_sum_slices(const float* part, int slices, int64_t n, float* out, bool add,
+                      cudaStream_t stream) {
+  TOTRI_KERNEL("sum of slices", stream,
+               sum_slices_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, stream>>>(
+                   part, slices, n, out, add));
+  return TOTRI_OK;
+}
+
 // The mesh gradient's copies have rows of a multiple of 4 bins.
 static int64_t padded_bins(int64_t T) { return (T + 3) & ~(int64_t)3; }
 size_t mesh_grad_scratch_bytes(int64_t S, int64_t L, int64_t T) {

@@ -576,6 +576,23 @@ int launch_bins_last(const float* in, float* out, int T, int Tp, int64_t row, in
 // scratch bytes those copies need.
 int64_t exh_grad_chunk_points(int64_t S, int64_t L, int64_t T);
 size_t exh_grad_scratch_bytes(int64_t S, int64_t L, int64_t T);
+// How a gather over S scan points x L lasers (the exhaustive backprojection and volume
+// gradient) runs within a workspace of ws_bytes: scan points per bins-last copy (0: read in
+// place), per launch (step) and per slice, and the slices of a launch, each of which
+// writes a volume of partial sums of its own (at part_at in the workspace) that are
+// then added in order: the result repeats bit for bit. Without room for partial sums
+// a launch is one slice.
+struct PairPlan {
+  int64_t chunk, step;
+  int per, slices;
+  size_t part_at, bytes;  // bytes: all that the plan uses
+};
+// ctas: CTAs to launch at least, blocks of them per slice, each of `least` points.
+PairPlan pair_plan(int64_t S, int64_t L, int64_t T, int64_t voxels, int64_t blocks, int64_t ctas,
+                   int64_t least, bool copies, size_t ws_bytes);
+// out[i] = (add ? out[i] : 0) + sum over slices, in order, of part[slice n + i].
+int launch_sum_slices(const float* part, int slices, int64_t n, float* out, bool add,
+                      cudaStream_t stream);
 // The same for the mesh gradient, whose copies have rows of a multiple of 4 bins.
 size_t mesh_grad_scratch_bytes(int64_t S, int64_t L, int64_t T);
 

@@ -58,8 +58,9 @@ def backprojection_exhaustive_velten_forward(transient, scan_points, laser_point
     (reference src/reconstruct/backprojection.cpp:36-49)."""
     _lib.require_cuda(transient, scan_points, laser_points, scan_origin, laser_origin, volume)
     out = dense_out(volume)
-    n = int(_lib.load().totri_backprojection_exhaustive_velten_scratch(
-        int(scan_points.shape[1]), int(laser_points.shape[1]), int(transient.shape[1])))
+    n = int(_lib.load().totri_backprojection_exhaustive_velten_workspace(
+        int(scan_points.shape[1]), int(laser_points.shape[1]), int(transient.shape[1]),
+        *[int(d) for d in volume.shape[1:]], float(bin_width)))
     ws = torch.empty(n, dtype=torch.uint8, device=volume.device) if n > 0 else None
     _call("totri_backprojection_exhaustive_velten_forward_ws",
           (transient.contiguous(), scan_points, laser_points, scan_origin, laser_origin, out),
