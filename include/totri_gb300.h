@@ -364,12 +364,18 @@ int totri_volume_exhaustive_grad_volume(const totri_array_t* transient_grad,
                                         float bin_offset, void* stream);
 
 /* The same with an optional workspace of
- * totri_volume_exhaustive_grad_scratch(S, L, T) bytes (at most 2 GiB; smaller
- * or null: transient_grad is read in place, more slowly), which holds bins-last
- * copies of transient_grad, one batch item and range of scan points at a time.
- * The results are the same up to FP32 summation order. */
+ * totri_volume_exhaustive_grad_scratch(S, L, T) bytes, which is enough for any
+ * volume (at most 2 GiB and some 10 MB), or of the bytes that a call with the volume
+ * [D, H, W] uses (..._grad_workspace). It holds bins-last copies of transient_grad,
+ * one batch item and range of scan points at a time, and the partial sums of a
+ * launch. With less room or null transient_grad is read in place and a launch is not
+ * split: more slowly, the results the same up to FP32 summation order. A call
+ * repeats bit for bit with the same workspace size. */
 size_t totri_volume_exhaustive_grad_scratch(int64_t num_scan_points, int64_t num_laser_points,
                                             int64_t num_bins);
+size_t totri_volume_exhaustive_grad_workspace(int64_t num_scan_points, int64_t num_laser_points,
+                                              int64_t num_bins, int64_t depth, int64_t height,
+                                              int64_t width);
 int totri_volume_exhaustive_grad_volume_ws(const totri_array_t* transient_grad,
                                            const totri_array_t* scan_points,
                                            const totri_array_t* laser_points,

@@ -366,3 +366,22 @@ def test_exhaustive_velten_repeats(cuda_lib, shape, S, L, T):
     ref = oracle.bp_exhaustive_velten(tr[0].cpu().numpy(), sp[0].cpu().numpy(),
                                       lp[0].cpu().numpy(), None, None, shape, START, END, 0.02, 0.0)
     assert rel(call()[0].cpu().numpy(), ref) < 1e-5
+
+
+@pytest.mark.parametrize("shape,S,L,T", [((24, 24, 24), 256, 36, 300), ((5, 9, 3), 41, 7, 400)])
+def test_exhaustive_volume_gradient_repeats(cuda_lib, shape, S, L, T):
+    """The slices of a launch are added in order; against the FP64 oracle 1e-5."""
+    g = np.random.default_rng(S)
+    sp, lp = cu(points(g, S).T[None]), cu(points(g, L).T[None])
+    none = torch.empty((1, 3, 0), device="cuda")
+    tg = cu(g.uniform(0.5, 1.5, (1, T, S, L)).astype(np.float32))
+
+    def call():
+        out = torch.full((1,) + shape, 7.0, device="cuda")
+        R.volume_render_exhaustive_grad_volume(tg, sp, lp, none, none, out, START, END, 0.02, 0.0)
+        return out
+
+    assert repeats(call)
+    ref = oracle.volume_exhaustive_adjoint(tg[0].cpu().numpy(), shape, sp[0].cpu().numpy(),
+                                           lp[0].cpu().numpy(), START, END, 0.02, 0.0)
+    assert rel(call()[0].cpu().numpy(), ref) < 1e-5

@@ -113,6 +113,7 @@ _SIGNATURES = {
     "totri_volume_exhaustive_forward": [_ArrP] * 6 + [_F3, _F3, _flt, _flt, _vp, _sz, _vp],
     "totri_volume_exhaustive_grad_volume": [_ArrP] * 6 + [_F3, _F3, _flt, _flt, _vp],
     "totri_volume_exhaustive_grad_scratch": [_i64, _i64, _i64],
+    "totri_volume_exhaustive_grad_workspace": [_i64] * 6,
     "totri_volume_exhaustive_grad_volume_ws": [_ArrP] * 6 + [_F3, _F3, _flt, _flt, _vp, _sz, _vp],
     "totri_backprojection_confocal_velten_forward": [_ArrP] * 4 + [_F3, _F3, _flt, _flt, _vp],
     "totri_backprojection_confocal_velten_adjoint": [_ArrP] * 4 + [_F3, _F3, _flt, _flt, _vp],
@@ -148,6 +149,7 @@ _RESTYPES = {
     "totri_mesh_mask_bytes": ctypes.c_size_t,
     "totri_volume_workspace": ctypes.c_size_t,
     "totri_volume_exhaustive_grad_scratch": ctypes.c_size_t,
+    "totri_volume_exhaustive_grad_workspace": ctypes.c_size_t,
     "totri_backprojection_exhaustive_velten_scratch": ctypes.c_size_t,
     "totri_backprojection_exhaustive_velten_workspace": ctypes.c_size_t,
     "totri_marching_cubes_workspace": ctypes.c_size_t,

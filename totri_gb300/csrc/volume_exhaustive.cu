@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(256, 4) adjoint_kernel(Geo g, int b, Pts sp, P
                                                          int s_end, int per_slice,
                                                          const float* __restrict__ tg,
                                                          int64_t cstep, int64_t bstep,
-                                                         float* __restrict__ vg, int accumulate) {
+                                                         float* __restrict__ vg, int add) {
   using u64 = unsigned long long;
   __shared__ float win[2][kLC][kRows];
   __shared__ float2 laser[kLC][256];  // distances of the thread's voxel ends to the lasers
@@ -340,9 +340,9 @@ __global__ void __launch_bounds__(256, 4) adjoint_kernel(Geo g, int b, Pts sp, P
     }
   }
   if (xi >= g.W || yi >= g.H || zi >= g.D) return;
-  float* dst = vg + (((size_t)b * g.D + zi) * g.H + yi) * g.W + xi;
-  if (accumulate) atomicAdd(dst, acc);
-  else *dst = acc;
+  // (a slice's volume is its own)
+  float* dst = vg + (((size_t)blockIdx.y * g.D + zi) * g.H + yi) * g.W + xi;
+  *dst = add ? *dst + acc : acc;
 }
 
 }  // namespace vexh
@@ -452,8 +452,28 @@ int totri_volume_exhaustive_forward(const totri_array_t* vol, const totri_array_
   return TOTRI_OK;
 }
 
+// Bins-last copies (one read and write of transient_grad, where a pair's reads in place
+// are a sector per voxel and bin); slices of the scan points until about 8 waves of
+// CTAs (4 per SM), with at least 8 scan points each (a slice repeats the lasers'
+// distances).
+static mesh::PairPlan grad_plan(int64_t S, int64_t L, int64_t T, int64_t D, int64_t H, int64_t W,
+                                size_t ws_bytes) {
+  const int64_t blocks = ceil_div(W, 8) * ceil_div(H, 8) * ceil_div(D, 4);
+  return mesh::pair_plan(S, L, T, D * H * W, blocks, 32 * (int64_t)tune::sm_count(), 8, true,
+                         ws_bytes);
+}
+
 size_t totri_volume_exhaustive_grad_scratch(int64_t S, int64_t L, int64_t T) {
-  return mesh::exh_grad_scratch_bytes(S, L, T);
+  // Partial sums of a launch: slices of at most 256 voxels per CTA, fewer than 2 x 32
+  // CTAs per SM where there is more than one.
+  const size_t partial = S < 16 ? 0 : sizeof(float) * 256 * 64 * (size_t)tune::sm_count();
+  return S > 0 && L > 0 && T > 0 ? mesh::exh_grad_scratch_bytes(S, L, T) + partial : 0;
+}
+
+size_t totri_volume_exhaustive_grad_workspace(int64_t S, int64_t L, int64_t T, int64_t D, int64_t H,
+                                              int64_t W) {
+  if (S <= 0 || L <= 0 || T <= 0 || D <= 0 || H <= 0 || W <= 0) return 0;
+  return grad_plan(S, L, T, D, H, W, SIZE_MAX).bytes;
 }
 
 int totri_volume_exhaustive_grad_volume_ws(const totri_array_t* tg,
@@ -488,38 +508,32 @@ int totri_volume_exhaustive_grad_volume_ws(const totri_array_t* tg,
     TOTRI_CUDA(cudaMemsetAsync(out, 0, sizeof(float) * n, stream));
     return TOTRI_OK;
   }
-  // Scan points per bins-last copy (all of them up to 2 GiB); 0: read in place.
-  // The copy costs one read and write of transient_grad, a pair's reads in place
-  // a sector per voxel and bin.
-  int64_t chunk = ws ? mesh::exh_grad_chunk_points(S, L, T) : 0;
-  if (ws_bytes < (size_t)chunk * L * T * sizeof(float)) chunk = 0;
-  const int64_t step = chunk > 0 ? chunk : S;
+  const mesh::PairPlan plan = grad_plan(S, L, T, g.D, g.H, g.W, ws ? ws_bytes : 0);
   const int64_t blocks = ceil_div(g.W, 8) * ceil_div(g.H, 8) * ceil_div(g.D, 4);
-  // slices of the scan points until about 8 waves of CTAs (4 per SM), with at
-  // least 8 scan points each (a slice repeats the lasers' distances)
-  const int64_t slices = std::max<int64_t>(
-      1, std::min<int64_t>(ceil_div(32 * (int64_t)tune::sm_count(), blocks), step / 8));
-  const int per = (int)ceil_div(step, slices);
-  const int accumulate = ceil_div(step, per) > 1 || step < S;
-  if (accumulate) TOTRI_CUDA(cudaMemsetAsync(out, 0, sizeof(float) * n, stream));
-  const int64_t row = S * L;
+  const int64_t row = S * L, nv = (int64_t)g.D * g.H * g.W;
+  float* copy = static_cast<float*>(ws);
+  float* part = reinterpret_cast<float*>(static_cast<char*>(ws) + plan.part_at);
   for (int b = 0; b < (int)B; ++b) {
     const float* tb = static_cast<const float*>(tg->data) + (int64_t)b * T * row;
-    for (int64_t sa = 0; sa < S; sa += step) {
-      const int64_t sb = std::min(S, sa + step);
-      const dim3 grid((unsigned)blocks, (unsigned)ceil_div(sb - sa, per));
-      if (chunk > 0) {
-        float* copy = static_cast<float*>(ws);
+    for (int64_t sa = 0; sa < S; sa += plan.step) {
+      const int64_t sb = std::min(S, sa + plan.step);
+      const int slices = (int)ceil_div(sb - sa, plan.per);
+      const dim3 grid((unsigned)blocks, (unsigned)slices);
+      float* sum = out + b * nv;
+      float* dst = slices > 1 ? part : sum;
+      const int add = slices == 1 && sa > 0;
+      if (plan.chunk > 0) {
         TOTRI_TRY(mesh::launch_bins_last(tb + sa * L, copy, (int)T, (int)T, row, (sb - sa) * L,
                                          stream));
         TOTRI_KERNEL("volume exhaustive adjoint", stream,
                      vexh::adjoint_kernel<<<grid, 256, 0, stream>>>(
-                         g, b, sp, lp, (int)sa, (int)sb, per, copy, T, 1, out, accumulate));
+                         g, b, sp, lp, (int)sa, (int)sb, plan.per, copy, T, 1, dst, add));
       } else {
         TOTRI_KERNEL("volume exhaustive adjoint", stream,
                      vexh::adjoint_kernel<<<grid, 256, 0, stream>>>(
-                         g, b, sp, lp, (int)sa, (int)sb, per, tb, 1, row, out, accumulate));
+                         g, b, sp, lp, (int)sa, (int)sb, plan.per, tb, 1, row, dst, add));
       }
+      if (slices > 1) TOTRI_TRY(mesh::launch_sum_slices(part, slices, nv, sum, sa > 0, stream));
     }
   }
   return TOTRI_OK;

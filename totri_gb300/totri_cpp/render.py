@@ -181,8 +181,9 @@ def volume_render_exhaustive_grad_volume(transient_grad, scan_points, laser_poin
     _lib.require_cuda(transient_grad, scan_points, laser_points, scan_origin, laser_origin,
                       volume_grad)
     out = dense_out(volume_grad)
-    n = int(_lib.load().totri_volume_exhaustive_grad_scratch(
-        int(scan_points.shape[2]), int(laser_points.shape[2]), int(transient_grad.shape[1])))
+    n = int(_lib.load().totri_volume_exhaustive_grad_workspace(
+        int(scan_points.shape[2]), int(laser_points.shape[2]), int(transient_grad.shape[1]),
+        *[int(d) for d in volume_grad.shape[1:]]))
     ws = torch.empty(n, dtype=torch.uint8, device=volume_grad.device) if n > 0 else None
     _vol_call("totri_volume_exhaustive_grad_volume_ws",
               (transient_grad.contiguous(), scan_points, laser_points, scan_origin,
