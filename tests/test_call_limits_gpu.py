@@ -385,3 +385,62 @@ def test_exhaustive_volume_gradient_repeats(cuda_lib, shape, S, L, T):
     ref = oracle.volume_exhaustive_adjoint(tg[0].cpu().numpy(), shape, sp[0].cpu().numpy(),
                                            lp[0].cpu().numpy(), START, END, 0.02, 0.0)
     assert rel(call()[0].cpu().numpy(), ref) < 1e-5
+
+
+def _pair_calls(S, L, T, shape):
+    """The exhaustive backprojection and volume gradient of the same sizes: (call, with
+    the workspace's use in it) each of an output tensor."""
+    g = np.random.default_rng(S)
+    sp, lp = cu(points(g, S)[None]), cu(points(g, L)[None])
+    tr = cu(g.integers(0, 16, (1, T, S, L)).astype(np.float32))
+    n1, n3 = torch.empty((1, 0, 3), device="cuda"), torch.empty((1, 3, 0), device="cuda")
+    return tr, {
+        "velten": lambda out: K.backprojection_exhaustive_velten_forward(
+            tr, sp, lp, n1, n1, out, START, END, 0.02, 0.0),
+        "volume": lambda out: R.volume_render_exhaustive_grad_volume(
+            tr, sp.transpose(1, 2), lp.transpose(1, 2), n3, n3, out, START, END, 0.02, 0.0)}
+
+
+@pytest.mark.parametrize("kind", ["velten", "volume"])
+def test_exhaustive_calls_without_memory_for_scratch(cuda_lib, kind, monkeypatch):
+    """Where the scratch cannot be allocated the transient is read in place (integers
+    and partial sums of a few hundred pairs: 1e-5)."""
+    shape = (1, 9, 10, 11)
+    _, calls = _pair_calls(33, 20, 200, shape)
+    want, got = torch.empty(shape, device="cuda"), torch.empty(shape, device="cuda")
+    calls[kind](want)
+    empty = torch.empty
+
+    def no_scratch(*args, **kw):
+        if kw.get("dtype") == torch.uint8:
+            raise torch.cuda.OutOfMemoryError("no memory")
+        return empty(*args, **kw)
+
+    monkeypatch.setattr(torch, "empty", no_scratch)
+    calls[kind](got)
+    assert float((got - want).norm() / want.norm()) < 1e-5
+
+
+def test_exhaustive_velten_takes_no_copies_that_it_does_not_use(cuda_lib):
+    """A volume of fewer voxels than bins is read in place: no copy of the transient."""
+    shape = (1, 8, 8, 8)
+    tr, calls = _pair_calls(100, 50, 2000, shape)
+    out = torch.empty(shape, device="cuda")
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    calls["velten"](out)
+    assert torch.cuda.max_memory_allocated() - before < tr.numel() * 4 // 4
+
+
+def test_exhaustive_calls_of_a_wrong_rank(cuda_lib):
+    """Refused by the entry point, as every other wrong shape."""
+    t = lambda *s: torch.zeros(s, device="cuda")
+    none = t(1, 0, 3)
+    with pytest.raises((ValueError, RuntimeError), match="dimensions"):
+        K.backprojection_exhaustive_velten_forward(t(5), t(3), t(3), none, none, t(1, 4, 4, 4),
+                                                   START, END, 0.02, 0.0)
+    with pytest.raises((ValueError, RuntimeError), match="dimensions"):
+        R.volume_render_exhaustive_grad_volume(t(1, 9, 2, 2), t(1, 3, 2), t(1, 3, 2),
+                                               t(1, 3, 0), t(1, 3, 0), t(4, 4), START, END, 0.02,
+                                               0.0)

@@ -25,6 +25,24 @@ def mesh_workspace(B, V, F, P, device, extra=0):
     return torch.empty(n + int(extra), dtype=torch.uint8, device=device)
 
 
+def pair_workspace(size, scan_points, laser_points, axis, transient, volume, *more):
+    """Scratch that `size` asks for (points per side on `axis`, bins, the volume's
+    shape, `more`) for an entry point that also runs without, more slowly: None where
+    nothing is needed, memory is short or a rank is wrong (which the entry point
+    reports)."""
+    if not (scan_points.dim() == laser_points.dim() == 3 and
+            transient.dim() == volume.dim() == 4):
+        return None
+    n = int(size(*[int(x) for x in (scan_points.shape[axis], laser_points.shape[axis],
+                                    transient.shape[1], *volume.shape[1:])], *more))
+    if n == 0:
+        return None
+    try:
+        return torch.empty(n, dtype=torch.uint8, device=volume.device)
+    except torch.cuda.OutOfMemoryError:
+        return None
+
+
 def exhaustive_grad_scratch(S, L, T):
     """Bytes of the exhaustive gradient's optional bins-last scratch."""
     return int(_lib.load().totri_mesh_exhaustive_grad_scratch(int(S), int(L), int(T)))

@@ -1,8 +1,6 @@
 """Drop-in for ``totri_cpp.reconstruct`` (reference src/totri.cpp:18-25)."""
-import torch
-
 from .. import _lib
-from ._common import dense_out, finish_out, ws_args
+from ._common import dense_out, finish_out, pair_workspace, ws_args
 
 
 def _call(name, tensors, a3, b3, bw, bo, device, extra=()):
@@ -58,10 +56,8 @@ def backprojection_exhaustive_velten_forward(transient, scan_points, laser_point
     (reference src/reconstruct/backprojection.cpp:36-49)."""
     _lib.require_cuda(transient, scan_points, laser_points, scan_origin, laser_origin, volume)
     out = dense_out(volume)
-    n = int(_lib.load().totri_backprojection_exhaustive_velten_workspace(
-        int(scan_points.shape[1]), int(laser_points.shape[1]), int(transient.shape[1]),
-        *[int(d) for d in volume.shape[1:]], float(bin_width)))
-    ws = torch.empty(n, dtype=torch.uint8, device=volume.device) if n > 0 else None
+    ws = pair_workspace(_lib.load().totri_backprojection_exhaustive_velten_workspace,
+                        scan_points, laser_points, 1, transient, volume, float(bin_width))
     _call("totri_backprojection_exhaustive_velten_forward_ws",
           (transient.contiguous(), scan_points, laser_points, scan_origin, laser_origin, out),
           volume_start, volume_end, bin_width, bin_offset, volume.device, extra=ws_args(ws))

@@ -8,7 +8,7 @@ import torch
 
 from .. import _lib
 from ._common import (check_device_status, dense_out, exhaustive_grad_scratch, finish_out,
-                      mesh_workspace, ws_args)
+                      mesh_workspace, pair_workspace, ws_args)
 
 
 def _mesh_call(name, tensors, bw, bo, model, points, extra=0):
@@ -181,10 +181,8 @@ def volume_render_exhaustive_grad_volume(transient_grad, scan_points, laser_poin
     _lib.require_cuda(transient_grad, scan_points, laser_points, scan_origin, laser_origin,
                       volume_grad)
     out = dense_out(volume_grad)
-    n = int(_lib.load().totri_volume_exhaustive_grad_workspace(
-        int(scan_points.shape[2]), int(laser_points.shape[2]), int(transient_grad.shape[1]),
-        *[int(d) for d in volume_grad.shape[1:]]))
-    ws = torch.empty(n, dtype=torch.uint8, device=volume_grad.device) if n > 0 else None
+    ws = pair_workspace(_lib.load().totri_volume_exhaustive_grad_workspace, scan_points,
+                        laser_points, 2, transient_grad, volume_grad)
     _vol_call("totri_volume_exhaustive_grad_volume_ws",
               (transient_grad.contiguous(), scan_points, laser_points, scan_origin,
                laser_origin, out), volume_start, volume_end, bin_width, bin_offset,
