@@ -571,9 +571,11 @@ __global__ void __launch_bounds__(32 * kListWarps, kOcc) visibility_list_kernel(
                                                                fr0 + kListFrontier, cand, lane,
                                                                list_cap);
           for (int base = 0; base < count; base += 32) {
-            const int kk = base + lane < count ? cand[base + lane] : -1;
+            const int kk = base + lane < count ? cand[base + lane] : k;
             bool in = false;
-            if (kk >= 0 && kk != k) {
+            if ((unsigned)kk >= (unsigned)n) {
+              atomicOr(sc.status, kStatusTraversalCap);
+            } else if (kk != k) {
               const float4* q = tri_at(sc, b, kk);
               const float4 t2 = __ldg(q + 2), t3 = __ldg(q + 3);
               in = shaft_box(h, t2.y, t2.z, t2.w, t3.x, t3.y, t3.z);
