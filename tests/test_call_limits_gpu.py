@@ -444,3 +444,51 @@ def test_exhaustive_calls_of_a_wrong_rank(cuda_lib):
         R.volume_render_exhaustive_grad_volume(t(1, 9, 2, 2), t(1, 3, 2), t(1, 3, 2),
                                                t(1, 3, 0), t(1, 3, 0), t(4, 4), START, END, 0.02,
                                                0.0)
+
+
+@pytest.mark.parametrize("vz", [1, 2, 4])
+@pytest.mark.parametrize("tile", [8, 16, 32])
+@pytest.mark.parametrize("T,bw,bo", [(300, 0.01, 0.0), (700, 0.003, 1.0), (64, 0.02, 3.9)])
+def test_every_tiled_velten_kernel_equals_the_untiled_one(cuda_lib, vz, tile, T, bw, bo):
+    """Each voxels-per-thread and points-per-tile kernel sums the same bins in the same
+    order as the kernel without windows: bit for bit, on real-valued transients."""
+    g = np.random.default_rng(T)
+    shape, S = (1, 19, 10, 21), 133
+    sp, so = cu(points(g, S)[None]), cu(points(g, S, -0.2)[None])
+    tr = cu(g.standard_normal((1, T, S)).astype(np.float32))
+    got, want = torch.empty(shape, device="cuda"), torch.empty(shape, device="cuda")
+    with tuned({"backprojection.velten.mode": 1}):
+        K.backprojection_confocal_velten_forward(tr, sp, so, want, START, END, bw, bo)
+    with tuned({"backprojection.velten.vz": vz, "backprojection.velten.points": tile}):
+        K.backprojection_confocal_velten_forward(tr, sp, so, got, START, END, bw, bo)
+    assert float(want.abs().sum()) > 0.0
+    assert torch.equal(got, want)
+
+
+def test_exhaustive_calls_over_several_ranges_of_scan_points(cuda_lib):
+    """A transient above 2 GiB: bins-last copies of 512 and then 88 scan points. The
+    backprojection of small integers (sums below 2^24) equals the one-voxel-per-thread
+    kernel bit for bit; the volume gradient of 30 scan points across the two ranges is
+    a sum of 27,000 FP32 terms of one sign in another order than the oracle's: 1e-4."""
+    S, L, T, shape = 600, 900, 1024, (1, 16, 8, 8)
+    g = np.random.default_rng(1)
+    spn, lpn = points(g, S), points(g, L)
+    sp, lp = cu(spn[None]), cu(lpn[None])
+    none = torch.empty((1, 0, 3), device="cuda")
+    tr = torch.randint(0, 16, (1, T, S, L), device="cuda", dtype=torch.uint8).float()
+    got, want = torch.empty(shape, device="cuda"), torch.empty(shape, device="cuda")
+    K.backprojection_exhaustive_velten_forward(tr, sp, lp, none, none, got, START, END, 0.005, 0.0)
+    with tuned({"backprojection.velten.pairs": 1}):
+        K.backprojection_exhaustive_velten_forward(tr, sp, lp, none, none, want, START, END, 0.005,
+                                                   0.0)
+    assert float(want.abs().sum()) > 0.0
+    assert torch.equal(got, want)
+    tr[:, :, :500] = 0.0
+    tr[:, :, 530:] = 0.0
+    none = torch.empty((1, 3, 0), device="cuda")
+    R.volume_render_exhaustive_grad_volume(tr, sp.transpose(1, 2), lp.transpose(1, 2), none, none,
+                                           got, START, END, 0.005, 0.0)
+    part = tr[0, :, 500:530].cpu().numpy()
+    ref = oracle.volume_exhaustive_adjoint(part, shape[1:], spn[500:530].T, lpn.T, START, END,
+                                           0.005, 0.0)
+    assert rel(got[0].cpu().numpy(), ref) < 1e-4

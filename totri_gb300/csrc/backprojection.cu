@@ -814,9 +814,9 @@ int totri_backprojection_confocal_velten_forward(const totri_array_t* transient,
   const bool tiled = tune::get("backprojection.velten.mode") != 1;
   int vz = tune::get("backprojection.velten.vz");
   if (vz <= 0) vz = 4;
-  if (vz != 1 && vz != 2 && vz != 4)
-    return fail(TOTRI_ERR_INVALID_ARGUMENT, "backprojection.velten.vz must be 1, 2 or 4");
-  if (vz == 1) vz = 2;  // voxels go in pairs
+  if (vz == 1) vz = 2;  // voxels go in pairs: 1 is taken as 2
+  if (vz != 2 && vz != 4)
+    return fail(TOTRI_ERR_INVALID_ARGUMENT, "backprojection.velten.vz must be 2 or 4");
   const dim3 grid((unsigned)ceil_div(g.W, bp::kBX), (unsigned)ceil_div(g.H, bp::kBY),
                   (unsigned)ceil_div(g.D, bp::kBZ * vz));
   // Points per tile (32, 16 or 8; "backprojection.velten.points" sets it): the
