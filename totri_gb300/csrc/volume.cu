@@ -427,9 +427,10 @@ __global__ void __launch_bounds__(32 * PT > 256 ? 32 * PT : 256) grad_mp_kernel(
                             radial += fmaf(4.f * w * df2, inv, slope) * (inv * g.dz);
                             axial += slope;
                           });
-      gx -= rec.z * ((p.wx - rec.x) * g.scale) * radial;
-      gy -= rec.z * ((p.wy - rec.y) * g.scale) * radial;
-      gz += rec.z * axial;
+      // (an infinite voxel or point without a sample adds nothing)
+      gx -= radial != 0.f ? rec.z * ((p.wx - rec.x) * g.scale) * radial : 0.f;
+      gy -= radial != 0.f ? rec.z * ((p.wy - rec.y) * g.scale) * radial : 0.f;
+      gz += axial != 0.f ? rec.z * axial : 0.f;
     }
   }
   for (int o = PT; o < 32; o <<= 1) {
