@@ -494,6 +494,33 @@ def test_exhaustive_calls_over_several_ranges_of_scan_points(cuda_lib):
     assert rel(got[0].cpu().numpy(), ref) < 1e-4
 
 
+@pytest.mark.parametrize("T", [150, 4100])
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("bw,bo,far", [(1e-30, 0.0, 0.0), (0.02, -1e8, 0.0), (0.02, 0.0, 3e37),
+                                       (0.02, 0.0, float("inf")), (1e-9, -3.0, 0.0)])
+def test_volume_gradients_of_bins_out_of_reach(cuda_lib, T, mode, bw, bo, far):
+    """First bins beyond 2^31 (a tiny bin width, an offset far below zero, points far
+    away): empty spans, so the near points alone are in the adjoint (1e-5 of the FP64
+    oracle) and the far ones get no gradient."""
+    g = np.random.default_rng(12)
+    shape, N = (5, 9, 40), 70
+    mp = np.stack([g.uniform(-1, 1, N), g.uniform(-1, 1, N), np.zeros(N)]).astype(np.float32)
+    y = g.uniform(0.5, 1.5, (N, T)).astype(np.float32)
+    vol = g.uniform(0.5, 1.5, shape).astype(np.float32)
+    org, size = (-0.5, -0.5, 0.5), (1.0, 1.0, 1.0)
+    near = np.ones(N, bool)
+    if far:
+        near[::3] = False
+        mp[0, ::3] = far
+    adj, gm = torch.full(shape, 7.0, device="cuda"), torch.full((3, N), 7.0, device="cuda")
+    with tuned({"volume.adjoint.mode": mode}):
+        R.volume_confocal_adjoint(adj, cu(mp), cu(y), org, size, bw, bo)
+    R.volume_confocal_grad_measurement_points(gm, cu(vol), cu(mp), cu(y), org, size, bw, bo)
+    ref = oracle.volume_confocal_adjoint(y[near], shape, mp[:, near], org, size, bw, bo)
+    assert rel(adj.cpu().numpy(), ref) < 1e-5
+    assert not bool(gm[:, torch.as_tensor(~near).cuda()].any())
+
+
 def test_volume_point_gradient_of_voxels_out_of_reach(cuda_lib):
     """An infinite voxel behind every point's samples adds nothing to their gradient
     (1e-4 of the FP64 oracle without it)."""

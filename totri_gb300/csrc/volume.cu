@@ -125,7 +125,8 @@ __device__ __forceinline__ int first_nonneg_bin(const Geo& g) {
 }
 
 // Bins whose centre's magnitude lies in [cl, ch] widened by eps bins: [p0, p1]
-// with non-negative centres (t >= tz) and [n0, n1] with negative ones (t < tz).
+// with non-negative centres (t >= tz) and [n0, n1] with negative ones (t < tz). A span
+// whose last bin is before its first is empty; its first may be any up to INT_MAX.
 // Every bin when the bin width is degenerate. A NaN bound gives empty spans.
 struct Spans {
   int p0, p1, n0, n1;
@@ -144,6 +145,14 @@ __device__ __forceinline__ Spans tc_spans(const Geo& g, int tz, float cl, float 
     s.n0 = max(__float2int_ru((-ch - g.bo) * g.inv_bw - eps), 0);
     s.n1 = min(__float2int_rd((-cl - g.bo) * g.inv_bw + eps), tz - 1);
   }
+  return s;
+}
+
+// The same spans with first bins of at most T, for walks that add a lane's offset to
+// them before the test for an empty span.
+__device__ __forceinline__ Spans within_bins(const Geo& g, Spans s) {
+  s.p0 = min(s.p0, g.T);
+  s.n0 = min(s.n0, g.T);
   return s;
 }
 
@@ -529,7 +538,7 @@ __device__ __forceinline__ Spans column_span(const Geo& g, int tz, float rho2, f
   float cl, ch;
   if (!tc_bounds(rho2, wz, g.oz + 0.5f / g.scale, g.oz + ((float)g.Z + 0.5f) / g.scale, cl, ch))
     return Spans{1, 0, 1, 0};
-  return tc_spans(g, tz, cl, ch, 1.f);
+  return within_bins(g, tc_spans(g, tz, cl, ch, 1.f));
 }
 
 // Largest |t bw + bo| over the bins of two spans (0 when both are empty).
@@ -971,7 +980,7 @@ __global__ void __launch_bounds__(256, 3) confocal_adjoint_columns_kernel(
       float cl, ch, unused;
       if (zn > 0 && zlo <= zhi && tc_bounds(ex * ex + ey * ey, lwz, zlo, zhi, cl, unused) &&
           tc_bounds(fx * fx + fy * fy, lwz, zlo, zhi, unused, ch))
-        sp = tc_spans(g, tz, cl, ch, span_eps(g, ch, lwz));
+        sp = within_bins(g, tc_spans(g, tz, cl, ch, span_eps(g, ch, lwz)));
       // sample_filtered's margin over the spans' largest |tc|
       const float dmax = 1.001f * span_tc_max(g, sp);
       const float zmax = fabsf(lwz) + dmax;
