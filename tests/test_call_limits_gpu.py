@@ -537,3 +537,12 @@ def test_volume_point_gradient_of_voxels_out_of_reach(cuda_lib):
     gm = torch.full((3, N), 7.0, device="cuda")
     R.volume_confocal_grad_measurement_points(gm, cu(vol), cu(mp), cu(y), org, size, 0.01, 0.0)
     assert rel(gm.cpu().numpy(), ref) < 1e-4
+
+
+def test_velten_of_no_bins(cuda_lib):
+    """A transient [1, 0, S], which has no address, gives zeros."""
+    out = torch.full((1, 5, 6, 7), 7.0, device="cuda")
+    K.backprojection_confocal_velten_forward(
+        torch.empty((1, 0, 9), device="cuda"), torch.zeros((1, 9, 3), device="cuda"),
+        torch.empty((1, 0, 3), device="cuda"), out, START, END, 0.02, 0.0)
+    assert not bool(out.any())

@@ -811,6 +811,10 @@ int totri_backprojection_confocal_velten_forward(const totri_array_t* transient,
   const int T = (int)transient->shape[1];
   const int64_t nv = (int64_t)g.D * g.H * g.W;
   if (nv == 0 || B == 0) return TOTRI_OK;
+  if (S == 0 || T == 0) {  // (an empty transient has no address to stage rows from)
+    TOTRI_CUDA(cudaMemsetAsync(volume->data, 0, sizeof(float) * (size_t)(B * nv), stream));
+    return TOTRI_OK;
+  }
   const bool tiled = tune::get("backprojection.velten.mode") != 1;
   int vz = tune::get("backprojection.velten.vz");
   if (vz <= 0) vz = 4;
