@@ -546,3 +546,30 @@ def test_velten_of_no_bins(cuda_lib):
         torch.empty((1, 0, 9), device="cuda"), torch.zeros((1, 9, 3), device="cuda"),
         torch.empty((1, 0, 3), device="cuda"), out, START, END, 0.02, 0.0)
     assert not bool(out.any())
+
+
+@pytest.mark.parametrize("unit", [1e-6, 1e-4, 1e3])
+def test_mesh_gradients_in_other_units(cuda_lib, unit):
+    """A scene of a metre in megametres, tens of kilometres and millimetres: both
+    gradients 1e-5 of the oracle, as in metres."""
+    g = np.random.default_rng(8)
+    v, f, m = sphere(1600, 3)
+    v = v * unit
+    sp, lp = points(g, 70) * np.float32(unit), points(g, 12) * np.float32(unit)
+    none, T, bw = torch.empty((1, 0, 3), device="cuda"), 150, 0.02 * unit
+    vn, fn, mn = (x[0].cpu().numpy() for x in (v, f, m))
+    vs, vl = mesh_masks(v, f, sp, lp)
+    vg, mg = torch.empty_like(v), torch.empty_like(m)
+    tg = g.standard_normal((T, 70)).astype(np.float32)
+    R.mesh_confocal_grad_verts(v, f, m, cu(sp[None]), none, cu(tg[None]), vg, mg, bw, 0.0, 0)
+    rv, rm = oracle.mesh_confocal_grad(vn, fn, mn, sp, None, vs, T, bw, 0.0, tg)
+    assert np.linalg.norm(rv) > 0.0
+    assert rel(vg[0].cpu().numpy(), rv) < 1e-5
+    assert rel(mg[0].cpu().numpy(), rm) < 1e-5
+    tg = g.standard_normal((T, 70, 12)).astype(np.float32)
+    R.mesh_exhaustive_grad_verts(v, f, m, cu(sp[None]), cu(lp[None]), none, none, cu(tg[None]),
+                                 vg, mg, bw, 0.0, 0)
+    rv, rm = oracle.mesh_exhaustive_grad(vn, fn, mn, sp, lp, None, None, vs, vl, T, bw, 0.0, tg)
+    assert np.linalg.norm(rv) > 0.0
+    assert rel(vg[0].cpu().numpy(), rv) < 1e-5
+    assert rel(mg[0].cpu().numpy(), rm) < 1e-5

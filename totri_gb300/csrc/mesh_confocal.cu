@@ -882,8 +882,9 @@ __global__ void __launch_bounds__(256, 2) grad_kernel(Scene sc, View3f sp, View3
       const fv3 p = mkv(sp.at(b, s, 0), sp.at(b, s, 1), sp.at(b, s, 2));
       const fv3 r = c - p;
       if (!(r.z > 0.f)) return;
-      const float nr = dot(nrm, r), rr = dot(r, r), rr2 = rr * rr;
-      const float alpha = vdiv(kf * (r.z * r.z) * (nr * nr), rr2 * rr2);
+      const float nr = dot(nrm, r), rr = dot(r, r);
+      // (the square of r.z nr / |r|^4: |r|^8 leaves the FP32 range in small units)
+      const float fall = vdiv(r.z * nr, rr * rr), alpha = kf * fall * fall;
       if (!(alpha > 0.f)) return;
       float i0, i1, i2;  // 1 / |v_m - p|
       auto path = [&](fv3 v, float& inv) {
@@ -952,7 +953,9 @@ __global__ void __launch_bounds__(256, 2) grad_kernel(Scene sc, View3f sp, View3
     fv3 acc[3] = {mkv(0.f, 0.f, 0.f), mkv(0.f, 0.f, 0.f), mkv(0.f, 0.f, 0.f)};
     float accm = 0.f;
     if (used) {
-      const fv3 jw = (vdiv(-1.f, nn) * sP) * nrm + mkv(t[3], t[4], t[5]);
+      // (1 / |n|^2 is first multiplied by n: with the sum it leaves the FP32 range in
+      // small units)
+      const fv3 jw = sP * (vdiv(-1.f, nn) * nrm) + mkv(t[3], t[4], t[5]);
       const fv3 g1 = cross(e2, jw), g2 = cross(jw, e1);
       const fv3 common = mkv(t[0], t[1], t[2]) + (t[6] * (1.f / 3.f)) * nrm + mkv(0.f, 0.f, t[7]);
       acc[0] = common - g1 - g2 + mkv(t[9], t[10], t[11]);

@@ -778,10 +778,10 @@ __global__ void __launch_bounds__(256, kOcc) exh_grad_face_kernel(
       if (tid < 9) {
         const int m = tid / 3, a = tid - 3 * m;
         // d alpha: w = sum P (wf + wv), wf = -n / |n|^2, through the normal's Jacobian
-        // (a face without a pair adds zeros, whatever its normal and albedo)
-        const float wf = tot[15] != 0.f ? vdiv(-1.f, nn) * tot[15] : 0.f;
+        // (a face without a pair adds zeros, whatever its normal and albedo; 1 / |n|^2 is
+        // first multiplied by n: with the sum it leaves the FP32 range in small units)
         fv3 w = mkv(tot[3], tot[4], tot[5]);
-        if (wf != 0.f) w = wf * nrm + w;
+        if (tot[15] != 0.f) w = tot[15] * (vdiv(-1.f, nn) * nrm) + w;
         const fv3 g1 = cross(v[2] - v[0], w), g2 = cross(w, v[1] - v[0]);
         const fv3 g = m == 0 ? -(g1 + g2) : (m == 1 ? g1 : g2);
         const float t = tot[a] + (a == 0 ? g.x : (a == 1 ? g.y : g.z)) + tot[6 + tid];
