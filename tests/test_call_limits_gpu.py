@@ -573,3 +573,25 @@ def test_mesh_gradients_in_other_units(cuda_lib, unit):
     assert np.linalg.norm(rv) > 0.0
     assert rel(vg[0].cpu().numpy(), rv) < 1e-5
     assert rel(mg[0].cpu().numpy(), rm) < 1e-5
+
+
+@pytest.mark.parametrize("P", [32, 64, 1024, 2048, 4096])
+@pytest.mark.parametrize("wall", ["grid", "jitter", "random", "line", "one"])
+def test_power_of_two_walls(cuda_lib, P, wall):
+    """Masks of 2^k wall points are the brute-force ones in either order of the points:
+    a 2^a x 2^b grid, one with its points moved, random points, points on a line and
+    all in one place; two items of different walls in a batch."""
+    g = np.random.default_rng(P)
+    v, f, _ = sphere(500, 3)
+    a = 1 << ((P.bit_length() - 1) // 2)
+    x, y = np.meshgrid(np.linspace(-1, 1, a), np.linspace(-1, 1, P // a), indexing="ij")
+    grid = np.stack([x.ravel(), y.ravel(), 0 * x.ravel()], 1).astype(np.float32)
+    pts = {"grid": grid, "random": points(g, P), "one": np.repeat(grid[:1], P, 0),
+           "jitter": grid + points(g, P) * np.float32(0.5 / a),
+           "line": grid * np.float32([1, 0, 0])}[wall]
+    both = cu(np.stack([pts, points(g, P)]))
+    v2, f2 = torch.cat([v, v]), torch.cat([f, f])
+    want = R.mesh_visibility(v2, f2, both, brute_force=True)
+    for lists in (0, 1):
+        with tuned({"mesh.visibility.list": lists}):
+            assert torch.equal(R.mesh_visibility(v2, f2, both), want)

@@ -319,9 +319,12 @@ __device__ __forceinline__ uint32_t hilbert2(uint32_t x, uint32_t y) {
 // together on grids of any size: visibility of 20,480 faces from 56 x 56 points
 // took 5.2 ms over blocks in Morton order, which jumps inside a block there, and
 // 3.9 ms now; from 40 x 40, 4.1 and 2.8 ms. Other points take the Morton order, as
-// all do with "mesh.visibility.morton" = 1, and so do 2^k points, whose grids' blocks
-// are whole in it (five meshes at 64 x 64 points: 5.13 ms in the mean, 5.27 along
-// the curve). scr is
+// all do with "mesh.visibility.morton" = 1, and so do 2^k points whose blocks are
+// whole in it, as those of a 2^a x 2^b grid are: if the blocks' boxes together cover at
+// most three quarters of the wall (64 x 64: 0.66; where blocks overlap, more). Seven
+// meshes of 20,480 faces from 64 x 64 points: 5.16 ms in the mean, 5.40 along the
+// curve; three from 4,096 random points 6.97 and 5.61, 5,000 faces from 1,024 random
+// points 1.53 and 0.79. scr is
 // [4][B][P] (keys, values, keys, values); the permutation (point indices in that
 // order) ends in the fourth quarter, and the first quarter is then set to -1: the
 // visibility kernel keeps each point's last occluder there (by the point's place).
@@ -355,22 +358,39 @@ __device__ __forceinline__ void point_order_item(const View3f& pts, int P, int B
   for (int a = 0; a < 3; ++a) ext[a] = iord(box[3 + a]) - iord(box[a]);
   const int thin = ext[0] <= ext[1] ? (ext[0] <= ext[2] ? 0 : 2) : (ext[1] <= ext[2] ? 1 : 2);
   const int ax = thin == 0 ? 1 : 0, ay = thin == 2 ? 1 : 2;
-  const bool flat = ext[thin] <= 0.25f * fminf(ext[ax], ext[ay]) && (P & (P - 1)) != 0 && !morton;
+  const bool flat = ext[thin] <= 0.25f * fminf(ext[ax], ext[ay]) && !morton;
   auto cell = [&](int i, int a, float cells) {
     float u = ext[a] > 0.f ? (pts.at(b, i, a) - iord(box[a])) / ext[a] : 0.f;
     u = fminf(fmaxf(u, 0.f), 1.f);
     if (!(u == u)) u = 0.f;
     return (uint32_t)fminf(u * cells, cells - 1.f);
   };
-  for (int i = threadIdx.x; i < P; i += blockDim.x) {
-    k0[i] = flat ? hilbert2(cell(i, ax, 32768.f), cell(i, ay, 32768.f))
-                 : (spread10(cell(i, 0, 1024.f)) << 2) | (spread10(cell(i, 1, 1024.f)) << 1) |
-                       spread10(cell(i, 2, 1024.f));
-    v0[i] = (uint32_t)i;
+  bool hilbert = flat && (P & (P - 1)) != 0;
+  for (;;) {
+    for (int i = threadIdx.x; i < P; i += blockDim.x) {
+      k0[i] = hilbert ? hilbert2(cell(i, ax, 32768.f), cell(i, ay, 32768.f))
+                      : (spread10(cell(i, 0, 1024.f)) << 2) | (spread10(cell(i, 1, 1024.f)) << 1) |
+                            spread10(cell(i, 2, 1024.f));
+      v0[i] = (uint32_t)i;
+    }
+    if (threadIdx.x == 0) box[6] = 0;
+    __syncthreads();
+    cta_radix_sort30(k0, v0, k1, v1, P, smem);
+    __syncthreads();
+    if (!flat || hilbert || P < 64) break;
+    // the blocks' boxes, one block per warp at a time
+    float* covered = reinterpret_cast<float*>(box + 6);
+    for (int i = threadIdx.x; i < P; i += blockDim.x) {
+      const float x = pts.at(b, v1[i], ax), y = pts.at(b, v1[i], ay);
+      const float area =
+          (warp_max_f(x) - warp_min_f(x)) * (warp_max_f(y) - warp_min_f(y));
+      if ((threadIdx.x & 31) == 0) atomicAdd(covered, area);
+    }
+    __syncthreads();
+    if (*covered <= 0.75f * ext[ax] * ext[ay]) break;
+    hilbert = true;
+    __syncthreads();  // (the area has been read)
   }
-  __syncthreads();
-  cta_radix_sort30(k0, v0, k1, v1, P, smem);
-  __syncthreads();
   for (int i = threadIdx.x; i < P; i += blockDim.x) k0[i] = ~0u;
 }
 
@@ -637,7 +657,7 @@ __global__ void edge_link_kernel(Scene sc) {
 __global__ void __launch_bounds__(kSortThreads) point_order_kernel(WallPoints w0, WallPoints w1,
                                                                   int B) {
   extern __shared__ __align__(16) uint32_t smem[];
-  __shared__ int box[6];
+  __shared__ int box[7];
   const WallPoints& w = blockIdx.y ? w1 : w0;
   point_order_item(w.pts, w.P, B, blockIdx.x, w.scratch, smem, box, w.morton);
 }
@@ -646,7 +666,7 @@ __global__ void __launch_bounds__(kSortThreads) point_order_kernel(WallPoints w0
 __global__ void __launch_bounds__(kSortThreads) sort_kernel(Scene sc, WallPoints w0,
                                                            WallPoints w1) {
   extern __shared__ __align__(16) uint32_t smem[];
-  __shared__ int box[6];
+  __shared__ int box[7];
   const int b = blockIdx.x;
   if (blockIdx.y > 0) {
     const WallPoints& w = blockIdx.y == 1 ? w0 : w1;
@@ -672,7 +692,7 @@ static_assert(17 * kSmallFaces <= kSortWords, "edge table and counters fit the s
 __global__ void __launch_bounds__(kSortThreads) build_small_kernel(Scene sc, BuildInputs in,
                                                                   WallPoints w0, WallPoints w1) {
   extern __shared__ __align__(16) uint32_t smem[];
-  __shared__ int box[6];
+  __shared__ int box[7];
   const int b = blockIdx.x, tid = threadIdx.x;
   if (blockIdx.y > 0) {
     const WallPoints& w = blockIdx.y == 1 ? w0 : w1;
