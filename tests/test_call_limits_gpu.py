@@ -50,7 +50,7 @@ def sphere(faces, seed):
 
 def mesh_masks(v, f, *walls):
     vn, fn = v[0].cpu().numpy(), f[0].cpu().numpy()
-    return [oracle.mesh_visibility(vn, fn, p) for p in walls]
+    return [oracle.mesh_visibility(vn, fn, p, bvh=f.shape[1] > 4000) for p in walls]
 
 
 @pytest.mark.parametrize("faces_per_block", [1, 2, 5, 32])
@@ -595,3 +595,34 @@ def test_power_of_two_walls(cuda_lib, P, wall):
     for lists in (0, 1):
         with tuned({"mesh.visibility.list": lists}):
             assert torch.equal(R.mesh_visibility(v2, f2, both), want)
+
+
+@pytest.mark.parametrize("faces,S,T", [(7800, 1024, 2048), (7800, 2304, 4100)])
+def test_confocal_columns_of_many_bins(cuda_lib, faces, S, T):
+    """The built-in choice above 2,048 bins, against the oracle (sums of a few FP32
+    terms of one sign per bin, as in the other renders: 1e-5)."""
+    g = np.random.default_rng(T)
+    v, f, m = sphere(faces, 5)
+    sp, bw = points(g, S), 5.12 / T
+    none = torch.empty((1, 0, 3), device="cuda")
+    out = torch.full((1, T, S), 7.0, device="cuda")
+    R.mesh_confocal_forward(v, f, m, cu(sp[None]), none, out, bw, 0.0, 0)
+    vn, fn, mn = (x[0].cpu().numpy() for x in (v, f, m))
+    ref = oracle.mesh_confocal_forward(vn, fn, mn, sp, None, *mesh_masks(v, f, sp), T, bw, 0.0)
+    assert rel(out[0].cpu().numpy(), ref) < 1e-5
+
+
+@pytest.mark.parametrize("faces,S,L,T", [(4200, 60, 20, 2049), (12300, 62, 119, 2049),
+                                         (4200, 60, 20, 4096), (1600, 40, 30, 4500)])
+def test_exhaustive_columns_of_many_bins(cuda_lib, faces, S, L, T):
+    """As above for the exhaustive render: tiles of 8 and 32 columns, long rows."""
+    g = np.random.default_rng(T)
+    v, f, m = sphere(faces, 5)
+    sp, lp, bw = points(g, S), points(g, L), 5.12 / T
+    none = torch.empty((1, 0, 3), device="cuda")
+    out = torch.full((1, T, S, L), 7.0, device="cuda")
+    R.mesh_exhaustive_forward(v, f, m, cu(sp[None]), cu(lp[None]), none, none, out, bw, 0.0, 0)
+    vn, fn, mn = (x[0].cpu().numpy() for x in (v, f, m))
+    ref = oracle.mesh_exhaustive_forward(vn, fn, mn, sp, lp, None, None,
+                                         *mesh_masks(v, f, sp, lp), T, bw, 0.0)
+    assert rel(out[0].cpu().numpy(), ref) < 1e-5

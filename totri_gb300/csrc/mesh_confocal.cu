@@ -1227,19 +1227,27 @@ int launch_confocal_splat(const Scene& sc, const View3f& sp, const View3f& so, i
   }
   // Columns (splat_columns_kernel with 8 scan points per tile) for large meshes and
   // for middling ones over few points, from 1,024 points on (us, the tiles below
-  // against it; 1,024, 2,304 and 4,096 points):
-  //   20,480 faces, 1,024 bins  335/232  586/296  761/544; 2,048: 434/343 527/423 1025/788
-  //   12,288 faces (a box), 2,048 bins, 6,767 points  936/867
-  //   5,000 faces, 1,024 bins   140/123  228/142  268/249; 2,048: 195/193 234/220 419/391
-  //   1,500 faces, 1,024 bins    68/66   104/74   124/131; 2,048: 104/113 121/124 216/216
-  //   700 faces, 512 bins        39/41    58/44    63/74
+  // against it on spheres; 1,024, 2,304 and 4,096 points):
+  //   20,448 faces, 1,024 bins  431/292  749/353  871/650; 2,048: 549/424 616/505 1091/924
+  //                 3,000 bins  456/523  802/611 1240/1130; 8,000: 913/1124 1637/1325 2726/2441
+  //   12,320 faces, 2,048 bins  376/331  436/382  747/658; 3,000: 330/419 580/482 897/825
+  //    7,920 faces, 2,048 bins  273/239  320/277  553/508; 3,000: 242/307 446/354 693/649
+  //    5,040 faces, 1,024 bins  147/132  235/146  277/265; 2,048: 206/209 240/230 421/414
+  //                 3,000 bins  194/273  364/306  559/542; 8,000: 497/619 874/707 1434/1257
+  //    3,024 faces, 1,024 bins  104/98   164/110  194/193; 2,048: 151/160 179/174 311/311
+  //    1,520 faces, 1,024 bins   72/70   104/82   122/136; 2,048: 109/114 130/131 226/225
+  //      700 faces, 512 bins     39/41    58/44    63/74
+  // Boxes of 4,800 to 20,172 faces: 0.47 to 0.98 of the tiles' time up to 2,048 bins,
+  // 0.80 to 1.04 above from 2,304 points, 1.13 to 1.55 there at 1,024. The spheres span 0.6
+  // m of 5.12; meshes that span 3 m, 19,880 faces: 0.90-0.92 at 2,048 bins, 0.87-0.99 above
+  // from 2,304 points; 5,040 faces: 1.02-1.08 and 0.87-1.07, which stay with the tiles.
   // Below 1,024 points its tiles leave SMs idle (20,480 faces, 256 points: 123/262),
   // and small meshes spend the time on the rows. With 32 points per tile: 670, 669
   // and 574 us in the first row. "mesh.confocal.splat.columns" = 1 turns it off, 8
   // and 32 select a tile, ".window" its bins.
   const int cols = tune::get("mesh.confocal.splat.columns");
   const int64_t all = (int64_t)S * sc.B;
-  const bool large = sc.F >= 12288 ? T <= 2048 : sc.F >= 4096 && T <= 1024;
+  const bool large = T <= 1024 ? sc.F >= 4096 : sc.F >= 7680 && (T <= 2048 || all >= 2304);
   const bool few = sc.F >= 1024 && all <= 16 * tune::sm_count() && T <= 1024;
   const int ct = cols > 0 ? cols : all >= 1024 && (large || few) ? 8 : 0;
   // (its sides and windows run forwards in time)

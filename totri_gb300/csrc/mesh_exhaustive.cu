@@ -889,7 +889,8 @@ constexpr int kColStage = 32 * (16 + 4 * kColScan);  // floats per warp
 // kConfocal: a column is a scan point, its path twice one length (L = 1, lp unused).
 // 20,480 faces x 4,096 points, 1,024 bins: 0.76 ms with blocks of 8 points whose
 // lanes met in the same bins, 0.54 ms.
-template <int CT, int kColWarps, bool kConfocal>
+// kWindows: T > W.
+template <int CT, int kColWarps, bool kConfocal, bool kWindows>
 __global__ void __launch_bounds__(32 * kColWarps, 32 / kColWarps) splat_columns_kernel(
     Scene sc, View3f sp, View3f lp, Origins org, int S, int L, float* __restrict__ out, int T,
     float bw, float bo, FastBins fb, int W) {
@@ -931,44 +932,52 @@ __global__ void __launch_bounds__(32 * kColWarps, 32 / kColWarps) splat_columns_
     const uint32_t m = ok ? (kConfocal ? __ldg(ms + ch) : __ldg(ms + ch) & __ldg(ml + ch)) : 0u;
     return n - ch * 32 >= 32 ? m : m & ((1u << (n - ch * 32)) - 1u);
   };
+  // The bins that the column's paths over a chunk can reach, [lo, hi] within [0, T)
+  // (all lanes).
+  auto reach = [&](int ch, int& lo, int& hi) {
+    const int k = min(ch * 32 + lane, n - 1);
+    const float4 s0r = __ldg(shade + 4 * k), s1r = __ldg(shade + 4 * k + 1);
+    const float4 s2r = __ldg(shade + 4 * k + 2);
+    // the chunk's box (a face with a NaN coordinate adds nothing)
+    const float bx0 = warp_min_f(fminf(fminf(s0r.x, s1r.x), s2r.x));
+    const float by0 = warp_min_f(fminf(fminf(s0r.y, s1r.y), s2r.y));
+    const float bz0 = warp_min_f(fminf(fminf(s0r.z, s1r.z), s2r.z));
+    const float bx1 = warp_max_f(fmaxf(fmaxf(s0r.x, s1r.x), s2r.x));
+    const float by1 = warp_max_f(fmaxf(fmaxf(s0r.y, s1r.y), s2r.y));
+    const float bz1 = warp_max_f(fmaxf(fmaxf(s0r.z, s1r.z), s2r.z));
+    auto near = [&](fv3 o) {
+      const float x = fmaxf(fmaxf(bx0 - o.x, o.x - bx1), 0.f);
+      const float y = fmaxf(fmaxf(by0 - o.y, o.y - by1), 0.f);
+      const float z = fmaxf(fmaxf(bz0 - o.z, o.z - bz1), 0.f);
+      return sqrtf(fmaf(x, x, fmaf(y, y, z * z)));
+    };
+    auto far = [&](fv3 o) {
+      const float x = fmaxf(bx1 - o.x, o.x - bx0), y = fmaxf(by1 - o.y, o.y - by0);
+      const float z = fmaxf(bz1 - o.z, o.z - bz0);
+      return sqrtf(fmaf(x, x, fmaf(y, y, z * z)));
+    };
+    // Each length and sum of the exact chain and of this one is within a few
+    // roundings of its value: 4e-6 of the terms and two bins cover them.
+    const float dn = near(p) + near(q), df = far(p) + far(q);
+    const float inv_bw = fb.inv_bw;
+    const float m = fmaf(4e-6f * inv_bw, df + od + fabsf(bo), 2.f);
+    const float clo = (dn + od - bo) * inv_bw - m, chi = (df + od - bo) * inv_bw + m;
+    // (NaN or infinite bounds: the whole range)
+    lo = clo > 0.f ? (clo < (float)T ? (int)clo : T) : 0;
+    hi = chi < (float)T ? (chi >= 0.f ? (int)chi : -1) : T - 1;
+  };
   __syncthreads();
   int w0 = 0, passes = 1;
-  if (T > W) {
+  if (kWindows) {
     int lo = T, hi = -1;
     for (int ch = warp; ch < nchu; ch += kColWarps) {
       const uint32_t bits = seen(ch);
       if (!__any_sync(0xffffffffu, bits != 0u)) continue;
-      const int k = min(ch * 32 + lane, n - 1);
-      const float4 s0r = __ldg(shade + 4 * k), s1r = __ldg(shade + 4 * k + 1);
-      const float4 s2r = __ldg(shade + 4 * k + 2);
-      // the chunk's box (a face with a NaN coordinate adds nothing)
-      const float bx0 = warp_min_f(fminf(fminf(s0r.x, s1r.x), s2r.x));
-      const float by0 = warp_min_f(fminf(fminf(s0r.y, s1r.y), s2r.y));
-      const float bz0 = warp_min_f(fminf(fminf(s0r.z, s1r.z), s2r.z));
-      const float bx1 = warp_max_f(fmaxf(fmaxf(s0r.x, s1r.x), s2r.x));
-      const float by1 = warp_max_f(fmaxf(fmaxf(s0r.y, s1r.y), s2r.y));
-      const float bz1 = warp_max_f(fmaxf(fmaxf(s0r.z, s1r.z), s2r.z));
+      int clo, chi;
+      reach(ch, clo, chi);
       if (bits == 0u) continue;
-      auto near = [&](fv3 o) {
-        const float x = fmaxf(fmaxf(bx0 - o.x, o.x - bx1), 0.f);
-        const float y = fmaxf(fmaxf(by0 - o.y, o.y - by1), 0.f);
-        const float z = fmaxf(fmaxf(bz0 - o.z, o.z - bz1), 0.f);
-        return sqrtf(fmaf(x, x, fmaf(y, y, z * z)));
-      };
-      auto far = [&](fv3 o) {
-        const float x = fmaxf(bx1 - o.x, o.x - bx0), y = fmaxf(by1 - o.y, o.y - by0);
-        const float z = fmaxf(bz1 - o.z, o.z - bz0);
-        return sqrtf(fmaf(x, x, fmaf(y, y, z * z)));
-      };
-      // Each length and sum of the exact chain and of this one is within a few
-      // roundings of its value: 4e-6 of the terms and two bins cover them.
-      const float dn = near(p) + near(q), df = far(p) + far(q);
-      const float inv_bw = fb.inv_bw;
-      const float m = fmaf(4e-6f * inv_bw, df + od + fabsf(bo), 2.f);
-      const float clo = (dn + od - bo) * inv_bw - m, chi = (df + od - bo) * inv_bw + m;
-      // (NaN or infinite bounds: the whole range)
-      lo = min(lo, clo > 0.f ? (clo < (float)T ? (int)clo : T) : 0);
-      hi = max(hi, chi < (float)T ? (chi >= 0.f ? (int)chi : -1) : T - 1);
+      lo = min(lo, clo);
+      hi = max(hi, chi);
     }
     atomicMin(&range[0][cl], lo);
     atomicMax(&range[1][cl], hi);
@@ -984,9 +993,16 @@ __global__ void __launch_bounds__(32 * kColWarps, 32 / kColWarps) splat_columns_
     __syncthreads();
     const Window<CT> win{hist + cl, w0, min(w0 + W, T)};
     for (int ch = warp; ch < nchu; ch += kColWarps) {
-      const uint32_t bits = seen(ch);
+      uint32_t bits = seen(ch);
       uint32_t any = __reduce_or_sync(0xffffffffu, bits);
       if (any == 0u) continue;
+      if (kWindows && passes > 1) {  // but for columns whose window the chunk cannot reach
+        int clo, chi;
+        reach(ch, clo, chi);
+        if (chi < w0 || clo >= w0 + W) bits = 0u;
+        any = __reduce_or_sync(0xffffffffu, bits);
+        if (any == 0u) continue;
+      }
       __syncwarp();  // the last chunk's stage has been read
       if ((any >> lane) & 1u) {
         const int k = ch * 32 + lane;
@@ -1089,7 +1105,8 @@ static int launch_columns(const Scene& sc, const View3f& sp, const View3f& lp,
       bw, bo, tune::get(kConfocal ? "mesh.confocal.exact" : "mesh.exhaustive.exact") != 1);
   const size_t smem = sizeof(float) * ((size_t)kColWarps * kColStage + (size_t)W * CT);
   const dim3 grid((unsigned)ceil_div((int64_t)S * L, CT), (unsigned)sc.B);
-  auto* kern = splat_columns_kernel<CT, kColWarps, kConfocal>;
+  auto* kern = T > W ? splat_columns_kernel<CT, kColWarps, kConfocal, true>
+                     : splat_columns_kernel<CT, kColWarps, kConfocal, false>;
   TOTRI_CUDA(tune::ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
   TOTRI_KERNEL(kConfocal ? "mesh confocal splat" : "mesh exhaustive splat", stream,
                kern<<<grid, 32 * kColWarps, smem, stream>>>(sc, sp, lp, org, S, L, out, T, bw, bo,
@@ -1202,24 +1219,39 @@ int launch_exhaustive_splat(const Scene& sc, const View3f& sp, const View3f& lp,
       default: return fail(TOTRI_ERR_INVALID_ARGUMENT, "laser tile must be 1, 4, 8, 16 or 32");
     }
   }
-  // Columns (splat_columns_kernel) up to the 2,048 bins that were measured, from
-  // 1,024 columns on (ms, the tiles below against 8 and 32 columns; 400 x 144, 64 x
-  // 144, 169 x 36 and 64 x 16 points):
+  // Columns (splat_columns_kernel) from 1,024 columns on (ms, the tiles below against 8
+  // and 32 columns; 400 x 144, 64 x 144, 169 x 36 and 64 x 16 points):
   //   20,000 faces, 1,024 bins  8.30 / 6.85 / 5.86   1.68 / 1.21 / 1.07
   //                             1.39 / 0.94 / 1.18   0.68 / 0.30 / 0.83
   //   20,000 faces, 2,048 bins 10.27 / 9.31 / 7.80   1.88 / 1.66 / 1.44
   //                             1.61 / 1.26 / 1.87   0.52 / 0.41 / 1.32
+  //                3,072 bins  13.70 /11.43 / 9.69   2.48 / 2.07 / 1.78
+  //                             2.03 / 1.64 / 1.88   0.64 / 0.54 / 0.98
+  //                4,096 bins  18.98 /13.38 /14.42   3.34 / 2.43 / 2.63
+  //                             2.76 / 1.91 / 2.81   0.73 / 0.63 / 1.45
+  //                6,000 bins  31.98 /16.88 /18.02   5.49 / 3.08 / 3.25
   //   5,000 faces, 1,024 bins   2.61 / 2.60 / 2.26   0.54 / 0.47 / 0.44
   //                             0.45 / 0.37 / 0.43   0.23 / 0.13 / 0.34
+  //                3,072 bins   5.39 / 5.31 / 4.65   0.99 / 0.97 / 0.91
+  //                4,096 bins   7.87 / 6.48 / 6.72   1.40 / 1.19 / 1.31
   //   1,500 faces, 1,024 bins   1.08 / 1.43 / 1.16   0.24 / 0.27 / 0.25
   //                             0.19 / 0.21 / 0.25   0.12 / 0.09 / 0.22
+  //                4,096 bins   4.36 / 3.62 / 4.30   0.79 / 0.66 / 0.79
   //   500 faces, 1,024 bins     0.58 / 0.92 / 0.65   0.13 / 0.17 / 0.14
   //                             0.10 / 0.13 / 0.15   0.06 / 0.05 / 0.12
-  // Small meshes spend the time on the rows, not on the faces: they take 8 columns
-  // only where the tiles leave SMs idle (up to 16 columns per SM and 1,024 bins, or
-  // 48 with two faces per bin: 0.16 against 0.15 ms for 1,500 faces, 512 bins, 169 x
-  // 36 points). A window of 496 bins leaves room for two CTAs per SM; a mesh whose
-  // paths span more than half of 2,048 bins needs a second pass over its faces.
+  //                3,072 bins   1.97 / 2.23 / 2.81   0.37 / 0.41 / 0.55
+  //                4,096 bins   3.12 / 2.83 / 3.62   0.56 / 0.51 / 0.69
+  // These are spheres, whose paths span 0.6 m of 5.12; a mesh that spans more than a
+  // window needs more passes over its faces, each over the chunks that its window
+  // reaches (20,000 faces that span 3 m, 400 x 144 points: 10.21 / 10.15 / 9.46 at 2,048
+  // bins, 14.2 / 12.9 / 13.4 at 3,072, 20.5 / 16.5 / 17.0 at 4,096; 5,000 faces 4.18 / 4.94
+  // / 4.95, 6.2 / 6.7 / 7.7 and 9.4 / 8.8 / 10.4). Hence above 2,048 bins only meshes of
+  // 12,288 faces, and from 4,096 bins on, where the tiles are one or two lasers wide,
+  // 8 columns from 1,500 faces. Small meshes spend the time on the rows, not on the
+  // faces: they take 8 columns only where the tiles leave SMs idle (up to 16 columns
+  // per SM and 1,024 bins, or 48 with two faces per bin: 0.16 against 0.15 ms for 1,500
+  // faces, 512 bins, 169 x 36 points). A window of 496 bins leaves room for two CTAs per
+  // SM.
   // "mesh.exhaustive.splat.columns" = 1 turns the kernel off, 8 and 32 select a
   // tile, ".window" its bins.
   const int cols = tune::get("mesh.exhaustive.splat.columns");
@@ -1228,13 +1260,14 @@ int launch_exhaustive_splat(const Scene& sc, const View3f& sp, const View3f& lp,
       (size_t)T * 4 <= budget) {
     const int64_t all = (int64_t)S * L * sc.B;
     const int sms = tune::sm_count();
-    const bool many = sc.F >= 4096;
+    const bool many = sc.F >= (T <= 2048 ? 4096 : 12288);
     const bool few = all <= 16 * sms && T <= 1024;
     const bool middling = all <= 48 * sms && sc.F >= 2 * T;
+    const bool rows = T >= 4096 && sc.F >= 1500;
     const int ct = cols > 1 ? cols
-                   : all < 1024 || T > 2048 || !(many || few || middling) ? 0
-                   : many && all >= 48 * sms                              ? 32
-                                                                          : 8;
+                   : all < 1024 || !(many || few || middling || rows) ? 0
+                   : many && !rows && all >= 48 * sms                 ? 32
+                                                                      : 8;
     const int W = tune::get("mesh.exhaustive.splat.window");
     if (ct != 0) return launch_tile<false>(ct, sc, sp, lp, org, S, L, out, T, bw, bo, W, stream);
   }
