@@ -626,3 +626,22 @@ def test_exhaustive_columns_of_many_bins(cuda_lib, faces, S, L, T):
     ref = oracle.mesh_exhaustive_forward(vn, fn, mn, sp, lp, None, None,
                                          *mesh_masks(v, f, sp, lp), T, bw, 0.0)
     assert rel(out[0].cpu().numpy(), ref) < 1e-5
+
+
+@pytest.mark.parametrize("shape,S,L,T", [((8, 8, 8), 160, 64, 256), ((3, 2, 2), 160, 33, 300),
+                                         ((8, 8, 8), 304, 5, 300), ((9, 7, 20), 61, 41, 900),
+                                         ((20, 20, 9), 3, 7, 2000)])
+@pytest.mark.parametrize("share", [0.002, 0.02, 0.2, 1.0])
+def test_exhaustive_volume_tiles(cuda_lib, shape, S, L, T, share):
+    """The built-in laser tiles (32, 8 and 1) with remainders and voxels shared by 1 to 32
+    threads: forward 1e-5 of the FP64 oracle."""
+    g = np.random.default_rng(S + L)
+    sp, lp = points(g, S), points(g, L)
+    vol = g.uniform(0.5, 1.5, shape) * (g.uniform(size=shape) < share)
+    vol.flat[0] = 1.0
+    vol, none = vol.astype(np.float32), torch.empty((1, 3, 0), device="cuda")
+    out = torch.full((1, T, S, L), 7.0, device="cuda")
+    R.volume_render_exhaustive_forward(cu(vol[None]), cu(sp.T[None]), cu(lp.T[None]), none, none,
+                                       out, START, END, 5.12 / T, 0.0)
+    ref = oracle.volume_exhaustive_forward(vol, sp.T, lp.T, T, START, END, 5.12 / T, 0.0)
+    assert rel(out[0].cpu().numpy(), ref) < 1e-5

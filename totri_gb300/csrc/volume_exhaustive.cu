@@ -129,9 +129,10 @@ __global__ void __launch_bounds__(256) forward_kernel(Geo g, int b, const float*
   for (int j = threadIdx.x; j < g.T * LT; j += blockDim.x) hist[j] = 0.f;
   __syncthreads();
   const uint32_t nnz = *count;
-  // a thread takes one occupied voxel at a time to every laser of the tile, in
-  // an order that starts at its lane: the lanes of a warp add to different
-  // histogram columns
+  // A thread takes one occupied voxel at a time to the lasers of the tile, in an order
+  // that starts at its lane: the lanes of a warp add to different histogram columns.
+  // Where the voxels are fewer than the threads, 2, 4 .. LT threads share a voxel's
+  // lasers.
   __shared__ float laser[LT][3];
   if (threadIdx.x < LT && l0 + (int)threadIdx.x < g.L) {
     const fv3 q = lp.at(b, l0 + threadIdx.x);
@@ -141,7 +142,10 @@ __global__ void __launch_bounds__(256) forward_kernel(Geo g, int b, const float*
   }
   __syncthreads();
   const fv3 sc = sp.at(b, s);
-  for (uint32_t v = threadIdx.x; v < nnz; v += blockDim.x) {
+  const int nl = min(LT, g.L - l0);
+  uint32_t share = 1;
+  while (share < LT && 2 * share * nnz <= blockDim.x) share *= 2;
+  for (uint32_t v = threadIdx.x / share; v < nnz; v += blockDim.x / share) {
     const uint32_t lin = __ldg(list + v);
     const int xi = (int)(lin % g.W), yi = (int)((lin / g.W) % g.H);
     const int zi = (int)(lin / ((uint32_t)g.W * g.H));
@@ -149,9 +153,9 @@ __global__ void __launch_bounds__(256) forward_kernel(Geo g, int b, const float*
     const float occ = __ldg(vol + lin);
     const float s0 = xlen(xsub3(sc, e.p0)), s1 = xlen(xsub3(sc, e.p1));
 #pragma unroll 1
-    for (int i = 0; i < LT; ++i) {
+    for (int i = 0; i < LT; i += share) {
       const int ll = (threadIdx.x + i) & (LT - 1);
-      if (l0 + ll >= g.L) continue;
+      if (ll >= nl) continue;
       const fv3 lc = mkv(laser[ll][0], laser[ll][1], laser[ll][2]);
       const Interval iv = interval<true>(g, xadd(s0, xlen(xsub3(lc, e.p0))),
                                    xadd(s1, xlen(xsub3(lc, e.p1))));
@@ -433,6 +437,7 @@ int totri_volume_exhaustive_forward(const totri_array_t* vol, const totri_array_
                      vb, nv, list, count));
     float* out = static_cast<float*>(transient->data);
     const size_t budget = 200 * 1024;
+    const int64_t fill = 2 * (int64_t)tune::sm_count();  // CTAs, two per SM
     const int want = tune::get("volume.exhaustive.lt");
     if (want == 1 || want == 8 || want == 32) {
       if ((size_t)g.T * want * 4 > budget)
@@ -442,11 +447,18 @@ int totri_volume_exhaustive_forward(const totri_array_t* vol, const totri_array_
       else TOTRI_TRY(launch_fwd<1>(g, b, vb, list, count, sp, lp, out, stream));
     } else if (want != 0) {
       return fail(TOTRI_ERR_INVALID_ARGUMENT, "laser tile must be 1, 8 or 32");
-    } else if ((size_t)g.T * 8 * 4 <= budget && L >= 4)
+    } else if ((size_t)g.T * 32 * 4 <= 40 * 1024 && L >= 32 && S * ceil_div(L, 32) >= fill)
+      // 32 lasers (a column per lane) where several CTAs fit an SM and there are CTAs
+      // for two per SM: 4 x 64 x 64 voxels x 100 x 100 points, 300 bins, 0.35 ms (5% of the
+      // voxels) and 4.7 ms (all), with 8 lasers 0.44 and 7.2; 32^3 x 64 x 64, 256 bins: 0.31
+      // and 0.15 ms.
+      TOTRI_TRY(launch_fwd<32>(g, b, vb, list, count, sp, lp, out, stream));
+    else if ((size_t)g.T * 8 * 4 <= budget && L >= 6 && S * ceil_div(L, 8) >= fill)
       // 8 lasers: several CTAs per SM up to 1,600 bins or so, and whole 32-byte
       // sectors of the output (36 lasers, 1,024 bins, 256 scan points x 2,150
-      // voxels: 0.25 ms; 32 lasers, one CTA per SM and a second tile of 4 lasers:
-      // 1.06 ms)
+      // voxels: 0.27 ms; 1 laser 0.35 ms; 32 lasers, one CTA per SM and a second tile
+      // of 4 lasers: 1.06 ms). Fewer CTAs or lasers: 1 laser (64^3 x 16 x 16 0.15 against
+      // 0.49 ms, 96^3 x 9 x 9 0.35 against 1.04; 32^3 x 1,024 x 4, 5: 0.15, 0.18 against 0.20).
       TOTRI_TRY(launch_fwd<8>(g, b, vb, list, count, sp, lp, out, stream));
     else if ((size_t)g.T * 4 <= budget)
       TOTRI_TRY(launch_fwd<1>(g, b, vb, list, count, sp, lp, out, stream));
