@@ -178,7 +178,8 @@ __global__ void __launch_bounds__(256) forward_kernel(Grid g, int b, Rbf r, int 
   using u64 = unsigned long long;
   constexpr int kFac = kBX + kBY + VZ;  // factors of one Gaussian: x | y | z
   constexpr int kHalf = 128;            // Gaussians whose factors are held at once
-  __shared__ float tile[kTile][5 + kA];  // x y z, exponent (hi, lo), attributes
+  __shared__ float tile[kTile][5];  // x y z, exponent (hi, lo)
+  __shared__ __align__(16) u64 rows[kTile][kA];  // attributes, each twice
   __shared__ __align__(16) float fac[kHalf][kFac];
   __shared__ float axis[kFac];  // the brick's voxel coordinates
   __shared__ int counts[8];
@@ -225,9 +226,12 @@ __global__ void __launch_bounds__(256) forward_kernel(Grid g, int b, Rbf r, int 
       const int sat = block_slot(keep && !finite, counts, &special);
       if (keep && !finite) at = cnt + sat;
     }
-    if (keep)
+    if (keep) {
 #pragma unroll
-      for (int c = 0; c < 5 + kA; ++c) tile[at][c] = val[c];
+      for (int c = 0; c < 5; ++c) tile[at][c] = val[c];
+#pragma unroll
+      for (int a = 0; a < kA; ++a) rows[at][a] = f2pack(val[5 + a], val[5 + a]);
+    }
     __syncthreads();
     for (int h0 = 0; h0 < cnt; h0 += kHalf) {
       const int hn = min(kHalf, cnt - h0);
@@ -245,8 +249,16 @@ __global__ void __launch_bounds__(256) forward_kernel(Grid g, int b, Rbf r, int 
         const u64 e2 = f2pack(exy, exy);
         const float4* ez = reinterpret_cast<const float4*>(&fac[i][kBX + kBY]);
         u64 ra[kA];
+        if constexpr (kA == 1) {
+          ra[0] = rows[h0 + i][0];
+        } else {
 #pragma unroll
-        for (int a = 0; a < kA; ++a) ra[a] = f2pack(tile[h0 + i][5 + a], tile[h0 + i][5 + a]);
+          for (int a = 0; a < kA; a += 2) {
+            const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(&rows[h0 + i][a]);
+            ra[a] = q.x;
+            ra[a + 1] = q.y;
+          }
+        }
 #pragma unroll
         for (int q = 0; q < VZ / 4; ++q) {
           const float4 z = ez[q];
@@ -256,7 +268,7 @@ __global__ void __launch_bounds__(256) forward_kernel(Grid g, int b, Rbf r, int 
             sum[2 * q + h] = f2add(sum[2 * q + h], w);
 #pragma unroll
             for (int a = 0; a < kA; ++a)
-              if (kA == 1 || a < A) attr[2 * q + h][a] = f2fma(w, ra[a], attr[2 * q + h][a]);
+              attr[2 * q + h][a] = f2fma(w, ra[a], attr[2 * q + h][a]);
           }
         }
       }
@@ -276,8 +288,7 @@ __global__ void __launch_bounds__(256) forward_kernel(Grid g, int b, Rbf r, int 
 #pragma unroll
         for (int a = 0; a < kA; ++a)
           if (a < A)
-            attr[v / 2][a] =
-                f2fma(w2, f2pack(tile[i][5 + a], tile[i][5 + a]), attr[v / 2][a]);
+            attr[v / 2][a] = f2fma(w2, rows[i][a], attr[v / 2][a]);
       }
     }
   }
