@@ -894,12 +894,13 @@ int totri_backprojection_confocal_velten_adjoint(const totri_array_t* volume,
   if (smem > 200 * 1024) return fail(TOTRI_ERR_UNSUPPORTED, "too many bins for one tile");
   TOTRI_CUDA(tune::ensure_dynamic_smem(
       reinterpret_cast<const void*>(bp::velten_adjoint_kernel), smem));
-  // 1,024 threads once the histogram leaves room for one CTA per SM only, else
-  // 512. A second grid dimension slices the voxels until about 8 waves of CTAs
+  // 1,024 threads once the histogram leaves room for one CTA per SM only, else 512,
+  // and not many more than there are columns (8^3 voxels x 16,384 points, 1,024 bins: 96
+  // us with 512, 67 with 128; nearly all voxels zero 86 and 63). A second grid dimension slices the voxels until about 8 waves of CTAs
   // are in flight, each slice with at least 16 columns per thread (zeroing and
   // flushing the histogram costs about what 1 or 2 take).
-  const int threads = smem > 100 * 1024 ? 1024 : 512;
   const int64_t units = (int64_t)ceil_div(g.D, bp::kAZ) * g.H * g.W;
+  const int threads = smem > 100 * 1024 ? 1024 : (units <= 128 ? 128 : (units <= 256 ? 256 : 512));
   const int64_t tiles = ceil_div(S, bp::kTS);
   const int64_t resident = (int64_t)tune::sm_count() *
                            std::max<int64_t>(1, std::min<int64_t>(2048 / threads,
