@@ -343,6 +343,22 @@ __device__ __forceinline__ void fill_bin_table(const Geo& g, float4* tab) {
   }
 }
 
+// f(p, t) for the n rows of T bins, t fastest, over the threads of the CTA (without a
+// division per element: the forward of 8^3 voxels, 16,384 rows of 4,096 bins, took 0.69 ms
+// with one and takes 0.56).
+template <class F>
+__device__ __forceinline__ void for_rows(int n, int T, F f) {
+  if (T <= 0) return;
+  int p = threadIdx.x / T, t = threadIdx.x - p * T;
+  const int dp = blockDim.x / T, dt = blockDim.x - dp * T;
+  while (p < n) {
+    f(p, t);
+    p += dp;
+    t += dt;
+    if (t >= T) t -= T, ++p;
+  }
+}
+
 // Confocal forward: a CTA takes PT points and a slice of the occupied voxels,
 // and keeps the points' bins in shared memory ([bin][point]: with 32 points the
 // lanes of a warp add to 32 banks). A thread walks one point over every
@@ -380,14 +396,12 @@ __global__ void __launch_bounds__(32 * PT > 256 ? 32 * PT : 256) confocal_forwar
     }
   }
   __syncthreads();
-  for (int j = threadIdx.x; j < PT * g.T; j += blockDim.x) {
-    const int p = j / g.T, t = j - p * g.T;
-    if (i0 + p >= N) break;
+  for_rows(min(PT, N - i0), g.T, [&](int p, int t) {
     float* dst = out + (size_t)(i0 + p) * g.T + t;
     const float h = hist[t * PT + p];
     if (gridDim.y == 1) *dst = h;
     else if (h != 0.f) atomicAdd(dst, h);
-  }
+  });
 }
 
 // d transient / d measurement points (volume_cuda.cu:189-265) with the same
@@ -404,10 +418,9 @@ __global__ void __launch_bounds__(32 * PT > 256 ? 32 * PT : 256) grad_mp_kernel(
   float4* tab = reinterpret_cast<float4*>(rows + (((size_t)PT * g.T + 3) & ~(size_t)3));
   __shared__ float sum[PT][3];
   const int i0 = blockIdx.x * PT;
-  for (int j = threadIdx.x; j < PT * g.T; j += blockDim.x) {
-    const int p = j / g.T, t = j - p * g.T;
+  for_rows(PT, g.T, [&](int p, int t) {
     rows[t * PT + p] = i0 + p < N ? __ldg(tg + (size_t)(i0 + p) * g.T + t) : 0.f;
-  }
+  });
   fill_bin_table(g, tab);
   if (threadIdx.x < PT) sum[threadIdx.x][0] = sum[threadIdx.x][1] = sum[threadIdx.x][2] = 0.f;
   __syncthreads();
