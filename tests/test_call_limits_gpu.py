@@ -645,3 +645,20 @@ def test_exhaustive_volume_tiles(cuda_lib, shape, S, L, T, share):
                                        out, START, END, 5.12 / T, 0.0)
     ref = oracle.volume_exhaustive_forward(vol, sp.T, lp.T, T, START, END, 5.12 / T, 0.0)
     assert rel(out[0].cpu().numpy(), ref) < 1e-5
+
+
+@pytest.mark.parametrize("N,T", [(1, 300), (5, 2048), (700, 1024), (700, 1025), (1300, 2049),
+                                 (90, 4097), (19, 9600), (3, 28200)])
+def test_point_gradient_tiles(cuda_lib, N, T):
+    """Tiles of 16, 8 and 4 points by the points and bins, and bin tables past shared
+    memory: 1e-4 of the FP64 oracle."""
+    g = np.random.default_rng(N + T)
+    shape, bw = (5, 6, 11), 3.0 / T
+    mp = np.stack([g.uniform(-1, 1, N), g.uniform(-1, 1, N), np.zeros(N)]).astype(np.float32)
+    vol = g.uniform(0.5, 1.5, shape).astype(np.float32)
+    y = g.uniform(0.5, 1.5, (N, T)).astype(np.float32)
+    org, size = (-0.5, -0.5, 0.5), (1.0, 1.0, 1.0)
+    gm = torch.full((3, N), 7.0, device="cuda")
+    R.volume_confocal_grad_measurement_points(gm, cu(vol), cu(mp), cu(y), org, size, bw, 0.0)
+    ref = oracle.volume_confocal_grad_mp(vol, mp, y, org, size, bw, 0.0)
+    assert rel(gm.cpu().numpy(), ref) < 1e-4

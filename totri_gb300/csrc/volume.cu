@@ -405,22 +405,20 @@ __global__ void __launch_bounds__(32 * PT > 256 ? 32 * PT : 256) confocal_forwar
 }
 
 // d transient / d measurement points (volume_cuda.cu:189-265) with the same
-// walks: a CTA holds its PT points' rows of transient_grad in shared memory,
-// a thread accumulates one point over its share of the voxels, and the shares
+// walks: a thread accumulates one point over its share of the voxels, and the shares
 // are reduced in shared memory (then added into a zeroed output when there are
-// several slices of the voxels). 41 x 37 x 53 voxels (10%) x 899 points x 500
-// bins: 0.55 -> 0.10 ms.
+// several slices of the voxels). 41 x 37 x 53 voxels (10%) x 899 points x 500 bins: 0.55
+// -> 0.10 ms. transient_grad is read in place, a voxel's few bins of a row: with the
+// rows in shared memory 1,024 bins took as long (0.92 to 1.02 of the time, by voxels and
+// points), 2,048 bins 1.3 to 3 times and 4,096 bins 2 to 7 times as long (16,384 rows for
+// the 10 voxels of an 8^3 volume 1.2 against 0.18 ms).
 template <int PT, bool kSigned>
 __global__ void __launch_bounds__(32 * PT > 256 ? 32 * PT : 256) grad_mp_kernel(
     Geo g, const float4* __restrict__ recs, const uint32_t* __restrict__ count, Points mp, int N,
     const float* __restrict__ tg, float* __restrict__ out, int64_t osc, int64_t osn) {
-  extern __shared__ __align__(16) float rows[];  // [T][PT], then the bin table
-  float4* tab = reinterpret_cast<float4*>(rows + (((size_t)PT * g.T + 3) & ~(size_t)3));
+  extern __shared__ float4 tab[];  // the bin table
   __shared__ float sum[PT][3];
   const int i0 = blockIdx.x * PT;
-  for_rows(PT, g.T, [&](int p, int t) {
-    rows[t * PT + p] = i0 + p < N ? __ldg(tg + (size_t)(i0 + p) * g.T + t) : 0.f;
-  });
   fill_bin_table(g, tab);
   if (threadIdx.x < PT) sum[threadIdx.x][0] = sum[threadIdx.x][1] = sum[threadIdx.x][2] = 0.f;
   __syncthreads();
@@ -433,7 +431,7 @@ __global__ void __launch_bounds__(32 * PT > 256 ? 32 * PT : 256) grad_mp_kernel(
   const int tz = kSigned ? first_nonneg_bin(g) : 0;
   if (i < N) {
     const WalkPoint p = walk_point(g, mp.at(0, i), mp.at(1, i), mp.at(2, i));
-    const float* col = rows + pl;
+    const float* row = tg + (size_t)i * g.T;
     for (uint32_t v = v0 + threadIdx.x / PT; v < v1; v += blockDim.x / PT) {
       const float4 rec = __ldg(recs + v);
       // with f2 = (depth / tc^2)^4 and w the interpolation weight, d(w f2) / d depth
@@ -443,7 +441,7 @@ __global__ void __launch_bounds__(32 * PT > 256 ? 32 * PT : 256) grad_mp_kernel(
       walk_voxel<kSigned>(g, tab, p, tz, rec.x, rec.y, __float_as_int(rec.w),
                           [&](int t, bool lower, float fr, float a, float b, float depth) {
                             const float w = lower ? 1.f - fr : fr, f1 = a * b;
-                            const float df2 = col[t * PT] * (f1 * f1);
+                            const float df2 = __ldg(row + t) * (f1 * f1);
                             const float slope = lower ? -g.scale * df2 : g.scale * df2;
                             const float inv = __fdividef(1.f, depth);
                             radial += fmaf(4.f * w * df2, inv, slope) * (inv * g.dz);
@@ -476,8 +474,8 @@ __global__ void __launch_bounds__(32 * PT > 256 ? 32 * PT : 256) grad_mp_kernel(
   }
 }
 
-// grad_mp_kernel for transients whose rows do not fit shared memory: every
-// sample by the exact chain, transient_grad read in place; one thread
+// grad_mp_kernel for bin tables that do not fit shared memory: every sample by the
+// exact chain; one thread
 // accumulates one point's gradient over a share of the voxels, reduced across
 // the kPT-strided threads in shared memory.
 __global__ void __launch_bounds__(256) grad_mp_wide_kernel(Geo g, const float4* __restrict__ recs,
@@ -1156,17 +1154,17 @@ int compact(const Geo& g, const float* vol, int64_t n, void* ws, size_t ws_bytes
 }
 
 // Points per CTA, threads, shared memory and slices of the occupied voxels for
-// the walks of confocal_forward_kernel and grad_mp_kernel. points 0: the rows of
-// 4 points do not fit.
+// the walks of confocal_forward_kernel (rows: the points' bins are in shared memory) and
+// grad_mp_kernel. points 0: the rows of 4 points, or the bin table, do not fit.
 struct WalkTile {
   int points, threads, slices;
   size_t smem;
 };
 
-WalkTile walk_tile(int64_t N, int T, int64_t voxels) {
+WalkTile walk_tile(int64_t N, int T, int64_t voxels, bool rows) {
   const size_t budget = 220 * 1024;
   const auto bytes = [&](int pt) {
-    return sizeof(float) * (((size_t)pt * T + 3) & ~(size_t)3) +
+    return (rows ? sizeof(float) * (((size_t)pt * T + 3) & ~(size_t)3) : 0) +
            sizeof(float4) * volume::bin_table(T);
   };
   WalkTile w{0, 0, 1, 0};
@@ -1184,6 +1182,14 @@ WalkTile walk_tile(int64_t N, int T, int64_t voxels) {
     break;
   }
   if (w.points == 0) return w;
+  // Without rows: smaller tiles until 8 slices make a CTA per SM, and until the points'
+  // rows fit half of the L1 cache (24^3 voxels, half of them, x 1,024 points: 2,048 bins
+  // 0.51 ms with 8 points, 1.11 with 16; 4,096 bins 0.95 with 4, 1.21 with 8, 2.05 with
+  // 16). From 6,400 bins on not even 4 rows do, and 16 points are the fastest.
+  while (!rows && want == 0 && w.points > 4 &&
+         (8 * ceil_div(N, w.points) < (int64_t)tune::sm_count() ||
+          (T <= 4096 && sizeof(float) * w.points * T > 64 * 1024)))
+    w.points /= 2;
   w.threads = std::max(256, 32 * w.points);
   w.smem = bytes(w.points);
   const int64_t resident = std::max<int64_t>(
@@ -1243,7 +1249,7 @@ int totri_volume_confocal_forward(const totri_array_t* vol, const totri_array_t*
   TOTRI_TRY(compact(g, static_cast<const float*>(vol->data), numel(vol), ws, ws_bytes, &recs,
                     &count, stream));
   float* out = static_cast<float*>(tr->data);
-  const WalkTile w = walk_tile(N, T, numel(vol));
+  const WalkTile w = walk_tile(N, T, numel(vol), true);
   if (w.slices > 1)
     TOTRI_CUDA(cudaMemsetAsync(out, 0, sizeof(float) * (size_t)N * T, stream));
   return for_walk_tile(w.points, g, [&](auto pt, auto sign) {
@@ -1423,8 +1429,8 @@ int totri_volume_confocal_grad_measurement_points(const totri_array_t* mpg,
                     &count, stream));
   float* out = static_cast<float*>(mpg->data);
   const int64_t osc = mpg->strides[0], osn = mpg->strides[1];
-  WalkTile w = walk_tile(N, T, numel(vol));
-  if (w.points == 0) {  // rows too long for shared memory
+  WalkTile w = walk_tile(N, T, numel(vol), false);
+  if (w.points == 0) {  // the bin table is too long for shared memory
     TOTRI_KERNEL("volume confocal grad points", stream,
                  volume::grad_mp_wide_kernel<<<(unsigned)ceil_div(N, volume::kPT), 256, 0, stream>>>(
                      g, recs, count, pts, N, static_cast<const float*>(tg->data), out, osc, osn));
