@@ -17,6 +17,7 @@
 //    the per-face gradient in registers, reduces it across the warp and issues
 //    12 atomics per face instead of 9 + 3M per visible pair.
 #include <algorithm>
+#include <cmath>
 
 #include "mesh.cuh"
 #include "mesh_kernels.cuh"
@@ -1241,13 +1242,22 @@ int launch_confocal_splat(const Scene& sc, const View3f& sp, const View3f& so, i
   // 0.80 to 1.04 above from 2,304 points, 1.13 to 1.55 there at 1,024. The spheres span 0.6
   // m of 5.12; meshes that span 3 m, 19,880 faces: 0.90-0.92 at 2,048 bins, 0.87-0.99 above
   // from 2,304 points; 5,040 faces: 1.02-1.08 and 0.87-1.07, which stay with the tiles.
+  // Above 1,024 bins two CTAs share an SM, and a second wave that is nearly empty costs
+  // as much as a full one (20,448 faces, 2,048 and 3,000 bins: 0.81 and 0.81 of the tiles'
+  // time at 2,401 points, 0.99 waves; 1.08 and 1.31 at 2,500, 1.03 waves; 1.29 and 1.22 at
+  // 2,704; 0.85 and 0.93 at 3,136; 0.86 and 0.92 at 4,096, 1.68 waves; at 1,024, 0.42 waves,
+  // 0.79 and 1.16).
   // Below 1,024 points its tiles leave SMs idle (20,480 faces, 256 points: 123/262),
   // and small meshes spend the time on the rows. With 32 points per tile: 670, 669
   // and 574 us in the first row. "mesh.confocal.splat.columns" = 1 turns it off, 8
   // and 32 select a tile, ".window" its bins.
   const int cols = tune::get("mesh.confocal.splat.columns");
   const int64_t all = (int64_t)S * sc.B;
-  const bool large = T <= 1024 ? sc.F >= 4096 : sc.F >= 7680 && (T <= 2048 || all >= 2304);
+  const double waves = (double)ceil_div(all, 8) / (2 * tune::sm_count());
+  const double filled = waves / std::ceil(waves);  // of all waves together
+  const bool large = T <= 1024 ? sc.F >= 4096
+                               : sc.F >= 7680 && (T <= 2048 ? waves <= 1.0 || filled >= 0.6
+                                                            : filled >= 0.8);
   const bool few = sc.F >= 1024 && all <= 16 * tune::sm_count() && T <= 1024;
   const int ct = cols > 0 ? cols : all >= 1024 && (large || few) ? 8 : 0;
   // (its sides and windows run forwards in time)
