@@ -378,13 +378,15 @@ __device__ __forceinline__ void point_order_item(const View3f& pts, int P, int B
     cta_radix_sort30(k0, v0, k1, v1, P, smem);
     __syncthreads();
     if (!flat || hilbert || P < 64) break;
-    // the blocks' boxes, one block per warp at a time
+    // the boxes of the blocks, or of 32 of them (one per warp), evenly spread
     float* covered = reinterpret_cast<float*>(box + 6);
-    for (int i = threadIdx.x; i < P; i += blockDim.x) {
-      const float x = pts.at(b, v1[i], ax), y = pts.at(b, v1[i], ay);
+    const int blocks = P / 32, every = max(blocks / 32, 1), at = (threadIdx.x >> 5) * every;
+    if (at < blocks) {
+      const int i = v1[at * 32 + (threadIdx.x & 31)];
+      const float x = pts.at(b, i, ax), y = pts.at(b, i, ay);
       const float area =
           (warp_max_f(x) - warp_min_f(x)) * (warp_max_f(y) - warp_min_f(y));
-      if ((threadIdx.x & 31) == 0) atomicAdd(covered, area);
+      if ((threadIdx.x & 31) == 0) atomicAdd(covered, every * area);
     }
     __syncthreads();
     if (*covered <= 0.75f * ext[ax] * ext[ay]) break;
