@@ -72,43 +72,12 @@ __device__ __forceinline__ Sample sample(const Geo& g, float wx, float wy, float
   return s;
 }
 
-// sample() with a filtered fast path: the depth from the hardware reciprocal
-// square root (within 6 u of the exact root, u = 2^-24) and z_hat from one
-// fused multiply-add. Against the exact chain z_hat moves by at most
-// scale 8 u (depth + |z| + |oz|) + 4 u |z_hat|, so where its fraction is
-// farther than that (with |wz| added) from 0 and 1 the fast floor is the
-// exact floor and the sample is kept; otherwise the exact sample() runs. The
-// d2 > 0 test is taken on the exact d2 either way. alpha and f2 are values
-// (few-ulp differences); every decision is the exact chain's. Used by the
-// adjoint (247 -> 195 ms on 128^3 x 16384 points x 1024 bins); the forward,
-// which only walks bins next to each occupied voxel's cell, ran 5% slower
-// with it and keeps sample().
-__device__ __forceinline__ Sample sample_filtered(const Geo& g, float wx, float wy, float wz,
-                                                  int t, float x, float y) {
-  if (g.exact) return sample(g, wx, wy, wz, t, x, y);
-  Sample s{false, 0, 0.f, 0.f, 0.f};
-  const float tc = xadd(xmul((float)t, g.bw), g.bo);
-  const float dx = xsub(wx, x), dy = xsub(wy, y);
-  const float d2 = xsub(xsub(xmul(tc, tc), xmul(dx, dx)), xmul(dy, dy));
-  if (!(d2 > 0.f)) return s;
-  const float depth = d2 * rsqrtf(d2);
-  const float z = wz + depth;
-  const float zh = fmaf(z - g.oz, g.scale, -0.5f);
-  const float fl = floorf(zh);
-  const float fr = zh - fl;
-  const float u = 5.9604645e-8f;
-  const float m = 8.f * u * g.scale * (depth + fabsf(wz) + fabsf(z) + fabsf(g.oz)) +
-                  4.f * u * fabsf(zh) + 1e-7f;
-  if (!(fr > m && fr < 1.f - m)) return sample(g, wx, wy, wz, t, x, y);
-  if (!(fl >= 0.f && fl + 1.f < (float)g.Z)) return s;
-  s.ok = true;
-  s.zi = (int)fl;
-  s.alpha = fr;
-  const float q = __fdividef(depth, tc * tc);
-  s.f1 = q * q;
-  s.f2 = s.f1 * s.f1;
-  return s;
-}
+// The kernels take a sample's cell from a fast path where it is sure to be the exact
+// chain's: with u = 2^-24, the depth from the hardware reciprocal square root (within 6 u
+// of the exact root) moves z_hat by at most 8 u scale (depth + |wz| + |z| + |oz|) + 4 u |z_hat|,
+// so where its fraction is farther than that margin from 0 and 1 (taken at the largest
+// magnitudes of a walk), the fast floor is the exact floor; elsewhere sample() decides.
+// alpha and f2 are values (few-ulp differences). "volume.exact" = 1: sample() always.
 
 // First bin whose centre t bw + bo (the sample chain's FP32 arithmetic) is not
 // negative; 0 unless the bin offset is negative. Bins before it have negative
@@ -236,7 +205,7 @@ __host__ __device__ constexpr int bin_table(int T) { return 2 * ((T + 3) / 4); }
 struct WalkPoint {
   float wx, wy, wz;
   float ea, eb;  // span_eps as ea ch + eb, at most 1
-  float ma, mb;  // sample_filtered's margin of a cell fraction as ma ch + mb
+  float ma, mb;  // the margin of a cell fraction as ma ch + mb
 };
 __device__ __forceinline__ WalkPoint walk_point(const Geo& g, float wx, float wy, float wz) {
   const float u = 5.9604645e-8f;
@@ -571,9 +540,8 @@ __device__ __forceinline__ float span_tc_max(const Geo& g, const Spans& s) {
 // margin) is done once per point by one lane for 32 points at a time and
 // handed to the warp with shuffles, instead of by all 32 lanes for every point
 // (148 ms for that version on 128^3 voxels x 16,384 points x 1,024 bins).
-// Samples are those of sample_filtered: the margin here bounds its
-// per-sample margin over every bin of the span, so the kept samples and every
-// decision are the exact chain's.
+// The margin bounds the fast path's over every bin of the span, so every decision is
+// the exact chain's.
 __global__ void __launch_bounds__(256) confocal_adjoint_kernel(Geo g, Points mp, int N,
                                                                const float* __restrict__ tr,
                                                                float* __restrict__ vol) {
@@ -600,7 +568,7 @@ __global__ void __launch_bounds__(256) confocal_adjoint_kernel(Geo g, Points mp,
       ddx = xmul(dx, dx);
       ddy = xmul(dy, dy);
       sp = column_span(g, tz, dx * dx + dy * dy, wz);
-      // sample_filtered's margin 8 u scale (depth + |wz| + |z| + |oz|) + 4 u |zh|
+      // the margin 8 u scale (depth + |wz| + |z| + |oz|) + 4 u |zh|
       // + 1e-7 with depth, |z| and |zh| at their largest over the spans' bins
       const float dmax = 1.001f * span_tc_max(g, sp);
       const float zmax = fabsf(wz) + dmax;
@@ -622,7 +590,7 @@ __global__ void __launch_bounds__(256) confocal_adjoint_kernel(Geo g, Points mp,
       for (int r = 0; r < 2; ++r) {
         const int t0 = r ? n0 : p0, t1 = r ? n1 : p1;
         for (int t = t0 + lane; t <= t1; t += 32) {
-          // sample_filtered with the point's constants
+          // the fast path with the point's constants
           const float tc = xadd(xmul((float)t, g.bw), g.bo);
           const float d2 = xsub(xsub(xmul(tc, tc), pddx), pddy);
           if (!(d2 > 0.f)) continue;
@@ -667,7 +635,7 @@ __global__ void __launch_bounds__(256) confocal_adjoint_kernel(Geo g, Points mp,
 // widened by eps bins, a bound on the FP32 rounding of the sample chain
 // against that inverse (64 u of the largest magnitudes, over the bin width,
 // plus 0.01, at most the one bin of column_span, inside which the per-point
-// margin holds). Each sample's decisions are the exact chain's (sample_filtered
+// margin holds). Each sample's decisions are the exact chain's (the fast path
 // with the per-point margin, as in confocal_adjoint_kernel), so every kept
 // sample is the forward's and each lands in exactly one lane.
 template <int CPL>
@@ -925,7 +893,7 @@ __device__ __forceinline__ void add_cluster_columns(const Geo& g, float* acc, in
 // of the lanes' column spans: every valid sample of a lane lies in its own
 // span, and a sample outside it is decided (and rejected) like any other, so
 // each (column, point, bin) is counted once. Decisions are the exact chain's
-// (sample_filtered's margin, taken over the largest |tc| of the union).
+// (the fast path's margin, taken over the largest |tc| of the union).
 // What bounds it: instruction issue and the four shared-memory accesses of a
 // sample's cell pair, about 25 warp instructions per warp-sample (55 with one
 // bin at a time in scalar instructions, the values handed out by shuffles and
@@ -992,7 +960,7 @@ __global__ void __launch_bounds__(256, 3) confocal_adjoint_columns_kernel(
       if (zn > 0 && zlo <= zhi && tc_bounds(ex * ex + ey * ey, lwz, zlo, zhi, cl, unused) &&
           tc_bounds(fx * fx + fy * fy, lwz, zlo, zhi, unused, ch))
         sp = within_bins(g, tc_spans(g, tz, cl, ch, span_eps(g, ch, lwz)));
-      // sample_filtered's margin over the spans' largest |tc|
+      // the margin over the spans' largest |tc|
       const float dmax = 1.001f * span_tc_max(g, sp);
       const float zmax = fabsf(lwz) + dmax;
       const float zhmax = (zmax + fabsf(g.oz)) * g.scale + 0.5f;
