@@ -662,3 +662,24 @@ def test_point_gradient_tiles(cuda_lib, N, T):
     R.volume_confocal_grad_measurement_points(gm, cu(vol), cu(mp), cu(y), org, size, bw, 0.0)
     ref = oracle.volume_confocal_grad_mp(vol, mp, y, org, size, bw, 0.0)
     assert rel(gm.cpu().numpy(), ref) < 1e-4
+
+
+@pytest.mark.parametrize("value", [float("inf"), -float("inf"), 3e38, float("nan")])
+def test_volume_adjoint_of_infinite_elements(cuda_lib, value):
+    """Elements of the transient that are infinite or huge give the
+    oracle's infinities and NaN (in FP32, as sums of the same products)."""
+    g = np.random.default_rng(14)
+    shape, N, T = (9, 10, 13), 40, 150
+    mp = np.stack([g.uniform(-1, 1, N), g.uniform(-1, 1, N), np.zeros(N)]).astype(np.float32)
+    y = g.uniform(0.5, 1.5, (N, T)).astype(np.float32)
+    y[3, 60], y[17, 75] = value, value
+    org, size = (-0.5, -0.5, 0.5), (1.0, 1.0, 1.0)
+    out = torch.full(shape, 7.0, device="cuda")
+    R.volume_confocal_adjoint(out, cu(mp), cu(y), org, size, 0.02, 0.0)
+    got = out.cpu().numpy()
+    ref = oracle.volume_confocal_adjoint(y, shape, mp, org, size, 0.02, 0.0)
+    with np.errstate(over="ignore"):
+        ref = ref.astype(np.float32)
+    for kind in (np.isnan, np.isposinf, np.isneginf):
+        assert np.array_equal(kind(got), kind(ref))
+    assert np.isfinite(ref).any() and (np.isfinite(value) or not np.isfinite(ref).all())

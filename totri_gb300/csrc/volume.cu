@@ -795,6 +795,9 @@ __device__ __forceinline__ void adj_walk(const Geo& g, const float4* __restrict_
   for (int c = t0 & ~3; c <= t1; c += 32) {
     __syncwarp();
     reinterpret_cast<float*>(vbuf)[lane] = val;
+    // (v - alpha v is NaN where v overflows: chunks with infinite or huge values go
+    // through the exact chain, whose (1 - alpha) v is not)
+    const float lim = __any_sync(0xffffffffu, !(fabsf(val) < 1e30f)) ? 0.f : p.lim;
     __syncwarp();
     if (c + 32 <= t1) val = c + 32 + lane < g.T ? __ldg(row + c + 32 + lane) : 0.f;
     const int n = min(32, t1 - c + 1);
@@ -829,11 +832,11 @@ __device__ __forceinline__ void adj_walk(const Geo& g, const float4* __restrict_
         u[2 * h + 1] = __float_as_uint(xb) - bias;
       }
       // (NaN fractions are passed over)
-      if (absmax3(absmax3(0.f, off[0], off[1]), off[2], off[3]) >= p.lim) {
+      if (absmax3(absmax3(0.f, off[0], off[1]), off[2], off[3]) >= lim) {
         unsigned slow = 0;
 #pragma unroll
         for (int q = 0; q < 4; ++q)
-          if (fabsf(off[q]) >= p.lim) slow |= 1u << q, u[q] = 0xffffffffu;
+          if (fabsf(off[q]) >= lim) slow |= 1u << q, u[q] = 0xffffffffu;
         do {
           const int q = __ffs(slow) - 1;
           slow &= slow - 1;
