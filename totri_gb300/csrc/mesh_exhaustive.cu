@@ -874,14 +874,15 @@ __device__ __forceinline__ float4 splat_record(fv3 v0, fv3 v1, fv3 v2, fv3 c, fv
 // lane, and then takes the faces one by one with all lanes (four by four with CT =
 // 8). The columns' bins are a window [w0, w0 + W) of the T, W rows of shared
 // memory: where T > W the CTA first bounds each column's path lengths over the
-// chunks it sees, and walks the faces again for every further W bins.
+// chunks it sees, and walks the faces again for every further W bins, but for the
+// chunks that the window cannot hold.
 // Instruction issue bounds it (72% of the slots at 26 warps per SM): of 8.8 ms for
 // 20,000 faces x 400 x 144 points and 2,048 bins with 16 warps, the tents took 4.0
 // (1.1 of it the compare-and-swap of a float add in shared memory), the laser
 // records 1.9, the corners 0.9 and the rest 2.2), as it did the CTA per scan point
 // and 4 lasers (10.3 ms), whose lanes met in the same bins and computed both
 // points' lengths for every pair. 32 warps over one window of 1,024 bins (one CTA
-// per SM) take 7.8 ms, as fewer columns need a second pass. The coordinates are
+// per SM) take 7.9 ms, as fewer columns need a second pass. The coordinates are
 // exh_pair_filtered's, bit for bit; exact ones from a square root per length and
 // a fixed division were 0.5 ms faster, but moved single bins by 1e-3.
 constexpr int kColScan = 2;  // scan points with records prepared per face

@@ -37,8 +37,9 @@
 //   "mesh.visibility.occupancy", ".chunks", ".seed", ".seed.steps", ".shaft.cap"
 //                               visibility launch shape and prefix (at its launcher)
 //   "volume.exact"              1: every volume sample takes the exact chain
-//   "volume.forward.points", ".slices" points per CTA (4, 8, 16, 32) and slices of the
-//                               voxels, forward and measurement-point gradient
+//   "volume.forward.points", ".slices" points per CTA (4, 8, 16, 32; below 4: the built-in
+//                               choice) and slices of the voxels, forward and
+//                               measurement-point gradient
 //   "volume.adjoint.mode"       0 lanes over 32 columns (default), 1 shared-memory
 //                               atomics, 2 lane-owned cells (up to 256 cells)
 //   "volume.adjoint.warps"      warps per CTA of the lanes-over-columns adjoint
@@ -46,7 +47,8 @@
 //   "volume.exhaustive.lt"      laser points per exhaustive volume CTA (1,8,32)
 //   "backprojection.velten.mode", ".vz", ".points"
 //                               1: one voxel per thread without windows / voxels per
-//                               thread (2, 4) / scan points per tile (8, 16, 32)
+//                               thread (2, 4; 1 is taken as 2) / scan points per tile
+//                               (8, 16, 32)
 //   "backprojection.velten.pairs" 1: one voxel per thread in the exhaustive Velten
 //   "rbf.cull"                  1: RBF kernels without the underflow cull
 #pragma once

@@ -901,8 +901,8 @@ __device__ __forceinline__ void add_cluster_columns(const Geo& g, float* acc, in
 // sample's cell pair, about 25 warp instructions per warp-sample (55 with one
 // bin at a time in scalar instructions, the values handed out by shuffles and
 // floor and conversion on the special-function units). 128^3 voxels x 16,384
-// points x 1,024 bins: 62.8 -> 39.5 ms, at
-// 73% of the shared-memory pipe's wavefronts.
+// points x 1,024 bins: 62.8 -> 40.1 ms, at 73% of the shared-memory pipe's wavefronts
+// (39.7 with a table of 1 / tc^8, which leaves the FP32 range in other units).
 // kSigned: there may be negative bin centres (a negative bin offset), whose bins
 // are a second walk of a point. kCluster: the point groups form a cluster
 // (add_cluster_columns).

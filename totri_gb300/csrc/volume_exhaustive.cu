@@ -197,7 +197,7 @@ __device__ __forceinline__ float clamp_finite(float x) {
 // shared memory (cp.async, the next scan point's while this one's are used). A window past kRows bins, or without
 // sound bounds, is read in place. 56 x 40 x 48 voxels x 256 scan points x 36
 // lasers, 1,024 bins: 21.8 ms (four square roots and eight divisions per pair,
-// every bin another sector of the in-place order) -> 3.65 ms,
+// every bin another sector of the in-place order) -> 3.68 ms,
 // at 91% of issue slots: about 50 instructions per pair and 5 per bin.
 constexpr int kLC = 8, kRows = 256;
 
