@@ -683,3 +683,21 @@ def test_volume_adjoint_of_infinite_elements(cuda_lib, value):
     for kind in (np.isnan, np.isposinf, np.isneginf):
         assert np.array_equal(kind(got), kind(ref))
     assert np.isfinite(ref).any() and (np.isfinite(value) or not np.isfinite(ref).all())
+
+
+@pytest.mark.parametrize("N,T,bo", [(256, 4097, 0.0), (1, 6001, 0.0), (7, 6400, -0.7),
+                                    (256, 6003, 0.0), (257, 6400, 0.0), (6, 9386, 0.0),
+                                    (6, 9387, 0.0)])
+def test_point_gradient_long_rows(cuda_lib, N, T, bo):
+    """Rows of few points in shared memory above 6,000 bins, as long as four fit: 1e-4 of
+    the FP64 oracle."""
+    g = np.random.default_rng(N + T)
+    shape, bw = (5, 6, 7), (3.0 - bo) / T
+    mp = np.stack([g.uniform(-1, 1, N), g.uniform(-1, 1, N), np.zeros(N)]).astype(np.float32)
+    vol = g.uniform(0.5, 1.5, shape).astype(np.float32)
+    y = g.uniform(0.5, 1.5, (N, T)).astype(np.float32)
+    org, size = (-0.5, -0.5, 0.5), (1.0, 1.0, 1.0)
+    gm = torch.full((3, N), 7.0, device="cuda")
+    R.volume_confocal_grad_measurement_points(gm, cu(vol), cu(mp), cu(y), org, size, bw, bo)
+    ref = oracle.volume_confocal_grad_mp(vol, mp, y, org, size, bw, bo)
+    assert rel(gm.cpu().numpy(), ref) < 1e-4

@@ -328,12 +328,10 @@ __global__ void __launch_bounds__(256) forward_kernel(Grid g, int b, Rbf r, int 
 // then x fold in the other axes' factors. Nothing is reduced across lanes, and a
 // Gaussian issues 4 + A atomics per brick. With fewer than 129 Gaussians left,
 // several warps share a batch of 32, split the brick's x and add up before the atomics.
-// What bounds it:
-// instruction issue, about 5.5 instructions per (Gaussian, voxel) with one
-// attribute. 4,096 Gaussians, 128^3 voxels: 3.15 -> 0.85 ms (1.05 with the
-// voxel coordinates taken per Gaussian and row), against a warp per two
-// Gaussians whose lanes took the voxels, one ex2 per pair and a shuffle
-// reduction per Gaussian and brick.
+// What bounds it: instruction issue, about 5.5 instructions per (Gaussian, voxel) with
+// one attribute. 4,096 Gaussians, 128^3 voxels: 3.15 -> 0.85 ms (1.05 with the voxel
+// coordinates taken per Gaussian and row), against a warp per two Gaussians whose lanes
+// took the voxels, one ex2 per pair and a shuffle reduction per Gaussian and brick.
 constexpr int kGB = 8;  // brick side
 
 // kA attributes at most.

@@ -377,17 +377,23 @@ __global__ void __launch_bounds__(32 * PT > 256 ? 32 * PT : 256) confocal_forwar
 // walks: a thread accumulates one point over its share of the voxels, and the shares
 // are reduced in shared memory (then added into a zeroed output when there are
 // several slices of the voxels). 41 x 37 x 53 voxels (10%) x 899 points x 500 bins: 0.55
-// -> 0.10 ms. transient_grad is read in place, a voxel's few bins of a row: with the
-// rows in shared memory 1,024 bins took as long (0.92 to 1.02 of the time, by voxels and
+// -> 0.10 ms. transient_grad is read in place, a voxel's few bins of a row, or its rows
+// are staged in shared memory (kRows: few points, long rows, see the launcher): with the
+// rows staged 1,024 bins took as long (0.92 to 1.02 of the time, by voxels and
 // points), 2,048 bins 1.3 to 3 times and 4,096 bins 2 to 7 times as long (16,384 rows for
 // the 10 voxels of an 8^3 volume 1.2 against 0.18 ms).
-template <int PT, bool kSigned>
+template <int PT, bool kSigned, bool kRows>
 __global__ void __launch_bounds__(32 * PT > 256 ? 32 * PT : 256) grad_mp_kernel(
     Geo g, const float4* __restrict__ recs, const uint32_t* __restrict__ count, Points mp, int N,
     const float* __restrict__ tg, float* __restrict__ out, int64_t osc, int64_t osn) {
-  extern __shared__ float4 tab[];  // the bin table
+  extern __shared__ __align__(16) float rows[];  // kRows: [T][PT]; then the bin table
+  float4* tab = reinterpret_cast<float4*>(rows + (kRows ? ((size_t)PT * g.T + 3) & ~(size_t)3 : 0));
   __shared__ float sum[PT][3];
   const int i0 = blockIdx.x * PT;
+  if (kRows)
+    for_rows(PT, g.T, [&](int p, int t) {
+      rows[t * PT + p] = i0 + p < N ? __ldg(tg + (size_t)(i0 + p) * g.T + t) : 0.f;
+    });
   fill_bin_table(g, tab);
   if (threadIdx.x < PT) sum[threadIdx.x][0] = sum[threadIdx.x][1] = sum[threadIdx.x][2] = 0.f;
   __syncthreads();
@@ -410,7 +416,8 @@ __global__ void __launch_bounds__(32 * PT > 256 ? 32 * PT : 256) grad_mp_kernel(
       walk_voxel<kSigned>(g, tab, p, tz, rec.x, rec.y, __float_as_int(rec.w),
                           [&](int t, bool lower, float fr, float a, float b, float depth) {
                             const float w = lower ? 1.f - fr : fr, f1 = a * b;
-                            const float df2 = __ldg(row + t) * (f1 * f1);
+                            const float y = kRows ? rows[t * PT + pl] : __ldg(row + t);
+                            const float df2 = y * (f1 * f1);
                             const float slope = lower ? -g.scale * df2 : g.scale * df2;
                             const float inv = __fdividef(1.f, depth);
                             radial += fmaf(4.f * w * df2, inv, slope) * (inv * g.dz);
@@ -444,9 +451,8 @@ __global__ void __launch_bounds__(32 * PT > 256 ? 32 * PT : 256) grad_mp_kernel(
 }
 
 // grad_mp_kernel for bin tables that do not fit shared memory: every sample by the
-// exact chain; one thread
-// accumulates one point's gradient over a share of the voxels, reduced across
-// the kPT-strided threads in shared memory.
+// exact chain; one thread accumulates one point's gradient over a share of the voxels,
+// reduced across the kPT-strided threads in shared memory.
 __global__ void __launch_bounds__(256) grad_mp_wide_kernel(Geo g, const float4* __restrict__ recs,
                                                       const uint32_t* __restrict__ count,
                                                       Points mp, int N,
@@ -1156,10 +1162,11 @@ WalkTile walk_tile(int64_t N, int T, int64_t voxels, bool rows) {
   // Without rows: smaller tiles until 8 slices make a CTA per SM, and until the points'
   // rows fit half of the L1 cache (24^3 voxels, half of them, x 1,024 points: 2,048 bins
   // 0.51 ms with 8 points, 1.11 with 16; 4,096 bins 0.95 with 4, 1.21 with 8, 2.05 with
-  // 16). From 6,400 bins on not even 4 rows do, and 16 points are the fastest.
+  // 16). Above, not even 4 rows do, and 16 points are the fastest (64^3 voxels x 2,048
+  // points x 5,000 bins 13.2 ms, 21.8 with 4) but for few points (256: 4.3 and 3.1 ms).
   while (!rows && want == 0 && w.points > 4 &&
          (8 * ceil_div(N, w.points) < (int64_t)tune::sm_count() ||
-          (T <= 4096 && sizeof(float) * w.points * T > 64 * 1024)))
+          (T <= (N <= 256 ? 6000 : 4096) && sizeof(float) * w.points * T > 64 * 1024)))
     w.points /= 2;
   w.threads = std::max(256, 32 * w.points);
   w.smem = bytes(w.points);
@@ -1400,7 +1407,17 @@ int totri_volume_confocal_grad_measurement_points(const totri_array_t* mpg,
                     &count, stream));
   float* out = static_cast<float*>(mpg->data);
   const int64_t osc = mpg->strides[0], osn = mpg->strides[1];
-  WalkTile w = walk_tile(N, T, numel(vol), false);
+  // Rows in shared memory for few and long ones only (us, in place against it, half of
+  // 24^3 voxels, and 2% of them): 6,400 bins, 64 points 667/490 and 66/70, 256 points
+  // 1,789/923 and 99/115, 1,024 points 4,091/2,607 and 200/279; 9,300 bins, 256 points
+  // 2,647/1,306 and 137/151. Half of 64^3 voxels x 6,400 bins, 1,024 points 9.9/16.4 ms.
+  WalkTile w{0, 0, 1, 0};
+  bool staged = T > 6000 && N <= 256;
+  if (staged) w = walk_tile(N, T, numel(vol), true);
+  if (w.points == 0) {
+    staged = false;
+    w = walk_tile(N, T, numel(vol), false);
+  }
   if (w.points == 0) {  // the bin table is too long for shared memory
     TOTRI_KERNEL("volume confocal grad points", stream,
                  volume::grad_mp_wide_kernel<<<(unsigned)ceil_div(N, volume::kPT), 256, 0, stream>>>(
@@ -1412,7 +1429,10 @@ int totri_volume_confocal_grad_measurement_points(const totri_array_t* mpg,
   else
     w.slices = 1;  // (the slices add into a zeroed output)
   return for_walk_tile(w.points, g, [&](auto pt, auto sign) {
-    const auto kernel = volume::grad_mp_kernel<decltype(pt)::value, decltype(sign)::value>;
+    constexpr int kPoints = decltype(pt)::value;
+    constexpr bool kSigned = decltype(sign)::value;
+    const auto kernel = staged ? volume::grad_mp_kernel<kPoints, kSigned, true>
+                               : volume::grad_mp_kernel<kPoints, kSigned, false>;
     TOTRI_CUDA(tune::ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), w.smem));
     const dim3 grid((unsigned)ceil_div(N, w.points), (unsigned)w.slices);
     TOTRI_KERNEL("volume confocal grad points", stream,
